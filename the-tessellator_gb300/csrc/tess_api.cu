@@ -147,8 +147,7 @@ struct Engine {
     double* d_spx = nullptr;
     double* d_spy = nullptr;
     double* d_spz = nullptr;
-    float* d_shi = nullptr;
-    float* d_slo = nullptr;
+    float4* d_pk = nullptr;
     uint32_t* d_sgroup = nullptr;
     TabEntry* d_table = nullptr;
     int* d_err = nullptr;
@@ -262,7 +261,7 @@ struct Engine {
         drop_graphs();
         dfree(d_xyz); dfree(d_groups); dfree(d_desc); dfree(d_chunk_diag); dfree(d_chunk_start);
         dfree(d_bounds); dfree(d_bin); dfree(d_rank); dfree(d_delims); dfree(d_scan_tmp);
-        dfree(d_sorted); dfree(d_inv); dfree(d_spx); dfree(d_spy); dfree(d_spz); dfree(d_shi); dfree(d_slo); dfree(d_sgroup);
+        dfree(d_sorted); dfree(d_inv); dfree(d_spx); dfree(d_spy); dfree(d_spz); dfree(d_pk); dfree(d_sgroup);
         dfree(d_table); dfree(d_err); dfree(d_check); dfree(d_vol); dfree(d_nface); dfree(d_fstart); dfree(d_status);
         dfree(d_fnbr); dfree(d_farea); dfree(d_fcursor);
         for (auto& l : d_list) dfree(l);
@@ -284,13 +283,14 @@ struct Engine {
         const int si = slots <= 2 ? 0 : (slots <= 4 ? 1 : 2);
         int& b = blocks_cache[precision][si][form];
         if (!b) {
-            const int wpb = wpb_for(precision, slots);
+            const int wpb = wpb_for(slots, form);
             b = clip_blocks_for(precision, slots, form, wpb, device);
         }
         return b;
     }
-    int wpb_for(int precision, int slots) const {
+    int wpb_for(int slots, int form) const {
         int w = cfg.warps_per_block;
+        if ((form & 3) == kFormLean) w = std::min(w, 4);   // its launch bound
         if (slots >= 8) w = std::min(w, 2);
         else if (slots >= 4) w = std::min(w, 4);
         return std::max(1, w);
@@ -426,8 +426,7 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     TRY(dalloc(&E.d_spx, n));
     TRY(dalloc(&E.d_spy, n));
     TRY(dalloc(&E.d_spz, n));
-    TRY(dalloc(&E.d_shi, 3 * n));
-    TRY(dalloc(&E.d_slo, 3 * n));
+    TRY(dalloc(&E.d_pk, 2 * n));
     TRY(dalloc(&E.d_table, E.table_total));
     E.table_alloc = E.table_total;
     TRY(dalloc(&E.d_err, 1));
@@ -472,8 +471,7 @@ GridBuffers grid_buffers(Engine& E) {
     g.spx = E.d_spx;
     g.spy = E.d_spy;
     g.spz = E.d_spz;
-    g.shi = E.d_shi;
-    g.slo = E.d_slo;
+    g.pk = E.d_pk;
     g.sgroup = E.d_sgroup;
     g.table = E.d_table;
     g.table_gaps = E.cfg.table_gaps;
@@ -599,13 +597,11 @@ ClipParams base_params(Engine& E) {
     p.spx = E.d_spx;
     p.spy = E.d_spy;
     p.spz = E.d_spz;
-    p.shi = E.d_shi;
-    p.slo = E.d_slo;
+    p.pk = E.d_pk;
     p.sorted = E.d_sorted;
     p.delims = E.d_delims;
     p.sgroup = E.d_sgroup;
     p.table = E.d_table;
-    p.bin = E.d_bin;
     p.total = E.total;
     p.vol = E.d_vol;
     p.nface = E.d_nface;
@@ -637,6 +633,7 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
     if (E.cfg.flags & TESS_FLAG_COUNTERS) CU(cudaMemsetAsync(E.d_work, 0, sizeof(unsigned long long) * 8, E.stream));
     ClipParams base = base_params(E);
     base.search_radius = radius;
+    base.has_radius = radius >= 0.0;
     base.target_group = group;
     const int s0 = E.cfg.slots_per_lane;
     int cursor = 0;
@@ -659,7 +656,7 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
         p.fail_count = cnt + L_FAIL;
         p.reasons = cnt + L_REASON;
         p.work_ctr = (E.cfg.flags & TESS_FLAG_COUNTERS) ? E.d_work : nullptr;
-        CU(launch_clip(p, prec, slots, form, E.wpb_for(prec, slots), E.blocks(prec, slots, form), E.stream));
+        CU(launch_clip(p, prec, slots, form, E.wpb_for(slots, form), E.blocks(prec, slots, form), E.stream));
         E.launches += 1;
         return TESS_OK;
     };
@@ -1094,6 +1091,7 @@ tess_status engine_geo(Engine& E, int precision, uint32_t gs, const double* poin
     for (int prec : {precision, (int)TESS_PRECISION_FP64}) {
         ClipParams p = base_params(E);
         p.search_radius = radius;
+        p.has_radius = radius >= 0.0;
         p.target_group = group;
         CU(cudaMemcpyAsync(E.d_one, &gs, sizeof(uint32_t), cudaMemcpyHostToDevice, E.stream));
         CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * 32, E.stream));
@@ -1220,7 +1218,7 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
         E.bnd_valid = true;
     }
     p.bnd = E.d_bnd;
-    p.shi = E.d_shi;
+    p.pk = E.d_pk;
     const double r2 = radius * radius;
     p.f32_filter = mode == RQ_REAL_RADIUS && std::isfinite(radius) && r2 >= 1e-30 && r2 <= 1e36;
     if (mode == RQ_CLOUD) {

@@ -11,8 +11,7 @@ cudaError_t launch_clip_f32x(const ClipParams& p, int slots, int form, int wpb, 
     const int base = form & 3;
     if (slots <= 2) {
         if (base == kFormHybrid) return launch_t<float, 2, false, kFormHybrid | kFormExact>(p, wpb, blocks, s);
-        return base == kFormLean ? launch_t<float, 2, false, kFormLean | kFormExact>(p, wpb, blocks, s)
-                                 : launch_t<float, 2, false, kFormStd | kFormExact>(p, wpb, blocks, s);
+        return launch_t<float, 2, false, kFormStd | kFormExact>(p, wpb, blocks, s);
     }
     if (slots <= 4) return launch_t<float, 4, false, kFormStd | kFormExact>(p, wpb, blocks, s);
     return launch_t<float, 8, false, kFormStd | kFormExact>(p, wpb, blocks, s);
@@ -23,8 +22,7 @@ int clip_blocks_f32x(int slots, int form, int wpb, int device) {
     const int base = form & 3;
     if (slots <= 2) {
         if (base == kFormHybrid) return blocks_t<float, 2, false, kFormHybrid | kFormExact>(wpb, device);
-        return base == kFormLean ? blocks_t<float, 2, false, kFormLean | kFormExact>(wpb, device)
-                                 : blocks_t<float, 2, false, kFormStd | kFormExact>(wpb, device);
+        return blocks_t<float, 2, false, kFormStd | kFormExact>(wpb, device);
     }
     if (slots <= 4) return blocks_t<float, 4, false, kFormStd | kFormExact>(wpb, device);
     return blocks_t<float, 8, false, kFormStd | kFormExact>(wpb, device);

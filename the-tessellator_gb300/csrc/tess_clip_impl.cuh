@@ -61,10 +61,8 @@ constexpr float kVertexErr = 1.5e-6f;
 // Load the next batch's table entries and bin ranges before cutting the
 // current batch (overlaps their latency, costs registers).
 constexpr bool kPrefetch = true;
-// Pre-test a window's candidates against the live vertices (re-run form)
-// when at least this many are within twice the cell radius.  The lean
-// first-pass form leaves it out: on uniform inputs windows are small and its
-// mere presence costs the hot loop registers.
+// Pre-test a window's candidates against the live vertices when at least
+// this many are within twice the cell radius.
 constexpr int kPretestMin = 2;
 // A site whose own bin holds at least ClipParams::seed_min points (12 by
 // default, autotuned per input) is seeded before the shell walk: every lane
@@ -333,8 +331,7 @@ __device__ __forceinline__ float vrad2(double x, double y, double z, double) {
     return __double2float_ru(x * x + y * y + z * z);
 }
 
-// Per-warp work counters (reported when ClipParams::work_ctr is set).  The
-// lean first-pass form does not count: the registers cost it 2%.
+// Per-warp work counters (reported when ClipParams::work_ctr is set).
 struct Work {
     unsigned tested = 0, cuts = 0, newv = 0, windows = 0, batches = 0;
 };
@@ -997,9 +994,6 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
     constexpr bool GUARD = sizeof(T) == 4;
     constexpr int BASE = FORM & 3;                                  // lean, std or hybrid
     constexpr bool EXACT = GUARD && (FORM & kFormExact) != 0;       // FP64-accurate finalize
-    // the lean first pass sends crowded cells to a seeded pass instead (the
-    // seeding code would cost its hot loop registers)
-    constexpr bool kSeedForm = BASE != kFormLean;
     // ---- diagram of this cell ----
     int d = 0;
     if (P.ndiag > 1 && !P.at_point) {
@@ -1039,8 +1033,9 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
             shy = __double2float_rn(uy); sly = __double2float_rn(uy - (double)shy);
             shz = __double2float_rn(uz); slz = __double2float_rn(uz - (double)shz);
         } else {
-            shx = P.shi[3ull * gs]; shy = P.shi[3ull * gs + 1]; shz = P.shi[3ull * gs + 2];
-            slx = P.slo[3ull * gs]; sly = P.slo[3ull * gs + 1]; slz = P.slo[3ull * gs + 2];
+            const float4 h = P.pk[2ull * gs], l = P.pk[2ull * gs + 1];
+            shx = h.x; shy = h.y; shz = h.z;
+            slx = l.x; sly = l.y; slz = l.z;
         }
     }
 
@@ -1057,23 +1052,11 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
     }
     C.lm[0] = 0xFFu;
     C.np = 6;
-    // The FP32 first pass sets up without the FP64 pipe (dozens of cycles per
-    // warp instruction on this part): box offsets from the FP32 pairs of the
-    // box and the site relative to the centre, one rounding each side of the
-    // sum (<= 2^-23 relative) plus the pairs' own ~2^-47 of the extent.
-    constexpr bool kF32Setup = BASE == kFormLean;
     if (lane < 6) {
         const int a = lane >> 1;
         const bool mx = lane & 1;
-        T offt;
-        if constexpr (kF32Setup) {
-            const float sh_a = a == 0 ? shx : (a == 1 ? shy : shz);
-            const float sl_a = a == 0 ? slx : (a == 1 ? sly : slz);
-            offt = mx ? ((D.bhi_hi[a] - sh_a) + (D.bhi_lo[a] - sl_a)) : ((sh_a - D.blo_hi[a]) + (sl_a - D.blo_lo[a]));
-        } else {
-            const double s_a = a == 0 ? sx : (a == 1 ? sy : sz);
-            offt = (T)(mx ? (bhi[a] - s_a) : (s_a - blo[a]));
-        }
+        const double s_a = a == 0 ? sx : (a == 1 ? sy : sz);
+        const T offt = (T)(mx ? (bhi[a] - s_a) : (s_a - blo[a]));
         const T sg = mx ? (T)1 : (T)-1;
         S.px[lane] = a == 0 ? sg : (T)0;
         S.py[lane] = a == 1 ? sg : (T)0;
@@ -1084,15 +1067,9 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
     }
     if (lane < 8) {
         const int bx = lane & 1, by = (lane >> 1) & 1, bz = (lane >> 2) & 1;
-        if constexpr (kF32Setup) {
-            C.vx[0] = bx ? ((D.bhi_hi[0] - shx) + (D.bhi_lo[0] - slx)) : ((D.blo_hi[0] - shx) + (D.blo_lo[0] - slx));
-            C.vy[0] = by ? ((D.bhi_hi[1] - shy) + (D.bhi_lo[1] - sly)) : ((D.blo_hi[1] - shy) + (D.blo_lo[1] - sly));
-            C.vz[0] = bz ? ((D.bhi_hi[2] - shz) + (D.bhi_lo[2] - slz)) : ((D.blo_hi[2] - shz) + (D.blo_lo[2] - slz));
-        } else {
-            C.vx[0] = (T)((bx ? bhi[0] : blo[0]) - sx);
-            C.vy[0] = (T)((by ? bhi[1] : blo[1]) - sy);
-            C.vz[0] = (T)((bz ? bhi[2] : blo[2]) - sz);
-        }
+        C.vx[0] = (T)((bx ? bhi[0] : blo[0]) - sx);
+        C.vy[0] = (T)((by ? bhi[1] : blo[1]) - sy);
+        C.vz[0] = (T)((bz ? bhi[2] : blo[2]) - sz);
         S.vx[lane] = C.vx[0];
         S.vy[lane] = C.vy[0];
         S.vz[lane] = C.vz[0];
@@ -1102,9 +1079,9 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
             S.fvz[lane % S_t::VD] = (float)C.vz[0];
         }
         if constexpr (GUARD) {
-            // the corner's rounding to FP32: 2^-24 relative per component from
-            // FP64, 2^-23 from the FP32 pairs (doubled here)
-            C.ve[0] = ((T)(kF32Setup ? 2.5e-7 : 1.2e-7) + (T)P.guard_rel) * (fabs(C.vx[0]) + fabs(C.vy[0]) + fabs(C.vz[0]));
+            // the corner's rounding to FP32: 2^-24 relative per component
+            // (doubled here)
+            C.ve[0] = ((T)1.2e-7 + (T)P.guard_rel) * (fabs(C.vx[0]) + fabs(C.vy[0]) + fabs(C.vz[0]));
             S.ve[lane] = C.ve[0];
         }
         S.vr[lane] = vrad2(C.vx[0], C.vy[0], C.vz[0], C.ve[0]);
@@ -1159,15 +1136,9 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
 
     // ---- the walk over bins in shell order (celery.rs:1023-1075) ----
     const int cpd = D.cpd;
-    int cbx, cby, cbz;
-    if constexpr (kF32Setup) {
-        // the site's bin from the binning pass (bit-exact axis_index there)
-        split_bin(P.bin[orig] - (uint32_t)bin_base, cpd, D.rcp_cpd, D.rcp_cpd2, cbx, cby, cbz);
-    } else {
-        cbx = axis_index(sx, D.glo[0], D.ghi[0], D.inv[0], cpd);
-        cby = axis_index(sy, D.glo[1], D.ghi[1], D.inv[1], cpd);
-        cbz = axis_index(sz, D.glo[2], D.ghi[2], D.inv[2], cpd);
-    }
+    const int cbx = axis_index(sx, D.glo[0], D.ghi[0], D.inv[0], cpd);
+    const int cby = axis_index(sy, D.glo[1], D.ghi[1], D.inv[1], cpd);
+    const int cbz = axis_index(sz, D.glo[2], D.ghi[2], D.inv[2], cpd);
     const double radius = P.search_radius;
     const bool has_radius = radius >= 0.0;
     const int64_t tgroup = P.target_group;
@@ -1176,9 +1147,10 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
     // The offset p - site of sorted point j and its squared length.
     auto cand = [&](uint32_t j, T& rx, T& ry, T& rz, T& r2) {
         if constexpr (GUARD) {
-            rx = (T)((P.shi[3ull * j] - shx) + (P.slo[3ull * j] - slx));
-            ry = (T)((P.shi[3ull * j + 1] - shy) + (P.slo[3ull * j + 1] - sly));
-            rz = (T)((P.shi[3ull * j + 2] - shz) + (P.slo[3ull * j + 2] - slz));
+            const float4 h = P.pk[2ull * j], l = P.pk[2ull * j + 1];
+            rx = (T)((h.x - shx) + (l.x - slx));
+            ry = (T)((h.y - shy) + (l.y - sly));
+            rz = (T)((h.z - shz) + (l.z - slz));
         } else {
             rx = (T)(P.spx[j] - sx);
             ry = (T)(P.spy[j] - sy);
@@ -1198,7 +1170,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
         // nothing later (the cell only shrinks), so only possible cutters
         // (and guard-band cases, which the serial test reports) go on to
         // the serial nearest-first loop.  Same arithmetic as cut().
-        if (BASE != kFormLean && __popc(km) >= kPretestMin) {
+        if (__popc(km) >= kPretestMin) {
             bool maycut = false;
             if (keep && sizeof(T) == 8) {
                 // FP64 form: the test in FP32 on the vertices' FP32 copies,
@@ -1279,13 +1251,11 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
             bisector(cx, cy, cz, c2, nx, ny, nz, off, rn);
             const int r = cut<T, K, GUARD, BASE == kFormHybrid>(S, C, nx, ny, nz, off, rn, cR, eC, cidb, cj, lane,
                                                                    P, fsite);
-            if constexpr (BASE != kFormLean) ++W.tested;
+            ++W.tested;
             if (r < 0) return -r;
             if (r > 0) {
-                if constexpr (BASE != kFormLean) {
-                    ++W.cuts;
-                    W.newv += (unsigned)(r - 1);
-                }
+                ++W.cuts;
+                W.newv += (unsigned)(r - 1);
                 const T R2b = R2;
                 if constexpr (sizeof(T) == 8) {
                     R2f = live_r2f(S, C, lane);
@@ -1319,7 +1289,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
         // same however few of its candidates are kept (clustered 4M in FP64:
         // 1,204 -> 1,070 ms).  In the FP32 forms the pre-test is cheap and
         // gathering did not pay (measured).
-        constexpr bool kGather = BASE != kFormLean && sizeof(T) == 8;
+        constexpr bool kGather = sizeof(T) == 8;
         unsigned nbuf = 0;
         for (unsigned w0 = 0;; w0 += 32) {
             const bool more = w0 < total;
@@ -1330,7 +1300,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
             int32_t cid = 0;
             bool near = false;
             if (!more) {
-            } else if (kSeedForm && direct) {
+            } else if (direct) {
                 j = S.sdj[lane];
                 keep = j != 0xFFFFFFFFu;
                 rx = S.sdx[lane];
@@ -1339,7 +1309,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
                 r2 = S.sd2[lane];
                 cid = S.sdcid[lane];
             } else {
-                if constexpr (BASE != kFormLean) ++W.windows;
+                ++W.windows;
                 const unsigned c = w0 + lane;
                 const T lim = (T)4 * R2 * (T)kStopMargin;
                 // the lane's bin: the last with prefix <= c (never an empty one)
@@ -1354,7 +1324,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
                     if constexpr (sizeof(T) == 8) keep = (j != self) && r2 > dup2 && (float)r2 < 4.f * R2f * (float)kStopMargin;
                     else keep = (j != self) && r2 > dup2 && r2 < lim;
                     if constexpr (GUARD) near = (j != self) && !(r2 > dup2);
-                    if constexpr (kSeedForm) keep = keep && j != seedj;
+                    keep = keep && j != seedj;
                     cid = (int32_t)(P.sorted[j] - pt_base);
                     if (keep && tgroup >= 0) keep = (int64_t)(P.sgroup ? P.sgroup[j] : 0u) == tgroup;
                 }
@@ -1414,17 +1384,9 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
     // test than the gap key: a point of bin (b + o) lies at least
     // |o| - 1 + f (o < 0) or o - f (o > 0) bin sides from the site on each
     // axis.  Off-grid sites (cells of external points) skip the test.
-    float fx, fy, fz;
-    if constexpr (kF32Setup) {
-        // (x - glo) * inv from the FP32 pairs: within D.frac_eps bins
-        fx = ((shx - D.glo_hi[0]) + (slx - D.glo_lo[0])) * D.inv_f[0] - (float)cbx;
-        fy = ((shy - D.glo_hi[1]) + (sly - D.glo_lo[1])) * D.inv_f[1] - (float)cby;
-        fz = ((shz - D.glo_hi[2]) + (slz - D.glo_lo[2])) * D.inv_f[2] - (float)cbz;
-    } else {
-        fx = (float)(__dmul_rn(sx - D.glo[0], D.inv[0]) - (double)cbx);
-        fy = (float)(__dmul_rn(sy - D.glo[1], D.inv[1]) - (double)cby);
-        fz = (float)(__dmul_rn(sz - D.glo[2], D.inv[2]) - (double)cbz);
-    }
+    const float fx = (float)(__dmul_rn(sx - D.glo[0], D.inv[0]) - (double)cbx);
+    const float fy = (float)(__dmul_rn(sy - D.glo[1], D.inv[1]) - (double)cby);
+    const float fz = (float)(__dmul_rn(sz - D.glo[2], D.inv[2]) - (double)cbz);
     const bool near_ok = fx >= -1e-3f && fx <= 1.001f && fy >= -1e-3f && fy <= 1.001f && fz >= -1e-3f &&
                          fz <= 1.001f && D.has_extent;
     const float bsx = D.size_f[0], bsy = D.size_f[1], bsz = D.size_f[2];
@@ -1451,17 +1413,14 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
     };
 
     // Phases of the walk:
-    //   0  crowded bins (seeded forms, when the site's own bin is crowded);
+    //   0  crowded bins (when the site's own bin is crowded);
     //   1  the sorted shell table, 32 entries per batch (one per lane); the
     //      next batch's entries and bin ranges are loaded before the current
     //      batch is cut, so their latency overlaps the cutting;
     //   2  Chebyshev rings beyond the table (sparse regions).
-    // The seeded forms run them as one loop with one call of process(), so
-    // their window and cut code is inlined once: with a copy per phase,
-    // instruction fetch limited them (and the single loop takes their
-    // crowded-bin pass from 238 to 214 ms on the clustered 4M set).  The lean
-    // first pass keeps a loop per phase: it has no phase 0, and the single
-    // loop's dispatch made it 8% slower.
+    // They run as one loop with one call of process(), so the window and cut
+    // code is inlined once: with a copy per phase, instruction fetch limited
+    // the pass (crowded bins of the clustered 4M set: 238 -> 214 ms).
     uint32_t t = 0;
     // a batch entry: offsets, key and, after the bin test, the sorted range
     struct Ent {
@@ -1482,7 +1441,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
             e.key = te.key;
             if (has_radius && gap_key(D.size, e.i, e.j, e.k) > radius) e.key = INFINITY;
             long long lb = bin_of(e.i, e.j, e.k);
-            if (kSeedForm && done && abs(e.i) <= 1 && abs(e.j) <= 1 && abs(e.k) <= 1 &&
+            if (done && abs(e.i) <= 1 && abs(e.j) <= 1 && abs(e.k) <= 1 &&
                 ((done >> ((e.i + 1) * 9 + (e.j + 1) * 3 + (e.k + 1))) & 1u))
                 lb = -1;   // handled among the crowded bins
             if (lb >= 0) {
@@ -1492,65 +1451,6 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
         }
     };
     int ph = 1;
-    if constexpr (!kSeedForm) {
-        Ent ea;
-        load_entry(lane, ea);
-        // lean first pass: a crowded own bin (table entry 0, lane 0's first
-        // entry) sends the cell to the seeded pass
-        if (BASE == kFormLean && P.list_dense && __shfl_sync(FULL, ea.cnt, 0) >= P.seed_min) status = ST_DENSE;
-        bool rings = false;
-        while (status == ST_OK) {
-            // The table key is rounded toward zero and the threshold up, so
-            // stopping on key >= thr never drops a bin that could hold a cutter.
-            const float thr = round_up_f((T)4 * R2 * (T)kStopMargin);
-            const unsigned ma = __ballot_sync(FULL, !(ea.key < thr));
-            const int na = ma ? __ffs(ma) - 1 : 32;
-            const unsigned ba = ea.beg;
-            unsigned ca = lane < na ? ea.cnt : 0u;
-            // re-test the bins against the current (smaller) radius
-            if (ca && near_ok && near2(ea.i, ea.j, ea.k) * (1.0f - 1e-4f) >= round_up_f((T)4 * R2)) ca = 0;
-            t += (uint32_t)na;
-            if (!ma) load_entry(t + lane, ea);
-            if constexpr (BASE != kFormLean) ++W.batches;
-            status = process(ba, ca, false);
-            if (status != ST_OK) break;
-            if (ma) {
-                rings = (t >= tab_len) && isfinite(D.tab_kmax);
-                break;
-            }
-        }
-        if (status == ST_OK && rings) {
-            for (int ring = 1; ring <= cpd - 1 && status == ST_OK; ++ring) {
-                double lbk = (double)(ring - 1) * D.min_size;
-                lbk = lbk * lbk;
-                if (lbk < D.tab_kmax) lbk = D.tab_kmax;
-                if (lbk >= 4.0 * (double)R2 * kStopMargin) break;
-                if (radius >= 0.0 && lbk > radius) break;
-                const uint32_t rs = 24u * (uint32_t)ring * (uint32_t)ring + 2u;
-                for (uint32_t r0 = 0; r0 < rs; r0 += 32) {
-                    const double thr = 4.0 * (double)R2 * kStopMargin;
-                    long long lb = -1;
-                    const uint32_t r = r0 + lane;
-                    if (r < rs) {
-                        int i, j, k;
-                        ring_offset(ring, r, i, j, k);
-                        const double key = gap_key(D.size, i, j, k);
-                        if (key > D.tab_kmax && key < thr && !(radius >= 0.0 && key > radius)) lb = bin_of(i, j, k);
-                    }
-                    if (!__any_sync(FULL, lb >= 0)) continue;
-                    if constexpr (BASE != kFormLean) ++W.batches;
-                    unsigned beg = 0, cnt = 0;
-                    if (lb >= 0) {
-                        beg = P.delims[lb];
-                        cnt = P.delims[lb + 1] - beg;
-                    }
-                    status = process(beg, cnt, false);
-                    if (status != ST_OK) break;
-                }
-            }
-        }
-        ph = 3;
-    }
     // ---- phase 0: crowded bins first ----
     // When the site's own bin is crowded, it and every crowded neighbour bin
     // still within reach are handled one at a time, nearest first, in two
@@ -1562,7 +1462,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
     // (their ranges and distances wait in shared memory: in registers they
     // would stay live through every later cut)
     bool seed_step = true;       // phase 0: the next step cuts a bin's seeds
-    if constexpr (kSeedForm) {
+    {
         const uint64_t sb = tess_chk(bin_base + ((uint64_t)cbx * cpd + cby) * cpd + cbz, P.nbins, P.check, CK_BIN);
         if (P.delims[sb + 1] - P.delims[sb] >= P.seed_min) {
             const int ti = lane / 9 - 1, tj = (lane / 3) % 3 - 1, tk = lane % 3 - 1;
@@ -1587,10 +1487,10 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
     bool loaded = false;                 // phase 1: the first batch is loaded
     S.ring = 1;
     S.r0 = 0;
-    while (kSeedForm && status == ST_OK) {
+    while (status == ST_OK) {
         unsigned ba = 0, ca = 0;
         bool direct = false;
-        if (kSeedForm && ph == 0) {
+        if (ph == 0) {
             if (seed_step) {
                 const unsigned pending = S.pending;
                 if (!pending) {
@@ -1640,12 +1540,6 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
             if (!loaded) {
                 load_entry(lane, ea);
                 loaded = true;
-                // lean first pass: a crowded own bin (table entry 0, lane 0's
-                // first entry) sends the cell to the seeded pass
-                if (BASE == kFormLean && P.list_dense && __shfl_sync(FULL, ea.cnt, 0) >= P.seed_min) {
-                    status = ST_DENSE;
-                    break;
-                }
             }
             // The table key is rounded toward zero and the threshold up, so
             // stopping on key >= thr never drops a bin that could hold a cutter.
@@ -1664,7 +1558,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
             } else {
                 load_entry(t + lane, ea);
             }
-            if constexpr (BASE != kFormLean) ++W.batches;
+            ++W.batches;
         } else if (ph == 2) {
             const int ring = S.ring;
             const uint32_t r0 = S.r0;
@@ -1691,7 +1585,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
             S.r0 = r0 + 32 < rs ? r0 + 32 : 0u;
             S.ring = r0 + 32 < rs ? ring : ring + 1;
             if (!__any_sync(FULL, lb >= 0)) continue;
-            if constexpr (BASE != kFormLean) ++W.batches;
+            ++W.batches;
             if (lb >= 0) {
                 ba = P.delims[lb];
                 ca = P.delims[lb + 1] - ba;
@@ -1700,7 +1594,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
             break;
         }
         status = process(ba, ca, direct);
-        if (kSeedForm && ph == 0 && seed_step) {
+        if (ph == 0 && seed_step) {
             // a crowded bin's windows are done
             seedj = 0xFFFFFFFFu;
             done |= 1u << S.cbin;
@@ -1769,12 +1663,13 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
                 } else {
                     const uint32_t j = tess_chk(S.psrc[p], P.npts, P.check, CK_POINT);
                     float sh, se;
-                    two_sum(P.shi[3ull * j], -shx, sh, se);
-                    two_sum(sh, (P.slo[3ull * j] - slx) + se, q0, l0);
-                    two_sum(P.shi[3ull * j + 1], -shy, sh, se);
-                    two_sum(sh, (P.slo[3ull * j + 1] - sly) + se, q1, l1);
-                    two_sum(P.shi[3ull * j + 2], -shz, sh, se);
-                    two_sum(sh, (P.slo[3ull * j + 2] - slz) + se, q2, l2);
+                    const float4 h = P.pk[2ull * j], l = P.pk[2ull * j + 1];
+                    two_sum(h.x, -shx, sh, se);
+                    two_sum(sh, (l.x - slx) + se, q0, l0);
+                    two_sum(h.y, -shy, sh, se);
+                    two_sum(sh, (l.y - sly) + se, q1, l1);
+                    two_sum(h.z, -shz, sh, se);
+                    two_sum(sh, (l.z - slz) + se, q2, l2);
                     float p0, e0, p1, e1, p2, e2, s01, t01, s2, t2;
                     two_prod(q0, q0, p0, e0);
                     two_prod(q1, q1, p1, e1);

@@ -422,15 +422,19 @@ __global__ void k_gather(GridBuffers g) {
     }
     const DiagDesc& D = g.diags[lo];
     const double u[3] = {x - D.ctr[0], y - D.ctr[1], z - D.ctr[2]};
+    float hi4[3], lo4[3];
     for (int a = 0; a < 3; ++a) {
         float h, l;
         if (!split_rn_int(u[a], h, l)) {
             h = __double2float_rn(u[a]);
             l = __double2float_rn(u[a] - (double)h);
         }
-        g.shi[3ull * s + a] = h;
-        g.slo[3ull * s + a] = l;
+        hi4[a] = h;
+        lo4[a] = l;
     }
+    // one 32-byte sector per point: what the clipping reads of a candidate
+    g.pk[2ull * s] = make_float4(hi4[0], hi4[1], hi4[2], __uint_as_float(i));
+    g.pk[2ull * s + 1] = make_float4(lo4[0], lo4[1], lo4[2], __uint_as_float(g.bin[i]));
     if (g.sgroup) g.sgroup[s] = g.groups[i];
 }
 

@@ -7,6 +7,8 @@
 //   grid     delims[total_bins + 1]     CSR offsets of the bin-sorted order
 //   sorted   sorted[total]              sorted position -> point (concatenated index)
 //            spx/spy/spz[total]         FP64 positions in sorted order (SoA)
+//            pk[2 * total]              per sorted point, one 32-byte sector: the FP32 pair of
+//                                       its position, its point index and its bin
 //            sgroup[total]              group ids in sorted order (optional)
 //   table    tab[...]                   per-diagram shell table (sorted offsets)
 //   results  vol[total], nface[total], fstart[total], status[total]  (point order)
@@ -176,8 +178,9 @@ struct GridBuffers {
     double* spx;
     double* spy;
     double* spz;
-    float* shi;                 // FP32 split of the sorted positions:
-    float* slo;                 // x = shi + slo, 3 floats per point each (AoS)
+    // FP32 split of the sorted positions relative to the centre, x = hi + lo:
+    // pk[2 s] = {hi, point index}, pk[2 s + 1] = {lo, global bin id}
+    float4* pk;
     uint32_t* sgroup;           // null when groups is null
     TabEntry* table;
     int table_gaps;
@@ -233,7 +236,7 @@ struct RadiusParams {
     uint32_t* out;              // fill pass: bin ids or original point indices
     int* err;                   // set to 1 when a query cell is out of range
     const uint32_t* qorder;     // processing order of the queries (spatially sorted), or null
-    const float* shi;           // FP32 high parts of the sorted positions (AoS), for the FP32 filter
+    const float4* pk;           // FP32 split of the sorted positions (see GridBuffers), for the FP32 filter
     int f32_filter;             // real radius: pre-filter candidates in FP32 (radius in range)
     // check_cell_in_range as a table: for gaps gx <= gtab_x, gy <= gtab_y, the
     // largest gz <= gtab_z whose squared gap distance is within radius^2
@@ -281,13 +284,11 @@ struct ClipParams {
     const double* spx;
     const double* spy;
     const double* spz;
-    const float* shi;               // x = shi + slo (FP32 pair), AoS
-    const float* slo;
+    const float4* pk;               // FP32 split of the sorted positions, point index, bin (see GridBuffers)
     const uint32_t* sorted;
     const uint32_t* delims;
     const uint32_t* sgroup;
     const TabEntry* table;
-    const uint32_t* bin;            // global bin of each point (original order)
     // work: sorted positions to process
     const uint32_t* work;          // null: 0 .. total-1
     const uint32_t* work_count;    // null: total
@@ -314,6 +315,7 @@ struct ClipParams {
     unsigned long long* work_ctr; // optional work counters (tested, cuts, new vertices, windows, batches)
     // options
     double search_radius;         // < 0: none
+    int has_radius;               // search_radius >= 0
     int64_t target_group;         // < 0: none
     float guard_rel;
     float verify_rel;
@@ -335,7 +337,8 @@ struct ClipParams {
 };
 
 // Forms of the clipping kernel:
-//   kFormLean    the FP32 first pass (2 slots per lane, no window pre-test);
+//   kFormLean    the FP32 first pass (tess_clip_lean.cu: 64 slots, a candidate
+//                plane per lane);
 //   kFormStd     the re-run passes and the plain FP64 form, with the window
 //                pre-test (cells next to dense clusters test hundreds of
 //                candidates);
@@ -348,6 +351,8 @@ struct ClipParams {
 //                areas and the volume in FP64 (FP64-accurate results)
 enum ClipForm : int { kFormLean = 0, kFormStd = 1, kFormHybrid = 2, kFormExact = 4 };
 cudaError_t launch_clip_f32(const ClipParams& p, int slots, int form, int wpb, int blocks, cudaStream_t s);
+cudaError_t launch_clip_lean(const ClipParams& p, int exact, int wpb, int blocks, cudaStream_t s);
+int clip_blocks_lean(int exact, int wpb, int device);
 cudaError_t launch_clip_f64(const ClipParams& p, int slots, int form, int wpb, int blocks, cudaStream_t s);
 int clip_blocks_f32(int slots, int form, int wpb, int device);
 int clip_blocks_f64(int slots, int form, int wpb, int device);

@@ -123,10 +123,10 @@ __device__ __forceinline__ void emit_stream(const RadiusParams& p, uint32_t beg,
             bool band = false;
             if (qt.on) {
                 if (valid) {
-                    const float* h = p.shi + 3 * (size_t)s;
-                    const float dx = __fsub_rn(qt.fx, h[0]);
-                    const float dy = __fsub_rn(qt.fy, h[1]);
-                    const float dz = __fsub_rn(qt.fz, h[2]);
+                    const float4 h = p.pk[2 * (size_t)s];
+                    const float dx = __fsub_rn(qt.fx, h.x);
+                    const float dy = __fsub_rn(qt.fy, h.y);
+                    const float dz = __fsub_rn(qt.fz, h.z);
                     const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
                     ok = d2 < qt.lo_thr;
                     band = !ok && !(d2 > qt.hi_thr);      // NaN lands in the band
