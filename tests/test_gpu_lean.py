@@ -1,0 +1,73 @@
+"""The FP32 first pass on the point sets where its walk over rows of bins can go wrong: axes without extent, oblong
+grids, sparse regions that need rings of rows far out (more rows than lanes in a ring), sizes around a window of 32
+candidates, extents outside FP32's range, and a search radius, all against the FP64 oracle with the bars of the parity
+tests (neighbour lists bit-exact; volumes 1e-6 relative in FP32, 1e-12 in MIXED)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+VOL_TOL = {"mixed": 1e-12, "fp32": 1e-6}
+
+
+def _rng(seed):
+    return np.random.default_rng(seed)
+
+
+def _clumps(n, clumps, seed, size=0.004, lone=40):
+    """Points in tight clumps and a few lone ones between them: most bins are empty."""
+    r = _rng(seed)
+    c = 0.05 + 0.9 * r.random((clumps, 3))
+    return np.concatenate([c[r.integers(0, clumps, n - lone)] + size * (r.random((n - lone, 3)) - 0.5), r.random((lone, 3))])
+
+
+def _flat(pts, axis, value):
+    pts[:, axis] = value
+    return pts
+
+
+SETS = {
+    **{f"uniform_{n}": (lambda n=n: _rng(n).random((n, 3)), (1, 1, 1)) for n in (1, 2, 3, 31, 32, 33, 34, 64, 65, 200)},
+    "plane_x": (lambda: _flat(_rng(1).random((300, 3)), 0, 0.25), (1, 1, 1)),
+    "plane_y": (lambda: _flat(_rng(2).random((300, 3)), 1, 0.5), (1, 1, 1)),
+    "plane_z": (lambda: _flat(_rng(3).random((300, 3)), 2, 0.75), (1, 1, 1)),
+    "line": (lambda: _flat(_flat(_rng(4).random((60, 3)), 0, 0.5), 2, 0.5), (1, 1, 1)),
+    "oblong_x": (lambda: _rng(5).random((3000, 3)) * [20, 1, 1], (20, 1, 1)),
+    "oblong_y": (lambda: _rng(6).random((3000, 3)) * [1, 20, 0.5], (1, 20, 0.5)),
+    "oblong_z": (lambda: _rng(7).random((3000, 3)) * [0.5, 1, 20], (0.5, 1, 20)),
+    "clumps_few": (lambda: _clumps(1500, 4, 8), (1, 1, 1)),
+    "clumps_many": (lambda: _clumps(20000, 60, 9), (1, 1, 1)),
+    "lone_corner": (lambda: np.concatenate([0.9 + 0.1 * _rng(10).random((4000, 3)), [[0.01, 0.02, 0.03]]]), (1, 1, 1)),
+}
+
+
+def _check(T, O, pts, hi, prec, ref_kw, **kw):
+    rv, ro, ri, _, _, _ = O.Diagram(pts, lo=[0, 0, 0], hi=list(hi)).compute_all(**ref_kw)
+    with T.Diagram(pts, container=T.Polyhedron(0, 0, 0, *hi)) as d:
+        d.compute_all(prec, **kw)
+        vol = d.volumes()
+        offs, nbr, _ = d.neighbors_csr()
+    assert np.array_equal(offs.astype(np.int64), ro)
+    assert np.array_equal(nbr.astype(np.int64), ri)
+    assert np.max(np.abs(vol - rv) / np.maximum(rv, 1e-300)) <= VOL_TOL[prec]
+
+
+@pytest.mark.parametrize("prec", ["fp32", "mixed"])
+@pytest.mark.parametrize("name", list(SETS))
+def test_point_sets(tess, oracle_mod, name, prec):
+    make, hi = SETS[name]
+    _check(tess, oracle_mod, np.ascontiguousarray(make(), dtype=np.float64), hi, prec, {})
+
+
+@pytest.mark.parametrize("prec", ["fp32", "mixed"])
+@pytest.mark.parametrize("radius", [0.0, 0.01, 0.09, 0.5])
+@pytest.mark.parametrize("name", ["uniform_200", "oblong_x", "clumps_few"])
+def test_search_radius(tess, oracle_mod, name, radius, prec):
+    make, hi = SETS[name]
+    _check(tess, oracle_mod, np.ascontiguousarray(make(), dtype=np.float64), hi, prec,
+           {"mode": oracle_mod.MODE_RADIUS, "radius": radius}, search_radius=radius)
+
+
+def test_extent_below_fp32(tess, oracle_mod):
+    """Bin sides below FP32's normal range: the pass hands every cell on."""
+    _check(tess, oracle_mod, _rng(11).random((100, 3)) * 1e-42, (1e-42, 1e-42, 1e-42), "fp32", {})

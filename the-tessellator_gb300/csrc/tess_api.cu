@@ -147,7 +147,8 @@ struct Engine {
     double* d_spx = nullptr;
     double* d_spy = nullptr;
     double* d_spz = nullptr;
-    float4* d_pk = nullptr;
+    float4* d_phi = nullptr;
+    float4* d_plo = nullptr;
     uint32_t* d_sgroup = nullptr;
     TabEntry* d_table = nullptr;
     int* d_err = nullptr;
@@ -261,7 +262,7 @@ struct Engine {
         drop_graphs();
         dfree(d_xyz); dfree(d_groups); dfree(d_desc); dfree(d_chunk_diag); dfree(d_chunk_start);
         dfree(d_bounds); dfree(d_bin); dfree(d_rank); dfree(d_delims); dfree(d_scan_tmp);
-        dfree(d_sorted); dfree(d_inv); dfree(d_spx); dfree(d_spy); dfree(d_spz); dfree(d_pk); dfree(d_sgroup);
+        dfree(d_sorted); dfree(d_inv); dfree(d_spx); dfree(d_spy); dfree(d_spz); dfree(d_phi); dfree(d_plo); dfree(d_sgroup);
         dfree(d_table); dfree(d_err); dfree(d_check); dfree(d_vol); dfree(d_nface); dfree(d_fstart); dfree(d_status);
         dfree(d_fnbr); dfree(d_farea); dfree(d_fcursor);
         for (auto& l : d_list) dfree(l);
@@ -426,7 +427,8 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     TRY(dalloc(&E.d_spx, n));
     TRY(dalloc(&E.d_spy, n));
     TRY(dalloc(&E.d_spz, n));
-    TRY(dalloc(&E.d_pk, 2 * n));
+    TRY(dalloc(&E.d_phi, n));
+    TRY(dalloc(&E.d_plo, n));
     TRY(dalloc(&E.d_table, E.table_total));
     E.table_alloc = E.table_total;
     TRY(dalloc(&E.d_err, 1));
@@ -471,7 +473,8 @@ GridBuffers grid_buffers(Engine& E) {
     g.spx = E.d_spx;
     g.spy = E.d_spy;
     g.spz = E.d_spz;
-    g.pk = E.d_pk;
+    g.phi = E.d_phi;
+    g.plo = E.d_plo;
     g.sgroup = E.d_sgroup;
     g.table = E.d_table;
     g.table_gaps = E.cfg.table_gaps;
@@ -597,7 +600,8 @@ ClipParams base_params(Engine& E) {
     p.spx = E.d_spx;
     p.spy = E.d_spy;
     p.spz = E.d_spz;
-    p.pk = E.d_pk;
+    p.phi = E.d_phi;
+    p.plo = E.d_plo;
     p.sorted = E.d_sorted;
     p.delims = E.d_delims;
     p.sgroup = E.d_sgroup;
@@ -1218,7 +1222,7 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
         E.bnd_valid = true;
     }
     p.bnd = E.d_bnd;
-    p.pk = E.d_pk;
+    p.phi = E.d_phi;
     const double r2 = radius * radius;
     p.f32_filter = mode == RQ_REAL_RADIUS && std::isfinite(radius) && r2 >= 1e-30 && r2 <= 1e36;
     if (mode == RQ_CLOUD) {
@@ -1862,7 +1866,7 @@ static tess_status batch_run(tess_batch* b, int prec) {
         CU(cudaEventRecord(ev.e[0], E.stream));
     }
     CU(cudaGraphLaunch(G, E.stream));
-    E.launches += kGridLaunches + (prec != TESS_PRECISION_FP64 ? 7 : 3);
+    E.launches += kGridLaunches + (prec != TESS_PRECISION_FP64 ? 8 : 3);
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     unsigned long long used = 0;
     unsigned counts[16];

@@ -213,36 +213,6 @@ __device__ __forceinline__ void two_prod(float a, float b, float& p, float& e) {
     e = __fmaf_rn(a, b, -p);
 }
 
-// q = b / d and r = b % d, exactly, for b < 2^32 and a quotient below 2^11
-// (bin coordinates: cpd <= 1625).  The FP32 estimate b * (1/d) carries three
-// roundings of 2^-24 relative, under 2e-4 on such a quotient, so its floor is
-// off by at most one and one correction step settles it.
-__device__ __forceinline__ void divmod_est(uint32_t b, uint32_t d, float rcp, uint32_t& q, uint32_t& r) {
-    long long qq = (long long)((float)b * rcp);
-    long long rr = (long long)b - qq * (long long)d;
-    if (rr < 0) {
-        --qq;
-        rr += d;
-    } else if (rr >= (long long)d) {
-        ++qq;
-        rr -= d;
-    }
-    q = (uint32_t)qq;
-    r = (uint32_t)rr;
-}
-
-// Bin coordinates of local bin id b = (x * cpd + y) * cpd + z
-// (get_cell_from_indices, celery.rs:317-325), without FP64.
-__device__ __forceinline__ void split_bin(uint32_t b, int cpd, float rcp, float rcp2, int& x, int& y, int& z) {
-    const uint32_t c = (uint32_t)cpd;
-    uint32_t qx, rx, qy, ry;
-    divmod_est(b, c * c, rcp2, qx, rx);
-    divmod_est(rx, c, rcp, qy, ry);
-    x = (int)qx;
-    y = (int)qy;
-    z = (int)ry;
-}
-
 // Signed distance n.v - offset.
 __device__ __forceinline__ float sdist(float nx, float ny, float nz, float off, float x, float y, float z) {
     return fmaf(nx, x, fmaf(ny, y, fmaf(nz, z, -off)));
@@ -313,7 +283,7 @@ __device__ __forceinline__ double recip_nr(double d) {
 // is one compare.  Planes beyond FP32's range take the FP64 root.
 __device__ __forceinline__ double tol_of(double n2) {
     const float n2f = (float)n2;
-    return n2f < 1e37f ? (double)(1e-12f * sqrtf(n2f)) : kTolerance * sqrt(n2);
+    return n2f >= FLT_MIN && n2f < 1e37f ? (double)(1e-12f * sqrtf(n2f)) : kTolerance * sqrt(n2);
 }
 
 __device__ __forceinline__ float round_up_f(float x) { return x; }
@@ -1033,7 +1003,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
             shy = __double2float_rn(uy); sly = __double2float_rn(uy - (double)shy);
             shz = __double2float_rn(uz); slz = __double2float_rn(uz - (double)shz);
         } else {
-            const float4 h = P.pk[2ull * gs], l = P.pk[2ull * gs + 1];
+            const float4 h = P.phi[gs], l = P.plo[gs];
             shx = h.x; shy = h.y; shz = h.z;
             slx = l.x; sly = l.y; slz = l.z;
         }
@@ -1133,6 +1103,9 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
         dup2 = d * d;
     }
     int status = ST_OK;
+    // a cell whose squared radius underflows in FP32 is FP64's
+    if constexpr (GUARD)
+        if (!(R2 >= FLT_MIN)) status = ST_GUARD;
 
     // ---- the walk over bins in shell order (celery.rs:1023-1075) ----
     const int cpd = D.cpd;
@@ -1147,7 +1120,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
     // The offset p - site of sorted point j and its squared length.
     auto cand = [&](uint32_t j, T& rx, T& ry, T& rz, T& r2) {
         if constexpr (GUARD) {
-            const float4 h = P.pk[2ull * j], l = P.pk[2ull * j + 1];
+            const float4 h = P.phi[j], l = P.plo[j];
             rx = (T)((h.x - shx) + (l.x - slx));
             ry = (T)((h.y - shy) + (l.y - sly));
             rz = (T)((h.z - shz) + (l.z - slz));
@@ -1663,7 +1636,7 @@ __device__ void run_cell(const ClipParams& P, Smem<T, K>& S, uint32_t gs, int la
                 } else {
                     const uint32_t j = tess_chk(S.psrc[p], P.npts, P.check, CK_POINT);
                     float sh, se;
-                    const float4 h = P.pk[2ull * j], l = P.pk[2ull * j + 1];
+                    const float4 h = P.phi[j], l = P.plo[j];
                     two_sum(h.x, -shx, sh, se);
                     two_sum(sh, (l.x - slx) + se, q0, l0);
                     two_sum(h.y, -shy, sh, se);

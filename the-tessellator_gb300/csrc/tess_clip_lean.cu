@@ -9,26 +9,30 @@
 //
 //   - The cell's vertices live in shared memory only.  When a window is
 //     loaded, every lane tests its own candidate's bisector against every live
-//     vertex and keeps the Outside ones as a 64-bit mask over the slots.
+//     vertex and keeps the touched ones (Outside or undecided) as a 64-bit mask
+//     over the slots.
 //   - Candidates whose mask is empty can never cut (the cell only shrinks) and
-//     cost nothing more.  The nearest candidate with a live Outside vertex is
+//     cost nothing more.  The nearest candidate with a live touched vertex is
 //     taken by one warp minimum; its mask is the cut's Outside set.
 //   - After a cut every lane tests its candidate against the new vertices
 //     alone (about four).
-//   - A vertex inside a candidate's guard band marks the candidate; a marked
-//     candidate is tested again, one vertex per lane, when its turn comes.
+//   - A vertex inside a candidate's guard band counts as touched; when its
+//     turn comes, the touched vertices are tested again, and one still inside
+//     the band hands the cell over (every such vertex is touched).
 //   - A window with few candidates within reach spreads the vertices of each
 //     test over several lanes.
 //
-// The candidates are cut in the same order, by the same arithmetic and with
-// the same Outside sets as a test of one candidate at a time against one
-// vertex per lane, which is what this pass did before: 49 tests per cell, of
-// which 32 cut nothing.
+// A test of one candidate at a time against one vertex per lane, as in
+// tess_clip_impl.cuh, takes 49 serial tests per cell, of which 32 cut nothing.
 //
-// What bounds it: instruction issue.  An ncu capture at 262,144 uniform points
-// counts 10.7 k warp instructions per cell at 72% issue utilisation with 20
-// warps per SM; before, 12.9 k at 63% with 16 (the vertices were in registers
-// too).  1,000,000 uniform points: 16.4 -> 11.9 ms.
+// What bounds it: instruction issue.  1,000,000 uniform points: 16.4 ms that
+// way with the vertices in registers (12.9 k warp instructions per cell, 16
+// warps per SM), 11.9 ms with a candidate per lane, 10.6 ms with the bins taken
+// as rows (three batches a cell instead of five) and the undecided vertices
+// found at the cut instead of in every test.  The code has to stay small: past
+// about 40 KB of it the warps, each at another place, wait for instructions.
+#include <climits>
+
 #include "tess_clip_impl.cuh"
 
 namespace tess {
@@ -56,6 +60,8 @@ struct Lean {
             float vr[kSlots];               // (|v| + e_v)^2
             float4 cand[32];                // a window's candidates within reach: plane ...
             float candn[32];                // ... and |normal|
+            float4 nv[32];                  // the new vertices of a cut, in order ...
+            alignas(4) uint8_t nvs[32];     // ... and their slots
             uint32_t boff[32];              // batch: start - prefix of the k-th bin that holds points
             uint16_t items[32];             // boundary edges of a cut with more than 32 edges
             uint8_t fl[kSlots + kSlots];    // free-slot stack (top = lowest free slot)
@@ -115,46 +121,69 @@ __device__ __forceinline__ void plane_test(const float4& v, float nx, float ny, 
     sd = sdist(nx, ny, nz, off, v.x, v.y, v.z);
     band = fmaf(rn, v.w, c0);
 }
-
-// Bins of one step of the walk beyond the table (Chebyshev rings), one per
-// lane.  Rare: kept out of line.  Returns false when the walk is over.
-__device__ __noinline__ bool ring_step(const ClipParams& P, const DiagDesc& D, float R2, int cbx, int cby, int cbz,
-                                       int lane, int& ring, uint32_t& r0, uint32_t& beg, uint32_t& cnt) {
-    beg = cnt = 0;
-    if (r0 == 0) {
-        double lbk = (double)(ring - 1) * D.min_size;
-        lbk = lbk * lbk;
-        if (lbk < D.tab_kmax) lbk = D.tab_kmax;
-        if (ring > D.cpd - 1 || lbk >= 4.0 * (double)R2 * kStopMargin || (P.search_radius >= 0.0 && lbk > P.search_radius))
-            return false;
-    }
-    const uint32_t rs = 24u * (uint32_t)ring * (uint32_t)ring + 2u;
-    const uint32_t r = r0 + lane;
-    if (r < rs) {
-        int i, j, k;
-        ring_offset(ring, r, i, j, k);
-        const double key = gap_key(D.size, i, j, k);
-        if (key > D.tab_kmax && key < 4.0 * (double)R2 * kStopMargin && !(P.search_radius >= 0.0 && key > P.search_radius)) {
-            const int x = cbx + i, y = cby + j, z = cbz + k, c = D.cpd;
-            if (x >= 0 && x < c && y >= 0 && y < c && z >= 0 && z < c) {
-                const uint64_t lb = tess_chk(D.bin_base + ((uint64_t)x * c + y) * c + z, P.nbins, P.check, CK_BIN);
-                beg = P.delims[lb];
-                cnt = P.delims[lb + 1] - beg;
-            }
-        }
-    }
-    r0 += 32;
-    if (r0 >= rs) {
-        r0 = 0;
-        ++ring;
-    }
-    return true;
+// Outside, or undecided in FP32.
+__device__ __forceinline__ bool touched(const float4& v, float nx, float ny, float nz, float off, float rn, float c0) {
+    float sd, band;
+    plane_test(v, nx, ny, nz, off, rn, c0, sd, band);
+    return sd >= -band;
 }
 
-// The exact search-radius test of a bin offset; out of line, few callers ask
-// for a radius.
-__device__ __noinline__ bool beyond_radius(const DiagDesc& D, double radius, int i, int j, int k) {
-    return gap_key(D.size, i, j, k) > radius;
+// The rows of bins (fixed x and y offset, running in z) in the order they are
+// walked, packed per lane: byte 0/1 the x/y offset in the first batch, byte
+// 2/3 in the second.
+//   first batch: lanes 2r, 2r + 1 the part of central row r below and above
+//     the 27 bins around the site's; lanes 18..29 the twelve rows at x or
+//     y offset +-2 beside them
+//   second batch: the corners (+-2, +-2), then the 24 rows of ring 3
+__device__ uint32_t row_plan(int lane) {
+    int ia = 0, ja = 0, ib = 0, jb = 0;
+    if (lane < 18) {
+        ia = (lane >> 1) / 3 - 1;
+        ja = (lane >> 1) % 3 - 1;
+    } else if (lane < 30) {
+        const int q = lane - 18, e = q % 3 - 1, f = (q / 3) & 1 ? 2 : -2;
+        ia = q < 6 ? f : e;
+        ja = q < 6 ? e : f;
+    }
+    if (lane < 4) {
+        ib = lane & 1 ? 2 : -2;
+        jb = lane & 2 ? 2 : -2;
+    } else if (lane < 28) {
+        const int q = lane - 4;
+        if (q < 14) {
+            ib = q < 7 ? -3 : 3;
+            jb = q % 7 - 3;
+        } else {
+            ib = (q - 14) % 5 - 2;
+            jb = q < 19 ? -3 : 3;
+        }
+    }
+    return (uint32_t)(ia & 0xFF) | (uint32_t)(ja & 0xFF) << 8 | (uint32_t)(ib & 0xFF) << 16 | (uint32_t)(jb & 0xFF) << 24;
+}
+// Row r of the 8 m rows of ring m (rows with max(|i|, |j|) = m).
+__device__ __forceinline__ void ring_row(int m, int r, int& i, int& j) {
+    const int side = 2 * m + 1;
+    if (r < 2 * side) {
+        i = r < side ? -m : m;
+        j = r % side - m;
+    } else {
+        r -= 2 * side;
+        i = r % (side - 2) - (m - 1);
+        j = r < side - 2 ? -m : m;
+    }
+}
+
+// A search radius (rare, out of line): the site's exact bin, and the end of
+// the bins of a row whose search-order key stays within it (the key grows
+// with the distance along the row).
+__device__ __noinline__ int exact_bin(const ClipParams& P, const DiagDesc& D, uint32_t gs, int a) {
+    const double x = a == 0 ? P.spx[gs] : (a == 1 ? P.spy[gs] : P.spz[gs]);
+    return axis_index(x, D.glo[a], D.ghi[a], D.inv[a], D.cpd);
+}
+__device__ __noinline__ int radius_reach(const DiagDesc& D, double radius, int i, int j, int k) {
+    const int step = k > 0 ? -1 : 1;
+    while (k != 0 && gap_key(D.size, i, j, k) > radius) k += step;
+    return (k == 0 && gap_key(D.size, i, j, 0) > radius) ? INT_MAX : k;
 }
 
 // A wall's distance from the site in FP64 (only cells that touch the box).
@@ -165,11 +194,11 @@ __device__ __noinline__ double wall_distance(const ClipParams& P, const DiagDesc
 }
 
 template <bool EXACT>
-__device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t gs, const DiagDesc& D, uint32_t& gen,
+__device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t gs, const DiagDesc& D, uint32_t plan, uint32_t& gen,
                                          int lane) {
     const unsigned lt = (1u << lane) - 1u;
     const uint32_t pt_base = D.pt_base;
-    const float4 site_h = P.pk[2ull * gs], site_l = P.pk[2ull * gs + 1];
+    const float4 site_h = P.phi[gs], site_l = P.plo[gs];
     const float shx = site_h.x, shy = site_h.y, shz = site_h.z;
     const float slx = site_l.x, sly = site_l.y, slz = site_l.z;
     const uint32_t orig = tess_chk(__float_as_uint(site_h.w), P.npts, P.check, CK_POINT);
@@ -229,96 +258,135 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
     }
     int status = ST_OK;
 
-    // ---- the walk over bins in shell order (celery.rs:1023-1075) ----
+    // ---- the walk: bins around the site, nearest rows first ----
+    // (ExpandingSearch, celery.rs:865-1075, visits single bins in key order;
+    // any order that covers the bins within twice the cell radius gives the
+    // same cell).  Bins of one x and y are contiguous in the sorted order along
+    // z, so a lane takes a whole row of them as one range:
+    //   batch 0   the 27 bins around the site's, no test
+    //   batch 1   the rest of those nine rows and the twelve rows beside them
+    //   batch 2   the four corner rows and ring 3
+    //   then      ring by ring (sparse regions)
+    // Rows and their ends beyond twice the current cell radius are left out.
     const int cpd = D.cpd;
-    const uint64_t bin_base = D.bin_base;
-    const uint32_t tab_len = D.tab_len;
-    const TabEntry* tab = P.table + D.tab_base;
-    int cbx, cby, cbz;
-    split_bin(__float_as_uint(site_l.w) - (uint32_t)bin_base, cpd, D.rcp_cpd, D.rcp_cpd2, cbx, cby, cbz);
-    // the site's place inside its bin (within D.frac_eps bins): a point of the
-    // bin at offset o > 0 is at least o - f bin sides away, o < 0 at least
-    // -o - 1 + f
-    const float fx = ((shx - D.glo_hi[0]) + (slx - D.glo_lo[0])) * D.inv_f[0] - (float)cbx;
-    const float fy = ((shy - D.glo_hi[1]) + (sly - D.glo_lo[1])) * D.inv_f[1] - (float)cby;
-    const float fz = ((shz - D.glo_hi[2]) + (slz - D.glo_lo[2])) * D.inv_f[2] - (float)cbz;
-    const bool near_ok = fx >= -1e-3f && fx <= 1.001f && fy >= -1e-3f && fy <= 1.001f && fz >= -1e-3f && fz <= 1.001f &&
-                         D.has_extent;
-    // a batch entry: its key, (1 - 1e-4) times the squared distance to the
-    // bin's nearest point, and its sorted range
-    float ekey, enear;
-    uint32_t ebeg, ecnt;
-    auto load_entry = [&](uint32_t idx) {
-        ekey = INFINITY;
-        enear = 0.f;
-        ebeg = ecnt = 0;
-        if (idx < tab_len) {
-            const TabEntry te = tab[idx];
-            const int i = te.i, j = te.j, k = te.k;
-            ekey = te.key;
-            if (P.has_radius && beyond_radius(D, P.search_radius, i, j, k)) ekey = INFINITY;
-            const int x = cbx + i, y = cby + j, z = cbz + k;
-            if (near_ok) {
-                const float feps = D.frac_eps;
-                const float fxc = fminf(fmaxf(fx, 0.f), 1.f), fyc = fminf(fmaxf(fy, 0.f), 1.f),
-                            fzc = fminf(fmaxf(fz, 0.f), 1.f);
-                const float dx = i > 0 ? fmaxf((float)i - fxc - feps, 0.f) : (i < 0 ? fmaxf((float)(-i - 1) + fxc - feps, 0.f) : 0.f);
-                const float dy = j > 0 ? fmaxf((float)j - fyc - feps, 0.f) : (j < 0 ? fmaxf((float)(-j - 1) + fyc - feps, 0.f) : 0.f);
-                const float dz = k > 0 ? fmaxf((float)k - fzc - feps, 0.f) : (k < 0 ? fmaxf((float)(-k - 1) + fzc - feps, 0.f) : 0.f);
-                const float ax = dx * D.size_f[0], ay = dy * D.size_f[1], az = dz * D.size_f[2];
-                enear = (ax * ax + ay * ay + az * az) * (1.0f - 1e-4f);
-            }
-            // bins beyond twice the cell radius hold no cutter
-            if (x >= 0 && x < cpd && y >= 0 && y < cpd && z >= 0 && z < cpd && !(near_ok && enear >= 4.f * R2)) {
-                const uint64_t lb = tess_chk(bin_base + ((uint64_t)x * cpd + y) * cpd + z, P.nbins, P.check, CK_BIN);
-                ebeg = P.delims[lb];
-                ecnt = P.delims[lb + 1] - ebeg;
-            }
-        }
-    };
-    // The next batch's entries are loaded before the current one is cut; the
-    // first turn of the loop only loads.
-    uint32_t t = 0xFFFFFFE0u;
-    int ring = 1;
-    uint32_t ring_r0 = 0;
-    bool table = true, last = false;
-    ekey = -INFINITY;
-    enear = INFINITY;
-    ebeg = ecnt = 0;
+    const float feps = D.frac_eps;
+    // the site in bin units (within feps), its bin and its place in it
+    const float inx = D.inv_s[0], iny = D.inv_s[1], inz = D.inv_s[2];
+    float px = ((shx - D.glo_hi[0]) + (slx - D.glo_lo[0])) * inx, py = ((shy - D.glo_hi[1]) + (sly - D.glo_lo[1])) * iny,
+          pz = ((shz - D.glo_hi[2]) + (slz - D.glo_lo[2])) * inz;
+    int cbx = min(max((int)px, 0), cpd - 1), cby = min(max((int)py, 0), cpd - 1), cbz = min(max((int)pz, 0), cpd - 1);
+    // an axis without extent has all its points in the last bin
+    if (inx == 0.f) px = cbx = cpd - 1;
+    if (iny == 0.f) py = cby = cpd - 1;
+    if (inz == 0.f) pz = cbz = cpd - 1;
+    if (P.has_radius) {
+        cbx = exact_bin(P, D, gs, 0);
+        cby = exact_bin(P, D, gs, 1);
+        cbz = exact_bin(P, D, gs, 2);
+    }
+    const float fx = fminf(fmaxf(px - (float)cbx, 0.f), 1.f), fy = fminf(fmaxf(py - (float)cby, 0.f), 1.f);
+    uint32_t pend = 0;               // batch 0: where my row's points that were not taken start
+    int m = 0, ring0 = 0;            // batch (0, 1, 2) or ring (4 on); first row of a ring's batch
+    // bin sides or a cell radius outside FP32's normal range
+    if (!D.lean_ok) status = ST_DENSE;
+    if (!(R2 >= FLT_MIN)) status = ST_GUARD;
     while (status == ST_OK) {
-        // ---- the next batch of bins, one per lane ----
-        uint32_t bbeg, bcnt;
-        if (table) {
-            if (last) break;
-            // the key is rounded toward zero and the threshold up: stopping on
-            // key >= thr never drops a bin that could hold a cutter
-            const float thr = 4.f * R2 * (float)kStopMargin;
-            const unsigned ma = __ballot_sync(FULL, !(ekey < thr));
-            const int na = ma ? __ffs(ma) - 1 : 32;
-            bbeg = ebeg;
-            bcnt = lane < na ? ecnt : 0u;
-            if (near_ok && enear >= 4.f * R2) bcnt = 0;
-            t += (uint32_t)na;
-            if (!ma) {
-                load_entry(t + lane);
-                if (t == 0) {
-                    // a crowded own bin (entry 0) sends the cell to the seeded pass
-                    if (P.list_dense && __shfl_sync(FULL, ecnt, 0) >= P.seed_min) status = ST_DENSE;
-                    continue;
-                }
-            } else {
-                // past the table: rings, unless it holds every offset
-                table = !(t >= tab_len && isfinite(D.tab_kmax));
-                last = true;
+        // ---- the next batch: one row of bins per lane ----
+        int i = 0, j = 0;
+        bool have;
+        if (m == 0) {
+            have = lane < 10;
+            if (lane < 9) {
+                i = lane / 3 - 1;
+                j = lane % 3 - 1;
             }
         } else {
-            if (!ring_step(P, D, R2, cbx, cby, cbz, lane, ring, ring_r0, bbeg, bcnt)) break;
+            if (m >= 2) {
+                // the farthest bin offset within reach
+                const float rc = 2.f * norm_up(R2) * 1.0001f;
+                const float rx_ = rc * inx + feps, ry_ = rc * iny + feps;
+                const float far = fmaxf(fmaxf(rx_ + fx, rx_ + 1.f - fx), fmaxf(ry_ + fy, ry_ + 1.f - fy));
+                if (!(far >= (float)m) || m >= cpd) break;
+            }
+            if (m <= 2) {
+                have = lane < (m == 1 ? 30 : 28);
+                const uint32_t w = m == 1 ? plan : plan >> 16;
+                i = (int8_t)w;
+                j = (int8_t)(w >> 8);
+            } else {
+                have = ring0 + lane < 8 * m;
+                ring_row(m, ring0 + lane, i, j);
+            }
+        }
+        uint32_t bbeg = 0, bcnt = 0;
+        const uint32_t from = __shfl_sync(FULL, pend, lane >> 1);
+        const int x = cbx + i, y = cby + j;
+        if (have && x >= 0 && x < cpd && y >= 0 && y < cpd) {
+            int kl = cbz, kh = cbz;
+            bool on = true;
+            if (m == 0) {
+                if (lane < 9) {
+                    kl = max(cbz - 1, 0);
+                    kh = min(cbz + 1, cpd - 1);
+                }
+            } else {
+                // distance to the row, each gap shortened by the in-bin
+                // position's error bound, and what is left of the reach along z
+                const float dx = fmaxf((i > 0 ? (float)i - fx : (i < 0 ? (float)(-i - 1) + fx : 0.f)) - feps, 0.f) * D.size_f[0];
+                const float dy = fmaxf((j > 0 ? (float)j - fy : (j < 0 ? (float)(-j - 1) + fy : 0.f)) - feps, 0.f) * D.size_f[1];
+                const float rem = 4.f * R2 * 1.0003f - (dx * dx + dy * dy);
+                on = rem > 0.f;
+                const float zr = fminf(norm_up(rem) * inz * 1.0001f + 2.f * feps, 4096.f);
+                kl = max((int)floorf(pz - zr), 0);
+                kh = min((int)floorf(pz + zr), cpd - 1);
+            }
+            if (P.has_radius) {
+                const int a = radius_reach(D, P.search_radius, i, j, min(kl - cbz, 0)), b = radius_reach(D, P.search_radius, i, j, max(kh - cbz, 0));
+                if (a == INT_MAX) on = false;
+                else {
+                    kl = max(kl, cbz + a);
+                    kh = min(kh, cbz + b);
+                }
+            }
+            const bool central = m == 1 && lane < 18;
+            if (central && !(lane & 1)) kh = min(kh, cbz - 2);            // below the 27 bins
+            if (central && (lane & 1)) {                                  // above them, and the points not taken
+                kl = min(cbz + 1, cpd - 1);
+                kh = max(kh, kl);
+            }
+            if (on && kl <= kh) {
+                const uint64_t row = D.bin_base + ((uint64_t)x * cpd + y) * cpd;
+                bbeg = P.delims[tess_chk(row + kl, P.nbins, P.check, CK_BIN)];
+                const uint32_t end = P.delims[tess_chk(row + kh, P.nbins, P.check, CK_BIN) + 1];
+                if (central && (lane & 1)) bbeg = from;
+                bcnt = end > bbeg ? end - bbeg : 0u;
+            }
+        }
+        if (m == 0) {
+            // a crowded own bin sends the cell to the seeded pass
+            if (P.list_dense && __shfl_sync(FULL, bcnt, 9) >= P.seed_min) status = ST_DENSE;
+            if (lane == 9) bcnt = 0;
         }
         // ---- its points as one stream, 32 per window ----
         const unsigned inc = warp_incl_scan_u(bcnt, lane);
-        const unsigned total = __shfl_sync(FULL, inc, 31);
-        if (total == 0) continue;
+        unsigned total = __shfl_sync(FULL, inc, 31);
         const unsigned pref = inc - bcnt;
+        if (m == 0) {
+            // whole windows only; the rest joins the next batch
+            if (total > 32) total &= ~31u;
+            pend = bbeg + min(max((int)(total - pref), 0), (int)bcnt);
+        }
+        // the batch after this one
+        if (m < 3) {
+            m = m == 2 ? 4 : m + 1;
+        } else {
+            ring0 += 32;
+            if (ring0 >= 8 * m) {
+                ++m;
+                ring0 = 0;
+            }
+        }
+        if (total == 0) continue;
         {
             const unsigned nz = __ballot_sync(FULL, bcnt > 0);
             if (bcnt) S.boff[__popc(nz & lt)] = bbeg - pref;
@@ -331,18 +399,18 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
             const unsigned c = w0 + lane;
             bool keep = false, near = false;
             float rx = 0.f, ry = 0.f, rz = 0.f, r2 = 0.f;
-            uint32_t j = 0;
+            uint32_t jp = 0;
             float lim = 4.f * R2 * (float)kStopMargin;
             if (c < total) {
-                j = tess_chk(S.boff[before + __popc(heads & (lt | (1u << lane))) - 1] + c, P.npts, P.check, CK_POINT);
-                const float4 h = P.pk[2ull * j], l = P.pk[2ull * j + 1];
+                jp = tess_chk(S.boff[before + __popc(heads & (lt | (1u << lane))) - 1] + c, P.npts, P.check, CK_POINT);
+                const float4 h = P.phi[jp], l = P.plo[jp];
                 rx = (h.x - shx) + (l.x - slx);
                 ry = (h.y - shy) + (l.y - sly);
                 rz = (h.z - shz) + (l.z - slz);
                 r2 = rx * rx + ry * ry + rz * rz;
-                keep = j != gs && r2 > dup2 && r2 < lim;
-                near = j != gs && !(r2 > dup2);
-                if (keep && P.target_group >= 0) keep = (int64_t)(P.sgroup ? P.sgroup[j] : 0u) == P.target_group;
+                keep = jp != gs && r2 > dup2 && r2 < lim;
+                near = jp != gs && !(r2 > dup2);
+                if (keep && P.target_group >= 0) keep = (int64_t)(P.sgroup ? P.sgroup[jp] : 0u) == P.target_group;
             }
             before += __popc(heads);
             // (near-)coincident points are decided in FP64
@@ -354,8 +422,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
             if (!km) continue;
             const float rn = norm_up(r2), off = 0.5f * r2;
             const float c0 = fmaf(rn, gr * rn, eC);
-            uint32_t t0, t1 = 0;                          // my candidate's Outside (or undecided) slots
-            unsigned flg;                                 // candidates with an undecided vertex
+            uint32_t t0, t1 = 0;                          // my candidate's touched slots
             {
                 // 2^sh lanes per candidate, each testing every 2^sh-th slot
                 const int rk = __popc(km & lt);
@@ -369,42 +436,38 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 const float nn = S.candn[lane >> sh];
                 const float cc = fmaf(nn, gr * nn, eC);
                 const int g = 1 << sh, v0 = lane & (g - 1);
-                uint32_t u0 = 0, u1 = 0, w0_ = 0, w1_ = 0;
-                const int s0 = 32 - __clz(l0);
-                for (int v = v0; v < s0; v += g) {
-                    float sd, band;
-                    plane_test(S.vtx[v], n.x, n.y, n.z, n.w, nn, cc, sd, band);
-                    if (sd >= -band) u0 |= 1u << v;
-                    if (fabsf(sd) <= band) w0_ |= 1u << v;
-                }
-                if (l1) {
+                // (two slots per turn; the one past the last is masked off, and
+                // v0 + g * turn stays below 64)
+                const int turns = (32 - __clz(l0) + g - 1) >> sh;
+                const float4* vp = S.vtx + v0;
+                uint32_t u0 = 0, bit = 1u << v0;
 #pragma unroll 1
-                    for (int v = v0; v < 32; v += g) {
-                        float sd, band;
-                        plane_test(S.vtx[32 + v], n.x, n.y, n.z, n.w, nn, cc, sd, band);
-                        if (sd >= -band) u1 |= 1u << v;
-                        if (fabsf(sd) <= band) w1_ |= 1u << v;
-                    }
+                for (int k = 0; k < turns; k += 2) {
+                    const float4 va = vp[0], vb = vp[g];
+                    if (touched(va, n.x, n.y, n.z, n.w, nn, cc)) u0 |= bit;
+                    bit = g < 32 ? bit << g : 0u;
+                    if (touched(vb, n.x, n.y, n.z, n.w, nn, cc)) u0 |= bit;
+                    bit = g < 32 ? bit << g : 0u;
+                    vp += 2 * g;
                 }
 #pragma unroll 1
                 for (int o = 1; o < g; o <<= 1) u0 |= __shfl_xor_sync(FULL, u0, o);
                 t0 = __shfl_sync(FULL, u0, rk << sh);
                 if (l1) {
+                    uint32_t u1 = 0;
+#pragma unroll 1
+                    for (int v = v0; v < 32; v += g)
+                        if (touched(S.vtx[32 + v], n.x, n.y, n.z, n.w, nn, cc)) u1 |= 1u << v;
 #pragma unroll 1
                     for (int o = 1; o < g; o <<= 1) u1 |= __shfl_xor_sync(FULL, u1, o);
                     t1 = __shfl_sync(FULL, u1, rk << sh);
-                }
-                flg = __ballot_sync(FULL, ((w0_ & l0) | (w1_ & l1)) != 0);
-                if (flg) {
-                    const unsigned gm = g == 32 ? FULL : (1u << g) - 1u;
-                    flg = __ballot_sync(FULL, keep && ((flg >> (rk << sh)) & gm) != 0);
                 }
             }
             // Nearest first: the closest candidate that may cut, by a warp
             // minimum of its distance (top 27 bits of r2, ties by lane).
             const unsigned mykey = (__float_as_uint(r2) & ~31u) | (unsigned)lane;
             for (;;) {
-                const bool act = keep && r2 < lim && ((((t0 & l0) | (t1 & l1)) != 0) || ((flg >> lane) & 1u));
+                const bool act = keep && r2 < lim && ((t0 & l0) | (t1 & l1)) != 0;
                 const unsigned best = __reduce_min_sync(FULL, act ? mykey : 0xFFFFFFFFu);
                 if (best == 0xFFFFFFFFu) break;
                 const int src = (int)(best & 31u);
@@ -412,35 +475,11 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 if (lane == src) {
                     S.pl[f] = make_float4(rx, ry, rz, off);
                     S.pn[f] = rn;
-                    S.psrc[f] = j;
+                    S.psrc[f] = jp;
                     keep = false;
                 }
                 km &= ~(1u << src);
-                uint32_t o0 = __shfl_sync(FULL, t0, src) & l0, o1 = __shfl_sync(FULL, t1, src) & l1;
-                if ((flg >> src) & 1u) {
-                    // one vertex per lane against this candidate
-                    __syncwarp();
-                    const float4 n = S.pl[f];
-                    const float nn = S.pn[f];
-                    const float cc = fmaf(nn, gr * nn, eC);
-                    float sd, band;
-                    plane_test(S.vtx[lane], n.x, n.y, n.z, n.w, nn, cc, sd, band);
-                    const bool lv = (l0 >> lane) & 1u;
-                    bool und = lv && fabsf(sd) <= band;
-                    o0 = __ballot_sync(FULL, lv && sd > 0.f);
-                    o1 = 0;
-                    if (l1) {
-                        plane_test(S.vtx[32 + lane], n.x, n.y, n.z, n.w, nn, cc, sd, band);
-                        const bool lv1 = (l1 >> lane) & 1u;
-                        und |= lv1 && fabsf(sd) <= band;
-                        o1 = __ballot_sync(FULL, lv1 && sd > 0.f);
-                    }
-                    if (__any_sync(FULL, und)) {
-                        status = ST_GUARD;
-                        break;
-                    }
-                    if (!(o0 | o1)) continue;
-                }
+                const uint32_t o0 = __shfl_sync(FULL, t0, src) & l0, o1 = __shfl_sync(FULL, t1, src) & l1;
                 // ---- cut by plane f: the Outside slots are o0, o1 ----
                 if (f >= kPlanes) {
                     status = ST_PCAP;
@@ -459,11 +498,13 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 if ((o0 >> lane) & 1u) S.fl[base + __popc(o0 & lt)] = (uint8_t)lane;
                 if ((o1 >> lane) & 1u) S.fl[base + R0 + __popc(o1 & lt)] = (uint8_t)(32 + lane);
                 __syncwarp();
+                const float4 pf = S.pl[f];
+                const float nf = S.pn[f], cf = fmaf(nf, gr * nf, eC);
                 // an edge of an Outside vertex whose neighbour is not Outside
                 // gets a new vertex: one lane per edge, or (large cuts) one
                 // lane per listed boundary edge
                 int a = 0, b = 0, y = 0, q = 0, B;      // y: the neighbour's slot | edge index << 6
-                bool bnd = false;
+                bool bnd = false, und = false;           // und: a touched vertex in the guard band
                 auto edge = [&](int x, int e) {
                     const uint2 tp = S.topo[x];
                     a = byte_of(tp.x, e);
@@ -474,7 +515,11 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 if (3 * R <= 32) {
                     if (lane < 3 * R) {
                         const int xi = (lane * 11) >> 5;          // lane / 3 for lane < 32
-                        bnd = edge(S.fl[base + xi], lane - 3 * xi);
+                        const int x = S.fl[base + xi];
+                        bnd = edge(x, lane - 3 * xi);
+                        float sd, band;
+                        plane_test(S.vtx[x], pf.x, pf.y, pf.z, pf.w, nf, cf, sd, band);
+                        und = sd <= band;
                     }
                     const unsigned bm = __ballot_sync(FULL, bnd);
                     B = __popc(bm);
@@ -490,6 +535,9 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                             x = S.fl[base + ei / 3];
                             e = ei % 3;
                             bd = edge(x, e);
+                            float sd, band;
+                            plane_test(S.vtx[x], pf.x, pf.y, pf.z, pf.w, nf, cf, sd, band);
+                            und |= sd <= band;
                         }
                         const unsigned bm = __ballot_sync(FULL, bd);
                         const int at = B + __popc(bm & lt);
@@ -504,6 +552,10 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                         edge(it & 0xFF, it >> 8);
                     }
                 }
+                if (__any_sync(FULL, und)) {
+                    status = ST_GUARD;
+                    break;
+                }
                 // more vertices than lanes or free slots: the larger forms
                 if (B > 32 || B > base + R) {
                     status = ST_VCAP;
@@ -516,7 +568,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 if (bnd) {
                     // the vertex of planes (a, b, f) by Cramer's rule; its error
                     // depends on its own conditioning only
-                    const float4 pa = S.pl[a], pb = S.pl[b], pf = S.pl[f];
+                    const float4 pa = S.pl[a], pb = S.pl[b];
                     const float bfx = pb.y * pf.z - pb.z * pf.y, bfy = pb.z * pf.x - pb.x * pf.z, bfz = pb.x * pf.y - pb.y * pf.x;
                     const float fax = pf.y * pa.z - pf.z * pa.y, fay = pf.z * pa.x - pf.x * pa.z, faz = pf.x * pa.y - pf.y * pa.x;
                     const float abx = pa.y * pb.z - pa.z * pb.y, aby = pa.z * pb.x - pa.x * pb.z, abz = pa.x * pb.y - pa.y * pb.x;
@@ -526,12 +578,13 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                     const float py = (pa.w * bfy + pb.w * fay + pf.w * aby) * inv;
                     const float pz = (pa.w * bfz + pb.w * faz + pf.w * abz) * inv;
                     const float x1 = fabsf(px) + fabsf(py) + fabsf(pz);
-                    float pe = kVertexErr * x1 * (S.pn[a] * S.pn[b] * S.pn[f]) * fabsf(inv);
+                    float pe = kVertexErr * x1 * (S.pn[a] * S.pn[b] * nf) * fabsf(inv);
                     // singular (or nearly): not a vertex to go on from
                     bad = !(pe < 1e30f);
                     pe += gr * x1;
                     slot = tess_chk((int)S.fl[base + R - 1 - q], kSlots, P.check, CK_SLOT);
-                    S.vtx[slot] = make_float4(px, py, pz, pe);
+                    S.vtx[slot] = S.nv[q] = make_float4(px, py, pz, pe);
+                    S.nvs[q] = (uint8_t)slot;
                     S.vr[slot] = vertex_r2(px, py, pz, pe);
                     // Y's edge back to X now leads to the new vertex's edge 0
                     reinterpret_cast<uint8_t*>(&S.topo[y & 63].y)[y >> 6] = (uint8_t)slot;
@@ -563,29 +616,28 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 // waiting candidates
                 float rr = ((l0 >> lane) & 1u) ? S.vr[lane] : 0.f;
                 if ((l1 >> lane) & 1u) rr = fmaxf(rr, S.vr[32 + lane]);
+                R2 = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(rr)));
                 if (km) {
-                    bool amb = false;
                     t0 &= ~n0;
                     t1 &= ~n1;
+                    if (!n1) {
 #pragma unroll 1
-                    for (uint32_t m = n0; m; m &= m - 1u) {
-                        const int s = __ffs(m) - 1;
-                        float sd, band;
-                        plane_test(S.vtx[s], rx, ry, rz, off, rn, c0, sd, band);
-                        if (sd >= -band) t0 |= 1u << s;
-                        amb |= fabsf(sd) <= band;
-                    }
+                        for (int q0 = 0; q0 < B; q0 += 4) {
+                            const uint32_t sl = *reinterpret_cast<const uint32_t*>(S.nvs + q0);
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                if (touched(S.nv[q0 + k], rx, ry, rz, off, rn, c0) && q0 + k < B) t0 |= 1u << byte_of(sl, k);
+                        }
+                    } else {
 #pragma unroll 1
-                    for (uint32_t m = n1; m; m &= m - 1u) {
-                        const int s = __ffs(m) - 1;
-                        float sd, band;
-                        plane_test(S.vtx[32 + s], rx, ry, rz, off, rn, c0, sd, band);
-                        if (sd >= -band) t1 |= 1u << s;
-                        amb |= fabsf(sd) <= band;
+                        for (int k = 0; k < B; ++k) {
+                            const int s = S.nvs[k];
+                            const bool hit = touched(S.nv[k], rx, ry, rz, off, rn, c0);
+                            if (hit && s < 32) t0 |= 1u << s;
+                            if (hit && s >= 32) t1 |= 1u << (s - 32);
+                        }
                     }
-                    flg |= __ballot_sync(FULL, keep && amb);
                 }
-                R2 = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(rr)));
                 lim = 4.f * R2 * (float)kStopMargin;
                 if (__any_sync(FULL, bad)) {
                     status = ST_DEGEN;
@@ -640,7 +692,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                         qz = a == 2 ? (mx ? 1.0 : -1.0) : 0.0;
                     } else {
                         const uint32_t j = tess_chk(S.psrc[p], P.npts, P.check, CK_POINT);
-                        id = (int32_t)(__float_as_uint(P.pk[2ull * j].w) - pt_base);
+                        id = (int32_t)(__float_as_uint(P.phi[j].w) - pt_base);
                         qx = P.spx[j] - P.spx[gs];
                         qy = P.spy[j] - P.spy[gs];
                         qz = P.spz[j] - P.spz[gs];
@@ -667,7 +719,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                         dist = hh;
                     } else {
                         const uint32_t j = tess_chk(S.psrc[p], P.npts, P.check, CK_POINT);
-                        const float4 h = P.pk[2ull * j], l = P.pk[2ull * j + 1];
+                        const float4 h = P.phi[j], l = P.plo[j];
                         id = (int32_t)(__float_as_uint(h.w) - pt_base);
                         float sh, se;
                         two_sum(h.x, -shx, sh, se);
@@ -919,6 +971,7 @@ __global__ void __launch_bounds__(128, 5) k_lean(ClipParams P) {
     const int lane = threadIdx.x & 31;
     if (P.grid_err && *P.grid_err == 1) return;   // non-finite input: nothing to clip
     for (int i = lane; i < kPlanes; i += 32) S.map[i] = 0;
+    const uint32_t plan = row_plan(lane);
     uint32_t gen = 0;
     int d = 0;                                    // diagram of the last cell
     const unsigned total = P.work_count ? *P.work_count : P.total;
@@ -939,7 +992,7 @@ __global__ void __launch_bounds__(128, 5) k_lean(ClipParams P) {
             }
             d = lo;
         }
-        run_lean<EXACT>(P, S, gs, P.diags[d], gen, lane);
+        run_lean<EXACT>(P, S, gs, P.diags[d], plan, gen, lane);
         w = __shfl_sync(FULL, wn, 0);
     }
 }

@@ -124,6 +124,7 @@ __global__ void k_grid_params(GridBuffers g) {
     DiagDesc& D = g.diags[d];
     const double c = (double)D.cpd;
     double m = DBL_MAX;
+    bool lean_ok = true;
     for (int a = 0; a < 3; ++a) {
         const double lo = ord_dec(g.bounds[6 * d + a]);
         const double hi = ord_dec(g.bounds[6 * d + 3 + a]);
@@ -147,9 +148,11 @@ __global__ void k_grid_params(GridBuffers g) {
         D.inv_f[a] = __double2float_rn(D.inv[a]);
         D.glo_f[a] = __double2float_rn(lo);
         D.size_f[a] = __double2float_rn(D.size[a]);
+        D.inv_s[a] = ext > 0.0 ? D.inv_f[a] : 0.f;
+        if (ext > 0.0)
+            lean_ok = lean_ok && D.size_f[a] >= FLT_MIN && D.size_f[a] <= FLT_MAX && D.inv_f[a] >= FLT_MIN && D.inv_f[a] <= FLT_MAX;
     }
-    D.rcp_cpd = 1.0f / (float)D.cpd;
-    D.rcp_cpd2 = 1.0f / ((float)D.cpd * (float)D.cpd);
+    D.lean_ok = lean_ok;
     // (x - glo) * inv from the FP32 pairs: one rounding of the difference, one
     // of inv, one of the product (u = 2^-24 each, relative to the result, at
     // most cpd bins), with a factor 4 in hand
@@ -432,9 +435,8 @@ __global__ void k_gather(GridBuffers g) {
         hi4[a] = h;
         lo4[a] = l;
     }
-    // one 32-byte sector per point: what the clipping reads of a candidate
-    g.pk[2ull * s] = make_float4(hi4[0], hi4[1], hi4[2], __uint_as_float(i));
-    g.pk[2ull * s + 1] = make_float4(lo4[0], lo4[1], lo4[2], __uint_as_float(g.bin[i]));
+    g.phi[s] = make_float4(hi4[0], hi4[1], hi4[2], __uint_as_float(i));
+    g.plo[s] = make_float4(lo4[0], lo4[1], lo4[2], 0.f);
     if (g.sgroup) g.sgroup[s] = g.groups[i];
 }
 

@@ -7,8 +7,8 @@
 //   grid     delims[total_bins + 1]     CSR offsets of the bin-sorted order
 //   sorted   sorted[total]              sorted position -> point (concatenated index)
 //            spx/spy/spz[total]         FP64 positions in sorted order (SoA)
-//            pk[2 * total]              per sorted point, one 32-byte sector: the FP32 pair of
-//                                       its position, its point index and its bin
+//            phi/plo[total]             FP32 pair of the sorted positions, 16 bytes each, the
+//                                       point's index in the high part's fourth word
 //            sgroup[total]              group ids in sorted order (optional)
 //   table    tab[...]                   per-diagram shell table (sorted offsets)
 //   results  vol[total], nface[total], fstart[total], status[total]  (point order)
@@ -98,9 +98,10 @@ struct DiagDesc {
     float inv_f[3];                      // inverse bin sides
     float glo_f[3];                      // point bounds' low corner, rounded to FP32
     float size_f[3];                     // bin sides
-    float rcp_cpd, rcp_cpd2;             // 1 / cpd, 1 / cpd^2 (bin id -> coordinates)
+    float inv_s[3];                      // inverse bin sides, 0 on an axis without extent
     float frac_eps;                      // bound on the FP32 in-bin position's error, in bins
     int32_t has_extent;                  // some bin side is nonzero (min_size > 0)
+    int32_t lean_ok;                     // inv_s and size_f are in FP32's normal range (or 0)
 };
 
 // Shell-table entry: a bin offset and its search-order key (celery.rs:423-427)
@@ -179,8 +180,9 @@ struct GridBuffers {
     double* spy;
     double* spz;
     // FP32 split of the sorted positions relative to the centre, x = hi + lo:
-    // pk[2 s] = {hi, point index}, pk[2 s + 1] = {lo, global bin id}
-    float4* pk;
+    // phi = {hi, point index}, plo = {lo, 0}
+    float4* phi;
+    float4* plo;
     uint32_t* sgroup;           // null when groups is null
     TabEntry* table;
     int table_gaps;
@@ -236,7 +238,7 @@ struct RadiusParams {
     uint32_t* out;              // fill pass: bin ids or original point indices
     int* err;                   // set to 1 when a query cell is out of range
     const uint32_t* qorder;     // processing order of the queries (spatially sorted), or null
-    const float4* pk;           // FP32 split of the sorted positions (see GridBuffers), for the FP32 filter
+    const float4* phi;          // FP32 high parts of the sorted positions (see GridBuffers), for the FP32 filter
     int f32_filter;             // real radius: pre-filter candidates in FP32 (radius in range)
     // check_cell_in_range as a table: for gaps gx <= gtab_x, gy <= gtab_y, the
     // largest gz <= gtab_z whose squared gap distance is within radius^2
@@ -284,7 +286,8 @@ struct ClipParams {
     const double* spx;
     const double* spy;
     const double* spz;
-    const float4* pk;               // FP32 split of the sorted positions, point index, bin (see GridBuffers)
+    const float4* phi;              // FP32 split of the sorted positions, point index (see GridBuffers)
+    const float4* plo;
     const uint32_t* sorted;
     const uint32_t* delims;
     const uint32_t* sgroup;

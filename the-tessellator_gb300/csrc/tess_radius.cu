@@ -123,7 +123,7 @@ __device__ __forceinline__ void emit_stream(const RadiusParams& p, uint32_t beg,
             bool band = false;
             if (qt.on) {
                 if (valid) {
-                    const float4 h = p.pk[2 * (size_t)s];
+                    const float4 h = p.phi[s];
                     const float dx = __fsub_rn(qt.fx, h.x);
                     const float dy = __fsub_rn(qt.fy, h.y);
                     const float dz = __fsub_rn(qt.fz, h.z);
