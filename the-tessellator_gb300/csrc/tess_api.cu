@@ -113,6 +113,11 @@ int64_t cells_per_dim(uint64_t n, double density) {
 // hybrid FP32 pass could not settle).
 enum { L_FP64 = 0, L_CAP1 = 1, L_CAP2 = 2, L_CAP64A = 3, L_CAP64B = 4, L_FP64B = 5, L_DENSE = 6, L_COUNT = 7,
        L_FAIL = 7, L_REASON = 8 };
+// The FP64 form's first pass runs in FP32 (tess_clip_lean.cu): a vertex whose
+// distance from a plane is within the FP32 error bound plus this is left to
+// the FP64 clipping, so that every decision the FP32 pass takes is the one the
+// reference's test (1e-12, vector3.rs:170-185) takes.
+constexpr float kFp64Tol = 1.01e-12f;
 // Kernels launched by one binning pass (launch_grid_build).
 constexpr uint64_t kGridLaunches = 11;
 
@@ -678,9 +683,7 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
         // hybrid form (guard-band tests decided in FP64); what that cannot
         // settle runs in the FP64 form.
         const bool two = s0 < 4, one = s0 < 8 && !norerun;
-        // (with TESS_FLAG_COUNTERS the first pass runs in the standard form:
-        // the lean form keeps no counters)
-        const bool lean = s0 <= 2 && !(E.cfg.flags & TESS_FLAG_COUNTERS);
+        const bool lean = s0 <= 2;
         TRY(pass(1, s0, (lean ? kFormLean : kFormStd) | X, sample, nullptr, L[L_FP64], cnt + L_FP64,
                  one ? L[L_CAP1] : nullptr, cnt + L_CAP1, lean ? L[L_DENSE] : nullptr, cnt + L_DENSE));
         if (lean)
@@ -702,7 +705,19 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
         TRY(pass(0, 8, kFormStd, L[L_CAP64B], cnt + L_CAP64B, nullptr, nullptr, nullptr, nullptr));
     } else {
         const bool two = s0 < 4, one = s0 < 8 && !norerun;
-        TRY(pass(0, s0, kFormStd, sample, nullptr, nullptr, nullptr, one ? L[L_CAP64A] : nullptr, cnt + L_CAP64A));
+        // FP64: the FP32 first pass with the FP64 finish settles the cells whose
+        // every plane test is decided in FP32 beyond its error bound and the
+        // reference's tolerance (see kFp64Tol); all others, crowded bins
+        // included, are clipped in FP64.
+        if (s0 <= 2) {
+            base.tol = kFp64Tol;
+            uint32_t* const rest = L[L_FP64B];
+            unsigned* const nrest = cnt + L_FP64B;
+            TRY(pass(1, 2, kFormLean | kFormExact, sample, nullptr, rest, nrest, rest, nrest, rest, nrest));
+            TRY(pass(0, 2, kFormStd, rest, nrest, nullptr, nullptr, one ? L[L_CAP64A] : nullptr, cnt + L_CAP64A));
+        } else {
+            TRY(pass(0, s0, kFormStd, sample, nullptr, nullptr, nullptr, one ? L[L_CAP64A] : nullptr, cnt + L_CAP64A));
+        }
         if (timing) CU(cudaEventRecord(ev[1], E.stream));
         if (one) {
             const int s1 = two ? 4 : 8;
@@ -1866,7 +1881,7 @@ static tess_status batch_run(tess_batch* b, int prec) {
         CU(cudaEventRecord(ev.e[0], E.stream));
     }
     CU(cudaGraphLaunch(G, E.stream));
-    E.launches += kGridLaunches + (prec != TESS_PRECISION_FP64 ? 8 : 3);
+    E.launches += kGridLaunches + (prec != TESS_PRECISION_FP64 ? 8 : 4);
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     unsigned long long used = 0;
     unsigned counts[16];

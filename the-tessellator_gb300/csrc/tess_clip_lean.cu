@@ -31,6 +31,14 @@
 // as rows (three batches a cell instead of five) and the undecided vertices
 // found at the cut instead of in every test.  The code has to stay small: past
 // about 40 KB of it the warps, each at another place, wait for instructions.
+//
+// With the FP64 finish (MIXED and the FP64 form) the faces' planes, vertices,
+// areas and the volume are computed in FP64 from the FP64 positions; only the
+// decisions which planes meet where are taken in FP32, each beyond its error
+// bound.  For the FP64 form the band is wider by the reference's tolerance, so
+// that every decision is the one its test takes in FP64.  250,007 uniform
+// points in that form: 12.6 -> 3.6 ms; the FP64 clipping it replaces spent
+// about 655 FP64 instructions on a cell, this finish about 130.
 #include <climits>
 
 #include "tess_clip_impl.cuh"
@@ -77,8 +85,8 @@ struct Lean {
             uint8_t face[kPlanes];          // planes that have a face
             uint8_t rank[kPlanes];          // position of the face in id order
         } s;
-        struct {                            // finalize, FP64-accurate
-            double qx[kPlanes], qy[kPlanes], qz[kPlanes], qh[kPlanes];
+        struct {                            // finalize, FP64
+            double2 qa[kPlanes], qb[kPlanes];   // face plane n.x = h: {n.x, n.y}, {n.z, h}
             double rx[kSlots], ry[kSlots], rz[kSlots];   // refined positions
             double area[kPlanes];
             alignas(16) int32_t ids[kPlanes + 4];
@@ -115,7 +123,7 @@ __device__ __forceinline__ float vertex_r2(float x, float y, float z, float e) {
 }
 
 // Signed distance of a vertex and the half-width of its guard band for the
-// plane (n, off) with |n| = rn; c0 = rn * guard_rel * rn + eC.
+// plane (n, off) with |n| = rn; c0 = rn (guard_rel * rn + tol) + eC.
 __device__ __forceinline__ void plane_test(const float4& v, float nx, float ny, float nz, float off, float rn,
                                            float c0, float& sd, float& band) {
     sd = sdist(nx, ny, nz, off, v.x, v.y, v.z);
@@ -193,8 +201,8 @@ __device__ __noinline__ double wall_distance(const ClipParams& P, const DiagDesc
     return (p & 1) ? D.bhi[a] - s : s - D.blo[a];
 }
 
-template <bool EXACT>
-__device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t gs, const DiagDesc& D, uint32_t plan, uint32_t& gen,
+template <bool EXACT, bool COUNT>
+__device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t gs, const DiagDesc& D, uint32_t plan, uint32_t& gen, Work& W,
                                          int lane) {
     const unsigned lt = (1u << lane) - 1u;
     const uint32_t pt_base = D.pt_base;
@@ -202,7 +210,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
     const float shx = site_h.x, shy = site_h.y, shz = site_h.z;
     const float slx = site_l.x, sly = site_l.y, slz = site_l.z;
     const uint32_t orig = tess_chk(__float_as_uint(site_h.w), P.npts, P.check, CK_POINT);
-    const float gr = P.guard_rel;
+    const float gr = P.guard_rel, tol = P.tol;
 
     // ---- the container box, translated by -site (polyhedron.rs:268-392) ----
     // Offsets from the FP32 pairs of the box and the site relative to the
@@ -387,6 +395,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
             }
         }
         if (total == 0) continue;
+        if constexpr (COUNT) ++W.batches;
         {
             const unsigned nz = __ballot_sync(FULL, bcnt > 0);
             if (bcnt) S.boff[__popc(nz & lt)] = bbeg - pref;
@@ -419,9 +428,13 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 break;
             }
             unsigned km = __ballot_sync(FULL, keep);      // candidates within reach
+            if constexpr (COUNT) {
+                ++W.windows;
+                W.tested += (unsigned)__popc(km);
+            }
             if (!km) continue;
             const float rn = norm_up(r2), off = 0.5f * r2;
-            const float c0 = fmaf(rn, gr * rn, eC);
+            const float c0 = fmaf(rn, fmaf(gr, rn, tol), eC);
             uint32_t t0, t1 = 0;                          // my candidate's touched slots
             {
                 // 2^sh lanes per candidate, each testing every 2^sh-th slot
@@ -434,7 +447,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 const int sh = __clz(__popc(km) - 1) - 27;
                 const float4 n = S.cand[lane >> sh];
                 const float nn = S.candn[lane >> sh];
-                const float cc = fmaf(nn, gr * nn, eC);
+                const float cc = fmaf(nn, fmaf(gr, nn, tol), eC);
                 const int g = 1 << sh, v0 = lane & (g - 1);
                 // (two slots per turn; the one past the last is masked off, and
                 // v0 + g * turn stays below 64)
@@ -499,7 +512,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 if ((o1 >> lane) & 1u) S.fl[base + R0 + __popc(o1 & lt)] = (uint8_t)(32 + lane);
                 __syncwarp();
                 const float4 pf = S.pl[f];
-                const float nf = S.pn[f], cf = fmaf(nf, gr * nf, eC);
+                const float nf = S.pn[f], cf = fmaf(nf, fmaf(gr, nf, tol), eC);
                 // an edge of an Outside vertex whose neighbour is not Outside
                 // gets a new vertex: one lane per edge, or (large cuts) one
                 // lane per listed boundary edge
@@ -555,6 +568,10 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 if (__any_sync(FULL, und)) {
                     status = ST_GUARD;
                     break;
+                }
+                if constexpr (COUNT) {
+                    ++W.cuts;
+                    W.newv += (unsigned)B;
                 }
                 // more vertices than lanes or free slots: the larger forms
                 if (B > 32 || B > base + R) {
@@ -698,10 +715,8 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                         qz = P.spz[j] - P.spz[gs];
                         qh = 0.5 * (qx * qx + qy * qy + qz * qz);
                     }
-                    S.d.qx[p] = qx;
-                    S.d.qy[p] = qy;
-                    S.d.qz[p] = qz;
-                    S.d.qh[p] = qh;
+                    S.d.qa[p] = make_double2(qx, qy);
+                    S.d.qb[p] = make_double2(qz, qh);
                 } else {
                     // as FP32 pairs without the FP64 pipe: q by a TwoSum of the
                     // points' high parts (error ~2^-46 of the distance from the
@@ -751,10 +766,10 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
         }
         if (lane < 3) ids[F + lane] = 0x7FFFFFFF;   // the ranks read groups of four
         __syncwarp();
-        // One Newton step per vertex: residuals of its three planes in
-        // double-float (or FP64), the correction solved in FP32 by Cramer's
-        // rule.  A correction beyond the vertex's error bound means the FP32
-        // vertex was not trustworthy: the cell re-runs.
+        // FP32: one Newton step per vertex, residuals of its three planes in
+        // double-float, the correction solved in FP32 by Cramer's rule.  FP64
+        // finish: the vertex solved from its planes in FP64.  A vertex that
+        // moves beyond its error bound was not trustworthy: the cell re-runs.
         auto resid = [&](const float4& h, const float4& l, float x, float y, float z) -> float {
             float p0, e0, p1, e1, p2, e2, s1, t1_, s2, t2, s3, t3;
             two_prod(h.x, x, p0, e0);
@@ -775,46 +790,38 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 const uint32_t tt = S.topo[s].x;
                 const int a = byte_of(tt, 0), b = byte_of(tt, 1), c = byte_of(tt, 2);
                 const float4 v = S.vtx[s];
-                float4 ha, hb, hc;
-                float ra, rb, rc;
+                float ddx, ddy, ddz;
                 if constexpr (EXACT) {
-                    const double x = v.x, y = v.y, z = v.z;
-                    ra = (float)(S.d.qh[a] - (S.d.qx[a] * x + S.d.qy[a] * y + S.d.qz[a] * z));
-                    rb = (float)(S.d.qh[b] - (S.d.qx[b] * x + S.d.qy[b] * y + S.d.qz[b] * z));
-                    rc = (float)(S.d.qh[c] - (S.d.qx[c] * x + S.d.qy[c] * y + S.d.qz[c] * z));
-                    ha = make_float4((float)S.d.qx[a], (float)S.d.qy[a], (float)S.d.qz[a], 0.f);
-                    hb = make_float4((float)S.d.qx[b], (float)S.d.qy[b], (float)S.d.qz[b], 0.f);
-                    hc = make_float4((float)S.d.qx[c], (float)S.d.qy[c], (float)S.d.qz[c], 0.f);
+                    const double2 a0 = S.d.qa[a], a1 = S.d.qb[a], b0 = S.d.qa[b], b1 = S.d.qb[b], c0_ = S.d.qa[c], c1 = S.d.qb[c];
+                    const double bcx = b0.y * c1.x - b1.x * c0_.y, bcy = b1.x * c0_.x - b0.x * c1.x, bcz = b0.x * c0_.y - b0.y * c0_.x;
+                    const double cax = c0_.y * a1.x - c1.x * a0.y, cay = c1.x * a0.x - c0_.x * a1.x, caz = c0_.x * a0.y - c0_.y * a0.x;
+                    const double abx = a0.y * b1.x - a1.x * b0.y, aby = a1.x * b0.x - a0.x * b1.x, abz = a0.x * b0.y - a0.y * b0.x;
+                    const double inv = recip_nr(a0.x * bcx + a0.y * bcy + a1.x * bcz);
+                    const double x = (a1.y * bcx + b1.y * cax + c1.y * abx) * inv;
+                    const double y = (a1.y * bcy + b1.y * cay + c1.y * aby) * inv;
+                    const double z = (a1.y * bcz + b1.y * caz + c1.y * abz) * inv;
+                    S.d.rx[s] = x;
+                    S.d.ry[s] = y;
+                    S.d.rz[s] = z;
+                    ddx = (float)x - v.x;
+                    ddy = (float)y - v.y;
+                    ddz = (float)z - v.z;
                 } else {
-                    ha = S.s.q[a];
-                    hb = S.s.q[b];
-                    hc = S.s.q[c];
-                    ra = resid(ha, S.s.ql[a], v.x, v.y, v.z);
-                    rb = resid(hb, S.s.ql[b], v.x, v.y, v.z);
-                    rc = resid(hc, S.s.ql[c], v.x, v.y, v.z);
-                }
-                const float bcx = hb.y * hc.z - hb.z * hc.y, bcy = hb.z * hc.x - hb.x * hc.z, bcz = hb.x * hc.y - hb.y * hc.x;
-                const float cax = hc.y * ha.z - hc.z * ha.y, cay = hc.z * ha.x - hc.x * ha.z, caz = hc.x * ha.y - hc.y * ha.x;
-                const float abx = ha.y * hb.z - ha.z * hb.y, aby = ha.z * hb.x - ha.x * hb.z, abz = ha.x * hb.y - ha.y * hb.x;
-                const float inv = rcp_ftz(ha.x * bcx + ha.y * bcy + ha.z * bcz);
-                const float ddx = (ra * bcx + rb * cax + rc * abx) * inv;
-                const float ddy = (ra * bcy + rb * cay + rc * aby) * inv;
-                const float ddz = (ra * bcz + rb * caz + rc * abz) * inv;
-                const float vl = 2.0f * v.w + vlim;
-                if (!(fabsf(ddx) <= vl && fabsf(ddy) <= vl && fabsf(ddz) <= vl)) vbad = true;
-                if constexpr (EXACT) {
-                    // a second step from x + d (exact in FP64): what is left is
-                    // the FP64 rounding of the residuals
-                    const double x1 = (double)v.x + (double)ddx, y1 = (double)v.y + (double)ddy, z1 = (double)v.z + (double)ddz;
-                    const float sa_ = (float)(S.d.qh[a] - (S.d.qx[a] * x1 + S.d.qy[a] * y1 + S.d.qz[a] * z1));
-                    const float sb_ = (float)(S.d.qh[b] - (S.d.qx[b] * x1 + S.d.qy[b] * y1 + S.d.qz[b] * z1));
-                    const float sc_ = (float)(S.d.qh[c] - (S.d.qx[c] * x1 + S.d.qy[c] * y1 + S.d.qz[c] * z1));
-                    S.d.rx[s] = x1 + (double)((sa_ * bcx + sb_ * cax + sc_ * abx) * inv);
-                    S.d.ry[s] = y1 + (double)((sa_ * bcy + sb_ * cay + sc_ * aby) * inv);
-                    S.d.rz[s] = z1 + (double)((sa_ * bcz + sb_ * caz + sc_ * abz) * inv);
-                } else {
+                    const float4 ha = S.s.q[a], hb = S.s.q[b], hc = S.s.q[c];
+                    const float ra = resid(ha, S.s.ql[a], v.x, v.y, v.z);
+                    const float rb = resid(hb, S.s.ql[b], v.x, v.y, v.z);
+                    const float rc = resid(hc, S.s.ql[c], v.x, v.y, v.z);
+                    const float bcx = hb.y * hc.z - hb.z * hc.y, bcy = hb.z * hc.x - hb.x * hc.z, bcz = hb.x * hc.y - hb.y * hc.x;
+                    const float cax = hc.y * ha.z - hc.z * ha.y, cay = hc.z * ha.x - hc.x * ha.z, caz = hc.x * ha.y - hc.y * ha.x;
+                    const float abx = ha.y * hb.z - ha.z * hb.y, aby = ha.z * hb.x - ha.x * hb.z, abz = ha.x * hb.y - ha.y * hb.x;
+                    const float inv = rcp_ftz(ha.x * bcx + ha.y * bcy + ha.z * bcz);
+                    ddx = (ra * bcx + rb * cax + rc * abx) * inv;
+                    ddy = (ra * bcy + rb * cay + rc * aby) * inv;
+                    ddz = (ra * bcz + rb * caz + rc * abz) * inv;
                     S.s.dv[s] = make_float4(ddx, ddy, ddz, 0.f);
                 }
+                const float vl = 2.0f * v.w + vlim;
+                if (!(fabsf(ddx) <= vl && fabsf(ddy) <= vl && fabsf(ddz) <= vl)) vbad = true;
             }
         }
         __syncwarp();
@@ -841,7 +848,8 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                     // The area from the face's projection on the plane normal to
                     // the dominant axis m of its normal (shoelace): w_m = 2 A
                     // q_m / |q|; the pyramid from the site is qh w_m / (6 q_m).
-                    const double q0 = S.d.qx[p], q1 = S.d.qy[p], q2 = S.d.qz[p];
+                    const double2 qa = S.d.qa[p], qb = S.d.qb[p];
+                    const double q0 = qa.x, q1 = qa.y, q2 = qb.x;
                     const int m = (fabs(q0) >= fabs(q1) && fabs(q0) >= fabs(q2)) ? 0 : (fabs(q1) >= fabs(q2) ? 1 : 2);
                     const double* X1 = m == 0 ? S.d.ry : (m == 1 ? S.d.rz : S.d.rx);
                     const double* X2 = m == 0 ? S.d.rz : (m == 1 ? S.d.rx : S.d.ry);
@@ -859,7 +867,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                     } while (at != st && steps <= kSlots);
                     const double inv_qm = 1.0 / qm;
                     S.d.area[i] = 0.5 * wm * inv_qm * sqrt(q0 * q0 + q1 * q1 + q2 * q2);
-                    vpart += S.d.qh[p] * wm * inv_qm * 0.5;
+                    vpart += qb.y * wm * inv_qm * 0.5;
                 } else {
                     // fan from the first vertex on refined positions:
                     // (x - anchor) = (x32 - a32) + (dx - da)
@@ -964,7 +972,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
 // 4 warps per block, five blocks per SM: 96 registers, no spills.  At
 // 1,000,000 uniform points: 13.3 ms with 16 warps per SM, 11.9 with 20, 12.4
 // with 24 (80 registers, 19% more instructions and the instruction cache full).
-template <bool EXACT>
+template <bool EXACT, bool COUNT>
 __global__ void __launch_bounds__(128, 5) k_lean(ClipParams P) {
     extern __shared__ __align__(16) unsigned char smraw[];
     Lean& S = reinterpret_cast<Lean*>(smraw)[threadIdx.x >> 5];
@@ -973,6 +981,7 @@ __global__ void __launch_bounds__(128, 5) k_lean(ClipParams P) {
     for (int i = lane; i < kPlanes; i += 32) S.map[i] = 0;
     const uint32_t plan = row_plan(lane);
     uint32_t gen = 0;
+    Work W;
     int d = 0;                                    // diagram of the last cell
     const unsigned total = P.work_count ? *P.work_count : P.total;
     // the next cell's number is fetched while a cell is worked on
@@ -992,12 +1001,21 @@ __global__ void __launch_bounds__(128, 5) k_lean(ClipParams P) {
             }
             d = lo;
         }
-        run_lean<EXACT>(P, S, gs, P.diags[d], plan, gen, lane);
+        run_lean<EXACT, COUNT>(P, S, gs, P.diags[d], plan, gen, W, lane);
         w = __shfl_sync(FULL, wn, 0);
+    }
+    if constexpr (COUNT) {
+        if (lane == 0) {
+            atomicAdd(&P.work_ctr[0], (unsigned long long)W.tested);
+            atomicAdd(&P.work_ctr[1], (unsigned long long)W.cuts);
+            atomicAdd(&P.work_ctr[2], (unsigned long long)W.newv);
+            atomicAdd(&P.work_ctr[3], (unsigned long long)W.windows);
+            atomicAdd(&P.work_ctr[4], (unsigned long long)W.batches);
+        }
     }
 }
 
-template <bool EXACT>
+template <bool EXACT, bool COUNT>
 cudaError_t configure(size_t bytes) {
     static std::mutex mu;
     static size_t configured[kMaxDevices] = {};
@@ -1007,26 +1025,26 @@ cudaError_t configure(size_t bytes) {
     std::lock_guard<std::mutex> lock(mu);
     size_t* slot = (dev >= 0 && dev < kMaxDevices) ? &configured[dev] : nullptr;
     if (slot && bytes <= *slot) return cudaSuccess;
-    e = cudaFuncSetAttribute(k_lean<EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    e = cudaFuncSetAttribute(k_lean<EXACT, COUNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e == cudaSuccess && slot) *slot = bytes;
     return e;
 }
 
-template <bool EXACT>
+template <bool EXACT, bool COUNT>
 cudaError_t launch(const ClipParams& p, int wpb, int blocks, cudaStream_t s) {
     const size_t sm = sizeof(Lean) * (size_t)wpb;
-    cudaError_t e = configure<EXACT>(sm);
+    cudaError_t e = configure<EXACT, COUNT>(sm);
     if (e != cudaSuccess) return e;
-    k_lean<EXACT><<<blocks, 32 * wpb, sm, s>>>(p);
+    k_lean<EXACT, COUNT><<<blocks, 32 * wpb, sm, s>>>(p);
     return cudaGetLastError();
 }
 
-template <bool EXACT>
+template <bool EXACT, bool COUNT>
 int blocks_for(int wpb, int device) {
     const size_t sm = sizeof(Lean) * (size_t)wpb;
     int per = 0, nsm = 0;
-    if (configure<EXACT>(sm) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lean<EXACT>, 32 * wpb, sm) != cudaSuccess)
+    if (configure<EXACT, COUNT>(sm) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lean<EXACT, COUNT>, 32 * wpb, sm) != cudaSuccess)
         per = 1;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
     cudaGetLastError();   // leave no sticky error behind a failed query
@@ -1036,12 +1054,17 @@ int blocks_for(int wpb, int device) {
 
 }  // namespace cliplean
 
+// TESS_FLAG_COUNTERS runs instances that count their work (the counters cost
+// the others registers); the results are the same.
 cudaError_t launch_clip_lean(const ClipParams& p, int exact, int wpb, int blocks, cudaStream_t s) {
-    return exact ? cliplean::launch<true>(p, wpb, blocks, s) : cliplean::launch<false>(p, wpb, blocks, s);
+    using namespace cliplean;
+    if (p.work_ctr) return exact ? launch<true, true>(p, wpb, blocks, s) : launch<false, true>(p, wpb, blocks, s);
+    return exact ? launch<true, false>(p, wpb, blocks, s) : launch<false, false>(p, wpb, blocks, s);
 }
 
 int clip_blocks_lean(int exact, int wpb, int device) {
-    return exact ? cliplean::blocks_for<true>(wpb, device) : cliplean::blocks_for<false>(wpb, device);
+    using namespace cliplean;
+    return exact ? blocks_for<true, false>(wpb, device) : blocks_for<false, false>(wpb, device);
 }
 
 }  // namespace tess

@@ -322,6 +322,7 @@ struct ClipParams {
     int64_t target_group;         // < 0: none
     float guard_rel;
     float verify_rel;
+    float tol;                    // FP32 first pass: plane tests nearer than this are undecided (FP64 form)
     uint32_t seed_min;            // own-bin count from which a cell is seeded (crowded bins)
     // single-cell geometry output (queries); null for bulk runs
     GeoOut* geo;
