@@ -118,8 +118,6 @@ enum { L_FP64 = 0, L_CAP1 = 1, L_CAP2 = 2, L_CAP64A = 3, L_CAP64B = 4, L_FP64B =
 // the FP64 clipping, so that every decision the FP32 pass takes is the one the
 // reference's test (1e-12, vector3.rs:170-185) takes.
 constexpr float kFp64Tol = 1.01e-12f;
-// Kernels launched by one binning pass (launch_grid_build).
-constexpr uint64_t kGridLaunches = 11;
 
 struct Engine {
     tess_config cfg{};
@@ -566,7 +564,7 @@ tess_status engine_build(Engine& E, bool check) {
         CU(cudaEventRecord(ev.e[0], E.stream));
     }
     CU(launch_grid_build(grid_buffers(E), E.stream, E.side, E.ev_fork, E.ev_join));
-    E.launches += kGridLaunches;
+    E.launches += grid_launches(E.total_bins);
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     if (check) {
         int err = 0;
@@ -1881,7 +1879,7 @@ static tess_status batch_run(tess_batch* b, int prec) {
         CU(cudaEventRecord(ev.e[0], E.stream));
     }
     CU(cudaGraphLaunch(G, E.stream));
-    E.launches += kGridLaunches + (prec != TESS_PRECISION_FP64 ? 8 : 4);
+    E.launches += grid_launches(E.total_bins) + (prec != TESS_PRECISION_FP64 ? 8 : 4);
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     unsigned long long used = 0;
     unsigned counts[16];

@@ -372,7 +372,10 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
         }
         if (m == 0) {
             // a crowded own bin sends the cell to the seeded pass
-            if (P.list_dense && __shfl_sync(FULL, bcnt, 9) >= P.seed_min) status = ST_DENSE;
+            if (P.list_dense && __shfl_sync(FULL, bcnt, 9) >= P.seed_min) {
+                status = ST_DENSE;
+                break;
+            }
             if (lane == 9) bcnt = 0;
         }
         // ---- its points as one stream, 32 per window ----

@@ -118,41 +118,49 @@ __device__ __forceinline__ int axis_index_fast(double x, const DiagDesc& D, int 
 }
 
 // CeleryCellInfo::new (celery.rs:153-181) from the bounds and the host's cpd.
-__global__ void k_grid_params(GridBuffers g) {
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= g.ndiag) return;
+// Four threads per diagram, one per axis and one idle: the FP64 divisions of
+// the axes run side by side.
+__global__ void __launch_bounds__(128) k_grid_params(GridBuffers g) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int d = min(t >> 2, g.ndiag - 1), a = min(t & 3, 2);
+    const bool mine = (t >> 2) < g.ndiag && (t & 3) < 3;
     DiagDesc& D = g.diags[d];
     const double c = (double)D.cpd;
-    double m = DBL_MAX;
-    bool lean_ok = true;
-    for (int a = 0; a < 3; ++a) {
-        const double lo = ord_dec(g.bounds[6 * d + a]);
-        const double hi = ord_dec(g.bounds[6 * d + 3 + a]);
-        D.glo[a] = lo;
-        D.ghi[a] = hi;
-        const double ctr = 0.5 * lo + 0.5 * hi;
-        D.ctr[a] = isfinite(ctr) ? ctr : 0.0;
-        const double ext = __dsub_rn(hi, lo);
-        D.size[a] = __ddiv_rn(ext, c);
-        D.inv[a] = __ddiv_rn(c, ext);
-        if (D.size[a] > 0.0) m = fmin(m, D.size[a]);
-        // FP32 forms for the FP32 clipping pass: offsets from the centre as
-        // FP32 pairs (48 bits), the bin sides and their inverses
-        const double gl = lo - D.ctr[a], bl = D.blo[a] - D.ctr[a], bh = D.bhi[a] - D.ctr[a];
-        D.glo_hi[a] = __double2float_rn(gl);
-        D.glo_lo[a] = __double2float_rn(gl - (double)D.glo_hi[a]);
-        D.blo_hi[a] = __double2float_rn(bl);
-        D.blo_lo[a] = __double2float_rn(bl - (double)D.blo_hi[a]);
-        D.bhi_hi[a] = __double2float_rn(bh);
-        D.bhi_lo[a] = __double2float_rn(bh - (double)D.bhi_hi[a]);
-        D.inv_f[a] = __double2float_rn(D.inv[a]);
-        D.glo_f[a] = __double2float_rn(lo);
-        D.size_f[a] = __double2float_rn(D.size[a]);
-        D.inv_s[a] = ext > 0.0 ? D.inv_f[a] : 0.f;
-        if (ext > 0.0)
-            lean_ok = lean_ok && D.size_f[a] >= FLT_MIN && D.size_f[a] <= FLT_MAX && D.inv_f[a] >= FLT_MIN && D.inv_f[a] <= FLT_MAX;
-    }
-    D.lean_ok = lean_ok;
+    const double lo = ord_dec(g.bounds[6 * d + a]);
+    const double hi = ord_dec(g.bounds[6 * d + 3 + a]);
+    const double half = 0.5 * lo + 0.5 * hi;
+    const double ctr = isfinite(half) ? half : 0.0;
+    const double ext = __dsub_rn(hi, lo);
+    const double size = __ddiv_rn(ext, c), inv = __ddiv_rn(c, ext);
+    const float size_f = __double2float_rn(size), inv_f = __double2float_rn(inv);
+    const bool ok_a = !(ext > 0.0) || (size_f >= FLT_MIN && size_f <= FLT_MAX && inv_f >= FLT_MIN && inv_f <= FLT_MAX);
+    const unsigned quad = (__ballot_sync(0xffffffffu, ok_a) >> (threadIdx.x & 28)) & 7u;
+    // the smallest nonzero bin side, through its order-preserving bits
+    unsigned long long m = size > 0.0 ? (unsigned long long)__double_as_longlong(size) : ~0ull;
+    m = min(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = min(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    if (!mine) return;
+    D.glo[a] = lo;
+    D.ghi[a] = hi;
+    D.ctr[a] = ctr;
+    D.size[a] = size;
+    D.inv[a] = inv;
+    // FP32 forms for the FP32 clipping pass: offsets from the centre as
+    // FP32 pairs (48 bits), the bin sides and their inverses
+    const double gl = lo - ctr, bl = D.blo[a] - ctr, bh = D.bhi[a] - ctr;
+    const float glf = __double2float_rn(gl), blf = __double2float_rn(bl), bhf = __double2float_rn(bh);
+    D.glo_hi[a] = glf;
+    D.glo_lo[a] = __double2float_rn(gl - (double)glf);
+    D.blo_hi[a] = blf;
+    D.blo_lo[a] = __double2float_rn(bl - (double)blf);
+    D.bhi_hi[a] = bhf;
+    D.bhi_lo[a] = __double2float_rn(bh - (double)bhf);
+    D.inv_f[a] = inv_f;
+    D.glo_f[a] = __double2float_rn(lo);
+    D.size_f[a] = size_f;
+    D.inv_s[a] = ext > 0.0 ? inv_f : 0.f;
+    if (a != 0) return;
+    D.lean_ok = quad == 7u;
     // (x - glo) * inv from the FP32 pairs: one rounding of the difference, one
     // of inv, one of the product (u = 2^-24 each, relative to the result, at
     // most cpd bins), with a factor 4 in hand
@@ -166,16 +174,17 @@ __global__ void k_grid_params(GridBuffers g) {
     // The table holds every offset of the grid when that fits; otherwise the
     // offsets with key <= kmax, and the walk continues ring by ring.
     const bool complete = cheb == D.cpd - 1 && (2 * cheb + 1) * (2 * cheb + 1) * (2 * cheb + 1) <= kMaxTable;
-    D.has_extent = m != DBL_MAX;
-    if (m == DBL_MAX) {          // every point identical: only the own bin holds points
+    D.has_extent = m != ~0ull;
+    if (m == ~0ull) {            // every point identical: only the own bin holds points
         D.min_size = 0.0;
         D.tab_kmax = INFINITY;
         D.cheb = 0;
     } else {
-        D.min_size = m;
+        const double ms = __longlong_as_double((long long)m);
+        D.min_size = ms;
         const int gaps = cheb - 1;
         D.tab_kmax = complete ? (double)INFINITY
-                              : __dmul_rn(__dmul_rn((double)gaps, m), __dmul_rn((double)gaps, m));
+                              : __dmul_rn(__dmul_rn((double)gaps, ms), __dmul_rn((double)gaps, ms));
     }
 }
 
@@ -272,6 +281,31 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_final(uint32_t* data, uin
     for (int k = 0; k < kScanItems; ++k) {
         if (base + k < n) data[base + k] = run;
         run += v[k];
+    }
+}
+
+// The whole scan by one block, for grids of few bins: one launch in place of
+// three (a 1,000-point grid's scan 10 -> 4 us with its launches).
+constexpr uint64_t kScanOneMax = 16384;
+__global__ void __launch_bounds__(kScanThreads) k_scan_one(uint32_t* data, uint32_t n) {
+    __shared__ uint32_t sh[33];
+    uint32_t carry = 0;
+    for (uint32_t base0 = 0; base0 < n; base0 += kScanThreads * kScanItems) {
+        const uint32_t base = base0 + threadIdx.x * kScanItems;
+        uint32_t v[kScanItems];
+        uint32_t s = 0;
+        for (int k = 0; k < kScanItems; ++k) {
+            v[k] = base + k < n ? data[base + k] : 0u;
+            s += v[k];
+        }
+        uint32_t ex;
+        const uint32_t tot = block_excl_scan(s, &ex, sh);
+        uint32_t run = carry + ex;
+        for (int k = 0; k < kScanItems; ++k) {
+            if (base + k < n) data[base + k] = run;
+            run += v[k];
+        }
+        carry += tot;
     }
 }
 
@@ -440,11 +474,6 @@ __global__ void k_gather(GridBuffers g) {
     if (g.sgroup) g.sgroup[s] = g.groups[i];
 }
 
-// ---- shell table (get_search_order, celery.rs:418-679) ----
-// One block per diagram: every offset within Chebyshev radius `cheb` whose key
-// is <= tab_kmax, sorted by (key, i, j, k) with a bitonic sort in shared memory.
-constexpr int kTabThreads = 1024;
-
 // The inverse permutation, point -> sorted position, for the queries that
 // start from a point's original index (radius queries by cell, single-cell
 // computes).  Built on first use after a binning pass rather than in it: its
@@ -454,75 +483,126 @@ __global__ void k_inverse(const uint32_t* sorted, uint32_t* inv, uint32_t n, int
         inv[tess_chk(sorted[s], n, check, CK_GRID)] = s;
 }
 
+// ---- shell table (get_search_order, celery.rs:418-679) ----
+// One block per diagram: every offset within Chebyshev radius `cheb` whose key
+// is <= tab_kmax, sorted by (key, i, j, k).  An offset's key depends on its gap
+// counts alone (0 for -1, 0 and 1, else |o| - 1), so only the at most 9^3 gap
+// triples are sorted, one per thread (the short steps of the network by
+// shuffles).  Each triple's offsets then take their place by the prefix sum of
+// the triples' sizes, and the offsets of equal keys order themselves by
+// counting.  Sorting all offsets in shared memory, with an FP64 key each, took
+// 97 us a block; this takes 13.
+constexpr int kTabThreads = 1024;
+constexpr int kTabGaps = 9;          // gap counts per axis: 0 .. table_gaps (at most 8)
 __global__ void __launch_bounds__(kTabThreads) k_table(GridBuffers g) {
-    __shared__ unsigned long long skey[kMaxTable];
-    __shared__ uint16_t sidx[kMaxTable];
-    __shared__ unsigned int count;
-    const int d = blockIdx.x;
+    __shared__ double sq[3][kTabGaps];
+    __shared__ unsigned long long skey[kTabThreads];
+    __shared__ uint16_t sid[kTabThreads];
+    __shared__ uint32_t wsum[kTabThreads / 32 + 1];
+    __shared__ uint32_t start[kTabThreads];      // first entry of the r-th triple
+    __shared__ uint16_t code[kMaxTable];         // an entry's offset, lexicographic
+    __shared__ uint16_t rank[kMaxTable];         // ... and the place of its triple
+    const int d = blockIdx.x, t = threadIdx.x, lane = t & 31;
     DiagDesc& D = g.diags[d];
-    const int c = D.cheb;
-    const int side = 2 * c + 1;
-    const int total = side * side * side;
-    if (threadIdx.x == 0) count = 0;
-    __syncthreads();
-    for (int t = threadIdx.x; t < total; t += blockDim.x) {
-        const int i = t / (side * side) - c;
-        const int j = (t / side) % side - c;
-        const int k = t % side - c;
-        const double key = gap_key(D.size, i, j, k);
-        if (key <= D.tab_kmax) {
-            unsigned int slot = atomicAdd(&count, 1u);
-            if (slot < (unsigned)kMaxTable) {
-                // keys >= 0 order as their bit patterns; self (-1) sorts first
-                skey[slot] = key < 0.0 ? 0ull : (unsigned long long)__double_as_longlong(key) + 1ull;
-                sidx[slot] = (uint16_t)t;   // t orders (i, j, k) lexicographically
-            }
-        }
+    const int c = D.cheb, side = 2 * c + 1;
+    const int ng = c > 0 ? c : 1;                // gap counts 0 .. ng - 1
+    if (t < 3 * ng) {
+        const double v = __dmul_rn((double)(t % ng), D.size[t / ng]);
+        sq[t / ng][t % ng] = __dmul_rn(v, v);
     }
     __syncthreads();
-    const unsigned cap = min((unsigned)kMaxTable, D.tab_cap);
-    if (count > cap && threadIdx.x == 0) atomicExch(g.error_flag, 2);
-    const int m = (int)min(count, cap);
-    int p2 = 1;
-    while (p2 < m) p2 <<= 1;
-    for (int t = m + threadIdx.x; t < p2; t += blockDim.x) {
-        skey[t] = ~0ull;
-        sidx[t] = 0xFFFF;
+    // the triple's key as ordered bits (gap_key's operations); ~0: not kept
+    unsigned long long key = ~0ull;
+    int id = t;
+    if (t < ng * ng * ng) {
+        const double k = __dadd_rn(__dadd_rn(sq[0][t / (ng * ng)], sq[1][(t / ng) % ng]), sq[2][t % ng]);
+        if (k <= D.tab_kmax) key = (unsigned long long)__double_as_longlong(k);
     }
-    __syncthreads();
-    for (int k2 = 2; k2 <= p2; k2 <<= 1) {
+    // bitonic sort of (key, id), ascending, one pair per thread
+    for (int k2 = 2; k2 <= kTabThreads; k2 <<= 1) {
         for (int j2 = k2 >> 1; j2 > 0; j2 >>= 1) {
-            for (int t = threadIdx.x; t < p2; t += blockDim.x) {
-                const int u = t ^ j2;
-                if (u > t) {
-                    const bool up = (t & k2) == 0;
-                    const unsigned long long ka = skey[t], kb = skey[u];
-                    const uint16_t ia = sidx[t], ib = sidx[u];
-                    const bool gt = (ka > kb) || (ka == kb && ia > ib);
-                    if (gt == up) {
-                        skey[t] = kb; skey[u] = ka;
-                        sidx[t] = ib; sidx[u] = ia;
-                    }
-                }
+            unsigned long long ok;
+            int oi;
+            if (j2 >= 32) {
+                skey[t] = key;
+                sid[t] = (uint16_t)id;
+                __syncthreads();
+                ok = skey[t ^ j2];
+                oi = sid[t ^ j2];
+                __syncthreads();
+            } else {
+                ok = __shfl_xor_sync(0xffffffffu, key, j2);
+                oi = __shfl_xor_sync(0xffffffffu, id, j2);
             }
-            __syncthreads();
+            const bool less = ok < key || (ok == key && oi < id);      // the partner's pair is smaller
+            const bool low = (t & j2) == 0, up = (t & k2) == 0;
+            if (less == (low == up)) {
+                key = ok;
+                id = oi;
+            }
         }
     }
-    for (int t = threadIdx.x; t < m; t += blockDim.x) {
-        const int e = sidx[t];
-        const int i = e / (side * side) - c;
-        const int j = (e / side) % side - c;
-        const int k = e % side - c;
-        const double key = gap_key(D.size, i, j, k);
-        TabEntry te;
-        te.key = key < 0.0 ? -1.0f : __double2float_rz(key);
-        te.i = (int8_t)i;
-        te.j = (int8_t)j;
-        te.k = (int8_t)k;
-        te.pad = 0;
-        g.table[D.tab_base + t] = te;
+    // the triple's offsets: {-1, 0, 1} for a gap of 0 (0 alone when the grid has
+    // one bin), {-g - 1, g + 1} otherwise
+    auto width = [&](int gap) { return gap ? 2u : (c > 0 ? 3u : 1u); };
+    auto pick = [&](int gap, uint32_t q) { return gap ? (q ? gap + 1 : -gap - 1) : (c > 0 ? (int)q - 1 : 0); };
+    const bool kept = key != ~0ull;
+    const int gi = id / (ng * ng), gj = (id / ng) % ng, gk = id % ng;
+    const uint32_t w0 = width(gi), w1 = width(gj), w2 = width(gk);
+    const uint32_t cnt = kept ? w0 * w1 * w2 : 0u;
+    uint32_t inc = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
     }
-    if (threadIdx.x == 0) D.tab_len = (uint32_t)m;
+    if (lane == 31) wsum[t >> 5] = inc;
+    skey[t] = key;
+    __syncthreads();
+    if (t < 32) {
+        const uint32_t v = wsum[t];
+        uint32_t i2 = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, i2, o);
+            if (lane >= o) i2 += u;
+        }
+        wsum[t] = i2 - v;
+        if (t == 31) wsum[32] = i2;
+    }
+    __syncthreads();
+    const uint32_t beg = wsum[t >> 5] + inc - cnt;
+    start[t] = beg;
+    const uint32_t total = wsum[32], cap = min((uint32_t)kMaxTable, D.tab_cap);
+    if (total > cap && t == 0) atomicExch(g.error_flag, 2);
+    const uint32_t m = min(total, cap);
+    for (uint32_t q = 0; q < cnt; ++q) {
+        if (beg + q >= m) break;
+        const int i = pick(gi, q / (w1 * w2)), j = pick(gj, (q / w2) % w1), k = pick(gk, q % w2);
+        code[beg + q] = (uint16_t)(((i + c) * side + (j + c)) * side + (k + c));
+        rank[beg + q] = (uint16_t)t;
+    }
+    __syncthreads();
+    const uint32_t self = (uint32_t)((c * side + c) * side + c);
+    for (uint32_t e = t; e < m; e += blockDim.x) {
+        // the entries of the same key: those of the triples around this one
+        int r0 = rank[e], r1 = r0;
+        const unsigned long long mine = skey[r0];
+        while (r0 > 0 && skey[r0 - 1] == mine) --r0;
+        while (r1 + 1 < kTabThreads && skey[r1 + 1] == mine) ++r1;
+        const uint32_t b = start[r0], n = r1 + 1 < kTabThreads ? min(start[r1 + 1], m) : m;
+        const uint32_t cd = code[e];
+        // (the own bin comes first: its key is -1)
+        uint32_t at = b;
+        if (cd != self)
+            for (uint32_t o = b; o < n; ++o) at += (code[o] < cd || code[o] == self) ? 1u : 0u;
+        TabEntry te;
+        te.key = cd == self ? -1.0f : __double2float_rz(__longlong_as_double((long long)mine));
+        te.i = (int8_t)((int)(cd / (side * side)) - c);
+        te.j = (int8_t)((int)((cd / side) % side) - c);
+        te.k = (int8_t)((int)(cd % side) - c);
+        te.pad = 0;
+        g.table[D.tab_base + at] = te;
+    }
+    if (t == 0) D.tab_len = m;
 }
 
 }  // namespace
@@ -552,9 +632,12 @@ __global__ void k_occupancy(const uint32_t* delims, uint64_t nbins, uint32_t cro
     }
 }
 
-__global__ void k_bounds_init(unsigned long long* b, int ndiag) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < 6 * ndiag) b[t] = (t % 6) < 3 ? ~0ull : 0ull;
+// Start values of a binning pass: bounds, histogram, error flag.
+__global__ void __launch_bounds__(256) k_grid_clear(GridBuffers g) {
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    if (t == 0) *g.error_flag = 0;
+    for (uint64_t i = t; i < 6ull * g.ndiag; i += stride) g.bounds[i] = (i % 6) < 3 ? ~0ull : 0ull;
+    for (uint64_t i = t; i <= g.total_bins; i += stride) g.delims[i] = 0u;
 }
 }  // namespace
 
@@ -594,18 +677,19 @@ cudaError_t launch_occupancy(const uint32_t* delims, uint64_t nbins, uint32_t cr
     return cudaGetLastError();
 }
 
+uint64_t grid_launches(uint64_t total_bins) { return total_bins + 1 <= kScanOneMax ? 9 : 11; }
+
 // Binning pass: bounds -> grid parameters -> shell tables -> histogram ->
 // scan -> scatter -> within-bin order -> gather.  A fixed launch sequence
 // (no host synchronisation), so it can be captured in a CUDA graph.
 cudaError_t launch_grid_build(const GridBuffers& g, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
                               cudaEvent_t join) {
     const int ndiag = g.ndiag;
-    k_bounds_init<<<(6 * ndiag + 255) / 256, 256, 0, s>>>(g.bounds, ndiag);
-    cudaMemsetAsync(g.delims, 0, sizeof(uint32_t) * (g.total_bins + 1), s);
-    cudaMemsetAsync(g.error_flag, 0, sizeof(int), s);
+    const uint64_t nclear = std::max<uint64_t>(6ull * ndiag, g.total_bins + 1);
+    k_grid_clear<<<(unsigned)std::min<uint64_t>((nclear + 1023) / 1024, 152u * 8u), 256, 0, s>>>(g);
     const int cblocks = (int)(g.nchunks < 4096u ? g.nchunks : 4096u);
     k_bounds<<<cblocks, kBoundsThreads, 0, s>>>(g);
-    k_grid_params<<<(ndiag + 127) / 128, 128, 0, s>>>(g);
+    k_grid_params<<<(4 * ndiag + 127) / 128, 128, 0, s>>>(g);
     // the shell tables need only the grid parameters: build them beside the
     // histogram, scan and scatter when a side stream is given
     const bool forked = side && fork && join;
@@ -621,9 +705,13 @@ cudaError_t launch_grid_build(const GridBuffers& g, cudaStream_t s, cudaStream_t
     const uint64_t nscan = g.total_bins + 1;
     const uint64_t per = (uint64_t)kScanThreads * kScanItems;
     const uint32_t nblk = (uint32_t)((nscan + per - 1) / per);
-    k_scan_partial<<<nblk, kScanThreads, 0, s>>>(g.delims, nscan, g.scan_tmp);
-    k_scan_sums<<<1, kScanThreads, 0, s>>>(g.scan_tmp, nblk);
-    k_scan_final<<<nblk, kScanThreads, 0, s>>>(g.delims, nscan, g.scan_tmp);
+    if (nscan <= kScanOneMax) {
+        k_scan_one<<<1, kScanThreads, 0, s>>>(g.delims, (uint32_t)nscan);
+    } else {
+        k_scan_partial<<<nblk, kScanThreads, 0, s>>>(g.delims, nscan, g.scan_tmp);
+        k_scan_sums<<<1, kScanThreads, 0, s>>>(g.scan_tmp, nblk);
+        k_scan_final<<<nblk, kScanThreads, 0, s>>>(g.delims, nscan, g.scan_tmp);
+    }
     k_scatter<<<(g.total + 255) / 256, 256, 0, s>>>(g);
     k_bin_order<<<(unsigned)((g.total_bins + 255) / 256), 256, 0, s>>>(g);
     k_gather<<<(g.total + 255) / 256, 256, 0, s>>>(g);
