@@ -48,26 +48,26 @@ typedef enum {
 } tess_status;
 
 typedef enum {
-    /* Plain FP64 clipping: the reference's arithmetic type (float.rs:78). */
+    /* FP64, the reference's arithmetic type (float.rs:78): faces, vertices,
+     * areas and volumes are computed in FP64.  Which planes cut the cell is
+     * decided in FP32 where the test is beyond its error bound and the
+     * reference's 1e-12 tolerance, else in FP64: the same decisions. */
     TESS_PRECISION_FP64 = 0,
-    /* FP32 clipping; a cell whose plane-side test lands inside the guard
-     * band, or whose FP32 vertices fail the FP64 check, is re-run in FP64.
+    /* FP32 clipping; a plane-side test inside the guard band is settled in
+     * FP64, and a cell whose FP32 vertices fail the check is re-run in FP64.
      * Volumes and areas are accumulated in FP64. */
     TESS_PRECISION_FP32_GUARD = 1,
     /* The FP32 + guard clipping (its exact topology and re-runs) with an
-     * FP64-accurate finish: every vertex is refined by two Newton steps on its
-     * three FP64 face planes, and face areas and volumes are accumulated in
-     * FP64 from those vertices.  Volumes are within 1e-11 relative of the
-     * FP64 form (the worst of 1,000,000 uniform cells: 1.8e-12; typically
-     * 1e-14), at close to the FP32 form's speed.
-     * Single-cell geometry queries run it as TESS_PRECISION_FP64. */
+     * FP64 finish: every vertex is solved in FP64 from its three face planes,
+     * and face areas and volumes are computed in FP64 from those vertices.
+     * (As TESS_PRECISION_FP64, without the reference's tolerance in the plane
+     * tests.)  Single-cell geometry queries run in FP64 in every precision. */
     TESS_PRECISION_MIXED = 2
 } tess_precision;
 
 /* Flags for tess_config.flags */
 #define TESS_FLAG_TIMING 1u     /* record per-pass device times (tess_stats)          */
-#define TESS_FLAG_COUNTERS 2u   /* count the clipping work (tess_stats); the FP32 first pass then runs
-                                   in its counting form, with the window pre-test (about 2% slower) */
+#define TESS_FLAG_COUNTERS 2u   /* count the clipping work (tess_stats; about 2% slower) */
 /* Flags that exercise the recovery paths (tests and diagnostics; results are
  * unchanged except as stated): */
 #define TESS_FLAG_SMALL_FACE_POOL 4u  /* start the face pool at 1,024 faces, so a compute
@@ -96,8 +96,9 @@ typedef struct {
     int32_t table_gaps;
     /* Warps per block of the clipping kernel (1..32). */
     int32_t warps_per_block;
-    /* Vertex slots per lane of the first clipping pass (2, 4 or 8):
-     * capacity = 32 x slots.  Overflowing cells re-run at the next size. */
+    /* Vertex slots per lane (2, 4 or 8).  The FP32 passes hold 64 vertices;
+     * cells beyond that are clipped in FP64 at 128 and then 255, with 8 at
+     * 255 at once. */
     int32_t slots_per_lane;
     /* CUDA device ordinal. */
     int32_t device;
@@ -114,7 +115,7 @@ typedef struct {
 typedef struct {
     uint64_t cells;             /* cells computed                                  */
     uint64_t faces;             /* faces over all cells                            */
-    uint64_t rerun_fp64;        /* FP32 cells re-run in FP64 (guard band / check)  */
+    uint64_t rerun_fp64;        /* cells with a test settled in FP64, or a failed check */
     uint64_t rerun_capacity;    /* cells re-run at a larger vertex capacity        */
     uint64_t failed;            /* cells with an error status                      */
     uint64_t table_entries;     /* shell-table entries (all diagrams)              */
@@ -136,8 +137,8 @@ typedef struct {
      * pass (with the scan of the counts) and of its fill pass. */
     double ms_query_count;
     double ms_query_fill;
-    /* FP32 form: of the rerun_fp64 cells, those the hybrid re-run (guard-band
-     * tests decided in FP64) could not settle, re-run entirely in FP64 */
+    /* of the rerun_fp64 cells, those that settling single tests in FP64 did
+     * not finish, clipped in FP64 as a whole */
     uint64_t rerun_fp64_full;
     /* FP32 form: cells whose own bin is crowded (>= crowded_bin points), taken out of
      * the first pass and computed by a pass that first cuts by the nearest

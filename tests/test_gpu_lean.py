@@ -1,13 +1,20 @@
-"""The FP32 first pass on the point sets where its walk over rows of bins can go wrong: axes without extent, oblong
+"""The FP32 passes on the point sets where their walk over rows of bins can go wrong: axes without extent, oblong
 grids, sparse regions that need rings of rows far out (more rows than lanes in a ring), sizes around a window of 32
-candidates, extents outside FP32's range, and a search radius, all against the FP64 oracle with the bars of the parity
-tests (neighbour lists bit-exact; volumes 1e-6 relative in FP32, 1e-12 in MIXED)."""
+candidates and around the size from which the plain, dense and careful passes share the work, extents outside FP32's
+range, and a search radius, all against the FP64 oracle with the bars of the parity tests (neighbour lists bit-exact;
+volumes 1e-6 relative in FP32, 1e-12 in MIXED and FP64)."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-VOL_TOL = {"mixed": 1e-12, "fp32": 1e-6}
+VOL_TOL = {"mixed": 1e-12, "fp64": 1e-12, "fp32": 1e-6}
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _rng(seed):
@@ -26,8 +33,16 @@ def _flat(pts, axis, value):
     return pts
 
 
+def _clustered(n):
+    from tessellator import workloads
+
+    return workloads.clustered(n, seed=3)
+
+
 SETS = {
     **{f"uniform_{n}": (lambda n=n: _rng(n).random((n, 3)), (1, 1, 1)) for n in (1, 2, 3, 31, 32, 33, 34, 64, 65, 200)},
+    **{f"uniform_{n}": (lambda n=n: _rng(n).random((n, 3)), (1, 1, 1)) for n in (32768, 32769)},
+    "clustered_40000": (lambda: _clustered(40_000), (1, 1, 1)),
     "plane_x": (lambda: _flat(_rng(1).random((300, 3)), 0, 0.25), (1, 1, 1)),
     "plane_y": (lambda: _flat(_rng(2).random((300, 3)), 1, 0.5), (1, 1, 1)),
     "plane_z": (lambda: _flat(_rng(3).random((300, 3)), 2, 0.75), (1, 1, 1)),
@@ -52,7 +67,7 @@ def _check(T, O, pts, hi, prec, ref_kw, **kw):
     assert np.max(np.abs(vol - rv) / np.maximum(rv, 1e-300)) <= VOL_TOL[prec]
 
 
-@pytest.mark.parametrize("prec", ["fp32", "mixed"])
+@pytest.mark.parametrize("prec", ["fp32", "mixed", "fp64"])
 @pytest.mark.parametrize("name", list(SETS))
 def test_point_sets(tess, oracle_mod, name, prec):
     make, hi = SETS[name]
@@ -71,3 +86,11 @@ def test_search_radius(tess, oracle_mod, name, radius, prec):
 def test_extent_below_fp32(tess, oracle_mod):
     """Bin sides below FP32's normal range: the pass hands every cell on."""
     _check(tess, oracle_mod, _rng(11).random((100, 3)) * 1e-42, (1e-42, 1e-42, 1e-42), "fp32", {})
+
+
+def test_checked_build():
+    """The plain, dense and careful passes through the bounds-checked library."""
+    env = dict(os.environ, TESS_LIB=os.path.join(ROOT, "the-tessellator_gb300", "tessellator", "libtessgpu_checked.so"))
+    r = subprocess.run([sys.executable, "-m", "pytest", os.path.abspath(__file__), "-q", "-x", "-m", "gpu", "-k",
+                        "uniform_32769 or clustered_40000 or clumps_many"], env=env, cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0 and "passed" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]

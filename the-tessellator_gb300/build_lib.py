@@ -22,7 +22,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "tessellator", "libtessgpu.so")
 OUT_CHECKED = os.path.join(HERE, "tessellator", "libtessgpu_checked.so")
 BUILD = os.path.join(ROOT, "_build", "tessgpu")
-SOURCES = ["tess_grid.cu", "tess_clip.cu", "tess_clip_f32.cu", "tess_clip_f32x.cu", "tess_clip_lean.cu", "tess_clip_f64.cu", "tess_api.cu",
+SOURCES = ["tess_grid.cu", "tess_clip.cu", "tess_clip_lean.cu", "tess_clip_f64.cu", "tess_api.cu",
            "tess_noalloc.cu", "tess_radius.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

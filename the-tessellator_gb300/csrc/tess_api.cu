@@ -108,11 +108,17 @@ int64_t cells_per_dim(uint64_t n, double density) {
     return (int64_t)v + 1;
 }
 
-// Work lists of the re-run passes: FP64 (cells the FP32 passes flagged),
-// CAP1/CAP2 (FP32 capacity), CAP64A/B (FP64 capacity), FP64B (cells the
-// hybrid FP32 pass could not settle).
-enum { L_FP64 = 0, L_CAP1 = 1, L_CAP2 = 2, L_CAP64A = 3, L_CAP64B = 4, L_FP64B = 5, L_DENSE = 6, L_COUNT = 7,
-       L_FAIL = 7, L_REASON = 8 };
+// Work lists: DENSE (cells of crowded bins), CARE (cells with undecided plane
+// tests), FULL (cells for the FP64 clipping), CAP64 (those beyond its first
+// capacity).
+enum { L_DENSE = 0, L_CARE = 1, L_FULL = 2, L_CAP64 = 3, L_COUNT = 4 };
+// d_counters: pass cursors, then list lengths and counts, then the cells each
+// status code was given to, in the FP32 and in the FP64 passes.
+enum { C_CURSOR = 0, C_LIST = 16, C_FAIL = 20, C_FLAG = 21, C_DENSE = 22, C_REASON32 = 32, C_REASON64 = 40, C_TOTAL = 48 };
+// Up to this many cells the careful pass runs over all of them: an input this
+// small is one wave of warps, whose time is a cell's latency, and a second
+// pass over a few cells would add its own.
+constexpr uint32_t kCarefulMax = 32768;
 // The FP64 form's first pass runs in FP32 (tess_clip_lean.cu): a vertex whose
 // distance from a plane is within the FP32 error bound plus this is left to
 // the FP64 clipping, so that every decision the FP32 pass takes is the one the
@@ -172,7 +178,7 @@ struct Engine {
     uint64_t pool_need = 0;
     unsigned long long* d_fcursor = nullptr;
     uint32_t* d_list[L_COUNT] = {};
-    unsigned* d_counters = nullptr;   // [0..15] cursors, [16..31] list counts
+    unsigned* d_counters = nullptr;   // C_* above
     unsigned long long* d_work = nullptr;  // work counters (TESS_FLAG_COUNTERS)
     uint64_t* d_offs = nullptr;
     int32_t* d_cnbr = nullptr;
@@ -242,7 +248,7 @@ struct Engine {
     const void* graph_host_nbr = nullptr;
     const void* graph_host_area = nullptr;
     uint64_t graph_host_cap = 0;
-    int blocks_cache[2][4][8] = {};   // [kernel type][slots][form, with the exact flag]
+    int blocks_cache[3][8] = {};   // [FP64 4 slots, FP64 8 slots, FP32][form, with the exact flag]
     // allocated capacities of the grid arrays a re-grid may grow
     uint64_t delims_alloc = 0, table_alloc = 0;
     // autotuning: the timing sample, the occupancy counters, and whether the
@@ -283,18 +289,14 @@ struct Engine {
         ev_fork = ev_join = nullptr;
     }
 
-    int blocks(int precision, int slots, int form = kFormStd) {
-        const int si = slots <= 2 ? 0 : (slots <= 4 ? 1 : 2);
-        int& b = blocks_cache[precision][si][form];
-        if (!b) {
-            const int wpb = wpb_for(slots, form);
-            b = clip_blocks_for(precision, slots, form, wpb, device);
-        }
+    int blocks(int slots, int form) {
+        int& b = blocks_cache[form == kFormStd ? (slots <= 4 ? 0 : 1) : 2][form];
+        if (!b) b = clip_blocks_for(slots, form, wpb_for(slots, form), device);
         return b;
     }
     int wpb_for(int slots, int form) const {
         int w = cfg.warps_per_block;
-        if ((form & 3) == kFormLean) w = std::min(w, 4);   // its launch bound
+        if ((form & 3) != kFormStd) w = std::min(w, 4);   // their launch bound
         if (slots >= 8) w = std::min(w, 2);
         else if (slots >= 4) w = std::min(w, 4);
         return std::max(1, w);
@@ -446,7 +448,7 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     TRY(dalloc(&E.d_farea, E.face_cap));
     TRY(dalloc(&E.d_fcursor, 1));
     for (auto& l : E.d_list) TRY(dalloc(&l, n));
-    TRY(dalloc(&E.d_counters, 32));
+    TRY(dalloc(&E.d_counters, C_TOTAL));
     TRY(dalloc(&E.d_work, 8));
     TRY(dalloc(&E.d_offs, n + 1));
     TRY(dalloc(&E.d_csr_tmp, csr_tmp_words(E.total)));
@@ -634,8 +636,8 @@ ClipParams base_params(Engine& E) {
 tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t group, bool timing,
                            cudaEvent_t* ev, const uint32_t* sample = nullptr, uint32_t nsample = 0) {
     unsigned* cur = E.d_counters;
-    unsigned* cnt = E.d_counters + 16;
-    CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * 32, E.stream));
+    unsigned* cnt = E.d_counters + C_LIST;
+    CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * C_TOTAL, E.stream));
     CU(cudaMemsetAsync(E.d_fcursor, 0, sizeof(unsigned long long), E.stream));
     if (E.cfg.flags & TESS_FLAG_COUNTERS) CU(cudaMemsetAsync(E.d_work, 0, sizeof(unsigned long long) * 8, E.stream));
     ClipParams base = base_params(E);
@@ -644,8 +646,14 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
     base.target_group = group;
     const int s0 = E.cfg.slots_per_lane;
     int cursor = 0;
-    // One launch over a work list (null: every cell).  Failed cells append to
-    // the FP64 list (guard, degenerate, verify) and the capacity list.
+    const bool fp64 = precision == TESS_PRECISION_FP64;
+    // the FP64 and MIXED forms finish in FP64
+    const int X = precision == TESS_PRECISION_FP32_GUARD ? 0 : kFormExact;
+    base.tol = fp64 ? kFp64Tol : 0.f;
+    base.fail_count = cur + C_FAIL;
+    base.flag_count = cur + C_FLAG;
+    base.work_ctr = (E.cfg.flags & TESS_FLAG_COUNTERS) ? E.d_work : nullptr;
+    // One launch over a work list (null: every cell).
     auto pass = [&](int prec, int slots, int form, const uint32_t* work, const unsigned* wcount, uint32_t* l64,
                     unsigned* c64, uint32_t* lcap, unsigned* ccap, uint32_t* ldense = nullptr,
                     unsigned* cdense = nullptr) -> tess_status {
@@ -655,15 +663,13 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
         p.work = work;
         p.work_count = wcount;
         if (work && !wcount) p.total = nsample;   // the first pass over a timing sample
-        p.cursor = cur + cursor++;
+        p.cursor = cur + C_CURSOR + cursor++;
         p.list_fp64 = l64;
         p.list_fp64_count = c64;
         p.list_cap = lcap;
         p.list_cap_count = ccap;
-        p.fail_count = cnt + L_FAIL;
-        p.reasons = cnt + L_REASON;
-        p.work_ctr = (E.cfg.flags & TESS_FLAG_COUNTERS) ? E.d_work : nullptr;
-        CU(launch_clip(p, prec, slots, form, E.wpb_for(slots, form), E.blocks(prec, slots, form), E.stream));
+        p.reasons = cur + (prec == 1 ? C_REASON32 : C_REASON64);
+        CU(launch_clip(p, slots, form, E.wpb_for(slots, form), E.blocks(slots, form), E.stream));
         E.launches += 1;
         return TESS_OK;
     };
@@ -672,60 +678,46 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
     // without capacity re-runs, the capacity lists are left out: an overflowing
     // cell is then reported as failed
     const bool norerun = E.cfg.flags & TESS_FLAG_NO_CAPACITY_RERUN;
-    if (precision == TESS_PRECISION_FP32_GUARD || precision == TESS_PRECISION_MIXED) {
-        // with the exact flag (MIXED) every FP32 pass finishes in FP64
-        const int X = precision == TESS_PRECISION_MIXED ? kFormExact : 0;
-        // FP32: the lean first pass (2 slots per lane) over every cell but
-        // those of crowded bins, which run seeded in the standard form;
-        // capacity re-runs at 4 and 8 slots; the flagged cells re-run in the
-        // hybrid form (guard-band tests decided in FP64); what that cannot
-        // settle runs in the FP64 form.
-        const bool two = s0 < 4, one = s0 < 8 && !norerun;
-        const bool lean = s0 <= 2;
-        TRY(pass(1, s0, (lean ? kFormLean : kFormStd) | X, sample, nullptr, L[L_FP64], cnt + L_FP64,
-                 one ? L[L_CAP1] : nullptr, cnt + L_CAP1, lean ? L[L_DENSE] : nullptr, cnt + L_DENSE));
-        if (lean)
-            TRY(pass(1, 2, kFormStd | X, L[L_DENSE], cnt + L_DENSE, L[L_FP64], cnt + L_FP64,
-                     norerun ? nullptr : L[L_CAP1], cnt + L_CAP1));
-        if (timing) CU(cudaEventRecord(ev[1], E.stream));
-        if (one) {
-            const int s1 = two ? 4 : 8;
-            TRY(pass(1, s1, kFormStd | X, L[L_CAP1], cnt + L_CAP1, L[L_FP64], cnt + L_FP64, two ? L[L_CAP2] : nullptr,
-                     cnt + L_CAP2));
-            if (two)
-                TRY(pass(1, 8, kFormStd | X, L[L_CAP2], cnt + L_CAP2, L[L_FP64], cnt + L_FP64, nullptr, nullptr));
-        }
-        TRY(pass(1, 2, kFormHybrid | X, L[L_FP64], cnt + L_FP64, L[L_FP64B], cnt + L_FP64B,
-                 norerun ? nullptr : L[L_FP64B], cnt + L_FP64B));
-        TRY(pass(0, 2, kFormStd, L[L_FP64B], cnt + L_FP64B, nullptr, nullptr, norerun ? nullptr : L[L_CAP64A],
-                 cnt + L_CAP64A));
-        TRY(pass(0, 4, kFormStd, L[L_CAP64A], cnt + L_CAP64A, nullptr, nullptr, L[L_CAP64B], cnt + L_CAP64B));
-        TRY(pass(0, 8, kFormStd, L[L_CAP64B], cnt + L_CAP64B, nullptr, nullptr, nullptr, nullptr));
+    uint32_t* const lcap = norerun ? nullptr : L[L_FULL];
+    // The FP32 first pass hands cells of crowded bins to the dense pass and both
+    // hand cells with an undecided plane test to the careful pass, which settles
+    // those tests in FP64; what that cannot settle, and cells beyond 64 vertices
+    // or 96 planes, are clipped in FP64 at 128 and 255 vertices.
+    const bool small = (sample ? nsample : E.total) <= kCarefulMax;
+    if (small) {
+        TRY(pass(1, 2, kFormCareful | X, sample, nullptr, L[L_FULL], cnt + L_FULL, lcap, cnt + L_FULL, nullptr, cur + C_DENSE));
     } else {
-        const bool two = s0 < 4, one = s0 < 8 && !norerun;
-        // FP64: the FP32 first pass with the FP64 finish settles the cells whose
-        // every plane test is decided in FP32 beyond its error bound and the
-        // reference's tolerance (see kFp64Tol); all others, crowded bins
-        // included, are clipped in FP64.
-        if (s0 <= 2) {
-            base.tol = kFp64Tol;
-            uint32_t* const rest = L[L_FP64B];
-            unsigned* const nrest = cnt + L_FP64B;
-            TRY(pass(1, 2, kFormLean | kFormExact, sample, nullptr, rest, nrest, rest, nrest, rest, nrest));
-            TRY(pass(0, 2, kFormStd, rest, nrest, nullptr, nullptr, one ? L[L_CAP64A] : nullptr, cnt + L_CAP64A));
-        } else {
-            TRY(pass(0, s0, kFormStd, sample, nullptr, nullptr, nullptr, one ? L[L_CAP64A] : nullptr, cnt + L_CAP64A));
-        }
-        if (timing) CU(cudaEventRecord(ev[1], E.stream));
-        if (one) {
-            const int s1 = two ? 4 : 8;
-            TRY(pass(0, s1, kFormStd, L[L_CAP64A], cnt + L_CAP64A, nullptr, nullptr, two ? L[L_CAP64B] : nullptr,
-                     cnt + L_CAP64B));
-            if (two) TRY(pass(0, 8, kFormStd, L[L_CAP64B], cnt + L_CAP64B, nullptr, nullptr, nullptr, nullptr));
-        }
+        TRY(pass(1, 2, kFormLean | X, sample, nullptr, L[L_CARE], cnt + L_CARE, lcap, cnt + L_FULL, L[L_DENSE], cnt + L_DENSE));
+    }
+    if (timing) CU(cudaEventRecord(ev[1], E.stream));
+    if (!small) {
+        TRY(pass(1, 2, kFormDense | X, L[L_DENSE], cnt + L_DENSE, L[L_CARE], cnt + L_CARE, lcap, cnt + L_FULL));
+        TRY(pass(1, 2, kFormCareful | X, L[L_CARE], cnt + L_CARE, L[L_FULL], cnt + L_FULL, lcap, cnt + L_FULL));
+    }
+    if (s0 < 8) {
+        TRY(pass(0, 4, kFormStd, L[L_FULL], cnt + L_FULL, nullptr, nullptr, norerun ? nullptr : L[L_CAP64], cnt + L_CAP64));
+        TRY(pass(0, 8, kFormStd, L[L_CAP64], cnt + L_CAP64, nullptr, nullptr, nullptr, nullptr));
+    } else {
+        TRY(pass(0, 8, kFormStd, L[L_FULL], cnt + L_FULL, nullptr, nullptr, nullptr, nullptr));
     }
     if (timing) CU(cudaEventRecord(ev[2], E.stream));
     return TESS_OK;
+}
+
+// The statistics of a finished compute from its counters.
+void read_counts(Engine& E, const unsigned* c, uint64_t faces) {
+    const unsigned *r32 = c + C_REASON32, *r64 = c + C_REASON64;
+    const uint64_t cap32 = (uint64_t)r32[ST_VCAP] + r32[ST_PCAP];
+    E.stats.cells = E.total;
+    E.stats.faces = faces;
+    E.stats.rerun_fp64 = (uint64_t)c[C_LIST + L_CARE] + c[C_FLAG];
+    E.stats.rerun_fp64_full = (uint64_t)c[C_LIST + L_FULL] - std::min<uint64_t>(cap32, c[C_LIST + L_FULL]);
+    E.stats.dense_cells = (uint64_t)c[C_LIST + L_DENSE] + c[C_DENSE];
+    E.stats.rerun_capacity = cap32 + c[C_LIST + L_CAP64];
+    E.stats.failed = c[C_FAIL];
+    E.stats.rerun_guard = (uint64_t)r32[ST_GUARD] + r64[ST_GUARD];
+    E.stats.rerun_verify = (uint64_t)r32[ST_VERIFY] + r64[ST_VERIFY];
+    E.stats.rerun_degenerate = (uint64_t)r32[ST_DEGEN] + r64[ST_DEGEN];
 }
 
 tess_status engine_autotune(Engine& E, int precision, bool batch, const char* cache_path, tess_tuning* out);
@@ -744,10 +736,10 @@ tess_status engine_compute(Engine& E, int precision, double radius, int64_t grou
     for (int attempt = 0; attempt < 4; ++attempt) {
         TRY(enqueue_passes(E, precision, radius, group, timing, ev.e));
         unsigned long long used = 0;
-        unsigned counts[16];
+        unsigned counts[C_TOTAL];
         int gerr = 0;
         CU(cudaMemcpyAsync(&used, E.d_fcursor, sizeof(used), cudaMemcpyDeviceToHost, E.stream));
-        CU(cudaMemcpyAsync(counts, E.d_counters + 16, sizeof(counts), cudaMemcpyDeviceToHost, E.stream));
+        CU(cudaMemcpyAsync(counts, E.d_counters, sizeof(counts), cudaMemcpyDeviceToHost, E.stream));
         CU(cudaMemcpyAsync(&gerr, E.d_err, sizeof(int), cudaMemcpyDeviceToHost, E.stream));
         CU(cudaStreamSynchronize(E.stream));
         if (gerr == 1) {
@@ -772,19 +764,7 @@ tess_status engine_compute(Engine& E, int precision, double radius, int64_t grou
             E.stats.face_pool_regrows += 1;
             continue;
         }
-        E.stats.cells = E.total;
-        E.stats.faces = used;
-        if (precision != TESS_PRECISION_FP64) {
-            E.stats.rerun_fp64 = counts[L_FP64];
-            E.stats.rerun_fp64_full = counts[L_FP64B];
-            E.stats.dense_cells = counts[L_DENSE];
-            E.stats.rerun_capacity = (uint64_t)counts[L_CAP1] + counts[L_CAP2] + counts[L_CAP64A] + counts[L_CAP64B];
-        } else {
-            E.stats.rerun_fp64 = 0;
-            E.stats.rerun_fp64_full = 0;
-            E.stats.dense_cells = 0;
-            E.stats.rerun_capacity = (uint64_t)counts[L_CAP64A] + counts[L_CAP64B];
-        }
+        read_counts(E, counts, used);
         if (E.ndiag == 1) {
             DiagDesc dd;
             CU(cudaMemcpy(&dd, E.d_desc, sizeof(DiagDesc), cudaMemcpyDeviceToHost));
@@ -800,8 +780,7 @@ tess_status engine_compute(Engine& E, int precision, double radius, int64_t grou
         E.last_precision = precision;
         E.last_radius = radius;
         E.last_group = group;
-        const uint64_t failed = counts[L_FAIL];
-        E.stats.failed = failed;
+        const uint64_t failed = counts[C_FAIL];
         if (E.cfg.flags & TESS_FLAG_COUNTERS) {
             unsigned long long w[8];
             CU(cudaMemcpy(w, E.d_work, sizeof(w), cudaMemcpyDeviceToHost));
@@ -811,9 +790,6 @@ tess_status engine_compute(Engine& E, int precision, double radius, int64_t grou
             E.stats.windows = w[3];
             E.stats.batches = w[4];
         }
-        E.stats.rerun_guard = counts[L_REASON + ST_GUARD];
-        E.stats.rerun_verify = counts[L_REASON + ST_VERIFY];
-        E.stats.rerun_degenerate = counts[L_REASON + ST_DEGEN];
         TRY(check_word(E));
         if (failed) return fail(TESS_E_OVERFLOW, "%llu cells could not be computed", (unsigned long long)failed);
         return TESS_OK;
@@ -1100,43 +1076,41 @@ tess_status engine_autotune(Engine& E, int precision, bool batch, const char* ca
     return TESS_OK;
 }
 
-// One cell's full geometry: re-run the cell alone (FP64 re-run if the FP32
-// form declines it) into the GeoOut buffer and copy it back.
-tess_status engine_geo(Engine& E, int precision, uint32_t gs, const double* point, double radius, int64_t group,
-                       const double* lo, const double* hi, GeoOut* out) {
+// One cell's full geometry: the cell alone through the FP64 clipping (in every
+// precision: one warp's latency is the same in FP32) into the GeoOut buffer,
+// copied back.
+tess_status engine_geo(Engine& E, uint32_t gs, const double* point, double radius, int64_t group, const double* lo,
+                       const double* hi, GeoOut* out) {
     CU(cudaSetDevice(E.device));
-    for (int prec : {precision, (int)TESS_PRECISION_FP64}) {
-        ClipParams p = base_params(E);
-        p.search_radius = radius;
-        p.has_radius = radius >= 0.0;
-        p.target_group = group;
-        CU(cudaMemcpyAsync(E.d_one, &gs, sizeof(uint32_t), cudaMemcpyHostToDevice, E.stream));
-        CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * 32, E.stream));
-        p.work = E.d_one;
-        p.work_count = nullptr;
-        p.total = 1;
-        p.cursor = E.d_counters;
-        p.geo = E.d_geo;
-        if (point) {
-            p.at_point = 1;
-            p.point[0] = point[0];
-            p.point[1] = point[1];
-            p.point[2] = point[2];
-        }
-        if (lo) {
-            p.box_override = 1;
-            for (int a = 0; a < 3; ++a) {
-                p.box[a] = lo[a];
-                p.box[3 + a] = hi[a];
-            }
-        }
-        CU(launch_clip(p, prec == TESS_PRECISION_FP32_GUARD ? 1 : 0, 8, kFormStd, 1, 1, E.stream));
-        CU(cudaMemcpyAsync(out, E.d_geo, sizeof(GeoOut), cudaMemcpyDeviceToHost, E.stream));
-        CU(cudaStreamSynchronize(E.stream));
-        TRY(check_word(E));
-        if (out->status == ST_OK) return TESS_OK;
-        if (prec == TESS_PRECISION_FP64) break;
+    ClipParams p = base_params(E);
+    p.search_radius = radius;
+    p.has_radius = radius >= 0.0;
+    p.target_group = group;
+    CU(cudaMemcpyAsync(E.d_one, &gs, sizeof(uint32_t), cudaMemcpyHostToDevice, E.stream));
+    CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * C_TOTAL, E.stream));
+    p.work = E.d_one;
+    p.work_count = nullptr;
+    p.total = 1;
+    p.cursor = E.d_counters;
+    p.geo = E.d_geo;
+    if (point) {
+        p.at_point = 1;
+        p.point[0] = point[0];
+        p.point[1] = point[1];
+        p.point[2] = point[2];
     }
+    if (lo) {
+        p.box_override = 1;
+        for (int a = 0; a < 3; ++a) {
+            p.box[a] = lo[a];
+            p.box[3 + a] = hi[a];
+        }
+    }
+    CU(launch_clip(p, 8, kFormStd, 1, 1, E.stream));
+    CU(cudaMemcpyAsync(out, E.d_geo, sizeof(GeoOut), cudaMemcpyDeviceToHost, E.stream));
+    CU(cudaStreamSynchronize(E.stream));
+    TRY(check_word(E));
+    if (out->status == ST_OK) return TESS_OK;
     return fail(TESS_E_OVERFLOW, "cell could not be computed (status %d)", out->status);
 }
 
@@ -1635,7 +1609,7 @@ static tess_status geo_for(tess_diagram* d, size_t i, GeoOut* g) {
     CU(cudaSetDevice(d->E.device));
     TRY(ensure_inv(d->E));
     CU(cudaMemcpy(&gs, d->E.d_inv + i, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    return engine_geo(d->E, d->E.last_precision, gs, nullptr, d->E.last_radius, d->E.last_group, nullptr, nullptr, g);
+    return engine_geo(d->E, gs, nullptr, d->E.last_radius, d->E.last_group, nullptr, nullptr, g);
 }
 
 tess_status tess_cell_vertices(tess_diagram* d, size_t i, double* xyz, size_t cap, size_t* count) {
@@ -1704,7 +1678,7 @@ static tess_status single_cell(tess_diagram* d, const size_t* i, const double* p
     }
     GeoOut* g = new (std::nothrow) GeoOut;
     if (!g) return fail(TESS_E_NOMEM, "host allocation failed");
-    tess_status st = engine_geo(d->E, (int)precision, gs, i ? nullptr : p, search_radius, target_group, lo, hi, g);
+    tess_status st = engine_geo(d->E, gs, i ? nullptr : p, search_radius, target_group, lo, hi, g);
     if (st == TESS_OK) geo_to_public(*g, out);
     delete g;
     return st;
@@ -1844,10 +1818,9 @@ static tess_status batch_run(tess_batch* b, int prec) {
                                  E.graph_host_cap != E.face_cap));
     if (stale) {
         // warm the per-kernel attributes and occupancy queries outside capture
-        for (int pr : {0, 1})
-            for (int s : {2, 4, 8})
-                for (int f : {(int)kFormLean, (int)kFormStd, (int)kFormHybrid})
-                    for (int x : {0, (int)kFormExact}) E.blocks(pr, s, f | x);
+        for (int k : {4, 8}) E.blocks(k, kFormStd);
+        for (int f : {(int)kFormLean, (int)kFormDense, (int)kFormCareful})
+            for (int x : {0, (int)kFormExact}) E.blocks(2, f | x);
         if (G) cudaGraphExecDestroy(G);
         G = nullptr;
         cudaGraph_t g = nullptr;
@@ -1879,13 +1852,13 @@ static tess_status batch_run(tess_batch* b, int prec) {
         CU(cudaEventRecord(ev.e[0], E.stream));
     }
     CU(cudaGraphLaunch(G, E.stream));
-    E.launches += grid_launches(E.total_bins) + (prec != TESS_PRECISION_FP64 ? 8 : 4);
+    E.launches += grid_launches(E.total_bins) + (E.total <= kCarefulMax ? 3 : 5) - (E.cfg.slots_per_lane >= 8 ? 1 : 0);
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     unsigned long long used = 0;
-    unsigned counts[16];
+    unsigned counts[C_TOTAL];
     int gerr = 0;
     CU(cudaMemcpyAsync(&used, E.d_fcursor, sizeof(used), cudaMemcpyDeviceToHost, E.stream));
-    CU(cudaMemcpyAsync(counts, E.d_counters + 16, sizeof(counts), cudaMemcpyDeviceToHost, E.stream));
+    CU(cudaMemcpyAsync(counts, E.d_counters, sizeof(counts), cudaMemcpyDeviceToHost, E.stream));
     CU(cudaMemcpyAsync(&gerr, E.d_err, sizeof(int), cudaMemcpyDeviceToHost, E.stream));
     CU(cudaStreamSynchronize(E.stream));
     TRY(check_word(E));
@@ -1913,22 +1886,12 @@ static tess_status batch_run(tess_batch* b, int prec) {
         E.graph = nullptr;
         return batch_run(b, prec);
     }
-    E.stats.cells = E.total;
-    E.stats.faces = used;
-    const bool f32 = prec != TESS_PRECISION_FP64;
-    E.stats.rerun_fp64 = f32 ? counts[L_FP64] : 0;
-    E.stats.rerun_fp64_full = f32 ? counts[L_FP64B] : 0;
-    E.stats.dense_cells = f32 ? counts[L_DENSE] : 0;
-    E.stats.rerun_capacity = (uint64_t)counts[L_CAP1] + counts[L_CAP2] + counts[L_CAP64A] + counts[L_CAP64B];
-    E.stats.failed = counts[L_FAIL];
-    E.stats.rerun_guard = counts[L_REASON + ST_GUARD];
-    E.stats.rerun_verify = counts[L_REASON + ST_VERIFY];
-    E.stats.rerun_degenerate = counts[L_REASON + ST_DEGEN];
+    read_counts(E, counts, used);
     E.computed = true;
     E.csr_valid = false;
     E.faces_on_host = host;
     E.last_precision = prec;
-    if (counts[L_FAIL]) return fail(TESS_E_OVERFLOW, "%u cells could not be computed", counts[L_FAIL]);
+    if (counts[C_FAIL]) return fail(TESS_E_OVERFLOW, "%u cells could not be computed", counts[C_FAIL]);
     return TESS_OK;
 }
 

@@ -1,5 +1,5 @@
 // tess_clip.cu -- dispatch to the clipping kernel instantiations
-// (tess_clip_f32.cu, tess_clip_f64.cu; kernel source tess_clip_impl.cuh) and
+// (tess_clip_lean.cu, FP32; tess_clip_f64.cu, kernel source tess_clip_impl.cuh) and
 // the CSR compaction of the per-cell face lists: offsets = exclusive scan of
 // the face counts, then a gather from the face pool into original cell order
 // (the bulk form of Cell::compute_faces, interface.rs:373-384).
@@ -133,14 +133,14 @@ __global__ void __launch_bounds__(256) k_csr_gather(const uint32_t* cnt, const u
 
 }  // namespace
 
-cudaError_t launch_clip(const ClipParams& p, int precision, int slots, int form, int wpb, int blocks,
-                        cudaStream_t s) {
-    return precision == 1 ? launch_clip_f32(p, slots, form, wpb, blocks, s)
-                          : launch_clip_f64(p, slots, form, wpb, blocks, s);
+cudaError_t launch_clip(const ClipParams& p, int slots, int form, int wpb, int blocks, cudaStream_t s) {
+    if ((form & 3) != kFormStd) return launch_clip_lean(p, form, wpb, blocks, s);
+    return launch_clip_f64(p, slots, wpb, blocks, s);
 }
 
-int clip_blocks_for(int precision, int slots, int form, int wpb, int device) {
-    return precision == 1 ? clip_blocks_f32(slots, form, wpb, device) : clip_blocks_f64(slots, form, wpb, device);
+int clip_blocks_for(int slots, int form, int wpb, int device) {
+    if ((form & 3) != kFormStd) return clip_blocks_lean(form, wpb, device);
+    return clip_blocks_f64(slots, wpb, device);
 }
 
 size_t csr_tmp_words(uint32_t n) {

@@ -1,11 +1,11 @@
-// tess_clip_lean.cu -- the FP32 first pass of the clipping: one Voronoi cell
-// per warp, with one candidate plane per lane.
+// tess_clip_lean.cu -- the FP32 clipping: one Voronoi cell per warp, with one
+// candidate plane per lane (Cell::compute_voronoi_cell, interface.rs:257-313).
 //
-// The cell, its container box, the error bounds and every decision are those
-// of the FP32 + guard form in tess_clip_impl.cuh (Cell::compute_voronoi_cell,
-// interface.rs:257-313); this pass runs over every cell and hands the ones it
-// cannot finish (guard-band tests, full tables, crowded bins) to the passes
-// there.  It differs in how a window of 32 candidates is worked off:
+// Positions, planes and classification are FP32, with a rigorous bound on each
+// plane test's error (see plane_test).  A test inside its bound is undecided:
+// the plain pass hands the cell on, the careful pass settles the test in FP64.
+// The bins around the site come as rows (see the walk), a window of 32
+// candidates is worked off as follows:
 //
 //   - The cell's vertices live in shared memory only.  When a window is
 //     loaded, every lane tests its own candidate's bisector against every live
@@ -50,6 +50,18 @@ using namespace clipk;
 
 constexpr int kSlots = 64;     // vertex slots
 constexpr int kPlanes = 96;    // planes, walls included
+constexpr int kNearZ = 2;      // the first three batches take the bins up to this offset along z
+
+// Instances of the pass:
+//   kPlain    over every cell; a cell with an undecided test or a crowded own
+//             bin goes on to the careful pass
+//   kCount    the same with work counters (they cost registers)
+//   kDense    over the cells of crowded bins: seeded, points gathered
+//   kCareful  as kDense, and undecided tests are settled in FP64 in place: over
+//             the cells the others handed on, or over every cell of a small
+//             input.  (An instance of its own: the settling makes the code
+//             half as large again, and the dense pass waits for instructions.)
+enum Mode : int { kPlain = 0, kCount = 1, kDense = 2, kCareful = 3 };
 
 struct Lean {
     float4 vtx[kSlots];             // vertex position, error bound
@@ -67,7 +79,8 @@ struct Lean {
             float pn[kPlanes + 1];          // |normal|
             float vr[kSlots];               // (|v| + e_v)^2
             float4 cand[32];                // a window's candidates within reach: plane ...
-            float candn[32];                // ... and |normal|
+            float candn[32];                // ... |normal| ...
+            uint32_t candj[32];             // ... and (careful) sorted index
             float4 nv[32];                  // the new vertices of a cut, in order ...
             alignas(4) uint8_t nvs[32];     // ... and their slots
             uint32_t boff[32];              // batch: start - prefix of the k-th bin that holds points
@@ -112,7 +125,9 @@ __device__ __forceinline__ float rcp_ftz(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-// Upper bound of sqrt(x), x >= 0 (sqrt_up): 0 gives 0, +inf and NaN +inf.
+// Upper bound of sqrt(x), x >= 0: rsqrt is within 2 ulp and the product adds
+// half an ulp, so the 2^-20 inflation keeps it above the exact root.  0 gives
+// 0, +inf and NaN +inf.
 __device__ __forceinline__ float norm_up(float x) {
     const float r = x * rsqrt_ftz(x) * 1.00000095367431640625f;
     return x == 0.f ? 0.f : (x < INFINITY ? r : INFINITY);
@@ -123,7 +138,23 @@ __device__ __forceinline__ float vertex_r2(float x, float y, float z, float e) {
 }
 
 // Signed distance of a vertex and the half-width of its guard band for the
-// plane (n, off) with |n| = rn; c0 = rn (guard_rel * rn + tol) + eC.
+// bisector n = r, off = r.r / 2 of the site and a point at r, rn = |r|:
+//   band = rn e + c0,  c0 = rn (guard_rel rn + tol) + eC,
+// where e is the vertex's error bound e_v, to which guard_rel |v|_1 is added at
+// its creation, and eC covers the hi/lo split of the positions.  A test with
+// |sd| <= band is undecided.  The bound, with u = 2^-24, r~ the FP32 offset
+// (|r~ - r| <= 2u |r|) and v~ the FP32 vertex (|v~ - v| <= e_v):
+//   fma chain rounding       3u (rn |v~|_1 + off)
+//   plane normal, vertex     2u rn |v|  +  rn e_v
+//   offset r.r / 2           3u rn^2
+// <= rn (e_v + 5u |v~|_1 + 4.5u rn), about rn (e_v + 3e-7 (|v~|_1 + rn)); the
+// default guard_rel 4e-7 leaves a third in hand.  eC: per component the offset
+// r~ = (hi_p - hi_s) + (lo_p - lo_s) is off by at most 2u |r| plus eta =
+// 6.1 u^2 (|site|_inf + R) (the lo parts' rounding, the hi subtraction's share
+// of it, the FP64 centring), which moves n.v - off by at most
+// eta (|v|_1 + 1.8 rn) <= 5.4 eta R.  R only shrinks, so the initial radius
+// bounds it for the whole cell.  Candidates nearer than 4 eta / u (plane error
+// above u / 4 relative, beyond the vertex error model) send the cell to FP64.
 __device__ __forceinline__ void plane_test(const float4& v, float nx, float ny, float nz, float off, float rn,
                                            float c0, float& sd, float& band) {
     sd = sdist(nx, ny, nz, off, v.x, v.y, v.z);
@@ -168,17 +199,29 @@ __device__ uint32_t row_plan(int lane) {
     }
     return (uint32_t)(ia & 0xFF) | (uint32_t)(ja & 0xFF) << 8 | (uint32_t)(ib & 0xFF) << 16 | (uint32_t)(jb & 0xFF) << 24;
 }
-// Row r of the 8 m rows of ring m (rows with max(|i|, |j|) = m).
-__device__ __forceinline__ void ring_row(int m, int r, int& i, int& j) {
-    const int side = 2 * m + 1;
-    if (r < 2 * side) {
-        i = r < side ? -m : m;
-        j = r % side - m;
+// Row r of batch 3 (both ends, two lanes each, of the rows up to ring 3) or of
+// the 8 m rows of ring m > 3 (rows with max(|i|, |j|) = m).  Packed offsets,
+// -1 past the last row.  Out of line: sparse regions and thin boxes.
+__device__ __noinline__ int far_row(int m, int r) {
+    int i, j;
+    if (m == 3) {
+        r >>= 1;
+        if (r >= 49) return -1;
+        i = r / 7 - 3;
+        j = r % 7 - 3;
     } else {
-        r -= 2 * side;
-        i = r % (side - 2) - (m - 1);
-        j = r < side - 2 ? -m : m;
+        if (r >= 8 * m) return -1;
+        const int side = 2 * m + 1;
+        if (r < 2 * side) {
+            i = r < side ? -m : m;
+            j = r % side - m;
+        } else {
+            r -= 2 * side;
+            i = r % (side - 2) - (m - 1);
+            j = r < side - 2 ? -m : m;
+        }
     }
+    return (i + 2048) << 12 | (j + 2048);
 }
 
 // A search radius (rare, out of line): the site's exact bin, and the end of
@@ -201,7 +244,78 @@ __device__ __noinline__ double wall_distance(const ClipParams& P, const DiagDesc
     return (p & 1) ? D.bhi[a] - s : s - D.blo[a];
 }
 
-template <bool EXACT, bool COUNT>
+// The vertex of planes a, b, c in FP64, by Cramer's rule on the walls and the
+// bisectors of the FP64 positions; cond = |n_a| |n_b| |n_c| / |det|, +inf when
+// the planes are singular.
+struct Vertex64 {
+    double x, y, z;
+    float cond;
+};
+__device__ __forceinline__ Vertex64 vertex_fp64(const Lean& S, const ClipParams& P, const DiagDesc& D, uint32_t gs,
+                                             uint32_t planes) {
+    const double sx = P.spx[gs], sy = P.spy[gs], sz = P.spz[gs];
+    double n[3][3], h[3];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        const int p = byte_of(planes, e);
+        if (p < 6) {
+            const int a = p >> 1;
+            const double sg = (p & 1) ? 1.0 : -1.0;
+            n[e][0] = a == 0 ? sg : 0.0;
+            n[e][1] = a == 1 ? sg : 0.0;
+            n[e][2] = a == 2 ? sg : 0.0;
+            const double s = a == 0 ? sx : (a == 1 ? sy : sz);
+            h[e] = (p & 1) ? D.bhi[a] - s : s - D.blo[a];
+        } else {
+            const uint32_t j = tess_chk(S.psrc[p], P.npts, P.check, CK_POINT);
+            n[e][0] = P.spx[j] - sx;
+            n[e][1] = P.spy[j] - sy;
+            n[e][2] = P.spz[j] - sz;
+            h[e] = 0.5 * (n[e][0] * n[e][0] + n[e][1] * n[e][1] + n[e][2] * n[e][2]);
+        }
+    }
+    const double bc0 = n[1][1] * n[2][2] - n[1][2] * n[2][1], bc1 = n[1][2] * n[2][0] - n[1][0] * n[2][2],
+                 bc2 = n[1][0] * n[2][1] - n[1][1] * n[2][0];
+    const double ca0 = n[2][1] * n[0][2] - n[2][2] * n[0][1], ca1 = n[2][2] * n[0][0] - n[2][0] * n[0][2],
+                 ca2 = n[2][0] * n[0][1] - n[2][1] * n[0][0];
+    const double ab0 = n[0][1] * n[1][2] - n[0][2] * n[1][1], ab1 = n[0][2] * n[1][0] - n[0][0] * n[1][2],
+                 ab2 = n[0][0] * n[1][1] - n[0][1] * n[1][0];
+    const double det = n[0][0] * bc0 + n[0][1] * bc1 + n[0][2] * bc2;
+    const double inv = recip_nr(det);
+    Vertex64 v;
+    v.x = (h[0] * bc0 + h[1] * ca0 + h[2] * ab0) * inv;
+    v.y = (h[0] * bc1 + h[1] * ca1 + h[2] * ab1) * inv;
+    v.z = (h[0] * bc2 + h[1] * ca2 + h[2] * ab2) * inv;
+    // one refinement step
+    const double r0 = h[0] - (n[0][0] * v.x + n[0][1] * v.y + n[0][2] * v.z);
+    const double r1 = h[1] - (n[1][0] * v.x + n[1][1] * v.y + n[1][2] * v.z);
+    const double r2 = h[2] - (n[2][0] * v.x + n[2][1] * v.y + n[2][2] * v.z);
+    v.x += (r0 * bc0 + r1 * ca0 + r2 * ab0) * inv;
+    v.y += (r0 * bc1 + r1 * ca1 + r2 * ab1) * inv;
+    v.z += (r0 * bc2 + r1 * ca2 + r2 * ab2) * inv;
+    auto norm = [](const double (&u)[3]) {
+        const float x = (float)u[0], y = (float)u[1], z = (float)u[2];
+        return norm_up(x * x + y * y + z * z);
+    };
+    v.cond = fabsf((float)inv) * norm(n[0]) * norm(n[1]) * norm(n[2]);
+    if (!(fabs(det) > 0.0)) v.cond = INFINITY;
+    return v;
+}
+
+// Side of the vertex of `planes` relative to the bisector of the site and
+// point j, decided in FP64 with the reference's test (vector3.rs:170-239,
+// tolerance 1e-12): 1 Outside, 0 not, -1 when the planes are singular.  Out of
+// line: few vertices need it.
+__device__ __noinline__ int side_fp64(const Lean& S, const ClipParams& P, const DiagDesc& D, uint32_t gs, uint32_t planes,
+                                      uint32_t j) {
+    const Vertex64 v = vertex_fp64(S, P, D, gs, planes);
+    if (!(v.cond < 1e12f)) return -1;
+    const double qx = P.spx[j] - P.spx[gs], qy = P.spy[j] - P.spy[gs], qz = P.spz[j] - P.spz[gs];
+    const double q2 = qx * qx + qy * qy + qz * qz;
+    return (qx * v.x + qy * v.y + qz * v.z - 0.5 * q2) / sqrt(q2) > kTolerance ? 1 : 0;
+}
+
+template <bool EXACT, int MODE>
 __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t gs, const DiagDesc& D, uint32_t plan, uint32_t& gen, Work& W,
                                          int lane) {
     const unsigned lt = (1u << lane) - 1u;
@@ -210,6 +324,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
     const float shx = site_h.x, shy = site_h.y, shz = site_h.z;
     const float slx = site_l.x, sly = site_l.y, slz = site_l.z;
     const uint32_t orig = tess_chk(__float_as_uint(site_h.w), P.npts, P.check, CK_POINT);
+    constexpr bool COUNT = MODE != kPlain, SEED = MODE >= kDense, CAREFUL = MODE == kCareful;
     const float gr = P.guard_rel, tol = P.tol;
 
     // ---- the container box, translated by -site (polyhedron.rs:268-392) ----
@@ -255,7 +370,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
     int np = 6;
     float R2 = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(r2l)));
     // the hi/lo split's share of a plane test's error, and the distance below
-    // which a candidate is handed to FP64 (derived in run_cell)
+    // which a candidate is handed to FP64 (see plane_test)
     float eC, dup2;
     {
         const float sa = fmaxf(fabsf(shx), fmaxf(fabsf(shy), fabsf(shz))) * 1.001f;
@@ -293,12 +408,78 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
         cbz = exact_bin(P, D, gs, 2);
     }
     const float fx = fminf(fmaxf(px - (float)cbx, 0.f), 1.f), fy = fminf(fmaxf(py - (float)cby, 0.f), 1.f);
+    const float fz = fminf(fmaxf(pz - (float)cbz, 0.f), 1.f);
+    // Careful: when the own bin is crowded, it and the crowded bins around it
+    // are seeded first, nearest first: each lane takes the nearest point of its
+    // stride of the bin, and the 32 are cut as one window.  Otherwise windows
+    // in storage order meet the nearest points late, after many cuts by farther
+    // ones (clustered inputs: 62 cuts a cell instead of 23).
+    uint32_t nbeg = 0, ncnt = 0;
+    float nd = INFINITY;
+    unsigned pending = 0;
+    bool undec = false;              // careful: a test was settled in FP64
+    if constexpr (SEED) {
+        const int ti = lane / 9 - 1, tj = (lane / 3) % 3 - 1, tk = lane % 3 - 1;
+        const int x = cbx + ti, y = cby + tj, z = cbz + tk;
+        if (lane < 27 && x >= 0 && x < cpd && y >= 0 && y < cpd && z >= 0 && z < cpd) {
+            const uint64_t lb = tess_chk(D.bin_base + ((uint64_t)x * cpd + y) * cpd + z, P.nbins, P.check, CK_BIN);
+            nbeg = P.delims[lb];
+            ncnt = P.delims[lb + 1] - nbeg;
+            const float dx = fmaxf((ti > 0 ? 1.f - fx : (ti < 0 ? fx : 0.f)) - feps, 0.f) * D.size_f[0];
+            const float dy = fmaxf((tj > 0 ? 1.f - fy : (tj < 0 ? fy : 0.f)) - feps, 0.f) * D.size_f[1];
+            const float dz = fmaxf((tk > 0 ? 1.f - fz : (tk < 0 ? fz : 0.f)) - feps, 0.f) * D.size_f[2];
+            nd = (dx * dx + dy * dy + dz * dz) * (1.0f - 1e-4f);
+        }
+        const unsigned crowded = __ballot_sync(FULL, ncnt >= P.seed_min);
+        if (__shfl_sync(FULL, ncnt, 13) >= P.seed_min) pending = crowded;
+    }
+    const bool seeded = SEED && pending != 0;
     uint32_t pend = 0;               // batch 0: where my row's points that were not taken start
     int m = 0, ring0 = 0;            // batch (0, 1, 2) or ring (4 on); first row of a ring's batch
     // bin sides or a cell radius outside FP32's normal range
-    if (!D.lean_ok) status = ST_DENSE;
+    if (!D.lean_ok) status = SEED ? ST_GUARD : ST_DENSE;
     if (!(R2 >= FLT_MIN)) status = ST_GUARD;
     while (status == ST_OK) {
+        float sx_ = 0.f, sy_ = 0.f, sz_ = 0.f, s2_ = INFINITY;   // careful: my seed
+        uint32_t sj_ = 0;
+        unsigned total, pref = 0;
+        uint32_t bbeg = 0, bcnt = 0;
+        const bool direct = SEED && pending != 0;
+        if (direct) {
+            // ---- the seeds of the nearest crowded bin left ----
+            const unsigned best = __reduce_min_sync(
+                FULL, ((pending >> lane) & 1u) ? ((__float_as_uint(nd) & ~31u) | (unsigned)lane) : 0xFFFFFFFFu);
+            const int cb = (int)(best & 31u);
+            pending &= ~(1u << cb);
+            if (cb != 13 && __shfl_sync(FULL, nd, cb) >= 4.f * R2) {
+                pending = 0;     // the others are farther
+                continue;
+            }
+            const uint32_t sbeg = __shfl_sync(FULL, nbeg, cb), scnt = __shfl_sync(FULL, ncnt, cb);
+            bool near = false;
+#pragma unroll 1
+            for (uint32_t q = lane; q < scnt; q += 32) {
+                const uint32_t j = tess_chk(sbeg + q, P.npts, P.check, CK_POINT);
+                const float4 h = P.phi[j], l = P.plo[j];
+                const float rx = (h.x - shx) + (l.x - slx), ry = (h.y - shy) + (l.y - sly), rz = (h.z - shz) + (l.z - slz);
+                const float r2 = rx * rx + ry * ry + rz * rz;
+                near |= j != gs && !(r2 > dup2);
+                bool take = j != gs && r2 > dup2 && r2 < s2_;
+                if (take && P.target_group >= 0) take = (int64_t)(P.sgroup ? P.sgroup[j] : 0u) == P.target_group;
+                if (take) {
+                    sx_ = rx;
+                    sy_ = ry;
+                    sz_ = rz;
+                    s2_ = r2;
+                    sj_ = j;
+                }
+            }
+            if (__any_sync(FULL, near)) {
+                status = ST_GUARD;
+                break;
+            }
+            total = 32;
+        } else {
         // ---- the next batch: one row of bins per lane ----
         int i = 0, j = 0;
         bool have;
@@ -310,11 +491,13 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
             }
         } else {
             if (m >= 2) {
-                // the farthest bin offset within reach
+                // the farthest bin offsets within reach
                 const float rc = 2.f * norm_up(R2) * 1.0001f;
-                const float rx_ = rc * inx + feps, ry_ = rc * iny + feps;
+                const float rx_ = rc * inx + feps, ry_ = rc * iny + feps, rz_ = rc * inz + feps;
                 const float far = fmaxf(fmaxf(rx_ + fx, rx_ + 1.f - fx), fmaxf(ry_ + fy, ry_ + 1.f - fy));
-                if (!(far >= (float)m) || m >= cpd) break;
+                if (m == 2 && !(far >= 2.f)) m = 3;
+                if (m == 3 && !(fmaxf(rz_ + fz, rz_ + 1.f - fz) >= (float)(kNearZ + 1))) m = 4;
+                if (m >= 4 && (!(far >= (float)m) || m >= cpd)) break;
             }
             if (m <= 2) {
                 have = lane < (m == 1 ? 30 : 28);
@@ -322,17 +505,18 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 i = (int8_t)w;
                 j = (int8_t)(w >> 8);
             } else {
-                have = ring0 + lane < 8 * m;
-                ring_row(m, ring0 + lane, i, j);
+                const int w = far_row(m, ring0 + lane);
+                have = w >= 0;
+                i = (w >> 12) - 2048;
+                j = (w & 4095) - 2048;
             }
         }
-        uint32_t bbeg = 0, bcnt = 0;
         const uint32_t from = __shfl_sync(FULL, pend, lane >> 1);
         const int x = cbx + i, y = cby + j;
         if (have && x >= 0 && x < cpd && y >= 0 && y < cpd) {
             int kl = cbz, kh = cbz;
             bool on = true;
-            if (m == 0) {
+            if (!SEED && m == 0) {
                 if (lane < 9) {
                     kl = max(cbz - 1, 0);
                     kh = min(cbz + 1, cpd - 1);
@@ -348,6 +532,13 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 kl = max((int)floorf(pz - zr), 0);
                 kh = min((int)floorf(pz + zr), cpd - 1);
             }
+            if (m == 1 || m == 2) {
+                kl = max(kl, cbz - kNearZ);
+                kh = min(kh, cbz + kNearZ);
+            } else if (m == 3) {
+                if (lane & 1) kl = max(kl, cbz + kNearZ + 1);
+                else kh = min(kh, cbz - kNearZ - 1);
+            }
             if (P.has_radius) {
                 const int a = radius_reach(D, P.search_radius, i, j, min(kl - cbz, 0)), b = radius_reach(D, P.search_radius, i, j, max(kh - cbz, 0));
                 if (a == INT_MAX) on = false;
@@ -355,6 +546,10 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                     kl = max(kl, cbz + a);
                     kh = min(kh, cbz + b);
                 }
+            }
+            if (SEED && m == 0) {
+                kl = max(kl, cbz - 1);
+                kh = min(kh, cbz + 1);
             }
             const bool central = m == 1 && lane < 18;
             if (central && !(lane & 1)) kh = min(kh, cbz - 2);            // below the 27 bins
@@ -366,13 +561,13 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 const uint64_t row = D.bin_base + ((uint64_t)x * cpd + y) * cpd;
                 bbeg = P.delims[tess_chk(row + kl, P.nbins, P.check, CK_BIN)];
                 const uint32_t end = P.delims[tess_chk(row + kh, P.nbins, P.check, CK_BIN) + 1];
-                if (central && (lane & 1)) bbeg = from;
+                if (central && (lane & 1) && from != 0xFFFFFFFFu) bbeg = from;
                 bcnt = end > bbeg ? end - bbeg : 0u;
             }
         }
         if (m == 0) {
             // a crowded own bin sends the cell to the seeded pass
-            if (P.list_dense && __shfl_sync(FULL, bcnt, 9) >= P.seed_min) {
+            if (!SEED && P.list_dense && __shfl_sync(FULL, bcnt, 9) >= P.seed_min) {
                 status = ST_DENSE;
                 break;
             }
@@ -380,19 +575,19 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
         }
         // ---- its points as one stream, 32 per window ----
         const unsigned inc = warp_incl_scan_u(bcnt, lane);
-        unsigned total = __shfl_sync(FULL, inc, 31);
-        const unsigned pref = inc - bcnt;
+        total = __shfl_sync(FULL, inc, 31);
+        pref = inc - bcnt;
         if (m == 0) {
             // whole windows only; the rest joins the next batch
             if (total > 32) total &= ~31u;
-            pend = bbeg + min(max((int)(total - pref), 0), (int)bcnt);
+            pend = bcnt ? bbeg + min(max((int)(total - pref), 0), (int)bcnt) : (SEED ? 0xFFFFFFFFu : bbeg);
         }
         // the batch after this one
         if (m < 3) {
-            m = m == 2 ? 4 : m + 1;
+            ++m;
         } else {
             ring0 += 32;
-            if (ring0 >= 8 * m) {
+            if (ring0 >= (m == 3 ? 98 : 8 * m)) {
                 ++m;
                 ring0 = 0;
             }
@@ -403,28 +598,123 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
             const unsigned nz = __ballot_sync(FULL, bcnt > 0);
             if (bcnt) S.boff[__popc(nz & lt)] = bbeg - pref;
         }
+        }
         __syncwarp();
-        unsigned before = 0;      // bins that began in earlier windows
-        for (unsigned w0 = 0; w0 < total; w0 += 32) {
-            const unsigned rel = pref - w0;
-            const unsigned heads = __reduce_or_sync(FULL, (bcnt && rel < 32u) ? 1u << rel : 0u);
-            const unsigned c = w0 + lane;
-            bool keep = false, near = false;
-            float rx = 0.f, ry = 0.f, rz = 0.f, r2 = 0.f;
-            uint32_t jp = 0;
+        unsigned before = 0;      // ranges that began in earlier windows
+        unsigned w0 = 0;
+        do {
+            float rx, ry, rz, r2;
+            uint32_t jp;
+            bool keep, near;
             float lim = 4.f * R2 * (float)kStopMargin;
-            if (c < total) {
-                jp = tess_chk(S.boff[before + __popc(heads & (lt | (1u << lane))) - 1] + c, P.npts, P.check, CK_POINT);
-                const float4 h = P.phi[jp], l = P.plo[jp];
-                rx = (h.x - shx) + (l.x - slx);
-                ry = (h.y - shy) + (l.y - sly);
-                rz = (h.z - shz) + (l.z - slz);
-                r2 = rx * rx + ry * ry + rz * rz;
-                keep = jp != gs && r2 > dup2 && r2 < lim;
-                near = jp != gs && !(r2 > dup2);
-                if (keep && P.target_group >= 0) keep = (int64_t)(P.sgroup ? P.sgroup[jp] : 0u) == P.target_group;
+            // Careful: the bounds of the cell's vertices and of their errors.  In
+            // clusters most points within twice the radius lie where the cell
+            // does not reach: a bisector beyond the box's support cannot touch
+            // a vertex (clustered inputs: 260 points a cell are within twice
+            // the radius, of which 22 cut).
+            float bl0 = 0.f, bl1 = 0.f, bl2 = 0.f, bh0 = 0.f, bh1 = 0.f, bh2 = 0.f, be = 0.f;
+            if constexpr (SEED) {
+                if (!direct) {
+                    float4 v = S.vtx[lane];
+                    bool lv = (l0 >> lane) & 1u;
+                    bl0 = bh0 = lv ? v.x : 0.f;      // the site is inside its bounds
+                    bl1 = bh1 = lv ? v.y : 0.f;
+                    bl2 = bh2 = lv ? v.z : 0.f;
+                    be = lv ? v.w : 0.f;
+                    if ((l1 >> lane) & 1u) {
+                        v = S.vtx[32 + lane];
+                        bl0 = fminf(bl0, v.x);
+                        bh0 = fmaxf(bh0, v.x);
+                        bl1 = fminf(bl1, v.y);
+                        bh1 = fmaxf(bh1, v.y);
+                        bl2 = fminf(bl2, v.z);
+                        bh2 = fmaxf(bh2, v.z);
+                        be = fmaxf(be, v.w);
+                    }
+                    // non-negative floats order like their bits
+                    auto top = [](float x) { return __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(fmaxf(x, 0.f)))); };
+                    bl0 = -top(-bl0);
+                    bl1 = -top(-bl1);
+                    bl2 = -top(-bl2);
+                    bh0 = top(bh0);
+                    bh1 = top(bh1);
+                    bh2 = top(bh2);
+                    be = top(be) + 1e-6f * norm_up(R2);   // and the support's own rounding
+                }
             }
-            before += __popc(heads);
+            auto reaches = [&](float x, float y, float z, float q2) {
+                const float h = fmaxf(x * bl0, x * bh0) + fmaxf(y * bl1, y * bh1) + fmaxf(z * bl2, z * bh2);
+                const float n = norm_up(q2);
+                return h + fmaf(n, be + fmaf(gr, n, tol), eC) >= 0.5f * q2;
+            };
+            // 32 points of the stream, one per lane
+            auto load = [&]() {
+                const unsigned rel = pref - w0;
+                const unsigned heads = __reduce_or_sync(FULL, (bcnt && rel < 32u) ? 1u << rel : 0u);
+                const unsigned c = w0 + lane;
+                keep = near = false;
+                rx = ry = rz = r2 = 0.f;
+                jp = 0;
+                if (c < total) {
+                    jp = tess_chk(S.boff[before + __popc(heads & (lt | (1u << lane))) - 1] + c, P.npts, P.check, CK_POINT);
+                    const float4 h = P.phi[jp], l = P.plo[jp];
+                    rx = (h.x - shx) + (l.x - slx);
+                    ry = (h.y - shy) + (l.y - sly);
+                    rz = (h.z - shz) + (l.z - slz);
+                    r2 = rx * rx + ry * ry + rz * rz;
+                    keep = jp != gs && r2 > dup2 && r2 < lim;
+                    near = jp != gs && !(r2 > dup2);
+                    if (keep && P.target_group >= 0) keep = (int64_t)(P.sgroup ? P.sgroup[jp] : 0u) == P.target_group;
+                    if constexpr (SEED) keep = keep && reaches(rx, ry, rz, r2);
+                }
+                return heads;
+            };
+            if (direct) {
+                rx = sx_;
+                ry = sy_;
+                rz = sz_;
+                r2 = s2_;
+                jp = sj_;
+                keep = s2_ < lim;
+                near = false;
+                w0 += 32;
+            } else if constexpr (SEED) {
+                // gather the points within reach until the window is full
+                // (crowded bins hold hundreds that are not)
+                unsigned nk = 0;
+                bool anynear = false;
+                do {
+                    const unsigned heads = load();
+                    const unsigned kk = __ballot_sync(FULL, keep);
+                    if (nk + __popc(kk) > 32u) break;
+                    if (keep) {
+                        const unsigned at = nk + __popc(kk & lt);
+                        S.cand[at] = make_float4(rx, ry, rz, r2);
+                        S.candj[at] = jp;
+                    }
+                    anynear |= near;
+                    nk += __popc(kk);
+                    before += __popc(heads);
+                    w0 += 32;
+                } while (w0 < total && nk < 24u);
+                __syncwarp();
+                near = anynear;
+                keep = (unsigned)lane < nk;
+                const float4 own = S.cand[lane];
+                rx = own.x;
+                ry = own.y;
+                rz = own.z;
+                r2 = own.w;
+                jp = S.candj[lane];
+                // (a seed that cut is a plane already)
+                if (seeded)
+#pragma unroll 1
+                    for (int p = 6; p < np; ++p) keep = keep && S.psrc[p] != jp;
+                __syncwarp();
+            } else {
+                before += __popc(load());
+                w0 += 32;
+            }
             // (near-)coincident points are decided in FP64
             if (__any_sync(FULL, near)) {
                 status = ST_GUARD;
@@ -481,13 +771,37 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
             }
             // Nearest first: the closest candidate that may cut, by a warp
             // minimum of its distance (top 27 bits of r2, ties by lane).
+            int decided = -1;        // careful: a candidate whose undecided tests were settled
             const unsigned mykey = (__float_as_uint(r2) & ~31u) | (unsigned)lane;
             for (;;) {
                 const bool act = keep && r2 < lim && ((t0 & l0) | (t1 & l1)) != 0;
                 const unsigned best = __reduce_min_sync(FULL, act ? mykey : 0xFFFFFFFFu);
                 if (best == 0xFFFFFFFFu) break;
                 const int src = (int)(best & 31u);
-                const int f = np;
+                int f = np;
+                if constexpr (SEED) {
+                    if (f >= kPlanes) {
+                        // the table is full: an id that no live vertex has any
+                        // more (planes cut away entirely leave them behind)
+                        uint32_t u0 = 0x3Fu, u1 = 0, u2 = 0;       // the walls stay
+#pragma unroll 1
+                        for (int k = 0; k < 2; ++k)
+                            if (((k ? l1 : l0) >> lane) & 1u) {
+                                const uint32_t tt = S.topo[32 * k + lane].x;
+#pragma unroll 1
+                                for (int e = 0; e < 3; ++e) {
+                                    const int p = byte_of(tt, e);
+                                    if (p < 32) u0 |= 1u << p;
+                                    else if (p < 64) u1 |= 1u << (p - 32);
+                                    else u2 |= 1u << (p - 64);
+                                }
+                            }
+                        u0 = ~__reduce_or_sync(FULL, u0);
+                        u1 = ~__reduce_or_sync(FULL, u1);
+                        u2 = ~__reduce_or_sync(FULL, u2);
+                        f = u0 ? __ffs(u0) - 1 : (u1 ? 31 + __ffs(u1) : (u2 ? 63 + __ffs(u2) : kPlanes));
+                    }
+                }
                 if (lane == src) {
                     S.pl[f] = make_float4(rx, ry, rz, off);
                     S.pn[f] = rn;
@@ -535,7 +849,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                         bnd = edge(x, lane - 3 * xi);
                         float sd, band;
                         plane_test(S.vtx[x], pf.x, pf.y, pf.z, pf.w, nf, cf, sd, band);
-                        und = sd <= band;
+                        und = sd <= band && (!CAREFUL || src != decided);
                     }
                     const unsigned bm = __ballot_sync(FULL, bnd);
                     B = __popc(bm);
@@ -553,7 +867,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                             bd = edge(x, e);
                             float sd, band;
                             plane_test(S.vtx[x], pf.x, pf.y, pf.z, pf.w, nf, cf, sd, band);
-                            und |= sd <= band;
+                            und |= sd <= band && (!CAREFUL || src != decided);
                         }
                         const unsigned bm = __ballot_sync(FULL, bd);
                         const int at = B + __popc(bm & lt);
@@ -569,9 +883,44 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                     }
                 }
                 if (__any_sync(FULL, und)) {
-                    status = ST_GUARD;
-                    break;
+                    if constexpr (!CAREFUL) {
+                        status = ST_GUARD;
+                        break;
+                    }
+                    undec = true;
+                    // settle the touched vertices in FP64, one lane each, and
+                    // choose again
+                    uint32_t d0 = 0, d1 = 0;
+                    bool fail = false;
+                    for (int r0 = 0; r0 < R; r0 += 32) {
+                        if (r0 + lane < R) {
+                            const int x = S.fl[base + r0 + lane];
+                            float sd, band;
+                            plane_test(S.vtx[x], pf.x, pf.y, pf.z, pf.w, nf, cf, sd, band);
+                            int side = 1;
+                            if (sd <= band) side = side_fp64(S, P, D, gs, S.topo[x].x, tess_chk(S.psrc[f], P.npts, P.check, CK_POINT));
+                            fail |= side < 0;
+                            if (side > 0 && x < 32) d0 |= 1u << x;
+                            if (side > 0 && x >= 32) d1 |= 1u << (x - 32);
+                        }
+                    }
+                    if (__any_sync(FULL, fail)) {
+                        status = ST_GUARD;
+                        break;
+                    }
+                    d0 = __reduce_or_sync(FULL, d0);
+                    d1 = __reduce_or_sync(FULL, d1);
+                    if (lane == src) {
+                        t0 = d0;
+                        t1 = d1;
+                        keep = true;
+                    }
+                    km |= 1u << src;
+                    decided = src;
+                    __syncwarp();
+                    continue;
                 }
+                decided = -1;
                 if constexpr (COUNT) {
                     ++W.cuts;
                     W.newv += (unsigned)B;
@@ -600,7 +949,8 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                     const float x1 = fabsf(px) + fabsf(py) + fabsf(pz);
                     float pe = kVertexErr * x1 * (S.pn[a] * S.pn[b] * nf) * fabsf(inv);
                     // singular (or nearly): not a vertex to go on from
-                    bad = !(pe < 1e30f);
+                    // (careful: beyond 0.03 the first-order bound is no bound)
+                    bad = CAREFUL ? !(pe <= 0.03f * x1) : !(pe < 1e30f);
                     pe += gr * x1;
                     slot = tess_chk((int)S.fl[base + R - 1 - q], kSlots, P.check, CK_SLOT);
                     S.vtx[slot] = S.nv[q] = make_float4(px, py, pz, pe);
@@ -631,12 +981,16 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 l0 = (l0 & ~o0) | n0;
                 l1 = (l1 & ~o1) | n1;
                 nfree = base + R - B;
-                np = f + 1;
+                np = SEED ? max(np, f + 1) : f + 1;
                 // the smaller cell's radius, and the new vertices against the
                 // waiting candidates
                 float rr = ((l0 >> lane) & 1u) ? S.vr[lane] : 0.f;
                 if ((l1 >> lane) & 1u) rr = fmaxf(rr, S.vr[32 + lane]);
+                const float R2b = R2;
                 R2 = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(rr)));
+                // a cut moves no vertex beyond the cell: a radius that grew
+                // means a wrong vertex
+                if constexpr (CAREFUL) bad |= !(R2 <= R2b * 1.001f);
                 if (km) {
                     t0 &= ~n0;
                     t1 &= ~n1;
@@ -665,7 +1019,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 }
             }
             if (status != ST_OK) break;
-        }
+        } while (w0 < total);
     }
 
     // ---- finalize: faces, areas, volume (polyhedron.rs:776-855) ----
@@ -771,8 +1125,8 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
         __syncwarp();
         // FP32: one Newton step per vertex, residuals of its three planes in
         // double-float, the correction solved in FP32 by Cramer's rule.  FP64
-        // finish: the vertex solved from its planes in FP64.  A vertex that
-        // moves beyond its error bound was not trustworthy: the cell re-runs.
+        // finish: the same step in FP64.  A vertex that moves beyond its error
+        // bound was not trustworthy: the cell re-runs.
         auto resid = [&](const float4& h, const float4& l, float x, float y, float z) -> float {
             float p0, e0, p1, e1, p2, e2, s1, t1_, s2, t2, s3, t3;
             two_prod(h.x, x, p0, e0);
@@ -800,15 +1154,23 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                     const double cax = c0_.y * a1.x - c1.x * a0.y, cay = c1.x * a0.x - c0_.x * a1.x, caz = c0_.x * a0.y - c0_.y * a0.x;
                     const double abx = a0.y * b1.x - a1.x * b0.y, aby = a1.x * b0.x - a0.x * b1.x, abz = a0.x * b0.y - a0.y * b0.x;
                     const double inv = recip_nr(a0.x * bcx + a0.y * bcy + a1.x * bcz);
-                    const double x = (a1.y * bcx + b1.y * cax + c1.y * abx) * inv;
-                    const double y = (a1.y * bcy + b1.y * cay + c1.y * aby) * inv;
-                    const double z = (a1.y * bcz + b1.y * caz + c1.y * abz) * inv;
-                    S.d.rx[s] = x;
-                    S.d.ry[s] = y;
-                    S.d.rz[s] = z;
-                    ddx = (float)x - v.x;
-                    ddy = (float)y - v.y;
-                    ddz = (float)z - v.z;
+                    // the residuals at the FP32 vertex, and the step that removes
+                    // them: its error is the residuals' rounding (solving for
+                    // the vertex itself loses 1 / det of it: 2e-12 of a thin
+                    // cell's volume against 1e-15)
+                    const double vx = v.x, vy = v.y, vz = v.z;
+                    const double ra = a1.y - (a0.x * vx + a0.y * vy + a1.x * vz);
+                    const double rb = b1.y - (b0.x * vx + b0.y * vy + b1.x * vz);
+                    const double rc = c1.y - (c0_.x * vx + c0_.y * vy + c1.x * vz);
+                    const double ex = (ra * bcx + rb * cax + rc * abx) * inv;
+                    const double ey = (ra * bcy + rb * cay + rc * aby) * inv;
+                    const double ez = (ra * bcz + rb * caz + rc * abz) * inv;
+                    S.d.rx[s] = vx + ex;
+                    S.d.ry[s] = vy + ey;
+                    S.d.rz[s] = vz + ez;
+                    ddx = (float)ex;
+                    ddy = (float)ey;
+                    ddz = (float)ez;
                 } else {
                     const float4 ha = S.s.q[a], hb = S.s.q[b], hc = S.s.q[c];
                     const float ra = resid(ha, S.s.ql[a], v.x, v.y, v.z);
@@ -918,6 +1280,13 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
     }
 
     // ---- outputs ----
+    if constexpr (CAREFUL) {
+        // as the first pass, it counts what the plain pass would hand on
+        if (lane == 0 && !P.work) {
+            if (seeded) atomicAdd(P.list_dense_count, 1u);
+            else if (undec || status == ST_GUARD || status == ST_DEGEN || status == ST_VERIFY) atomicAdd(P.flag_count, 1u);
+        }
+    }
     if (status != ST_OK) {
         if (lane == 0) {
             uint32_t* list = nullptr;
@@ -975,8 +1344,8 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
 // 4 warps per block, five blocks per SM: 96 registers, no spills.  At
 // 1,000,000 uniform points: 13.3 ms with 16 warps per SM, 11.9 with 20, 12.4
 // with 24 (80 registers, 19% more instructions and the instruction cache full).
-template <bool EXACT, bool COUNT>
-__global__ void __launch_bounds__(128, 5) k_lean(ClipParams P) {
+template <bool EXACT, int MODE>
+__global__ void __launch_bounds__(128, MODE == kCareful ? 4 : 5) k_lean(ClipParams P) {
     extern __shared__ __align__(16) unsigned char smraw[];
     Lean& S = reinterpret_cast<Lean*>(smraw)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -1004,11 +1373,11 @@ __global__ void __launch_bounds__(128, 5) k_lean(ClipParams P) {
             }
             d = lo;
         }
-        run_lean<EXACT, COUNT>(P, S, gs, P.diags[d], plan, gen, W, lane);
+        run_lean<EXACT, MODE>(P, S, gs, P.diags[d], plan, gen, W, lane);
         w = __shfl_sync(FULL, wn, 0);
     }
-    if constexpr (COUNT) {
-        if (lane == 0) {
+    if constexpr (MODE != kPlain) {
+        if (lane == 0 && P.work_ctr) {
             atomicAdd(&P.work_ctr[0], (unsigned long long)W.tested);
             atomicAdd(&P.work_ctr[1], (unsigned long long)W.cuts);
             atomicAdd(&P.work_ctr[2], (unsigned long long)W.newv);
@@ -1018,7 +1387,7 @@ __global__ void __launch_bounds__(128, 5) k_lean(ClipParams P) {
     }
 }
 
-template <bool EXACT, bool COUNT>
+template <bool EXACT, int MODE>
 cudaError_t configure(size_t bytes) {
     static std::mutex mu;
     static size_t configured[kMaxDevices] = {};
@@ -1028,26 +1397,26 @@ cudaError_t configure(size_t bytes) {
     std::lock_guard<std::mutex> lock(mu);
     size_t* slot = (dev >= 0 && dev < kMaxDevices) ? &configured[dev] : nullptr;
     if (slot && bytes <= *slot) return cudaSuccess;
-    e = cudaFuncSetAttribute(k_lean<EXACT, COUNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    e = cudaFuncSetAttribute(k_lean<EXACT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e == cudaSuccess && slot) *slot = bytes;
     return e;
 }
 
-template <bool EXACT, bool COUNT>
+template <bool EXACT, int MODE>
 cudaError_t launch(const ClipParams& p, int wpb, int blocks, cudaStream_t s) {
     const size_t sm = sizeof(Lean) * (size_t)wpb;
-    cudaError_t e = configure<EXACT, COUNT>(sm);
+    cudaError_t e = configure<EXACT, MODE>(sm);
     if (e != cudaSuccess) return e;
-    k_lean<EXACT, COUNT><<<blocks, 32 * wpb, sm, s>>>(p);
+    k_lean<EXACT, MODE><<<blocks, 32 * wpb, sm, s>>>(p);
     return cudaGetLastError();
 }
 
-template <bool EXACT, bool COUNT>
+template <bool EXACT, int MODE>
 int blocks_for(int wpb, int device) {
     const size_t sm = sizeof(Lean) * (size_t)wpb;
     int per = 0, nsm = 0;
-    if (configure<EXACT, COUNT>(sm) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lean<EXACT, COUNT>, 32 * wpb, sm) != cudaSuccess)
+    if (configure<EXACT, MODE>(sm) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lean<EXACT, MODE>, 32 * wpb, sm) != cudaSuccess)
         per = 1;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
     cudaGetLastError();   // leave no sticky error behind a failed query
@@ -1057,17 +1426,29 @@ int blocks_for(int wpb, int device) {
 
 }  // namespace cliplean
 
-// TESS_FLAG_COUNTERS runs instances that count their work (the counters cost
-// the others registers); the results are the same.
-cudaError_t launch_clip_lean(const ClipParams& p, int exact, int wpb, int blocks, cudaStream_t s) {
+// form: kFormLean (the plain pass; with TESS_FLAG_COUNTERS its counting
+// instance, the results are the same), kFormDense or kFormCareful, with
+// kFormExact for the FP64 finish.
+cudaError_t launch_clip_lean(const ClipParams& p, int form, int wpb, int blocks, cudaStream_t s) {
     using namespace cliplean;
-    if (p.work_ctr) return exact ? launch<true, true>(p, wpb, blocks, s) : launch<false, true>(p, wpb, blocks, s);
-    return exact ? launch<true, false>(p, wpb, blocks, s) : launch<false, false>(p, wpb, blocks, s);
+    const bool x = form & kFormExact;
+    switch (form & 3) {
+        case kFormCareful: return x ? launch<true, kCareful>(p, wpb, blocks, s) : launch<false, kCareful>(p, wpb, blocks, s);
+        case kFormDense: return x ? launch<true, kDense>(p, wpb, blocks, s) : launch<false, kDense>(p, wpb, blocks, s);
+        default: break;
+    }
+    if (p.work_ctr) return x ? launch<true, kCount>(p, wpb, blocks, s) : launch<false, kCount>(p, wpb, blocks, s);
+    return x ? launch<true, kPlain>(p, wpb, blocks, s) : launch<false, kPlain>(p, wpb, blocks, s);
 }
 
-int clip_blocks_lean(int exact, int wpb, int device) {
+int clip_blocks_lean(int form, int wpb, int device) {
     using namespace cliplean;
-    return exact ? blocks_for<true, false>(wpb, device) : blocks_for<false, false>(wpb, device);
+    const bool x = form & kFormExact;
+    switch (form & 3) {
+        case kFormCareful: return x ? blocks_for<true, kCareful>(wpb, device) : blocks_for<false, kCareful>(wpb, device);
+        case kFormDense: return x ? blocks_for<true, kDense>(wpb, device) : blocks_for<false, kDense>(wpb, device);
+        default: return x ? blocks_for<true, kPlain>(wpb, device) : blocks_for<false, kPlain>(wpb, device);
+    }
 }
 
 }  // namespace tess

@@ -317,6 +317,7 @@ struct ClipParams {
     unsigned int* list_cap_count;
     uint32_t* list_dense;         // lean first pass: cells of crowded bins, or null
     unsigned int* list_dense_count;
+    unsigned int* flag_count;     // careful pass over every cell: cells with an undecided FP32 test
     unsigned int* fail_count;     // cells left with an error status
     unsigned int* reasons;        // per status code: cells routed or failed for it
     unsigned long long* work_ctr; // optional work counters (tested, cuts, new vertices, windows, batches)
@@ -344,30 +345,24 @@ struct ClipParams {
     uint64_t nbins;
 };
 
-// Forms of the clipping kernel:
-//   kFormLean    the FP32 first pass (tess_clip_lean.cu: 64 slots, a candidate
-//                plane per lane);
-//   kFormStd     the re-run passes and the plain FP64 form, with the window
-//                pre-test (cells next to dense clusters test hundreds of
-//                candidates);
-//   kFormHybrid  FP32, 2 slots per lane, with the pre-test, for cells the
-//                first pass flagged: a plane test in the guard band is
-//                decided in FP64 for the vertices concerned (each recomputed
-//                from its three planes) instead of re-running the cell.
-//   kFormExact   a flag on the FP32 forms: the finalize refines every vertex
-//                with a second FP64-residual Newton step and accumulates face
-//                areas and the volume in FP64 (FP64-accurate results)
-enum ClipForm : int { kFormLean = 0, kFormStd = 1, kFormHybrid = 2, kFormExact = 4 };
-cudaError_t launch_clip_f32(const ClipParams& p, int slots, int form, int wpb, int blocks, cudaStream_t s);
-cudaError_t launch_clip_lean(const ClipParams& p, int exact, int wpb, int blocks, cudaStream_t s);
-int clip_blocks_lean(int exact, int wpb, int device);
-cudaError_t launch_clip_f64(const ClipParams& p, int slots, int form, int wpb, int blocks, cudaStream_t s);
-int clip_blocks_f32(int slots, int form, int wpb, int device);
-int clip_blocks_f64(int slots, int form, int wpb, int device);
-// precision: 0 FP64, 1 FP32.  slots: 2, 4 or 8.
-cudaError_t launch_clip(const ClipParams& p, int precision, int slots, int form, int warps_per_block,
-                        int blocks, cudaStream_t s);
-int clip_blocks_for(int precision, int slots, int form, int warps_per_block, int device);
+// Forms of the clipping:
+//   kFormLean     the FP32 first pass (tess_clip_lean.cu: 64 slots, a candidate
+//                 plane per lane);
+//   kFormDense    the same over the cells of crowded bins, seeded;
+//   kFormCareful  the same over the cells those hand on (and over every cell of
+//                 a small input), with undecided plane tests settled in FP64;
+//   kFormStd      FP64 clipping (tess_clip_f64.cu), for what neither settles
+//                 and for single cells;
+//   kFormExact    a flag on the first three: faces, vertices, areas and volume
+//                 computed in FP64 (the MIXED and FP64 forms)
+enum ClipForm : int { kFormLean = 0, kFormStd = 1, kFormDense = 2, kFormCareful = 3, kFormExact = 4 };
+cudaError_t launch_clip_lean(const ClipParams& p, int form, int wpb, int blocks, cudaStream_t s);
+int clip_blocks_lean(int form, int wpb, int device);
+cudaError_t launch_clip_f64(const ClipParams& p, int slots, int wpb, int blocks, cudaStream_t s);
+int clip_blocks_f64(int slots, int wpb, int device);
+// slots (kFormStd): vertex slots per lane, 4 or 8.
+cudaError_t launch_clip(const ClipParams& p, int slots, int form, int warps_per_block, int blocks, cudaStream_t s);
+int clip_blocks_for(int slots, int form, int warps_per_block, int device);
 // CSR offsets (3 launches) and the gather into them (1 launch).
 cudaError_t launch_csr_offsets(const uint32_t* nface, uint32_t n, uint64_t* offs, uint64_t* scan_tmp,
                                cudaStream_t s);
