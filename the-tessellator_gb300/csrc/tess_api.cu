@@ -114,7 +114,9 @@ int64_t cells_per_dim(uint64_t n, double density) {
 enum { L_DENSE = 0, L_CARE = 1, L_FULL = 2, L_CAP64 = 3, L_COUNT = 4 };
 // d_counters: pass cursors, then list lengths and counts, then the cells each
 // status code was given to, in the FP32 and in the FP64 passes.
-enum { C_CURSOR = 0, C_LIST = 16, C_FAIL = 20, C_FLAG = 21, C_DENSE = 22, C_REASON32 = 32, C_REASON64 = 40, C_TOTAL = 48 };
+enum { C_CURSOR = 0, C_LIST = 16, C_FAIL = 20, C_FLAG = 21, C_DENSE = 22, C_REASON32 = 32, C_REASON64 = 40,
+       C_TOTAL = 48,      // cleared for each compute, with the face cursor behind it ...
+       C_FACES = 48, C_ERR = 50, C_BYTES = 208 };   // ... and the binning's error flag, read back together
 // Up to this many cells the careful pass runs over all of them: an input this
 // small is one wave of warps, whose time is a cell's latency, and a second
 // pass over a few cells would add its own.
@@ -160,7 +162,7 @@ struct Engine {
     float4* d_plo = nullptr;
     uint32_t* d_sgroup = nullptr;
     TabEntry* d_table = nullptr;
-    int* d_err = nullptr;
+    int* d_err = nullptr;       // in d_counters
     int* d_check = nullptr;     // checked build: out-of-range index sites (CheckSite bits)
     bool inv_valid = false;     // d_inv matches the current binning
     // results
@@ -176,7 +178,12 @@ struct Engine {
     bool pool_fixed = false;
     bool faces_on_host = false;
     uint64_t pool_need = 0;
-    unsigned long long* d_fcursor = nullptr;
+    unsigned long long* d_fcursor = nullptr;   // in d_counters
+    // what the host reads back: mapped pinned memory that kernels write (a
+    // 16-byte aligned block of C_BYTES, and the bounds' error flag behind it)
+    unsigned* h_ret = nullptr;
+    unsigned* d_ret = nullptr;
+    cudaEvent_t ev_bounds = nullptr;
     uint32_t* d_list[L_COUNT] = {};
     unsigned* d_counters = nullptr;   // C_* above
     unsigned long long* d_work = nullptr;  // work counters (TESS_FLAG_COUNTERS)
@@ -272,8 +279,10 @@ struct Engine {
         dfree(d_xyz); dfree(d_groups); dfree(d_desc); dfree(d_chunk_diag); dfree(d_chunk_start);
         dfree(d_bounds); dfree(d_bin); dfree(d_rank); dfree(d_delims); dfree(d_scan_tmp);
         dfree(d_sorted); dfree(d_inv); dfree(d_spx); dfree(d_spy); dfree(d_spz); dfree(d_phi); dfree(d_plo); dfree(d_sgroup);
-        dfree(d_table); dfree(d_err); dfree(d_check); dfree(d_vol); dfree(d_nface); dfree(d_fstart); dfree(d_status);
-        dfree(d_fnbr); dfree(d_farea); dfree(d_fcursor);
+        dfree(d_table); dfree(d_check); dfree(d_vol); dfree(d_nface); dfree(d_fstart); dfree(d_status);
+        dfree(d_fnbr); dfree(d_farea);
+        if (h_ret) cudaFreeHost(h_ret);
+        h_ret = nullptr;
         for (auto& l : d_list) dfree(l);
         dfree(d_counters); dfree(d_work); dfree(d_offs); dfree(d_cnbr); dfree(d_carea); dfree(d_csr_tmp);
         dfree(d_geo); dfree(d_one);
@@ -285,8 +294,9 @@ struct Engine {
         if (side) cudaStreamDestroy(side);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
+        if (ev_bounds) cudaEventDestroy(ev_bounds);
         side = nullptr;
-        ev_fork = ev_join = nullptr;
+        ev_fork = ev_join = ev_bounds = nullptr;
     }
 
     int blocks(int slots, int form) {
@@ -387,6 +397,9 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     CU(cudaStreamCreateWithFlags(&E.side, cudaStreamNonBlocking));
     CU(cudaEventCreateWithFlags(&E.ev_fork, cudaEventDisableTiming));
     CU(cudaEventCreateWithFlags(&E.ev_join, cudaEventDisableTiming));
+    CU(cudaEventCreateWithFlags(&E.ev_bounds, cudaEventDisableTiming));
+    CU(cudaHostAlloc((void**)&E.h_ret, 256, cudaHostAllocMapped));
+    CU(cudaHostGetDevicePointer((void**)&E.d_ret, E.h_ret, 0));
     E.ndiag = diags.size();
     uint64_t total = 0, bins = 0, tab = 0;
     std::vector<uint32_t> cdiag, cstart;
@@ -436,7 +449,6 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     TRY(dalloc(&E.d_plo, n));
     TRY(dalloc(&E.d_table, E.table_total));
     E.table_alloc = E.table_total;
-    TRY(dalloc(&E.d_err, 1));
     TRY(dalloc(&E.d_check, 1));
     CU(cudaMemsetAsync(E.d_check, 0, sizeof(int), E.stream));
     TRY(dalloc(&E.d_vol, n));
@@ -446,9 +458,10 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     E.face_cap = (E.cfg.flags & TESS_FLAG_SMALL_FACE_POOL) ? 1024 : (uint64_t)n * 20 + 4096;
     TRY(dalloc(&E.d_fnbr, E.face_cap));
     TRY(dalloc(&E.d_farea, E.face_cap));
-    TRY(dalloc(&E.d_fcursor, 1));
     for (auto& l : E.d_list) TRY(dalloc(&l, n));
-    TRY(dalloc(&E.d_counters, C_TOTAL));
+    TRY(dalloc(&E.d_counters, C_BYTES / sizeof(unsigned)));
+    E.d_fcursor = reinterpret_cast<unsigned long long*>(E.d_counters + C_FACES);
+    E.d_err = reinterpret_cast<int*>(E.d_counters + C_ERR);
     TRY(dalloc(&E.d_work, 8));
     TRY(dalloc(&E.d_offs, n + 1));
     TRY(dalloc(&E.d_csr_tmp, csr_tmp_words(E.total)));
@@ -484,6 +497,7 @@ GridBuffers grid_buffers(Engine& E) {
     g.table = E.d_table;
     g.table_gaps = E.cfg.table_gaps;
     g.error_flag = E.d_err;
+    g.host_flag = reinterpret_cast<int*>(E.d_ret + C_BYTES / sizeof(unsigned));
     g.check = E.d_check;
     return g;
 }
@@ -557,7 +571,10 @@ static tess_status copy_async(Engine& E, void* dst, const void* src, size_t n) {
     return TESS_OK;
 }
 
-tess_status engine_build(Engine& E, bool check) {
+// src: device memory to take the points from, or null (they are in d_xyz).
+// With check, returns once the input is read and found finite; the rest of the
+// pass is on the stream.
+tess_status engine_build(Engine& E, bool check, const double* src = nullptr) {
     CU(cudaSetDevice(E.device));
     TimingEvents ev;
     const bool timing = E.cfg.flags & TESS_FLAG_TIMING;
@@ -565,21 +582,20 @@ tess_status engine_build(Engine& E, bool check) {
         CU(ev.create(2));
         CU(cudaEventRecord(ev.e[0], E.stream));
     }
-    CU(launch_grid_build(grid_buffers(E), E.stream, E.side, E.ev_fork, E.ev_join));
+    GridBuffers gb = grid_buffers(E);
+    gb.src = src;
+    CU(launch_grid_build(gb, E.stream, E.side, E.ev_fork, E.ev_join, check ? E.ev_bounds : nullptr));
     E.launches += grid_launches(E.total_bins);
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     if (check) {
-        int err = 0;
-        CU(cudaMemcpyAsync(&err, E.d_err, sizeof(int), cudaMemcpyDeviceToHost, E.stream));
-        CU(cudaStreamSynchronize(E.stream));
-        if (err) {
+        CU(cudaEventSynchronize(E.ev_bounds));
+        if (*reinterpret_cast<volatile int*>(E.h_ret + C_BYTES / sizeof(unsigned))) {
             // the grid describes the bad points: nothing may use it until a
             // build succeeds
             E.built = false;
             E.computed = false;
             E.csr_valid = false;
-            if (err == 1) return fail(TESS_E_INVALID, "input coordinates must be finite");
-            return fail(TESS_E_CUDA, "shell table exceeded its capacity");
+            return fail(TESS_E_INVALID, "input coordinates must be finite");
         }
     }
     if (timing) {
@@ -637,8 +653,7 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
                            cudaEvent_t* ev, const uint32_t* sample = nullptr, uint32_t nsample = 0) {
     unsigned* cur = E.d_counters;
     unsigned* cnt = E.d_counters + C_LIST;
-    CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * C_TOTAL, E.stream));
-    CU(cudaMemsetAsync(E.d_fcursor, 0, sizeof(unsigned long long), E.stream));
+    CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * C_TOTAL + sizeof(unsigned long long), E.stream));
     if (E.cfg.flags & TESS_FLAG_COUNTERS) CU(cudaMemsetAsync(E.d_work, 0, sizeof(unsigned long long) * 8, E.stream));
     ClipParams base = base_params(E);
     base.search_radius = radius;
@@ -704,6 +719,19 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
     return TESS_OK;
 }
 
+// Waits for the compute on the stream and reads its counters, face count and
+// the binning's error flag back: one small copy by a kernel into mapped memory.
+tess_status read_back(Engine& E, const unsigned** counts, unsigned long long* faces, int* err) {
+    if (!E.sm_count) CU(cudaDeviceGetAttribute(&E.sm_count, cudaDevAttrMultiProcessorCount, E.device));
+    CU(launch_copy_bytes(E.d_ret, E.d_counters, C_BYTES, E.sm_count, E.stream));
+    E.launches += 1;
+    CU(cudaStreamSynchronize(E.stream));
+    *counts = E.h_ret;
+    memcpy(faces, E.h_ret + C_FACES, sizeof(*faces));
+    memcpy(err, E.h_ret + C_ERR, sizeof(*err));
+    return TESS_OK;
+}
+
 // The statistics of a finished compute from its counters.
 void read_counts(Engine& E, const unsigned* c, uint64_t faces) {
     const unsigned *r32 = c + C_REASON32, *r64 = c + C_REASON64;
@@ -736,12 +764,10 @@ tess_status engine_compute(Engine& E, int precision, double radius, int64_t grou
     for (int attempt = 0; attempt < 4; ++attempt) {
         TRY(enqueue_passes(E, precision, radius, group, timing, ev.e));
         unsigned long long used = 0;
-        unsigned counts[C_TOTAL];
+        const unsigned* counts = nullptr;
         int gerr = 0;
-        CU(cudaMemcpyAsync(&used, E.d_fcursor, sizeof(used), cudaMemcpyDeviceToHost, E.stream));
-        CU(cudaMemcpyAsync(counts, E.d_counters, sizeof(counts), cudaMemcpyDeviceToHost, E.stream));
-        CU(cudaMemcpyAsync(&gerr, E.d_err, sizeof(int), cudaMemcpyDeviceToHost, E.stream));
-        CU(cudaStreamSynchronize(E.stream));
+        TRY(read_back(E, &counts, &used, &gerr));
+        if (gerr == 2) return fail(TESS_E_CUDA, "shell table exceeded its capacity");
         if (gerr == 1) {
             // the device points were rebuilt without a check and hold a
             // non-finite coordinate: the clipping kernels did nothing
@@ -765,11 +791,6 @@ tess_status engine_compute(Engine& E, int precision, double radius, int64_t grou
             continue;
         }
         read_counts(E, counts, used);
-        if (E.ndiag == 1) {
-            DiagDesc dd;
-            CU(cudaMemcpy(&dd, E.d_desc, sizeof(DiagDesc), cudaMemcpyDeviceToHost));
-            E.stats.table_entries = dd.tab_len;
-        }
         if (timing) {
             E.stats.ms_clip = ev.ms(0, 1);
             E.stats.ms_rerun = ev.ms(1, 2);
@@ -806,12 +827,10 @@ tess_status engine_csr(Engine& E) {
     TimingEvents ev;
     const bool timing = E.cfg.flags & TESS_FLAG_TIMING;
     if (timing) CU(ev.create(2));
-    // offsets first (to size the outputs), then the gather
     if (timing) CU(cudaEventRecord(ev.e[0], E.stream));
     CU(launch_csr_offsets(E.d_nface, E.total, E.d_offs, E.d_csr_tmp, E.stream));
-    uint64_t total = 0;
-    CU(cudaMemcpyAsync(&total, E.d_offs + E.total, sizeof(uint64_t), cudaMemcpyDeviceToHost, E.stream));
-    CU(cudaStreamSynchronize(E.stream));
+    // every face of the pool belongs to one cell: their number is the last offset
+    const uint64_t total = E.stats.faces;
     if (total > E.csr_cap || !E.d_cnbr) {
         dfree(E.d_cnbr);
         dfree(E.d_carea);
@@ -821,7 +840,7 @@ tess_status engine_csr(Engine& E) {
     }
     CU(launch_csr_gather(E.d_nface, E.d_fstart, E.d_fnbr, E.d_farea, E.total, E.d_offs, E.d_cnbr, E.d_carea,
                          E.stream));
-    E.launches += 4;
+    E.launches += csr_offset_launches(E.total) + 1;
     if (timing) {
         CU(cudaEventRecord(ev.e[1], E.stream));
         CU(cudaEventSynchronize(ev.e[1]));
@@ -1402,6 +1421,8 @@ static tess_status create_common(const double* xyz, bool on_device, size_t n, co
     std::vector<DiagDesc> v{D};
     tess_status st = engine_init(h->E, cfg, v, xyz, on_device, groups);
     if (st == TESS_OK) st = engine_build(h->E, true);
+    // the copies of the caller's and of local buffers have ended
+    if (st == TESS_OK && cudaStreamSynchronize(h->E.stream) != cudaSuccess) st = fail(TESS_E_CUDA, "building the grid");
     if (st != TESS_OK) {
         delete h;
         return st;
@@ -1520,6 +1541,13 @@ tess_status tess_host_free(void* ptr) {
 tess_status tess_diagram_stats(const tess_diagram* d, tess_stats* out) {
     if (!d || !out) return fail(TESS_E_INVALID, "NULL argument");
     *out = d->E.stats;
+    if (d->E.stats.cells) {     // the shell table's length of the last binning
+        DiagDesc D;
+        CU(cudaSetDevice(d->E.device));
+        CU(cudaStreamSynchronize(d->E.stream));
+        CU(cudaMemcpy(&D, d->E.d_desc, sizeof(D), cudaMemcpyDeviceToHost));
+        out->table_entries = D.tab_len;
+    }
     out->launches = d->E.launches;
     return TESS_OK;
 }
@@ -1528,6 +1556,12 @@ tess_status tess_diagram_update_points(tess_diagram* d, const double* xyz, int o
     if (!d || !xyz) return fail(TESS_E_INVALID, "NULL argument");
     Engine& E = d->E;
     CU(cudaSetDevice(E.device));
+    // points in this device's memory are copied by the bounds kernel, which
+    // reads them all anyway
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, xyz) != cudaSuccess) cudaGetLastError();
+    else if (a.type == cudaMemoryTypeDevice && a.device == E.device && !(reinterpret_cast<uintptr_t>(xyz) & 7u))
+        return engine_build(E, true, xyz);
     TRY(copy_async(E, E.d_xyz, xyz, sizeof(double) * 3 * (size_t)E.total));
     return engine_build(E, true);
 }
@@ -1537,6 +1571,7 @@ tess_status tess_diagram_celery(const tess_diagram* d, uint32_t* cells, uint32_t
     if (!d) return fail(TESS_E_INVALID, "diagram is NULL");
     const Engine& E = d->E;
     CU(cudaSetDevice(E.device));
+    CU(cudaStreamSynchronize(E.stream));   // the binning may still run
     if (cells) CU(cudaMemcpy(cells, E.d_bin, sizeof(uint32_t) * E.total, cudaMemcpyDeviceToHost));
     if (sorted_indices) CU(cudaMemcpy(sorted_indices, E.d_sorted, sizeof(uint32_t) * E.total, cudaMemcpyDeviceToHost));
     if (delimiters)
@@ -1548,6 +1583,7 @@ tess_status tess_diagram_grid(const tess_diagram* d, int64_t* cpd, double bounds
     if (!d) return fail(TESS_E_INVALID, "diagram is NULL");
     DiagDesc D;
     CU(cudaSetDevice(d->E.device));
+    CU(cudaStreamSynchronize(d->E.stream));   // the binning may still run
     CU(cudaMemcpy(&D, d->E.d_desc, sizeof(D), cudaMemcpyDeviceToHost));
     if (cpd) *cpd = D.cpd;
     if (bounds)
@@ -1729,10 +1765,19 @@ tess_status tess_neighbors_csr(tess_diagram* d, uint64_t* offs, int32_t* nbr, do
     return csr_out(d->E, offs, nbr, area, cap, total);
 }
 
+// Results handed out as device pointers: on the library's own stream, which the
+// caller cannot order against, they are complete; on the caller's stream they
+// are in its order.
+static tess_status results_ready(Engine& E) {
+    if (E.own_stream) CU(cudaStreamSynchronize(E.stream));
+    return TESS_OK;
+}
+
 tess_status tess_results_device(tess_diagram* d, const double** volumes, const uint64_t** offs,
                                 const int32_t** nbr, const double** area, size_t* total) {
     if (!d) return fail(TESS_E_INVALID, "diagram is NULL");
     TRY(engine_csr(d->E));
+    TRY(results_ready(d->E));
     if (volumes) *volumes = d->E.d_vol;
     if (offs) *offs = d->E.d_offs;
     if (nbr) *nbr = d->E.d_cnbr;
@@ -1796,6 +1841,8 @@ tess_status tess_batch_create(size_t ndiag, const uint64_t* pt_offsets, const do
     if (!h) return fail(TESS_E_NOMEM, "host allocation failed");
     tess_status st = engine_init(h->E, cfg, v, xyz, false, nullptr);
     if (st == TESS_OK) st = engine_build(h->E, true);
+    // the copies of the caller's and of local buffers have ended
+    if (st == TESS_OK && cudaStreamSynchronize(h->E.stream) != cudaSuccess) st = fail(TESS_E_CUDA, "building the grid");
     if (st != TESS_OK) {
         delete h;
         return st;
@@ -1855,12 +1902,9 @@ static tess_status batch_run(tess_batch* b, int prec) {
     E.launches += grid_launches(E.total_bins) + (E.total <= kCarefulMax ? 3 : 5) - (E.cfg.slots_per_lane >= 8 ? 1 : 0);
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     unsigned long long used = 0;
-    unsigned counts[C_TOTAL];
+    const unsigned* counts = nullptr;
     int gerr = 0;
-    CU(cudaMemcpyAsync(&used, E.d_fcursor, sizeof(used), cudaMemcpyDeviceToHost, E.stream));
-    CU(cudaMemcpyAsync(counts, E.d_counters, sizeof(counts), cudaMemcpyDeviceToHost, E.stream));
-    CU(cudaMemcpyAsync(&gerr, E.d_err, sizeof(int), cudaMemcpyDeviceToHost, E.stream));
-    CU(cudaStreamSynchronize(E.stream));
+    TRY(read_back(E, &counts, &used, &gerr));
     TRY(check_word(E));
     if (timing) E.stats.ms_clip = ev.ms(0, 1);
     if (gerr == 1) {
@@ -1987,6 +2031,7 @@ tess_status tess_batch_results_device(tess_batch* b, const double** volumes, con
                                       const int32_t** nbr, const double** area, size_t* total) {
     if (!b) return fail(TESS_E_INVALID, "batch is NULL");
     TRY(engine_csr(b->E));
+    TRY(results_ready(b->E));
     if (volumes) *volumes = b->E.d_vol;
     if (offs) *offs = b->E.d_offs;
     if (nbr) *nbr = b->E.d_cnbr;

@@ -86,21 +86,52 @@ __global__ void __launch_bounds__(kCsrThreads) k_csr_final(const uint32_t* cnt, 
     if (blockIdx.x == 0 && threadIdx.x == 0) offs[n] = sums[gridDim.x];
 }
 
-// One warp per 32 consecutive cells: their CSR range is contiguous, so the
+// The whole scan by one block, for few cells: one launch in place of three.
+constexpr uint32_t kCsrOneMax = 16384;
+__global__ void __launch_bounds__(kCsrThreads) k_csr_one(const uint32_t* cnt, uint32_t n, uint64_t* offs) {
+    __shared__ unsigned long long sh[33];
+    __shared__ unsigned long long tot;
+    unsigned long long carry = 0;
+    for (uint32_t b0 = 0; b0 < n; b0 += kCsrThreads * kCsrItems) {
+        const uint32_t base = b0 + threadIdx.x * kCsrItems;
+        uint32_t v[kCsrItems];
+        unsigned long long s = 0;
+        for (int k = 0; k < kCsrItems; ++k) {
+            v[k] = base + k < n ? cnt[base + k] : 0u;
+            s += v[k];
+        }
+        const unsigned long long ex = block_excl_scan64(s, sh);
+        if (threadIdx.x == kCsrThreads - 1) tot = ex + s;
+        unsigned long long run = carry + ex;
+        for (int k = 0; k < kCsrItems; ++k) {
+            if (base + k < n) offs[base + k] = run;
+            run += v[k];
+        }
+        __syncthreads();
+        carry += tot;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) offs[n] = carry;
+}
+
+// One warp per C consecutive cells: their CSR range is contiguous, so the
 // warp writes it as one coalesced stream; each output element finds its cell
 // (lane) by a binary search over the warp's prefix sums of the face counts
-// and reads from that cell's contiguous run in the face pool.
+// and reads from that cell's contiguous run in the face pool.  C = 32 where
+// that fills the GPU; small inputs take C = 4 (1,000 cells: 4 blocks of 16 us
+// with 32 a warp).
+template <int C>
 __global__ void __launch_bounds__(256) k_csr_gather(const uint32_t* cnt, const uint64_t* fstart,
                                                     const int32_t* fnbr, const double* farea, uint32_t n,
                                                     const uint64_t* offs, int32_t* nbr, double* area) {
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const uint64_t c0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull;
+    const uint64_t c0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * C;
     if (c0 >= n) return;                          // whole warps leave together
     const uint64_t i = c0 + lane;
     uint32_t c = 0;
     uint64_t src = 0;
-    if (i < n) {
+    if (lane < C && i < n) {
         c = cnt[i];
         src = fstart[i];
     }
@@ -117,7 +148,7 @@ __global__ void __launch_bounds__(256) k_csr_gather(const uint32_t* cnt, const u
         const uint32_t t = o + lane;
         int L = 0;
 #pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
+        for (int step = C / 2; step > 0; step >>= 1) {
             const uint32_t v = __shfl_sync(kFull, incl, L + step - 1);
             if (v <= t) L += step;
         }
@@ -143,6 +174,12 @@ int clip_blocks_for(int slots, int form, int wpb, int device) {
     return clip_blocks_f64(slots, wpb, device);
 }
 
+// From this many cells a warp of the gather takes 32 (38,912 warps fill the GPU's
+// 152 x 64 four times over), below it 4.
+constexpr uint32_t kCsrWide = 262144;
+
+uint64_t csr_offset_launches(uint32_t n) { return n <= kCsrOneMax ? 1 : 3; }
+
 size_t csr_tmp_words(uint32_t n) {
     const uint64_t per = (uint64_t)kCsrThreads * kCsrItems;
     return (size_t)((n + per - 1) / per) + 2;
@@ -150,6 +187,10 @@ size_t csr_tmp_words(uint32_t n) {
 
 cudaError_t launch_csr_offsets(const uint32_t* nface, uint32_t n, uint64_t* offs, uint64_t* scan_tmp,
                                cudaStream_t s) {
+    if (n <= kCsrOneMax) {
+        k_csr_one<<<1, kCsrThreads, 0, s>>>(nface, n, offs);
+        return cudaGetLastError();
+    }
     const uint64_t per = (uint64_t)kCsrThreads * kCsrItems;
     const uint32_t nb = (uint32_t)((n + per - 1) / per);
     unsigned long long* sums = reinterpret_cast<unsigned long long*>(scan_tmp);
@@ -162,7 +203,12 @@ cudaError_t launch_csr_offsets(const uint32_t* nface, uint32_t n, uint64_t* offs
 cudaError_t launch_csr_gather(const uint32_t* nface, const uint64_t* fstart, const int32_t* face_nbr,
                               const double* face_area, uint32_t n, const uint64_t* offs, int32_t* nbr_out,
                               double* area_out, cudaStream_t s) {
-    k_csr_gather<<<(n + 255) / 256, 256, 0, s>>>(nface, fstart, face_nbr, face_area, n, offs, nbr_out, area_out);
+    const uint64_t warps = n >= kCsrWide ? ((uint64_t)n + 31) / 32 : ((uint64_t)n + 3) / 4;
+    const unsigned blocks = (unsigned)((warps + 7) / 8);
+    if (n >= kCsrWide)
+        k_csr_gather<32><<<blocks, 256, 0, s>>>(nface, fstart, face_nbr, face_area, n, offs, nbr_out, area_out);
+    else
+        k_csr_gather<4><<<blocks, 256, 0, s>>>(nface, fstart, face_nbr, face_area, n, offs, nbr_out, area_out);
     return cudaGetLastError();
 }
 

@@ -41,9 +41,12 @@ __global__ void __launch_bounds__(kBoundsThreads) k_bounds(GridBuffers g) {
         unsigned long long mn[3] = {~0ull, ~0ull, ~0ull};
         unsigned long long mx[3] = {0ull, 0ull, 0ull};
         bool bad = false;
+        const double* const in = g.src ? g.src : g.xyz;
         for (uint32_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
             for (int a = 0; a < 3; ++a) {
-                const unsigned long long b = (unsigned long long)__double_as_longlong(g.xyz[3ull * i + a]);
+                const double v = in[3ull * i + a];
+                if (g.src) g.xyz[3ull * i + a] = v;
+                const unsigned long long b = (unsigned long long)__double_as_longlong(v);
                 bad |= ((b >> 52) & 0x7FFull) == 0x7FFull;
                 const unsigned long long e = (b >> 63) ? ~b : (b | 0x8000000000000000ull);
                 mn[a] = min(mn[a], e);
@@ -139,6 +142,7 @@ __global__ void __launch_bounds__(128) k_grid_params(GridBuffers g) {
     unsigned long long m = size > 0.0 ? (unsigned long long)__double_as_longlong(size) : ~0ull;
     m = min(m, __shfl_xor_sync(0xffffffffu, m, 1));
     m = min(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    if (t == 0 && g.host_flag) *g.host_flag = *g.error_flag;
     if (!mine) return;
     D.glo[a] = lo;
     D.ghi[a] = hi;
@@ -683,13 +687,14 @@ uint64_t grid_launches(uint64_t total_bins) { return total_bins + 1 <= kScanOneM
 // scan -> scatter -> within-bin order -> gather.  A fixed launch sequence
 // (no host synchronisation), so it can be captured in a CUDA graph.
 cudaError_t launch_grid_build(const GridBuffers& g, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
-                              cudaEvent_t join) {
+                              cudaEvent_t join, cudaEvent_t bounds_done) {
     const int ndiag = g.ndiag;
     const uint64_t nclear = std::max<uint64_t>(6ull * ndiag, g.total_bins + 1);
     k_grid_clear<<<(unsigned)std::min<uint64_t>((nclear + 1023) / 1024, 152u * 8u), 256, 0, s>>>(g);
     const int cblocks = (int)(g.nchunks < 4096u ? g.nchunks : 4096u);
     k_bounds<<<cblocks, kBoundsThreads, 0, s>>>(g);
     k_grid_params<<<(4 * ndiag + 127) / 128, 128, 0, s>>>(g);
+    if (bounds_done) cudaEventRecord(bounds_done, s);
     // the shell tables need only the grid parameters: build them beside the
     // histogram, scan and scatter when a side stream is given
     const bool forked = side && fork && join;

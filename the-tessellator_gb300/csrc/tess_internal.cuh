@@ -160,7 +160,8 @@ __device__ __forceinline__ double gap_key(const double size[3], int i, int j, in
 
 // ---- launchers (tess_grid.cu) ----
 struct GridBuffers {
-    const double* xyz;          // concatenated points, AoS
+    double* xyz;                // concatenated points, AoS
+    const double* src;          // device memory to take the points from (copied to xyz on the way), or null
     const uint32_t* groups;     // point groups or null
     DiagDesc* diags;
     int ndiag;
@@ -187,6 +188,7 @@ struct GridBuffers {
     TabEntry* table;
     int table_gaps;
     int* error_flag;            // set when an input coordinate is not finite
+    int* host_flag;             // its value after the bounds, in mapped host memory, or null
     int* check;                 // checked build: the check word
 };
 // Points per block of the bounds and histogram kernels: 2,048 keep small inputs
@@ -198,8 +200,11 @@ constexpr int kScanThreads = 1024;
 // side/fork/join (optional): a second stream and two events; the shell
 // table is then built on the side stream while the histogram, scan and
 // scatter run (fork after the grid parameters, join before returning).
+// bounds_done (optional) is recorded when the input is read and host_flag is
+// written.
 cudaError_t launch_grid_build(const GridBuffers& g, cudaStream_t s, cudaStream_t side = nullptr,
-                              cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
+                              cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr,
+                              cudaEvent_t bounds_done = nullptr);
 // Kernels launched by one binning pass.
 uint64_t grid_launches(uint64_t total_bins);
 // inv[sorted[s]] = s for s < n (the point -> sorted position map, on demand).
@@ -370,6 +375,7 @@ cudaError_t launch_csr_gather(const uint32_t* nface, const uint64_t* fstart, con
                               const double* face_area, uint32_t n, const uint64_t* offs, int32_t* nbr_out,
                               double* area_out, cudaStream_t s);
 size_t csr_tmp_words(uint32_t n);
+uint64_t csr_offset_launches(uint32_t n);   // kernels of launch_csr_offsets
 
 // Sets the calling thread's last error message (printf format).
 void set_error(const char* fmt, ...);
