@@ -41,7 +41,7 @@ def _clustered(n):
 
 SETS = {
     **{f"uniform_{n}": (lambda n=n: _rng(n).random((n, 3)), (1, 1, 1)) for n in (1, 2, 3, 31, 32, 33, 34, 64, 65, 200)},
-    **{f"uniform_{n}": (lambda n=n: _rng(n).random((n, 3)), (1, 1, 1)) for n in (32768, 32769)},
+    **{f"uniform_{n}": (lambda n=n: _rng(n).random((n, 3)), (1, 1, 1)) for n in (8192, 8193)},
     "clustered_40000": (lambda: _clustered(40_000), (1, 1, 1)),
     "plane_x": (lambda: _flat(_rng(1).random((300, 3)), 0, 0.25), (1, 1, 1)),
     "plane_y": (lambda: _flat(_rng(2).random((300, 3)), 1, 0.5), (1, 1, 1)),
@@ -92,5 +92,5 @@ def test_checked_build():
     """The plain, dense and careful passes through the bounds-checked library."""
     env = dict(os.environ, TESS_LIB=os.path.join(ROOT, "the-tessellator_gb300", "tessellator", "libtessgpu_checked.so"))
     r = subprocess.run([sys.executable, "-m", "pytest", os.path.abspath(__file__), "-q", "-x", "-m", "gpu", "-k",
-                        "uniform_32769 or clustered_40000 or clumps_many"], env=env, cwd=ROOT, capture_output=True, text=True)
+                        "uniform_8193 or clustered_40000 or clumps_many"], env=env, cwd=ROOT, capture_output=True, text=True)
     assert r.returncode == 0 and "passed" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]

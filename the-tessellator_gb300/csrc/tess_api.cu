@@ -117,10 +117,12 @@ enum { L_DENSE = 0, L_CARE = 1, L_FULL = 2, L_CAP64 = 3, L_COUNT = 4 };
 enum { C_CURSOR = 0, C_LIST = 16, C_FAIL = 20, C_FLAG = 21, C_DENSE = 22, C_REASON32 = 32, C_REASON64 = 40,
        C_TOTAL = 48,      // cleared for each compute, with the face cursor behind it ...
        C_FACES = 48, C_ERR = 50, C_BYTES = 208 };   // ... and the binning's error flag, read back together
-// Up to this many cells the careful pass runs over all of them: an input this
-// small is one wave of warps, whose time is a cell's latency, and a second
-// pass over a few cells would add its own.
-constexpr uint32_t kCarefulMax = 32768;
+// Up to this many cells the careful pass runs over all of them: a few waves of
+// warps, whose time is a cell's latency, and a second pass over a few cells
+// would add its own (uniform points, careful alone against plain and careful:
+// 3,000 0.113 / 0.134 ms, 10,000 0.205 / 0.204, 30,000 0.52 / 0.41).  Such
+// inputs have one launch of the FP64 clipping behind it, not two.
+constexpr uint32_t kCarefulMax = 8192;
 // The FP64 form's first pass runs in FP32 (tess_clip_lean.cu): a vertex whose
 // distance from a plane is within the FP32 error bound plus this is left to
 // the FP64 clipping, so that every decision the FP32 pass takes is the one the
@@ -404,13 +406,14 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     uint64_t total = 0, bins = 0, tab = 0;
     std::vector<uint32_t> cdiag, cstart;
     TRY(layout_grid(diags, E.cfg.bin_density, E.cfg.table_gaps, &bins, &tab));
+    for (const DiagDesc& D : diags) total += D.n;
+    const uint32_t chunk = chunk_points(total);
     for (size_t d = 0; d < diags.size(); ++d) {
         const DiagDesc& D = diags[d];
-        for (uint32_t s = 0; s < D.n; s += kChunk) {
+        for (uint64_t s = 0; s < D.n; s += chunk) {
             cdiag.push_back((uint32_t)d);
-            cstart.push_back(D.pt_base + s);
+            cstart.push_back(D.pt_base + (uint32_t)s);
         }
-        total += D.n;
     }
     if (total >= 0xFFFFFFF0ull) return fail(TESS_E_INVALID, "too many points (%llu)", (unsigned long long)total);
     E.total = (uint32_t)total;
@@ -434,7 +437,7 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     TRY(dalloc(&E.d_chunk_start, E.nchunks));
     CU(cudaMemcpyAsync(E.d_chunk_diag, cdiag.data(), sizeof(uint32_t) * E.nchunks, cudaMemcpyHostToDevice, E.stream));
     CU(cudaMemcpyAsync(E.d_chunk_start, cstart.data(), sizeof(uint32_t) * E.nchunks, cudaMemcpyHostToDevice, E.stream));
-    TRY(dalloc(&E.d_bounds, 6 * E.ndiag));
+    TRY(dalloc(&E.d_bounds, 6 * E.ndiag + 1));
     TRY(dalloc(&E.d_bin, n));
     TRY(dalloc(&E.d_rank, n));
     TRY(dalloc(&E.d_delims, E.total_bins + 1));
@@ -482,6 +485,8 @@ GridBuffers grid_buffers(Engine& E) {
     g.chunk_start = E.d_chunk_start;
     g.nchunks = E.nchunks;
     g.bounds = E.d_bounds;
+    g.tickets = reinterpret_cast<unsigned*>(E.d_bounds + 6 * E.ndiag);
+    g.chunk = chunk_points(E.total);
     g.bin = E.d_bin;
     g.rank = E.d_rank;
     g.delims = E.d_delims;
@@ -585,7 +590,7 @@ tess_status engine_build(Engine& E, bool check, const double* src = nullptr) {
     GridBuffers gb = grid_buffers(E);
     gb.src = src;
     CU(launch_grid_build(gb, E.stream, E.side, E.ev_fork, E.ev_join, check ? E.ev_bounds : nullptr));
-    E.launches += grid_launches(E.total_bins);
+    E.launches += grid_launches(E.total_bins, E.ndiag);
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     if (check) {
         CU(cudaEventSynchronize(E.ev_bounds));
@@ -709,7 +714,7 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
         TRY(pass(1, 2, kFormDense | X, L[L_DENSE], cnt + L_DENSE, L[L_CARE], cnt + L_CARE, lcap, cnt + L_FULL));
         TRY(pass(1, 2, kFormCareful | X, L[L_CARE], cnt + L_CARE, L[L_FULL], cnt + L_FULL, lcap, cnt + L_FULL));
     }
-    if (s0 < 8) {
+    if (s0 < 8 && !small) {
         TRY(pass(0, 4, kFormStd, L[L_FULL], cnt + L_FULL, nullptr, nullptr, norerun ? nullptr : L[L_CAP64], cnt + L_CAP64));
         TRY(pass(0, 8, kFormStd, L[L_CAP64], cnt + L_CAP64, nullptr, nullptr, nullptr, nullptr));
     } else {
@@ -1899,7 +1904,7 @@ static tess_status batch_run(tess_batch* b, int prec) {
         CU(cudaEventRecord(ev.e[0], E.stream));
     }
     CU(cudaGraphLaunch(G, E.stream));
-    E.launches += grid_launches(E.total_bins) + (E.total <= kCarefulMax ? 3 : 5) - (E.cfg.slots_per_lane >= 8 ? 1 : 0);
+    E.launches += grid_launches(E.total_bins, E.ndiag) + (E.total <= kCarefulMax ? 2 : (E.cfg.slots_per_lane >= 8 ? 4 : 5)) + 1;
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     unsigned long long used = 0;
     const unsigned* counts = nullptr;

@@ -430,10 +430,10 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
             const float dz = fmaxf((tk > 0 ? 1.f - fz : (tk < 0 ? fz : 0.f)) - feps, 0.f) * D.size_f[2];
             nd = (dx * dx + dy * dy + dz * dz) * (1.0f - 1e-4f);
         }
-        const unsigned crowded = __ballot_sync(FULL, ncnt >= P.seed_min);
-        if (__shfl_sync(FULL, ncnt, 13) >= P.seed_min) pending = crowded;
+        const unsigned many = __ballot_sync(FULL, ncnt >= P.seed_min);
+        if (__shfl_sync(FULL, ncnt, 13) >= P.seed_min) pending = many;
     }
-    const bool seeded = SEED && pending != 0;
+    const bool crowded = SEED && pending != 0;
     uint32_t pend = 0;               // batch 0: where my row's points that were not taken start
     int m = 0, ring0 = 0;            // batch (0, 1, 2) or ring (4 on); first row of a ring's batch
     // bin sides or a cell radius outside FP32's normal range
@@ -614,7 +614,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
             // the radius, of which 22 cut).
             float bl0 = 0.f, bl1 = 0.f, bl2 = 0.f, bh0 = 0.f, bh1 = 0.f, bh2 = 0.f, be = 0.f;
             if constexpr (SEED) {
-                if (!direct) {
+                if (crowded && !direct) {
                     float4 v = S.vtx[lane];
                     bool lv = (l0 >> lane) & 1u;
                     bl0 = bh0 = lv ? v.x : 0.f;      // the site is inside its bounds
@@ -665,7 +665,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                     keep = jp != gs && r2 > dup2 && r2 < lim;
                     near = jp != gs && !(r2 > dup2);
                     if (keep && P.target_group >= 0) keep = (int64_t)(P.sgroup ? P.sgroup[jp] : 0u) == P.target_group;
-                    if constexpr (SEED) keep = keep && reaches(rx, ry, rz, r2);
+                    if constexpr (SEED) keep = keep && (!crowded || reaches(rx, ry, rz, r2));
                 }
                 return heads;
             };
@@ -707,7 +707,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 r2 = own.w;
                 jp = S.candj[lane];
                 // (a seed that cut is a plane already)
-                if (seeded)
+                if (crowded)
 #pragma unroll 1
                     for (int p = 6; p < np; ++p) keep = keep && S.psrc[p] != jp;
                 __syncwarp();
@@ -1283,7 +1283,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
     if constexpr (CAREFUL) {
         // as the first pass, it counts what the plain pass would hand on
         if (lane == 0 && !P.work) {
-            if (seeded) atomicAdd(P.list_dense_count, 1u);
+            if (crowded) atomicAdd(P.list_dense_count, 1u);
             else if (undec || status == ST_GUARD || status == ST_DEGEN || status == ST_VERIFY) atomicAdd(P.flag_count, 1u);
         }
     }

@@ -27,17 +27,105 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
     return v;
 }
 
+// CeleryCellInfo::new (celery.rs:153-181) from the bounds and the host's cpd.
+// Four threads per diagram (t / 4), one per axis and one idle: the FP64
+// divisions of the axes run side by side.  Whole warps.
+__device__ __forceinline__ void grid_params(const GridBuffers& g, int t) {
+    const int d = min(t >> 2, g.ndiag - 1), a = min(t & 3, 2);
+    const bool mine = (t >> 2) < g.ndiag && (t & 3) < 3;
+    DiagDesc& D = g.diags[d];
+    const double c = (double)D.cpd;
+    const double lo = ord_dec(__ldcg(&g.bounds[6 * d + a]));
+    const double hi = ord_dec(__ldcg(&g.bounds[6 * d + 3 + a]));
+    const double half = 0.5 * lo + 0.5 * hi;
+    const double ctr = isfinite(half) ? half : 0.0;
+    const double ext = __dsub_rn(hi, lo);
+    const double size = __ddiv_rn(ext, c), inv = __ddiv_rn(c, ext);
+    const float size_f = __double2float_rn(size), inv_f = __double2float_rn(inv);
+    const bool ok_a = !(ext > 0.0) || (size_f >= FLT_MIN && size_f <= FLT_MAX && inv_f >= FLT_MIN && inv_f <= FLT_MAX);
+    const unsigned quad = (__ballot_sync(0xffffffffu, ok_a) >> (threadIdx.x & 28)) & 7u;
+    // the smallest nonzero bin side, through its order-preserving bits
+    unsigned long long m = size > 0.0 ? (unsigned long long)__double_as_longlong(size) : ~0ull;
+    m = min(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = min(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    if (t == 0 && g.host_flag) *g.host_flag = __ldcg(g.error_flag);
+    if (!mine) return;
+    D.glo[a] = lo;
+    D.ghi[a] = hi;
+    D.ctr[a] = ctr;
+    D.size[a] = size;
+    D.inv[a] = inv;
+    // FP32 forms for the FP32 clipping pass: offsets from the centre as
+    // FP32 pairs (48 bits), the bin sides and their inverses
+    const double gl = lo - ctr, bl = D.blo[a] - ctr, bh = D.bhi[a] - ctr;
+    const float glf = __double2float_rn(gl), blf = __double2float_rn(bl), bhf = __double2float_rn(bh);
+    D.glo_hi[a] = glf;
+    D.glo_lo[a] = __double2float_rn(gl - (double)glf);
+    D.blo_hi[a] = blf;
+    D.blo_lo[a] = __double2float_rn(bl - (double)blf);
+    D.bhi_hi[a] = bhf;
+    D.bhi_lo[a] = __double2float_rn(bh - (double)bhf);
+    D.inv_f[a] = inv_f;
+    D.glo_f[a] = __double2float_rn(lo);
+    D.size_f[a] = size_f;
+    D.inv_s[a] = ext > 0.0 ? inv_f : 0.f;
+    if (a != 0) return;
+    D.lean_ok = quad == 7u;
+    // (x - glo) * inv from the FP32 pairs: one rounding of the difference, one
+    // of inv, one of the product (u = 2^-24 each, relative to the result, at
+    // most cpd bins), with a factor 4 in hand
+    D.frac_eps = 4.0f * 5.9604645e-8f * (float)D.cpd + 1e-6f;
+    // Table extent: every offset whose key is <= (gaps * m)^2 has all gap
+    // counts <= gaps, hence |offset| <= gaps + 1 on every axis.
+    int cheb = g.table_gaps + 1;
+    if (cheb > D.cpd - 1) cheb = D.cpd - 1;
+    if (cheb < 0) cheb = 0;
+    D.cheb = cheb;
+    // The table holds every offset of the grid when that fits; otherwise the
+    // offsets with key <= kmax, and the walk continues ring by ring.
+    const bool complete = cheb == D.cpd - 1 && (2 * cheb + 1) * (2 * cheb + 1) * (2 * cheb + 1) <= kMaxTable;
+    D.has_extent = m != ~0ull;
+    if (m == ~0ull) {            // every point identical: only the own bin holds points
+        D.min_size = 0.0;
+        D.tab_kmax = INFINITY;
+        D.cheb = 0;
+    } else {
+        const double ms = __longlong_as_double((long long)m);
+        D.min_size = ms;
+        const int gaps = cheb - 1;
+        D.tab_kmax = complete ? (double)INFINITY
+                              : __dmul_rn(__dmul_rn((double)gaps, ms), __dmul_rn((double)gaps, ms));
+    }
+}
+
+__global__ void __launch_bounds__(128) k_grid_params(GridBuffers g) {
+    grid_params(g, (int)(blockIdx.x * blockDim.x + threadIdx.x));
+}
+
+// True in every thread of the last block of a grid to get here: what the other
+// blocks wrote before is visible (through L2).
+__device__ bool last_block(unsigned* ticket) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    __threadfence();
+    return last;
+}
+
 // CeleryBounds::new (celery.rs:81-125): per-chunk min/max of the coordinates'
 // order-preserving integer codes (ord_enc: the same order as the doubles),
 // merged with 64-bit atomics.  Non-finite inputs (exponent all ones) raise
-// error_flag.
+// error_flag.  A single diagram's grid parameters are computed by the last
+// block (a launch of their own takes 5 us, 2% of a 1,000-point pass).
 __global__ void __launch_bounds__(kBoundsThreads) k_bounds(GridBuffers g) {
     __shared__ unsigned long long red[6][kBoundsThreads / 32];
     for (uint32_t c = blockIdx.x; c < g.nchunks; c += gridDim.x) {
         const uint32_t d = g.chunk_diag[c];
         const uint32_t beg = g.chunk_start[c];
         const DiagDesc& D = g.diags[d];
-        const uint32_t end = min(beg + kChunk, D.pt_base + D.n);
+        const uint32_t end = min(beg + g.chunk, D.pt_base + D.n);
         unsigned long long mn[3] = {~0ull, ~0ull, ~0ull};
         unsigned long long mx[3] = {0ull, 0ull, 0ull};
         bool bad = false;
@@ -69,6 +157,7 @@ __global__ void __launch_bounds__(kBoundsThreads) k_bounds(GridBuffers g) {
         }
         __syncthreads();
     }
+    if (g.ndiag == 1 && last_block(&g.tickets[0]) && threadIdx.x < 32) grid_params(g, threadIdx.x);
 }
 
 // x rounded toward zero to FP32 by integer operations (within 2^-23 |x|).
@@ -120,104 +209,6 @@ __device__ __forceinline__ int axis_index_fast(double x, const DiagDesc& D, int 
     return 0;
 }
 
-// CeleryCellInfo::new (celery.rs:153-181) from the bounds and the host's cpd.
-// Four threads per diagram, one per axis and one idle: the FP64 divisions of
-// the axes run side by side.
-__global__ void __launch_bounds__(128) k_grid_params(GridBuffers g) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int d = min(t >> 2, g.ndiag - 1), a = min(t & 3, 2);
-    const bool mine = (t >> 2) < g.ndiag && (t & 3) < 3;
-    DiagDesc& D = g.diags[d];
-    const double c = (double)D.cpd;
-    const double lo = ord_dec(g.bounds[6 * d + a]);
-    const double hi = ord_dec(g.bounds[6 * d + 3 + a]);
-    const double half = 0.5 * lo + 0.5 * hi;
-    const double ctr = isfinite(half) ? half : 0.0;
-    const double ext = __dsub_rn(hi, lo);
-    const double size = __ddiv_rn(ext, c), inv = __ddiv_rn(c, ext);
-    const float size_f = __double2float_rn(size), inv_f = __double2float_rn(inv);
-    const bool ok_a = !(ext > 0.0) || (size_f >= FLT_MIN && size_f <= FLT_MAX && inv_f >= FLT_MIN && inv_f <= FLT_MAX);
-    const unsigned quad = (__ballot_sync(0xffffffffu, ok_a) >> (threadIdx.x & 28)) & 7u;
-    // the smallest nonzero bin side, through its order-preserving bits
-    unsigned long long m = size > 0.0 ? (unsigned long long)__double_as_longlong(size) : ~0ull;
-    m = min(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    m = min(m, __shfl_xor_sync(0xffffffffu, m, 2));
-    if (t == 0 && g.host_flag) *g.host_flag = *g.error_flag;
-    if (!mine) return;
-    D.glo[a] = lo;
-    D.ghi[a] = hi;
-    D.ctr[a] = ctr;
-    D.size[a] = size;
-    D.inv[a] = inv;
-    // FP32 forms for the FP32 clipping pass: offsets from the centre as
-    // FP32 pairs (48 bits), the bin sides and their inverses
-    const double gl = lo - ctr, bl = D.blo[a] - ctr, bh = D.bhi[a] - ctr;
-    const float glf = __double2float_rn(gl), blf = __double2float_rn(bl), bhf = __double2float_rn(bh);
-    D.glo_hi[a] = glf;
-    D.glo_lo[a] = __double2float_rn(gl - (double)glf);
-    D.blo_hi[a] = blf;
-    D.blo_lo[a] = __double2float_rn(bl - (double)blf);
-    D.bhi_hi[a] = bhf;
-    D.bhi_lo[a] = __double2float_rn(bh - (double)bhf);
-    D.inv_f[a] = inv_f;
-    D.glo_f[a] = __double2float_rn(lo);
-    D.size_f[a] = size_f;
-    D.inv_s[a] = ext > 0.0 ? inv_f : 0.f;
-    if (a != 0) return;
-    D.lean_ok = quad == 7u;
-    // (x - glo) * inv from the FP32 pairs: one rounding of the difference, one
-    // of inv, one of the product (u = 2^-24 each, relative to the result, at
-    // most cpd bins), with a factor 4 in hand
-    D.frac_eps = 4.0f * 5.9604645e-8f * (float)D.cpd + 1e-6f;
-    // Table extent: every offset whose key is <= (gaps * m)^2 has all gap
-    // counts <= gaps, hence |offset| <= gaps + 1 on every axis.
-    int cheb = g.table_gaps + 1;
-    if (cheb > D.cpd - 1) cheb = D.cpd - 1;
-    if (cheb < 0) cheb = 0;
-    D.cheb = cheb;
-    // The table holds every offset of the grid when that fits; otherwise the
-    // offsets with key <= kmax, and the walk continues ring by ring.
-    const bool complete = cheb == D.cpd - 1 && (2 * cheb + 1) * (2 * cheb + 1) * (2 * cheb + 1) <= kMaxTable;
-    D.has_extent = m != ~0ull;
-    if (m == ~0ull) {            // every point identical: only the own bin holds points
-        D.min_size = 0.0;
-        D.tab_kmax = INFINITY;
-        D.cheb = 0;
-    } else {
-        const double ms = __longlong_as_double((long long)m);
-        D.min_size = ms;
-        const int gaps = cheb - 1;
-        D.tab_kmax = complete ? (double)INFINITY
-                              : __dmul_rn(__dmul_rn((double)gaps, ms), __dmul_rn((double)gaps, ms));
-    }
-}
-
-// get_cells (celery.rs:342-354) + histogram.  rank = arrival order in the bin.
-__global__ void k_bin_count(GridBuffers g) {
-    for (uint32_t c = blockIdx.x; c < g.nchunks; c += gridDim.x) {
-        const uint32_t d = g.chunk_diag[c];
-        const uint32_t beg = g.chunk_start[c];
-        const DiagDesc& D = g.diags[d];
-        const uint32_t end = min(beg + kChunk, D.pt_base + D.n);
-        const int cpd = D.cpd;
-        for (uint32_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
-            const double x = g.xyz[3ull * i], y = g.xyz[3ull * i + 1], z = g.xyz[3ull * i + 2];
-            bool okx = true, oky = true, okz = true;
-            int bx = axis_index_fast(x, D, 0, cpd, okx);
-            int by = axis_index_fast(y, D, 1, cpd, oky);
-            int bz = axis_index_fast(z, D, 2, cpd, okz);
-            // the exact FP64 formula for the few coordinates near a boundary
-            if (!okx) bx = axis_index(x, D.glo[0], D.ghi[0], D.inv[0], cpd);
-            if (!oky) by = axis_index(y, D.glo[1], D.ghi[1], D.inv[1], cpd);
-            if (!okz) bz = axis_index(z, D.glo[2], D.ghi[2], D.inv[2], cpd);
-            // get_cell_from_indices, celery.rs:317-325
-            const uint64_t b = tess_chk(D.bin_base + ((uint64_t)bx * cpd + by) * cpd + bz, g.total_bins, g.check, CK_GRID);
-            g.bin[i] = (uint32_t)b;
-            g.rank[i] = atomicAdd(&g.delims[b], 1u);
-        }
-    }
-}
-
 // ---- exclusive scan of the bin counts -> delimiters (celery.rs:372-414) ----
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
     const int l = threadIdx.x & 31;
@@ -245,6 +236,62 @@ __device__ uint32_t block_excl_scan(uint32_t v, uint32_t* out, uint32_t* sh) {
     uint32_t total = sh[32];
     __syncthreads();
     return total;
+}
+
+// The whole scan by one block (of any size): carry by carry.
+__device__ void scan_by_block(uint32_t* data, uint32_t n, uint32_t* sh) {
+    uint32_t carry = 0;
+    for (uint32_t base0 = 0; base0 < n; base0 += blockDim.x * kScanItems) {
+        const uint32_t base = base0 + threadIdx.x * kScanItems;
+        uint32_t v[kScanItems];
+        uint32_t s = 0;
+        for (int k = 0; k < kScanItems; ++k) {
+            v[k] = base + k < n ? __ldcg(&data[base + k]) : 0u;
+            s += v[k];
+        }
+        uint32_t ex;
+        const uint32_t tot = block_excl_scan(s, &ex, sh);
+        uint32_t run = carry + ex;
+        for (int k = 0; k < kScanItems; ++k) {
+            if (base + k < n) data[base + k] = run;
+            run += v[k];
+        }
+        carry += tot;
+    }
+}
+// Grids of few bins: up to kScanLastMax the last block of the histogram scans
+// them, up to kScanOneMax one block in a launch of its own, three launches
+// beyond.
+constexpr uint64_t kScanLastMax = 4096, kScanOneMax = 16384;
+
+// get_cells (celery.rs:342-354) + histogram.  rank = arrival order in the bin.
+__global__ void __launch_bounds__(256) k_bin_count(GridBuffers g) {
+    for (uint32_t c = blockIdx.x; c < g.nchunks; c += gridDim.x) {
+        const uint32_t d = g.chunk_diag[c];
+        const uint32_t beg = g.chunk_start[c];
+        const DiagDesc& D = g.diags[d];
+        const uint32_t end = min(beg + g.chunk, D.pt_base + D.n);
+        const int cpd = D.cpd;
+        for (uint32_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
+            const double x = g.xyz[3ull * i], y = g.xyz[3ull * i + 1], z = g.xyz[3ull * i + 2];
+            bool okx = true, oky = true, okz = true;
+            int bx = axis_index_fast(x, D, 0, cpd, okx);
+            int by = axis_index_fast(y, D, 1, cpd, oky);
+            int bz = axis_index_fast(z, D, 2, cpd, okz);
+            // the exact FP64 formula for the few coordinates near a boundary
+            if (!okx) bx = axis_index(x, D.glo[0], D.ghi[0], D.inv[0], cpd);
+            if (!oky) by = axis_index(y, D.glo[1], D.ghi[1], D.inv[1], cpd);
+            if (!okz) bz = axis_index(z, D.glo[2], D.ghi[2], D.inv[2], cpd);
+            // get_cell_from_indices, celery.rs:317-325
+            const uint64_t b = tess_chk(D.bin_base + ((uint64_t)bx * cpd + by) * cpd + bz, g.total_bins, g.check, CK_GRID);
+            g.bin[i] = (uint32_t)b;
+            g.rank[i] = atomicAdd(&g.delims[b], 1u);
+        }
+    }
+    if (g.total_bins + 1 <= kScanLastMax) {
+        __shared__ uint32_t sh[33];
+        if (last_block(&g.tickets[1])) scan_by_block(g.delims, (uint32_t)g.total_bins + 1, sh);
+    }
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_partial(uint32_t* data, uint64_t n, uint32_t* sums) {
@@ -288,29 +335,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_final(uint32_t* data, uin
     }
 }
 
-// The whole scan by one block, for grids of few bins: one launch in place of
-// three (a 1,000-point grid's scan 10 -> 4 us with its launches).
-constexpr uint64_t kScanOneMax = 16384;
 __global__ void __launch_bounds__(kScanThreads) k_scan_one(uint32_t* data, uint32_t n) {
     __shared__ uint32_t sh[33];
-    uint32_t carry = 0;
-    for (uint32_t base0 = 0; base0 < n; base0 += kScanThreads * kScanItems) {
-        const uint32_t base = base0 + threadIdx.x * kScanItems;
-        uint32_t v[kScanItems];
-        uint32_t s = 0;
-        for (int k = 0; k < kScanItems; ++k) {
-            v[k] = base + k < n ? data[base + k] : 0u;
-            s += v[k];
-        }
-        uint32_t ex;
-        const uint32_t tot = block_excl_scan(s, &ex, sh);
-        uint32_t run = carry + ex;
-        for (int k = 0; k < kScanItems; ++k) {
-            if (base + k < n) data[base + k] = run;
-            run += v[k];
-        }
-        carry += tot;
-    }
+    scan_by_block(data, n, sh);
 }
 
 // get_sorted_indices (celery.rs:357-369): counting-sort scatter.
@@ -640,6 +667,7 @@ __global__ void k_occupancy(const uint32_t* delims, uint64_t nbins, uint32_t cro
 __global__ void __launch_bounds__(256) k_grid_clear(GridBuffers g) {
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     if (t == 0) *g.error_flag = 0;
+    if (t < 2) g.tickets[t] = 0u;
     for (uint64_t i = t; i < 6ull * g.ndiag; i += stride) g.bounds[i] = (i % 6) < 3 ? ~0ull : 0ull;
     for (uint64_t i = t; i <= g.total_bins; i += stride) g.delims[i] = 0u;
 }
@@ -681,7 +709,9 @@ cudaError_t launch_occupancy(const uint32_t* delims, uint64_t nbins, uint32_t cr
     return cudaGetLastError();
 }
 
-uint64_t grid_launches(uint64_t total_bins) { return total_bins + 1 <= kScanOneMax ? 9 : 11; }
+uint64_t grid_launches(uint64_t total_bins, size_t ndiag) {
+    return 7 + (ndiag > 1 ? 1 : 0) + (total_bins + 1 <= kScanLastMax ? 0 : (total_bins + 1 <= kScanOneMax ? 1 : 3));
+}
 
 // Binning pass: bounds -> grid parameters -> shell tables -> histogram ->
 // scan -> scatter -> within-bin order -> gather.  A fixed launch sequence
@@ -693,7 +723,7 @@ cudaError_t launch_grid_build(const GridBuffers& g, cudaStream_t s, cudaStream_t
     k_grid_clear<<<(unsigned)std::min<uint64_t>((nclear + 1023) / 1024, 152u * 8u), 256, 0, s>>>(g);
     const int cblocks = (int)(g.nchunks < 4096u ? g.nchunks : 4096u);
     k_bounds<<<cblocks, kBoundsThreads, 0, s>>>(g);
-    k_grid_params<<<(4 * ndiag + 127) / 128, 128, 0, s>>>(g);
+    if (ndiag > 1) k_grid_params<<<(4 * ndiag + 127) / 128, 128, 0, s>>>(g);   // else by k_bounds
     if (bounds_done) cudaEventRecord(bounds_done, s);
     // the shell tables need only the grid parameters: build them beside the
     // histogram, scan and scatter when a side stream is given
@@ -710,7 +740,9 @@ cudaError_t launch_grid_build(const GridBuffers& g, cudaStream_t s, cudaStream_t
     const uint64_t nscan = g.total_bins + 1;
     const uint64_t per = (uint64_t)kScanThreads * kScanItems;
     const uint32_t nblk = (uint32_t)((nscan + per - 1) / per);
-    if (nscan <= kScanOneMax) {
+    if (nscan <= kScanLastMax) {
+        // by k_bin_count
+    } else if (nscan <= kScanOneMax) {
         k_scan_one<<<1, kScanThreads, 0, s>>>(g.delims, (uint32_t)nscan);
     } else {
         k_scan_partial<<<nblk, kScanThreads, 0, s>>>(g.delims, nscan, g.scan_tmp);

@@ -167,10 +167,12 @@ struct GridBuffers {
     int ndiag;
     uint32_t total;             // total points
     uint64_t total_bins;
-    const uint32_t* chunk_diag; // per kChunk points: diagram id
+    uint32_t chunk;             // chunk_points(total)
+    const uint32_t* chunk_diag; // per chunk: diagram id
     const uint32_t* chunk_start;
     uint32_t nchunks;
     unsigned long long* bounds; // 6 per diagram (encoded)
+    unsigned* tickets;          // 2: blocks done, for the work of a last block
     uint32_t* bin;
     uint32_t* rank;
     uint32_t* delims;           // total_bins + 1
@@ -191,9 +193,11 @@ struct GridBuffers {
     int* host_flag;             // its value after the bounds, in mapped host memory, or null
     int* check;                 // checked build: the check word
 };
-// Points per block of the bounds and histogram kernels: 2,048 keep small inputs
-// on many SMs (884,736 points: 432 blocks instead of 108).
-constexpr uint32_t kChunk = 2048;
+// Points per block of the bounds and histogram kernels: one per thread up to
+// 131,072 points (512 blocks), where a block's rounds are the kernels' time
+// (1,000 points: 17 us in both with 2,048); 2,048 beyond.
+constexpr uint32_t kChunkSmall = 256, kChunkLarge = 2048;
+constexpr uint32_t chunk_points(uint64_t total) { return total <= 131072 ? kChunkSmall : kChunkLarge; }
 constexpr int kScanItems = 8;       // items per thread in the scan
 constexpr int kScanThreads = 1024;
 
@@ -206,7 +210,7 @@ cudaError_t launch_grid_build(const GridBuffers& g, cudaStream_t s, cudaStream_t
                               cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr,
                               cudaEvent_t bounds_done = nullptr);
 // Kernels launched by one binning pass.
-uint64_t grid_launches(uint64_t total_bins);
+uint64_t grid_launches(uint64_t total_bins, size_t ndiag);
 // inv[sorted[s]] = s for s < n (the point -> sorted position map, on demand).
 cudaError_t launch_inverse(const uint32_t* sorted, uint32_t* inv, uint32_t n, int* check, cudaStream_t s);
 // n bytes from src to dst by the SMs (16-byte aligned pointers; either may be
