@@ -9,6 +9,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <new>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -194,8 +195,11 @@ struct Engine {
     double* d_carea = nullptr;
     uint64_t csr_cap = 0;
     uint64_t* d_csr_tmp = nullptr;
+    // one cell's geometry (single-cell queries), in the same mapped memory;
+    // held by one query at a time
+    GeoOut* h_geo = nullptr;
     GeoOut* d_geo = nullptr;
-    uint32_t* d_one = nullptr;
+    std::mutex geo_mu;
     // radius queries: query positions / cells, per-query counts and offsets,
     // scan scratch, results, and the search-order prefix of the last radius
     double* d_rq = nullptr;
@@ -287,7 +291,6 @@ struct Engine {
         h_ret = nullptr;
         for (auto& l : d_list) dfree(l);
         dfree(d_counters); dfree(d_work); dfree(d_offs); dfree(d_cnbr); dfree(d_carea); dfree(d_csr_tmp);
-        dfree(d_geo); dfree(d_one);
         dfree(d_rq); dfree(d_rcell); dfree(d_rcnt); dfree(d_roffs); dfree(d_rtmp); dfree(d_rout); dfree(d_rtab);
         dfree(d_rerr); dfree(d_gtab); dfree(d_bnd); dfree(d_qbin); dfree(d_qrank); dfree(d_qorder); dfree(d_qcnt); dfree(d_qcoff); dfree(d_qtmp);
         dfree(d_sample); dfree(d_occ);
@@ -400,8 +403,10 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     CU(cudaEventCreateWithFlags(&E.ev_fork, cudaEventDisableTiming));
     CU(cudaEventCreateWithFlags(&E.ev_join, cudaEventDisableTiming));
     CU(cudaEventCreateWithFlags(&E.ev_bounds, cudaEventDisableTiming));
-    CU(cudaHostAlloc((void**)&E.h_ret, 256, cudaHostAllocMapped));
+    CU(cudaHostAlloc((void**)&E.h_ret, 256 + sizeof(GeoOut), cudaHostAllocMapped));
     CU(cudaHostGetDevicePointer((void**)&E.d_ret, E.h_ret, 0));
+    E.h_geo = reinterpret_cast<GeoOut*>(reinterpret_cast<char*>(E.h_ret) + 256);
+    E.d_geo = reinterpret_cast<GeoOut*>(reinterpret_cast<char*>(E.d_ret) + 256);
     E.ndiag = diags.size();
     uint64_t total = 0, bins = 0, tab = 0;
     std::vector<uint32_t> cdiag, cstart;
@@ -468,8 +473,6 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     TRY(dalloc(&E.d_work, 8));
     TRY(dalloc(&E.d_offs, n + 1));
     TRY(dalloc(&E.d_csr_tmp, csr_tmp_words(E.total)));
-    TRY(dalloc(&E.d_geo, 1));
-    TRY(dalloc(&E.d_one, 1));
     return TESS_OK;
 }
 
@@ -1100,23 +1103,24 @@ tess_status engine_autotune(Engine& E, int precision, bool batch, const char* ca
     return TESS_OK;
 }
 
-// One cell's full geometry: the cell alone through the FP64 clipping (in every
-// precision: one warp's latency is the same in FP32) into the GeoOut buffer,
-// copied back.
-tess_status engine_geo(Engine& E, uint32_t gs, const double* point, double radius, int64_t group, const double* lo,
-                       const double* hi, GeoOut* out) {
+// One cell's full geometry in E.h_geo, which the caller holds E.geo_mu for: the
+// cell alone through the careful pass's FP64 finish (in every precision), and
+// through the FP64 clipping when that cannot settle it, written by the kernel
+// into mapped memory.
+tess_status engine_geo(Engine& E, const size_t* i, const double* point, double radius, int64_t group, const double* lo,
+                       const double* hi) {
     CU(cudaSetDevice(E.device));
     ClipParams p = base_params(E);
     p.search_radius = radius;
     p.has_radius = radius >= 0.0;
     p.target_group = group;
-    CU(cudaMemcpyAsync(E.d_one, &gs, sizeof(uint32_t), cudaMemcpyHostToDevice, E.stream));
-    CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * C_TOTAL, E.stream));
-    p.work = E.d_one;
-    p.work_count = nullptr;
+    p.tol = kFp64Tol;
     p.total = 1;
-    p.cursor = E.d_counters;
     p.geo = E.d_geo;
+    if (i) {
+        TRY(ensure_inv(E));
+        p.work = E.d_inv + *i;
+    }
     if (point) {
         p.at_point = 1;
         p.point[0] = point[0];
@@ -1130,12 +1134,17 @@ tess_status engine_geo(Engine& E, uint32_t gs, const double* point, double radiu
             p.box[3 + a] = hi[a];
         }
     }
-    CU(launch_clip(p, 8, kFormStd, 1, 1, E.stream));
-    CU(cudaMemcpyAsync(out, E.d_geo, sizeof(GeoOut), cudaMemcpyDeviceToHost, E.stream));
+    CU(launch_cell_lean(p, E.stream));
     CU(cudaStreamSynchronize(E.stream));
+    if (E.h_geo->status != ST_OK) {
+        CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * C_TOTAL, E.stream));
+        p.cursor = E.d_counters;
+        CU(launch_clip(p, 8, kFormStd, 1, 1, E.stream));
+        CU(cudaStreamSynchronize(E.stream));
+    }
     TRY(check_word(E));
-    if (out->status == ST_OK) return TESS_OK;
-    return fail(TESS_E_OVERFLOW, "cell could not be computed (status %d)", out->status);
+    if (E.h_geo->status == ST_OK) return TESS_OK;
+    return fail(TESS_E_OVERFLOW, "cell could not be computed (status %d)", E.h_geo->status);
 }
 
 
@@ -1644,57 +1653,46 @@ tess_status tess_cell_original_index(const tess_diagram* d, size_t i, size_t* or
     return TESS_OK;
 }
 
-static tess_status geo_for(tess_diagram* d, size_t i, GeoOut* g) {
-    TRY(cell_check(d, i));
-    uint32_t gs = 0;
-    CU(cudaSetDevice(d->E.device));
-    TRY(ensure_inv(d->E));
-    CU(cudaMemcpy(&gs, d->E.d_inv + i, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    return engine_geo(d->E, gs, nullptr, d->E.last_radius, d->E.last_group, nullptr, nullptr, g);
+// Cell i of the last compute, in E.h_geo (E.geo_mu held).
+static tess_status geo_for(tess_diagram* d, size_t i) {
+    return engine_geo(d->E, &i, nullptr, d->E.last_radius, d->E.last_group, nullptr, nullptr);
 }
 
 tess_status tess_cell_vertices(tess_diagram* d, size_t i, double* xyz, size_t cap, size_t* count) {
-    GeoOut* g = new (std::nothrow) GeoOut;
-    if (!g) return fail(TESS_E_NOMEM, "host allocation failed");
-    tess_status st = geo_for(d, i, g);
-    if (st == TESS_OK) {
-        if (count) *count = (size_t)g->nv;
-        if ((size_t)g->nv > cap) st = fail(TESS_E_CAPACITY, "cell %zu has %d vertices, capacity %zu", i, g->nv, cap);
-        else if (xyz) memcpy(xyz, g->verts, sizeof(double) * 3 * g->nv);
-    }
-    delete g;
-    return st;
+    TRY(cell_check(d, i));
+    std::lock_guard<std::mutex> lock(d->E.geo_mu);
+    TRY(geo_for(d, i));
+    const GeoOut* g = d->E.h_geo;
+    if (count) *count = (size_t)g->nv;
+    if ((size_t)g->nv > cap) return fail(TESS_E_CAPACITY, "cell %zu has %d vertices, capacity %zu", i, g->nv, cap);
+    if (xyz) memcpy(xyz, g->verts, sizeof(double) * 3 * g->nv);
+    return TESS_OK;
 }
 
 tess_status tess_cell_face_vertices(tess_diagram* d, size_t i, size_t face, double* xyz, size_t cap,
                                     size_t* count) {
-    GeoOut* g = new (std::nothrow) GeoOut;
-    if (!g) return fail(TESS_E_NOMEM, "host allocation failed");
-    tess_status st = geo_for(d, i, g);
-    if (st == TESS_OK) {
-        if (face >= (size_t)g->nf) {
-            st = fail(TESS_E_INVALID, "face %zu out of range (%d faces)", face, g->nf);
-        } else {
-            const int b = g->face_off[face], e = g->face_off[face + 1];
-            if (count) *count = (size_t)(e - b);
-            if ((size_t)(e - b) > cap) st = fail(TESS_E_CAPACITY, "face has %d vertices, capacity %zu", e - b, cap);
-            else if (xyz)
-                for (int t = b; t < e; ++t) memcpy(xyz + 3 * (t - b), g->verts + 3 * g->face_vtx[t], 3 * sizeof(double));
-        }
-    }
-    delete g;
-    return st;
+    TRY(cell_check(d, i));
+    std::lock_guard<std::mutex> lock(d->E.geo_mu);
+    TRY(geo_for(d, i));
+    const GeoOut* g = d->E.h_geo;
+    if (face >= (size_t)g->nf) return fail(TESS_E_INVALID, "face %zu out of range (%d faces)", face, g->nf);
+    const int b = g->face_off[face], e = g->face_off[face + 1];
+    if (count) *count = (size_t)(e - b);
+    if ((size_t)(e - b) > cap) return fail(TESS_E_CAPACITY, "face has %d vertices, capacity %zu", e - b, cap);
+    if (xyz)
+        for (int t = b; t < e; ++t) memcpy(xyz + 3 * (t - b), g->verts + 3 * g->face_vtx[t], 3 * sizeof(double));
+    return TESS_OK;
 }
 
 static void geo_to_public(const GeoOut& g, tess_cell_geometry* out) {
     out->volume = g.volume;
     out->nvertices = g.nv;
     out->nfaces = g.nf;
-    memcpy(out->vertices, g.verts, sizeof(out->vertices));
-    memcpy(out->face_neighbor, g.face_nbr, sizeof(out->face_neighbor));
-    memcpy(out->face_area, g.face_area, sizeof(out->face_area));
-    memcpy(out->face_offset, g.face_off, sizeof(out->face_offset));
-    memcpy(out->face_vertex, g.face_vtx, sizeof(out->face_vertex));
+    memcpy(out->vertices, g.verts, sizeof(double) * 3 * g.nv);
+    memcpy(out->face_neighbor, g.face_nbr, sizeof(int32_t) * g.nf);
+    memcpy(out->face_area, g.face_area, sizeof(double) * g.nf);
+    memcpy(out->face_offset, g.face_off, sizeof(int32_t) * (g.nf + 1));
+    memcpy(out->face_vertex, g.face_vtx, sizeof(int32_t) * g.face_off[g.nf]);
 }
 
 static tess_status single_cell(tess_diagram* d, const size_t* i, const double* p, tess_precision precision,
@@ -1708,21 +1706,15 @@ static tess_status single_cell(tess_diagram* d, const size_t* i, const double* p
         (int)precision != TESS_PRECISION_MIXED)
         return fail(TESS_E_INVALID, "unknown precision %d", (int)precision);
     if (std::isnan(search_radius)) return fail(TESS_E_INVALID, "search_radius is NaN");
-    uint32_t gs = 0;
-    CU(cudaSetDevice(d->E.device));
     if (i) {
         if (*i >= d->n) return fail(TESS_E_INVALID, "cell index %zu out of range (n = %u)", *i, d->n);
-        TRY(ensure_inv(d->E));
-        CU(cudaMemcpy(&gs, d->E.d_inv + *i, sizeof(uint32_t), cudaMemcpyDeviceToHost));
     } else if (!std::isfinite(p[0]) || !std::isfinite(p[1]) || !std::isfinite(p[2])) {
         return fail(TESS_E_INVALID, "point must be finite");
     }
-    GeoOut* g = new (std::nothrow) GeoOut;
-    if (!g) return fail(TESS_E_NOMEM, "host allocation failed");
-    tess_status st = engine_geo(d->E, gs, i ? nullptr : p, search_radius, target_group, lo, hi, g);
-    if (st == TESS_OK) geo_to_public(*g, out);
-    delete g;
-    return st;
+    std::lock_guard<std::mutex> lock(d->E.geo_mu);
+    TRY(engine_geo(d->E, i, i ? nullptr : p, search_radius, target_group, lo, hi));
+    geo_to_public(*d->E.h_geo, out);
+    return TESS_OK;
 }
 
 tess_status tess_cell_compute(tess_diagram* d, size_t i, tess_precision precision, double search_radius,

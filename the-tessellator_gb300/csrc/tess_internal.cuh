@@ -366,6 +366,10 @@ struct ClipParams {
 //                 computed in FP64 (the MIXED and FP64 forms)
 enum ClipForm : int { kFormLean = 0, kFormStd = 1, kFormDense = 2, kFormCareful = 3, kFormExact = 4 };
 cudaError_t launch_clip_lean(const ClipParams& p, int form, int wpb, int blocks, cudaStream_t s);
+// One cell with its geometry into p.geo (readable by the host once the stream
+// is done): point *p.work of the single diagram, or the site p.point.  Any
+// status but ST_OK means the FP64 form has to take it.
+cudaError_t launch_cell_lean(const ClipParams& p, cudaStream_t s);
 int clip_blocks_lean(int form, int wpb, int device);
 cudaError_t launch_clip_f64(const ClipParams& p, int slots, int wpb, int blocks, cudaStream_t s);
 int clip_blocks_f64(int slots, int wpb, int device);
