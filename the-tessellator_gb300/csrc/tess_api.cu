@@ -118,6 +118,10 @@ enum { L_DENSE = 0, L_CARE = 1, L_FULL = 2, L_CAP64 = 3, L_COUNT = 4 };
 enum { C_CURSOR = 0, C_LIST = 16, C_FAIL = 20, C_FLAG = 21, C_DENSE = 22, C_REASON32 = 32, C_REASON64 = 40,
        C_TOTAL = 48,      // cleared for each compute, with the face cursor behind it ...
        C_FACES = 48, C_ERR = 50, C_BYTES = 208 };   // ... and the binning's error flag, read back together
+// Behind them in E.h_ret: the binning's early error flag, and a radius query's
+// total and error words.
+enum { RET_FLAG = C_BYTES / 4, RET_TOTAL = 56, RET_ERR = 58, RET_BYTES = 256 };
+static_assert(RET_FLAG < RET_TOTAL && 4 * (RET_ERR + 2) <= RET_BYTES, "layout of the read-back block");
 // Up to this many cells the careful pass runs over all of them: a few waves of
 // warps, whose time is a cell's latency, and a second pass over a few cells
 // would add its own (uniform points, careful alone against plain and careful:
@@ -195,11 +199,12 @@ struct Engine {
     double* d_carea = nullptr;
     uint64_t csr_cap = 0;
     uint64_t* d_csr_tmp = nullptr;
-    // one cell's geometry (single-cell queries), in the same mapped memory;
-    // held by one query at a time
+    // one cell's geometry (single-cell queries), in the same mapped memory.  A
+    // handle may be read from several threads: its query buffers are held by
+    // one query at a time
     GeoOut* h_geo = nullptr;
     GeoOut* d_geo = nullptr;
-    std::mutex geo_mu;
+    std::mutex query_mu;
     // radius queries: query positions / cells, per-query counts and offsets,
     // scan scratch, results, and the search-order prefix of the last radius
     double* d_rq = nullptr;
@@ -213,6 +218,8 @@ struct Engine {
     uint64_t* d_rtmp = nullptr;
     size_t rtmp_cap = 0;
     uint32_t* d_rout = nullptr;
+    uint32_t* d_rstage = nullptr; // results listed by the first pass
+    size_t rstage_cap = 0;
     size_t rout_cap = 0;
     short4* d_rtab = nullptr;
     size_t rtab_cap = 0;
@@ -228,7 +235,7 @@ struct Engine {
     bool hgrid_valid = false;
     int16_t* d_gtab = nullptr;    // gap table of the last box-query radius
     size_t gtab_cap = 0;
-    bool gtab_valid = false, gtab_present = false;
+    bool gtab_valid = false, gtab_present = false, gtab_tie = false;
     uint64_t gtab_radius_bits = 0;
     int gtab_dim[3] = {};
     // spatial order of large query batches
@@ -291,7 +298,7 @@ struct Engine {
         h_ret = nullptr;
         for (auto& l : d_list) dfree(l);
         dfree(d_counters); dfree(d_work); dfree(d_offs); dfree(d_cnbr); dfree(d_carea); dfree(d_csr_tmp);
-        dfree(d_rq); dfree(d_rcell); dfree(d_rcnt); dfree(d_roffs); dfree(d_rtmp); dfree(d_rout); dfree(d_rtab);
+        dfree(d_rq); dfree(d_rcell); dfree(d_rcnt); dfree(d_roffs); dfree(d_rtmp); dfree(d_rstage); dfree(d_rout); dfree(d_rtab);
         dfree(d_rerr); dfree(d_gtab); dfree(d_bnd); dfree(d_qbin); dfree(d_qrank); dfree(d_qorder); dfree(d_qcnt); dfree(d_qcoff); dfree(d_qtmp);
         dfree(d_sample); dfree(d_occ);
         if (own_stream && stream) cudaStreamDestroy(stream);
@@ -403,10 +410,10 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     CU(cudaEventCreateWithFlags(&E.ev_fork, cudaEventDisableTiming));
     CU(cudaEventCreateWithFlags(&E.ev_join, cudaEventDisableTiming));
     CU(cudaEventCreateWithFlags(&E.ev_bounds, cudaEventDisableTiming));
-    CU(cudaHostAlloc((void**)&E.h_ret, 256 + sizeof(GeoOut), cudaHostAllocMapped));
+    CU(cudaHostAlloc((void**)&E.h_ret, RET_BYTES + sizeof(GeoOut), cudaHostAllocMapped));
     CU(cudaHostGetDevicePointer((void**)&E.d_ret, E.h_ret, 0));
-    E.h_geo = reinterpret_cast<GeoOut*>(reinterpret_cast<char*>(E.h_ret) + 256);
-    E.d_geo = reinterpret_cast<GeoOut*>(reinterpret_cast<char*>(E.d_ret) + 256);
+    E.h_geo = reinterpret_cast<GeoOut*>(reinterpret_cast<char*>(E.h_ret) + RET_BYTES);
+    E.d_geo = reinterpret_cast<GeoOut*>(reinterpret_cast<char*>(E.d_ret) + RET_BYTES);
     E.ndiag = diags.size();
     uint64_t total = 0, bins = 0, tab = 0;
     std::vector<uint32_t> cdiag, cstart;
@@ -453,7 +460,7 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     TRY(dalloc(&E.d_spx, n));
     TRY(dalloc(&E.d_spy, n));
     TRY(dalloc(&E.d_spz, n));
-    TRY(dalloc(&E.d_phi, n));
+    TRY(dalloc(&E.d_phi, n + 3));   // (radius queries read four at a time)
     TRY(dalloc(&E.d_plo, n));
     TRY(dalloc(&E.d_table, E.table_total));
     E.table_alloc = E.table_total;
@@ -505,7 +512,7 @@ GridBuffers grid_buffers(Engine& E) {
     g.table = E.d_table;
     g.table_gaps = E.cfg.table_gaps;
     g.error_flag = E.d_err;
-    g.host_flag = reinterpret_cast<int*>(E.d_ret + C_BYTES / sizeof(unsigned));
+    g.host_flag = reinterpret_cast<int*>(E.d_ret + RET_FLAG);
     g.check = E.d_check;
     return g;
 }
@@ -597,7 +604,7 @@ tess_status engine_build(Engine& E, bool check, const double* src = nullptr) {
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     if (check) {
         CU(cudaEventSynchronize(E.ev_bounds));
-        if (*reinterpret_cast<volatile int*>(E.h_ret + C_BYTES / sizeof(unsigned))) {
+        if (*reinterpret_cast<volatile int*>(E.h_ret + RET_FLAG)) {
             // the grid describes the bad points: nothing may use it until a
             // build succeeds
             E.built = false;
@@ -1103,7 +1110,7 @@ tess_status engine_autotune(Engine& E, int precision, bool batch, const char* ca
     return TESS_OK;
 }
 
-// One cell's full geometry in E.h_geo, which the caller holds E.geo_mu for: the
+// One cell's full geometry in E.h_geo, which the caller holds E.query_mu for: the
 // cell alone through the careful pass's FP64 finish (in every precision), and
 // through the FP64 clipping when that cannot settle it, written by the kernel
 // into mapped memory.
@@ -1150,8 +1157,13 @@ tess_status engine_geo(Engine& E, const size_t* i, const double* point, double r
 
 // Largest search-order prefix a neighbour-cloud call may enumerate.
 constexpr size_t kMaxRadiusTable = (size_t)1 << 26;
-// Query batches at least this large are processed in spatial order.
-constexpr size_t kOrderMin = 65536;
+// Query batches at least this large are processed in spatial order: with a
+// warp per query, and with a lane per query (which keeps four times as many reads
+// in flight; 1,000,000 points: 262,144 queries 191 us as they come and 221 in
+// order, 524,288 290 and 288, 1,000,000 460 and 428).
+constexpr size_t kOrderMin = 65536, kOrderMinLane = 524288;
+// Most entries (of 4 bytes) of the lists that a radius query's first pass keeps.
+constexpr size_t kMaxStage = (size_t)1 << 29;
 // Largest gap table (entries of int16) for box queries; beyond it the
 // kernel evaluates the gap distance per bin in FP64.
 constexpr size_t kMaxGapTable = 65536;
@@ -1166,9 +1178,10 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     if (!E.built) return fail(TESS_E_STATE, "the diagram has no grid");
     if (nq >= 0xFFFFFFFFull) return fail(TESS_E_INVALID, "too many queries (%zu)", nq);
     if (nq && !by_cell && !qxyz) return fail(TESS_E_INVALID, "query positions are NULL");
+    std::lock_guard<std::mutex> lock(E.query_mu);
     CU(cudaSetDevice(E.device));
     if (!E.sm_count) CU(cudaDeviceGetAttribute(&E.sm_count, cudaDevAttrMultiProcessorCount, E.device));
-    if (!E.d_rerr) TRY(dalloc(&E.d_rerr, 1));
+    if (!E.d_rerr) TRY(dalloc(&E.d_rerr, 2));
     RadiusParams p{};
     p.desc = E.d_desc;
     p.delims = E.d_delims;
@@ -1178,8 +1191,6 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     p.spz = E.d_spz;
     p.sgroup = E.d_sgroup;
     p.xyz = E.d_xyz;
-    TRY(ensure_inv(E));
-    p.inv = E.d_inv;
     p.nq = (uint32_t)nq;
     p.radius = radius;
     p.group = group;
@@ -1219,7 +1230,7 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     if (need_gap_tab) {
         std::vector<int16_t> gt;
         E.gtab_present = build_gap_table(D.size, D.inv, D.cpd, radius, kMaxGapTable, gt, &E.gtab_dim[0],
-                                         &E.gtab_dim[1], &E.gtab_dim[2]);
+                                         &E.gtab_dim[1], &E.gtab_dim[2], &E.gtab_tie);
         if (E.gtab_present) {
             TRY(ensure(&E.d_gtab, E.gtab_cap, gt.size()));
             CU(cudaMemcpyAsync(E.d_gtab, gt.data(), sizeof(int16_t) * gt.size(), cudaMemcpyHostToDevice, E.stream));
@@ -1233,6 +1244,7 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
         p.gtab_x = E.gtab_dim[0];
         p.gtab_y = E.gtab_dim[1];
         p.gtab_z = E.gtab_dim[2];
+        p.gtab_tie = E.gtab_tie;
     }
     if (!E.bnd_valid) {
         const int cpd = E.hdesc[0].cpd;
@@ -1269,8 +1281,18 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     TRY(ensure(&E.d_rtmp, E.rtmp_cap, tmp_words));
     p.count = E.d_rcnt;
     p.offs = E.d_roffs;
+    if (out && cap && nq && E.hgrid_valid) {
+        // a bounded workspace, and none when memory is short: the second pass
+        // then finds the results again
+        const size_t len = radius_stage_len(mode, (uint32_t)nq, E.total, D, radius), entries = len * ((nq + 31) / 32 * 32);
+        if (len && entries <= kMaxStage && ensure(&E.d_rstage, E.rstage_cap, entries) == TESS_OK) {
+            p.stage = E.d_rstage;
+            p.stage_len = (uint32_t)len;
+        }
+        cudaGetLastError();   // leave no error behind a failed allocation
+    }
     const int blocks = (int)std::max<size_t>(1, std::min<size_t>((nq + 7) / 8, (size_t)E.sm_count * 16));
-    CU(cudaMemsetAsync(E.d_rerr, 0, sizeof(int), E.stream));
+    CU(cudaMemsetAsync(E.d_rerr, 0, 2 * sizeof(int), E.stream));
     const bool timing = E.cfg.flags & TESS_FLAG_TIMING;
     TimingEvents tev;
     cudaEvent_t* ev = tev.e;
@@ -1279,7 +1301,7 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     uint64_t tot = 0;
     if (nq) {
         if (timing) CU(cudaEventRecord(ev[0], E.stream));
-        if (nq >= kOrderMin && (p.qxyz || p.qcell)) {
+        if (nq >= (mode == RQ_CELL_RADIUS || mode == RQ_REAL_RADIUS ? kOrderMinLane : kOrderMin) && (p.qxyz || p.qcell)) {
             // process large batches in coarse-bin order: neighbouring warps then
             // read the same candidate bins
             QueryOrder o{};
@@ -1305,14 +1327,16 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
         CU(launch_radius(p, mode, false, blocks, E.stream));
         CU(launch_csr_offsets(E.d_rcnt, (uint32_t)nq, E.d_roffs, E.d_rtmp, E.stream));
         if (timing) CU(cudaEventRecord(ev[1], E.stream));
-        CU(cudaMemcpyAsync(&tot, E.d_roffs + nq, sizeof(uint64_t), cudaMemcpyDeviceToHost, E.stream));
+        CU(cudaMemcpyAsync(E.h_ret + RET_TOTAL, E.d_roffs + nq, sizeof(uint64_t), cudaMemcpyDeviceToHost, E.stream));
         E.launches += 4;
     }
-    int err = 0;
-    CU(cudaMemcpyAsync(&err, E.d_rerr, sizeof(int), cudaMemcpyDeviceToHost, E.stream));
+    int err[2];
+    CU(cudaMemcpyAsync(E.h_ret + RET_ERR, E.d_rerr, sizeof(err), cudaMemcpyDeviceToHost, E.stream));
     CU(cudaStreamSynchronize(E.stream));
+    if (nq) memcpy(&tot, E.h_ret + RET_TOTAL, sizeof(tot));
+    memcpy(err, E.h_ret + RET_ERR, sizeof(err));
     if (timing && nq) E.stats.ms_query_count = tev.ms(0, 1);
-    if (err) return fail(TESS_E_INVALID, "a query cell index is out of range (n = %u)", E.total);
+    if (err[0]) return fail(TESS_E_INVALID, "a query cell index is out of range (n = %u)", E.total);
     if (total) *total = (size_t)tot;
     if (offs) {
         if (nq) {
@@ -1337,6 +1361,7 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
         TRY(ensure(&E.d_rout, E.rout_cap, tot));
         p.out = E.d_rout;
     }
+    p.unlisted = err[1];
     if (timing) CU(cudaEventRecord(ev[1], E.stream));
     CU(launch_radius(p, mode, true, blocks, E.stream));
     if (timing) CU(cudaEventRecord(ev[2], E.stream));
@@ -1653,14 +1678,14 @@ tess_status tess_cell_original_index(const tess_diagram* d, size_t i, size_t* or
     return TESS_OK;
 }
 
-// Cell i of the last compute, in E.h_geo (E.geo_mu held).
+// Cell i of the last compute, in E.h_geo (E.query_mu held).
 static tess_status geo_for(tess_diagram* d, size_t i) {
     return engine_geo(d->E, &i, nullptr, d->E.last_radius, d->E.last_group, nullptr, nullptr);
 }
 
 tess_status tess_cell_vertices(tess_diagram* d, size_t i, double* xyz, size_t cap, size_t* count) {
     TRY(cell_check(d, i));
-    std::lock_guard<std::mutex> lock(d->E.geo_mu);
+    std::lock_guard<std::mutex> lock(d->E.query_mu);
     TRY(geo_for(d, i));
     const GeoOut* g = d->E.h_geo;
     if (count) *count = (size_t)g->nv;
@@ -1672,7 +1697,7 @@ tess_status tess_cell_vertices(tess_diagram* d, size_t i, double* xyz, size_t ca
 tess_status tess_cell_face_vertices(tess_diagram* d, size_t i, size_t face, double* xyz, size_t cap,
                                     size_t* count) {
     TRY(cell_check(d, i));
-    std::lock_guard<std::mutex> lock(d->E.geo_mu);
+    std::lock_guard<std::mutex> lock(d->E.query_mu);
     TRY(geo_for(d, i));
     const GeoOut* g = d->E.h_geo;
     if (face >= (size_t)g->nf) return fail(TESS_E_INVALID, "face %zu out of range (%d faces)", face, g->nf);
@@ -1711,7 +1736,7 @@ static tess_status single_cell(tess_diagram* d, const size_t* i, const double* p
     } else if (!std::isfinite(p[0]) || !std::isfinite(p[1]) || !std::isfinite(p[2])) {
         return fail(TESS_E_INVALID, "point must be finite");
     }
-    std::lock_guard<std::mutex> lock(d->E.geo_mu);
+    std::lock_guard<std::mutex> lock(d->E.query_mu);
     TRY(engine_geo(d->E, i, i ? nullptr : p, search_radius, target_group, lo, hi));
     geo_to_public(*d->E.h_geo, out);
     return TESS_OK;

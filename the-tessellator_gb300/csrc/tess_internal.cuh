@@ -238,7 +238,6 @@ struct RadiusParams {
     const double* spz;
     const uint32_t* sgroup;     // groups in sorted order, or null (all 0)
     const double* xyz;          // points, AoS, original order
-    const uint32_t* inv;        // point -> sorted position
     const double* qxyz;         // query positions (AoS), or null: queries are cells
     const uint32_t* qcell;      // cloud query cells (original index), or null: every cell
     uint32_t nq;
@@ -249,7 +248,7 @@ struct RadiusParams {
     uint32_t* count;            // count pass: results per query
     const uint64_t* offs;       // fill pass: CSR offsets per query
     uint32_t* out;              // fill pass: bin ids or original point indices
-    int* err;                   // set to 1 when a query cell is out of range
+    int* err;                   // [0] set to 1 when a query cell is out of range, [1] by a query with more than stage_len results
     const uint32_t* qorder;     // processing order of the queries (spatially sorted), or null
     const float4* phi;          // FP32 high parts of the sorted positions (see GridBuffers), for the FP32 filter
     int f32_filter;             // real radius: pre-filter candidates in FP32 (radius in range)
@@ -258,10 +257,21 @@ struct RadiusParams {
     // (-1: none); null: the FP64 formula per bin
     const int16_t* gtab;
     int gtab_x, gtab_y, gtab_z;
+    // counting pass, one query per lane: result k < stage_len of the query at
+    // place i of the processing order, at stage[(i / 32 * stage_len + k) * 32 + i % 32]
+    uint32_t* stage;
+    uint32_t stage_len;
+    int unlisted;               // fill pass: some query has more results than are listed
+    int gtab_tie;               // some squared gap distance is at most 1% above radius^2
     // bin boundaries per axis: bnd[a * cpd + i] (1 <= i < cpd) is the order
     // code (ord_enc) of the smallest double whose axis_index is >= i
     const unsigned long long* bnd;
 };
+
+// RadiusParams::stage_len for a batch of nq queries of a diagram of n points:
+// room for half as many results again as a uniform density gives a query (its
+// Poisson tail: 16 on top); 0: nothing is listed.
+uint32_t radius_stage_len(int mode, uint32_t nq, uint32_t n, const DiagDesc& D, double radius);
 
 // Fills RadiusParams::bnd for diagram 0 (3 * cpd entries).
 cudaError_t launch_axis_bounds(const DiagDesc* desc, int cpd, unsigned long long* bnd, cudaStream_t s);
@@ -290,7 +300,7 @@ bool build_radius_table(const double size[3], int cpd, double radius, size_t max
 // The gap table of RadiusParams::gtab for this radius; false if the radius is
 // not finite and non-negative or the table would exceed max_entries.
 bool build_gap_table(const double size[3], const double inv[3], int cpd, double radius, size_t max_entries,
-                     std::vector<int16_t>& out, int* gx, int* gy, int* gz);
+                     std::vector<int16_t>& out, int* gx, int* gy, int* gz, bool* tie);
 
 // ---- launchers (tess_clip.cu) ----
 struct ClipParams {

@@ -15,8 +15,9 @@
 //                   order up to the first key above r (celery.rs:1023-1075),
 //                   optionally filtered by group.
 //
-// One warp answers one query.  The warp takes 32 candidate bins at a time
-// (box cells or search-order entries), keeps the ones in range, and then
+// Large batches of the two point queries take a lane per query (k_radius_lane,
+// below); else one warp answers one query.  The warp takes 32 candidate bins at
+// a time (box cells or search-order entries), keeps the ones in range, and then
 // walks the kept bins' points as one concatenated stream, 32 points per step:
 // a warp prefix sum of the bins' counts maps each lane to its bin.  Results
 // stay in the reference's order (bins in query order, sorted_indices order
@@ -27,6 +28,7 @@
 // and points found are the reference's exactly.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "tess_internal.cuh"
 
@@ -34,6 +36,13 @@ namespace tess {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
+// Queries from which a lane answers one.  1,000,000 points, 16 results each,
+// whole calls: 4,000 queries 89 us by warps and 109 by lanes, 8,192 about 105 and
+// 104, 16,384 137 and 120, 65,535 213 and 112.
+constexpr uint32_t kLaneMin = 8192;
+constexpr uint32_t kLongRun = 64;     // points of a row from which a warp shares them
+constexpr int kLaneThreads = 128;     // threads of such a block
+constexpr int kLaneRows = 16;         // rows listed at a time
 
 __device__ __forceinline__ double sq_rn(double a) { return __dmul_rn(a, a); }
 
@@ -58,12 +67,12 @@ struct QueryTest {
 // Kept out of line: inlined, the compiler predicates these FP64 operations
 // into every candidate step, and predicated-off FP64 instructions still take
 // the (slow) FP64 pipe's issue slots.
-__device__ __noinline__ bool exact_within(const RadiusParams& p, const QueryTest& qt, uint32_t s) {
+__device__ __noinline__ bool exact_within(const RadiusParams& p, double x, double y, double z, double r2, uint32_t s) {
     // distance_squared(x, y, z, point), celery.rs:700-702
-    const double dx = __dsub_rn(qt.x, p.spx[s]);
-    const double dy = __dsub_rn(qt.y, p.spy[s]);
-    const double dz = __dsub_rn(qt.z, p.spz[s]);
-    return __dadd_rn(__dadd_rn(sq_rn(dx), sq_rn(dy)), sq_rn(dz)) <= qt.r2;
+    const double dx = __dsub_rn(x, p.spx[s]);
+    const double dy = __dsub_rn(y, p.spy[s]);
+    const double dz = __dsub_rn(z, p.spz[s]);
+    return __dadd_rn(__dadd_rn(sq_rn(dx), sq_rn(dy)), sq_rn(dz)) <= r2;
 }
 
 // Up to 32 runs (one per lane: first element `beg`, length `c`) as one
@@ -135,7 +144,7 @@ __device__ __forceinline__ void emit_stream(const RadiusParams& p, uint32_t beg,
                 band = valid;
                 ok = false;
             }
-            if (__any_sync(kFull, band) && band) ok = exact_within(p, qt, s);
+            if (__any_sync(kFull, band) && band) ok = exact_within(p, qt.x, qt.y, qt.z, qt.r2, s);
         }
         if (MODE == RQ_CLOUD && ok && p.group >= 0) ok = (int64_t)(p.sgroup ? p.sgroup[s] : 0u) == p.group;
         const unsigned bal = __ballot_sync(kFull, ok);
@@ -395,6 +404,360 @@ __global__ void __launch_bounds__(256) k_radius(RadiusParams p) {
     }
 }
 
+// The bin indices of k_radius_lane that FP32 leaves open, exactly: bit 3 a + e of
+// `open` is axis a's e-th of the query's own bin, the box's low and its high end.
+__device__ __noinline__ int exact_index(const RadiusParams& p, double c, int a, int e, int top) {
+    const DiagDesc& D = p.desc[0];
+    unsigned long long v = (unsigned long long)__double_as_longlong(e == 0 ? c : __dadd_rn(c, e == 2 ? p.radius : -p.radius));
+    if (e != 0) {
+        const unsigned long long clamp = (unsigned long long)__double_as_longlong(e == 2 ? D.ghi[a] : D.glo[a]);
+        const unsigned long long cc = (clamp >> 63) ? ~clamp : (clamp | 0x8000000000000000ull);
+        const unsigned long long ve = (v >> 63) ? ~v : (v | 0x8000000000000000ull);
+        if (is_nan_bits(v) || !(e == 2 ? ve < cc : ve > cc)) v = clamp;
+    }
+    return axis_index_table(v, p.bnd + a * D.cpd, D.cpd, top);
+}
+
+// Square root to 2 ulp, of a positive number.
+__device__ __forceinline__ float sqrt_near(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Whether point s is within the radius of query q, exactly (rare).
+__device__ __noinline__ bool exact_query(const RadiusParams& p, uint32_t q, uint32_t s) {
+    const double* c = p.qxyz + 3 * (size_t)q;
+    return exact_within(p, c[0], c[1], c[2], sq_rn(p.radius), s);
+}
+
+// RQ_REAL_RADIUS and RQ_CELL_RADIUS with one query per lane: the same rows and
+// the same order of the results.  A warp per query spends its instructions on
+// finding the query's bins and on mapping lanes to them (300 for 110 points); a
+// lane per query does that once for 32 queries.  Further:
+//   - The bins come from FP32 places; what is too near a boundary is looked up.
+//   - Only bins that the ball reaches are read (85 points instead of 110 with a
+//     radius of one bin).
+//   - The rows are listed first; then each lane goes through its own points,
+//     four at a time, whatever row the others are at.
+//   - A counting pass of real radius queries also lists each query's first
+//     p.stage_len results, so that only the queries with more of them are found
+//     again by a second pass (542 -> 421 us).
+//   - A long row of a few lanes (clusters) is taken by the whole warp.
+// 1,000,000 queries with 16 results each among 1,000,000 points: the two passes
+// 1,650 us by warps; this one 225 and k_radius_place 45.  Bound by the latency
+// and the wavefronts of the scattered 16-byte reads (L1 63% busy, issue 55%):
+// 24 warps per SM; 20 and 28 are no faster, nor is reading four points ahead.
+template <int MODE, bool FILL>
+__global__ void __launch_bounds__(kLaneThreads, 6) k_radius_lane(RadiusParams p) {
+    static_assert(MODE == RQ_REAL_RADIUS || MODE == RQ_CELL_RADIUS, "other queries take a warp each");
+    constexpr bool REAL = MODE == RQ_REAL_RADIUS;
+    __shared__ uint2 rows[kLaneRows][kLaneThreads];
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const uint64_t at = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    bool have = at < p.nq;
+    const uint32_t q = have ? (p.qorder ? p.qorder[at] : (uint32_t)at) : 0u;
+    if (FILL && have && p.stage_len) have = p.count[q] > p.stage_len;   // (the others are listed)
+    if (!__any_sync(kFull, have)) return;
+    const DiagDesc& D = p.desc[0];
+    const int cpd = D.cpd;
+    const uint64_t bin_base = D.bin_base;
+    const uint32_t pt_base = D.pt_base;
+    const double x = p.qxyz[3 * (size_t)q], y = p.qxyz[3 * (size_t)q + 1], z = p.qxyz[3 * (size_t)q + 2];
+    const float fr = (float)p.radius, r2f = (float)sq_rn(p.radius);
+
+    // The query in FP32, relative to the diagram's centre and in bins.  Its place
+    // in bins is known within feps: 2^-23 of the position, 2^-24 of the corner
+    // and three roundings, at most 6 2^-24 cpd on the grid (8 taken), in
+    // proportion off it; the same for the radius; and the FP64 rounding of c - r.
+    const float qx = f64_to_f32_rz(__dadd_rn(x, -D.ctr[0])), qy = f64_to_f32_rz(__dadd_rn(y, -D.ctr[1])),
+                qz = f64_to_f32_rz(__dadd_rn(z, -D.ctr[2]));
+    const float px = (qx - D.glo_hi[0]) * D.inv_s[0], py = (qy - D.glo_hi[1]) * D.inv_s[1], pz = (qz - D.glo_hi[2]) * D.inv_s[2];
+    const float away = fabsf(px) + fabsf(py) + fabsf(pz);
+    const float inv_most = fmaxf(D.inv_s[0], fmaxf(D.inv_s[1], D.inv_s[2]));
+    const float glo_most = fmaxf(fabsf(D.glo_f[0]), fmaxf(fabsf(D.glo_f[1]), fabsf(D.glo_f[2])));
+    const float feps = 8.0f * 5.9604645e-8f * (float)cpd + 1e-6f + 1e-6f * away + 4e-7f * fabsf(fr) * inv_most +
+                       1e-15f * glo_most * inv_most;
+    const bool grid = D.lean_ok && D.inv_s[0] > 0.f && D.inv_s[1] > 0.f && D.inv_s[2] > 0.f && away < 1e6f && feps < 0.25f;
+
+    // the query's bin and the box's ends.  A place further than feps from the
+    // bin boundaries between 1 and cpd - 1 has its index; the others are
+    // looked up.
+    unsigned open = 0;
+    auto index = [&](float u, int bit) {
+        const float f = floorf(u), fr_ = u - f;
+        const bool inner = u > 1.f - feps && u < (float)(cpd - 1) + feps;
+        if (!grid || !(u == u) || (inner && (fr_ < feps || fr_ > 1.f - feps))) open |= 1u << bit;
+        return min(max((int)f, 0), cpd - 1);
+    };
+    const float rx = fr * D.inv_s[0], ry = fr * D.inv_s[1], rz = fr * D.inv_s[2];
+    int xi = index(px, 0), i0 = index(px - rx, 1), i1 = index(px + rx, 2);
+    int yi = index(py, 3), j0 = index(py - ry, 4), j1 = index(py + ry, 5);
+    int zi = index(pz, 6), k0 = index(pz - rz, 7), k1 = index(pz + rz, 8);
+    if (open) {
+        int top = 1;
+        while (2 * top < cpd) top *= 2;
+#pragma unroll 1
+        for (; open; open &= open - 1u) {
+            const int bit = __ffs(open) - 1, a = bit / 3;
+            const int v = exact_index(p, p.qxyz[3 * (size_t)q + a], a, bit - 3 * a, top);
+            if (bit == 0) xi = v;
+            if (bit == 1) i0 = v;
+            if (bit == 2) i1 = v;
+            if (bit == 3) yi = v;
+            if (bit == 4) j0 = v;
+            if (bit == 5) j1 = v;
+            if (bit == 6) zi = v;
+            if (bit == 7) k0 = v;
+            if (bit == 8) k1 = v;
+        }
+    }
+
+    // FP32 filter: the error band of k_radius (the distance is summed from
+    // -r^2 up, the same roundings)
+    float band = INFINITY;      // nothing decided in FP32
+    bool filter = false;
+    if (REAL && p.f32_filter) {
+        float m = fmaxf(fmaxf(fabsf(qx), fabsf(qy)), fabsf(qz));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) m = fmaxf(m, fmaxf(fabsf(D.glo_hi[a]), fabsf(D.glo_hi[a] + D.size_f[a] * (float)cpd)));
+        m *= 1.0001f;
+        const float e = 6.0e-8f * (3.0f * m + 2.1f * fr);
+        filter = m < 1.0e18f;
+        if (filter) band = 2.0f * (3.5f * fr * e + 3.0f * e * e) + 1.0e-6f * r2f;
+    }
+    // Real radius: of the box's bins only those that the ball may reach.
+    const bool tight = REAL && filter && grid;
+    // A bin whose gap distance is beyond the radius is beyond the ball, so the gap
+    // test leaves nothing out that the ball does not, unless some gap distance
+    // is the radius to within the ball's margin (in squares 5e-4 and 6 feps).
+    const bool gaps = !tight || !p.gtab || p.gtab_tie || !(feps < 1e-3f);
+    const float fx = fminf(fmaxf(px - (float)xi, 0.f), 1.f), fy = fminf(fmaxf(py - (float)yi, 0.f), 1.f);
+    const float sx = D.size_f[0], sy = D.size_f[1], inz = D.inv_s[2];
+
+    // the results' places: one after the other, or (listed) a warp's first
+    // results, its second ones, ... side by side
+    constexpr uint32_t kStep = FILL ? 1 : 32;
+    using Place = std::conditional_t<FILL, uint64_t, uint32_t>;     // (the lists have at most 2^31 entries)
+    Place out = 0, end = 0;
+    uint32_t cnt = 0;
+    if (FILL && have) out = p.offs[q];
+    if (!FILL && have) {
+        out = (uint32_t)(at - lane) * p.stage_len + lane;
+        end = out + 32 * p.stage_len;
+    }
+    uint32_t* const results = FILL ? p.out : p.stage;
+    const int ny = j1 - j0 + 1, nx = i1 - i0 + 1;
+    const int nrows = have && nx > 0 && ny > 0 && k1 >= k0 ? nx * ny : 0;
+    const int gz_need = max(max(zi - k0, k1 - zi) - 1, 0);
+    int i = i0, j = j0;
+    // the points of row (i, j) that the query has to look at; on to the next row
+    auto row = [&](uint32_t& beg, uint32_t& c) {
+        const int di = i - xi, dj = j - yi;
+        const uint32_t first = ((uint32_t)i * (uint32_t)cpd + (uint32_t)j) * (uint32_t)cpd;
+        if (++j > j1) {
+            j = j0;
+            ++i;
+        }
+        int kl = k0, kh = k1;
+        if (tight) {
+            const float dx = fmaxf((di > 0 ? (float)di - fx : (di < 0 ? (float)(-di - 1) + fx : 0.f)) - feps, 0.f) * sx;
+            const float dy = fmaxf((dj > 0 ? (float)dj - fy : (dj < 0 ? (float)(-dj - 1) + fy : 0.f)) - feps, 0.f) * sy;
+            const float rem = r2f * 1.0003f - (dx * dx + dy * dy);
+            if (!(rem > 0.f)) return;
+            const float zr = fminf(sqrt_near(rem) * inz * 1.0001f + 2.f * feps, 4e6f);
+            kl = max(kl, (int)floorf(pz - zr));
+            kh = min(kh, (int)floorf(pz + zr));
+        }
+        if (gaps) {
+            const int gx = max(abs(di) - 1, 0), gy = max(abs(dj) - 1, 0);
+            int T = -1, from = 0;
+            if (p.gtab && gx <= p.gtab_x && gy <= p.gtab_y) {
+                T = __ldg(p.gtab + gx * (p.gtab_y + 1) + gy);
+                from = T == p.gtab_z ? p.gtab_z + 1 : gz_need + 1;
+            }
+            for (int gz = from; gz <= gz_need; ++gz) {
+                if (!(gap_ds(gx, gy, gz, D.size[0], D.size[1], D.size[2]) <= sq_rn(p.radius))) break;
+                T = gz;
+            }
+            kl = max(kl, zi - T - 1);
+            kh = min(kh, zi + T + 1);
+            if (T < 0) return;
+        }
+        if (kl > kh) return;
+        beg = p.delims[bin_base + first + (uint32_t)kl];
+        c = p.delims[bin_base + first + (uint32_t)kh + 1] - beg;
+    };
+    // the first c points from s on, four at most: which are results.  (Reads all
+    // four: the array has three entries more than points.)
+    auto load = [&](uint32_t s, float4 (&h)[4]) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) h[k] = p.phi[s + k];
+    };
+    auto test = [&](uint32_t s, uint32_t c, const float4 (&h)[4]) {
+        const unsigned all = c >= 4 ? 15u : (1u << c) - 1u;
+        if (!REAL) return all;
+        // t = d^2 - r^2; a result has t < 0, |t| within the band decides nothing
+        unsigned in = 0;
+        float t[4], least = filter ? INFINITY : 0.f;
+#pragma unroll
+        for (int k = 3; k >= 0; --k) {
+            const float dx = __fsub_rn(qx, h[k].x), dy = __fsub_rn(qy, h[k].y), dz = __fsub_rn(qz, h[k].z);
+            t[k] = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmaf_rn(dz, dz, -r2f)));
+            in = __funnelshift_l(__float_as_uint(t[k]), in, 1);
+            least = fminf(least, fabsf(t[k]));
+        }
+        in &= all;
+        if (least <= band)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (!(fabsf(t[k]) > band) && ((all >> k) & 1u))
+                    in = (in & ~(1u << k)) | (exact_query(p, q, s + k) ? 1u << k : 0u);
+        return in;
+    };
+    auto put = [&](unsigned ok, const float4 (&h)[4]) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (((ok >> u) & 1u) && (FILL || out < end)) {
+                results[out] = __float_as_uint(h[u].w) - pt_base;
+                out += kStep;
+            }
+        cnt += __popc(ok);
+    };
+    const int most = __reduce_max_sync(kFull, nrows);
+#pragma unroll 1
+    for (int t0 = 0; t0 < most; t0 += kLaneRows) {
+        // ---- the next rows that hold points ----
+        int n = 0;
+        bool has_long = false;
+#pragma unroll 1
+        for (int t = t0; t < min(t0 + kLaneRows, nrows); ++t) {
+            uint32_t beg = 0, c = 0;
+            row(beg, c);
+            if (!REAL && !FILL) {
+                cnt += c;
+            } else if (c) {
+                rows[n++][threadIdx.x] = make_uint2(beg, c);
+                has_long |= c >= kLongRun;
+            }
+        }
+        if (!REAL && !FILL) continue;
+        if (!__any_sync(kFull, has_long)) {
+            // ---- each lane its own points, four at a time ----
+            int k = 0;
+            uint32_t s = 0, c = 0;
+            uint2 e = k < n ? rows[k++][threadIdx.x] : make_uint2(0u, 0u);
+            for (;;) {
+                if (c == 0) {
+                    s = e.x;
+                    c = e.y;
+                    if (c == 0) break;
+                    e = k < n ? rows[k++][threadIdx.x] : make_uint2(0u, 0u);
+                }
+                float4 h[4];
+                load(s, h);
+                put(test(s, c, h), h);
+                s += 4;
+                c = c > 4 ? c - 4 : 0;
+            }
+            __syncwarp();
+            continue;
+        }
+        // ---- row by row; a long row of a few lanes is taken by the warp ----
+        const int rounds = __reduce_max_sync(kFull, n);
+#pragma unroll 1
+        for (int k = 0; k < rounds; ++k) {
+            const uint2 e = k < n ? rows[k][threadIdx.x] : make_uint2(0, 0);
+            uint32_t c = e.y;
+            unsigned longs = __ballot_sync(kFull, c >= kLongRun);
+            if (__popc(longs) <= 16) {
+                if (c >= kLongRun) c = 0;
+#pragma unroll 1
+                for (; longs; longs &= longs - 1u) {
+                    const int src = __ffs(longs) - 1;
+                    const uint32_t sb = __shfl_sync(kFull, e.x, src), sc = __shfl_sync(kFull, e.y, src);
+                    const uint32_t uq = __shfl_sync(kFull, q, src);
+                    const float vx = __shfl_sync(kFull, qx, src), vy = __shfl_sync(kFull, qy, src), vz = __shfl_sync(kFull, qz, src);
+                    const float vb = __shfl_sync(kFull, band, src);
+                    const Place o = __shfl_sync(kFull, out, src), oe = __shfl_sync(kFull, end, src);
+                    uint32_t found = 0;
+#pragma unroll 1
+                    for (uint32_t b = 0; b < sc; b += 32) {
+                        const uint32_t s = sb + b + lane;
+                        bool ok = b + lane < sc;
+                        float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (ok) {
+                            h = p.phi[s];
+                            if (REAL) {
+                                const float dx = __fsub_rn(vx, h.x), dy = __fsub_rn(vy, h.y), dz = __fsub_rn(vz, h.z);
+                                const float t = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmaf_rn(dz, dz, -r2f)));
+                                ok = fabsf(t) > vb ? t < 0.f : exact_query(p, uq, s);
+                            }
+                        }
+                        const unsigned bal = __ballot_sync(kFull, ok);
+                        const uint64_t to = o + (uint64_t)(found + __popc(bal & lt)) * kStep;
+                        if (ok && (FILL || to < oe)) results[to] = __float_as_uint(h.w) - pt_base;
+                        found += __popc(bal);
+                    }
+                    if (lane == src) {
+                        out = FILL ? o + found : (Place)min((uint64_t)oe, o + (uint64_t)found * kStep);
+                        cnt += found;
+                    }
+                }
+            }
+#pragma unroll 1
+            for (uint32_t b = 0; b < c; b += 4) {
+                float4 h[4];
+                load(e.x + b, h);
+                put(test(e.x + b, c - b, h), h);
+            }
+            __syncwarp();
+        }
+    }
+    if (!FILL && have) {
+        p.count[q] = cnt;
+        if (p.stage_len && cnt > p.stage_len) p.err[1] = 1;     // left to a second pass
+    }
+}
+
+// The listed results to their places: a warp takes the lists of a warp of
+// k_radius_lane, 32 results of each at a time, through shared memory, so that
+// both sides are read and written in runs.
+__global__ void __launch_bounds__(kLaneThreads) k_radius_place(RadiusParams p) {
+    __shared__ uint32_t tiles[kLaneThreads / 32][32][33];
+    uint32_t(*tile)[33] = tiles[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const uint64_t at = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t c = 0;
+    unsigned long long to = 0;
+    if (at < p.nq) {
+        const uint32_t q = p.qorder ? p.qorder[at] : (uint32_t)at;
+        c = p.count[q];
+        to = p.offs[q];
+        if (c > p.stage_len) c = 0;
+    }
+    const uint32_t most = __reduce_max_sync(kFull, c);
+    const uint32_t* from = p.stage + (at - lane) * p.stage_len + lane;
+#pragma unroll 1
+    for (uint32_t k0 = 0; k0 < most; k0 += 32) {
+#pragma unroll 8
+        for (uint32_t k = 0; k < 32; ++k)
+            if (k0 + k < c) tile[k][lane] = from[(size_t)(k0 + k) * 32];
+        __syncwarp();
+        const uint32_t k = lane & 15;
+#pragma unroll 4
+        for (int j = 0; j < 32; j += 2) {
+            const int src = j + (lane >> 4);
+            const uint32_t n = __shfl_sync(kFull, c, src);
+            uint32_t* const o = p.out + __shfl_sync(kFull, to, src) + k0;
+            if (k0 + k < n) o[k] = tile[k][src];
+            if (k0 + k + 16 < n) o[k + 16] = tile[k + 16][src];
+        }
+        __syncwarp();
+    }
+}
+
 // Position of query wq (a given position, or the position of a given cell).
 __device__ __forceinline__ bool query_position(const RadiusParams& p, uint32_t wq, double& x, double& y, double& z) {
     if (p.qxyz) {
@@ -419,14 +782,12 @@ __global__ void __launch_bounds__(256) k_query_bin(RadiusParams p, QueryOrder o)
         double x = 0.0, y = 0.0, z = 0.0;
         uint32_t c = 0;
         if (query_position(p, q, x, y, z)) {
-            int top = 1;
-            while (2 * top < D.cpd) top *= 2;
-            const uint32_t ix =
-                (uint32_t)axis_index_table((unsigned long long)__double_as_longlong(x), p.bnd, D.cpd, top) >> shift;
-            const uint32_t iy = (uint32_t)axis_index_table((unsigned long long)__double_as_longlong(y),
-                                                           p.bnd + D.cpd, D.cpd, top) >> shift;
-            const uint32_t iz = (uint32_t)axis_index_table((unsigned long long)__double_as_longlong(z),
-                                                           p.bnd + 2 * D.cpd, D.cpd, top) >> shift;
+            // (the order is for locality only: FP32 places)
+            auto place = [&](double v, int a) {
+                const float u = (f64_to_f32_rz(__dadd_rn(v, -D.ctr[a])) - D.glo_hi[a]) * D.inv_s[a];
+                return (uint32_t)min(max((int)u, 0), D.cpd - 1) >> shift;
+            };
+            const uint32_t ix = place(x, 0), iy = place(y, 1), iz = place(z, 2);
             c = (ix * (uint32_t)o.cpdc + iy) * (uint32_t)o.cpdc + iz;
         }
         o.qbin[q] = c;
@@ -441,6 +802,21 @@ __global__ void __launch_bounds__(256) k_query_scatter(uint32_t nq, QueryOrder o
 
 template <int MODE>
 cudaError_t launch_mode(const RadiusParams& p, bool fill, int blocks, cudaStream_t s) {
+    if constexpr (MODE == RQ_REAL_RADIUS || MODE == RQ_CELL_RADIUS) {
+        if (p.nq >= kLaneMin) {
+            const unsigned nb = (unsigned)(((uint64_t)p.nq + kLaneThreads - 1) / kLaneThreads);
+            if (fill && p.stage_len) {
+                k_radius_place<<<nb, kLaneThreads, 0, s>>>(p);
+                const cudaError_t e = cudaGetLastError();
+                if (e != cudaSuccess || !p.unlisted) return e;
+            }
+            if (fill)
+                k_radius_lane<MODE, true><<<nb, kLaneThreads, 0, s>>>(p);
+            else
+                k_radius_lane<MODE, false><<<nb, kLaneThreads, 0, s>>>(p);
+            return cudaGetLastError();
+        }
+    }
     if (fill)
         k_radius<MODE, true><<<blocks, 256, 0, s>>>(p);
     else
@@ -487,6 +863,14 @@ struct RadiusEntry {
 };
 
 }  // namespace
+
+uint32_t radius_stage_len(int mode, uint32_t nq, uint32_t n, const DiagDesc& D, double radius) {
+    if (mode != RQ_REAL_RADIUS || nq < kLaneMin) return 0;
+    double mean = n * 4.1887902047863910 * radius * radius * radius;
+    for (int a = 0; a < 3; ++a) mean /= D.size[a] * D.cpd;
+    if (!(mean >= 0.0 && mean <= 200.0)) return 0;
+    return ((uint32_t)(1.6 * mean) + 16 + 7) / 8 * 8;
+}
 
 cudaError_t launch_radius(const RadiusParams& p, int mode, bool fill, int blocks, cudaStream_t s) {
     if (p.nq == 0) return cudaSuccess;
@@ -548,7 +932,8 @@ bool build_radius_table(const double size[3], int cpd, double radius, size_t max
 }
 
 bool build_gap_table(const double size[3], const double inv[3], int cpd, double radius, size_t max_entries,
-                     std::vector<int16_t>& out, int* gx, int* gy, int* gz) {
+                     std::vector<int16_t>& out, int* gx, int* gy, int* gz, bool* tie) {
+    *tie = false;
     if (!(radius >= 0.0) || std::isinf(radius)) return false;
     // The box of find_cells_in_radius spans at most ceil(r * inv) + 1 bins on
     // either side of the query's bin, so gaps stay below ceil(r * inv) + 1.
@@ -565,7 +950,11 @@ bool build_gap_table(const double size[3], const double inv[3], int cpd, double 
         for (int j = 0; j <= g[1]; ++j) {
             int best = -1;
             for (int k = 0; k <= g[2]; ++k) {           // the distance grows with k
-                if (!(host_gap_ds(size, i, j, k) <= r2)) break;
+                const double ds = host_gap_ds(size, i, j, k);
+                if (!(ds <= r2)) {
+                    *tie = *tie || !(ds > r2 * 1.01);
+                    break;
+                }
                 best = k;
             }
             out[(size_t)i * (size_t)(g[1] + 1) + (size_t)j] = (int16_t)best;
