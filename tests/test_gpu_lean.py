@@ -1,6 +1,7 @@
 """The FP32 passes on the point sets where their walk over rows of bins can go wrong: axes without extent, oblong
 grids, sparse regions that need rings of rows far out (more rows than lanes in a ring), sizes around a window of 32
-candidates and around the size from which the plain, dense and careful passes share the work, extents outside FP32's
+candidates and around the size from which the plain, dense and careful passes share the work, lone points beside a cloud
+of thousands (handed on for the length of their batches), extents outside FP32's
 range, and a search radius, all against the FP64 oracle with the bars of the parity tests (neighbour lists bit-exact;
 volumes 1e-6 relative in FP32, 1e-12 in MIXED and FP64)."""
 import os
@@ -52,6 +53,7 @@ SETS = {
     "oblong_z": (lambda: _rng(7).random((3000, 3)) * [0.5, 1, 20], (0.5, 1, 20)),
     "clumps_few": (lambda: _clumps(1500, 4, 8), (1, 1, 1)),
     "clumps_many": (lambda: _clumps(20000, 60, 9), (1, 1, 1)),
+    "beside_cloud": (lambda: _clumps(12000, 2, 12, size=0.15, lone=2000), (1, 1, 1)),
     "lone_corner": (lambda: np.concatenate([0.9 + 0.1 * _rng(10).random((4000, 3)), [[0.01, 0.02, 0.03]]]), (1, 1, 1)),
 }
 
