@@ -43,6 +43,7 @@ __device__ unsigned long long block_excl_scan64(unsigned long long v, unsigned l
 
 __global__ void __launch_bounds__(kCsrThreads) k_csr_partial(const uint32_t* cnt, uint32_t n,
                                                              unsigned long long* sums) {
+    after_previous();
     __shared__ unsigned long long sh[33];
     const uint64_t base = ((uint64_t)blockIdx.x * kCsrThreads + threadIdx.x) * kCsrItems;
     unsigned long long s = 0;
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(kCsrThreads) k_csr_partial(const uint32_t* cnt
 }
 
 __global__ void __launch_bounds__(kCsrThreads) k_csr_sums(unsigned long long* sums, uint32_t nb) {
+    after_previous();
     __shared__ unsigned long long sh[33];
     unsigned long long carry = 0;
     for (uint32_t b0 = 0; b0 < nb; b0 += kCsrThreads) {
@@ -70,6 +72,7 @@ __global__ void __launch_bounds__(kCsrThreads) k_csr_sums(unsigned long long* su
 
 __global__ void __launch_bounds__(kCsrThreads) k_csr_final(const uint32_t* cnt, uint32_t n,
                                                            const unsigned long long* sums, uint64_t* offs) {
+    after_previous();
     __shared__ unsigned long long sh[33];
     const uint64_t base = ((uint64_t)blockIdx.x * kCsrThreads + threadIdx.x) * kCsrItems;
     uint32_t v[kCsrItems];
@@ -124,6 +127,7 @@ template <int C>
 __global__ void __launch_bounds__(256) k_csr_gather(const uint32_t* cnt, const uint64_t* fstart,
                                                     const int32_t* fnbr, const double* farea, uint32_t n,
                                                     const uint64_t* offs, int32_t* nbr, double* area) {
+    after_previous();
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const uint64_t c0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * C;
@@ -195,8 +199,8 @@ cudaError_t launch_csr_offsets(const uint32_t* nface, uint32_t n, uint64_t* offs
     const uint32_t nb = (uint32_t)((n + per - 1) / per);
     unsigned long long* sums = reinterpret_cast<unsigned long long*>(scan_tmp);
     k_csr_partial<<<nb, kCsrThreads, 0, s>>>(nface, n, sums);
-    k_csr_sums<<<1, kCsrThreads, 0, s>>>(sums, nb);
-    k_csr_final<<<nb, kCsrThreads, 0, s>>>(nface, n, sums, offs);
+    launch_after(k_csr_sums, 1, kCsrThreads, 0, s, sums, nb);
+    launch_after(k_csr_final, nb, kCsrThreads, 0, s, nface, n, sums, offs);
     return cudaGetLastError();
 }
 
@@ -206,9 +210,9 @@ cudaError_t launch_csr_gather(const uint32_t* nface, const uint64_t* fstart, con
     const uint64_t warps = n >= kCsrWide ? ((uint64_t)n + 31) / 32 : ((uint64_t)n + 3) / 4;
     const unsigned blocks = (unsigned)((warps + 7) / 8);
     if (n >= kCsrWide)
-        k_csr_gather<32><<<blocks, 256, 0, s>>>(nface, fstart, face_nbr, face_area, n, offs, nbr_out, area_out);
+        launch_after(k_csr_gather<32>, blocks, 256, 0, s, nface, fstart, face_nbr, face_area, n, offs, nbr_out, area_out);
     else
-        k_csr_gather<4><<<blocks, 256, 0, s>>>(nface, fstart, face_nbr, face_area, n, offs, nbr_out, area_out);
+        launch_after(k_csr_gather<4>, blocks, 256, 0, s, nface, fstart, face_nbr, face_area, n, offs, nbr_out, area_out);
     return cudaGetLastError();
 }
 

@@ -1493,6 +1493,7 @@ __device__ void run_cell(const ClipParams& P, Smem<K>& S, uint32_t gs, int lane,
 // K = 2: 8 warps per block, two blocks per SM (registers capped at 128).
 template <int K, bool GEO>
 __global__ void __launch_bounds__(K == 2 ? 256 : 128, K == 2 ? 2 : 1) k_clip(ClipParams P) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smraw[];
     Smem<K>& S = reinterpret_cast<Smem<K>*>(smraw)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -1542,8 +1543,7 @@ cudaError_t launch_t(const ClipParams& p, int wpb, int blocks, cudaStream_t s) {
     const size_t sm = sizeof(Smem<K>) * (size_t)wpb;
     cudaError_t e = configure_smem<K, GEO>(sm);
     if (e != cudaSuccess) return e;
-    k_clip<K, GEO><<<blocks, 32 * wpb, sm, s>>>(p);
-    return cudaGetLastError();
+    return launch_after(k_clip<K, GEO>, blocks, 32 * wpb, sm, s, p);
 }
 
 template <int K, bool GEO>

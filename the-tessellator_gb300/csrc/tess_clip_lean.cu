@@ -1451,6 +1451,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
 // with 24 (80 registers, 19% more instructions and the instruction cache full).
 template <bool EXACT, int MODE>
 __global__ void __launch_bounds__(128, MODE == kCareful ? 4 : 5) k_lean(ClipParams P) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smraw[];
     Lean& S = reinterpret_cast<Lean*>(smraw)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -1531,8 +1532,7 @@ cudaError_t launch(const ClipParams& p, int wpb, int blocks, cudaStream_t s) {
     const size_t sm = sizeof(Lean) * (size_t)wpb;
     cudaError_t e = configure<EXACT, MODE>(sm);
     if (e != cudaSuccess) return e;
-    k_lean<EXACT, MODE><<<blocks, 32 * wpb, sm, s>>>(p);
-    return cudaGetLastError();
+    return launch_after(k_lean<EXACT, MODE>, blocks, 32 * wpb, sm, s, p);
 }
 
 template <bool EXACT, int MODE>

@@ -120,6 +120,7 @@ __device__ bool last_block(unsigned* ticket) {
 // error_flag.  A single diagram's grid parameters are computed by the last
 // block (a launch of their own takes 5 us, 2% of a 1,000-point pass).
 __global__ void __launch_bounds__(kBoundsThreads) k_bounds(GridBuffers g) {
+    after_previous();
     __shared__ unsigned long long red[6][kBoundsThreads / 32];
     for (uint32_t c = blockIdx.x; c < g.nchunks; c += gridDim.x) {
         const uint32_t d = g.chunk_diag[c];
@@ -266,6 +267,7 @@ constexpr uint64_t kScanLastMax = 4096, kScanOneMax = 16384;
 
 // get_cells (celery.rs:342-354) + histogram.  rank = arrival order in the bin.
 __global__ void __launch_bounds__(256) k_bin_count(GridBuffers g) {
+    after_previous();
     for (uint32_t c = blockIdx.x; c < g.nchunks; c += gridDim.x) {
         const uint32_t d = g.chunk_diag[c];
         const uint32_t beg = g.chunk_start[c];
@@ -295,6 +297,7 @@ __global__ void __launch_bounds__(256) k_bin_count(GridBuffers g) {
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_partial(uint32_t* data, uint64_t n, uint32_t* sums) {
+    after_previous();
     __shared__ uint32_t sh[33];
     const uint64_t base = (uint64_t)blockIdx.x * kScanThreads * kScanItems + (uint64_t)threadIdx.x * kScanItems;
     uint32_t s = 0;
@@ -305,6 +308,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_partial(uint32_t* data, u
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_sums(uint32_t* sums, uint32_t nblocks) {
+    after_previous();
     __shared__ uint32_t sh[33];
     uint32_t carry = 0;
     for (uint32_t b0 = 0; b0 < nblocks; b0 += kScanThreads) {
@@ -318,6 +322,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(uint32_t* sums, uint
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_final(uint32_t* data, uint64_t n, const uint32_t* sums) {
+    after_previous();
     __shared__ uint32_t sh[33];
     const uint64_t base = (uint64_t)blockIdx.x * kScanThreads * kScanItems + (uint64_t)threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
@@ -336,12 +341,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_final(uint32_t* data, uin
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_one(uint32_t* data, uint32_t n) {
+    after_previous();
     __shared__ uint32_t sh[33];
     scan_by_block(data, n, sh);
 }
 
 // get_sorted_indices (celery.rs:357-369): counting-sort scatter.
 __global__ void k_scatter(GridBuffers g) {
+    after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.total) return;
     const uint32_t b = tess_chk(g.bin[i], g.total_bins, g.check, CK_GRID);
@@ -394,6 +401,7 @@ __device__ void block_bitonic_sort(uint32_t* a, I n) {
 // in shared memory up to kSortSmem points, in place beyond.
 constexpr uint32_t kSortSmem = 4096;
 __global__ void __launch_bounds__(256) k_bin_order(GridBuffers g) {
+    after_previous();
     __shared__ uint32_t big[256];
     __shared__ uint32_t nbig;
     __shared__ uint32_t buf[kSortSmem];
@@ -474,6 +482,7 @@ __device__ __forceinline__ bool split_rn_int(double u, float& hi, float& lo) {
 // centre: the split keeps 48 bits of that offset, so its error scales with
 // the diagram's extent rather than with the coordinates' distance from 0.
 __global__ void k_gather(GridBuffers g) {
+    after_previous();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.total) return;
     const uint32_t i = tess_chk(g.sorted[s], g.total, g.check, CK_GRID);
@@ -682,7 +691,8 @@ cudaError_t launch_inverse(const uint32_t* sorted, uint32_t* inv, uint32_t n, in
 // Bulk copy by the SMs: 16-byte loads and stores, grid-stride, then the tail
 // byte by byte.  Either side may be pinned host memory (its device address):
 // the SMs then move the bytes over the host link themselves.
-__global__ void k_copy_bytes(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, size_t n) {
+__global__ void k_copy_bytes(const uint8_t* src, uint8_t* dst, size_t n) {
+    after_previous();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t n16 = n / 16;
@@ -698,8 +708,7 @@ cudaError_t launch_copy_bytes(void* dst, const void* src, size_t n, int sms, cud
     // to fill the host link (≈ 192 GB/s measured either way)
     const size_t want = (n / 16 + 255) / 256;
     const int blocks = (int)std::max<size_t>(1, std::min<size_t>(want, (size_t)4 * (sms > 0 ? sms : 152)));
-    k_copy_bytes<<<blocks, 256, 0, s>>>(static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), n);
-    return cudaGetLastError();
+    return launch_after(k_copy_bytes, blocks, 256, 0, s, static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), n);
 }
 
 cudaError_t launch_occupancy(const uint32_t* delims, uint64_t nbins, uint32_t crowd, unsigned long long* out,
@@ -722,7 +731,7 @@ cudaError_t launch_grid_build(const GridBuffers& g, cudaStream_t s, cudaStream_t
     const uint64_t nclear = std::max<uint64_t>(6ull * ndiag, g.total_bins + 1);
     k_grid_clear<<<(unsigned)std::min<uint64_t>((nclear + 1023) / 1024, 152u * 8u), 256, 0, s>>>(g);
     const int cblocks = (int)(g.nchunks < 4096u ? g.nchunks : 4096u);
-    k_bounds<<<cblocks, kBoundsThreads, 0, s>>>(g);
+    launch_after(k_bounds, cblocks, kBoundsThreads, 0, s, g);
     if (ndiag > 1) k_grid_params<<<(4 * ndiag + 127) / 128, 128, 0, s>>>(g);   // else by k_bounds
     if (bounds_done) cudaEventRecord(bounds_done, s);
     // the shell tables need only the grid parameters: build them beside the
@@ -736,22 +745,22 @@ cudaError_t launch_grid_build(const GridBuffers& g, cudaStream_t s, cudaStream_t
     } else {
         k_table<<<ndiag, kTabThreads, 0, s>>>(g);
     }
-    k_bin_count<<<cblocks, 256, 0, s>>>(g);
+    launch_after(k_bin_count, cblocks, 256, 0, s, g);
     const uint64_t nscan = g.total_bins + 1;
     const uint64_t per = (uint64_t)kScanThreads * kScanItems;
     const uint32_t nblk = (uint32_t)((nscan + per - 1) / per);
     if (nscan <= kScanLastMax) {
         // by k_bin_count
     } else if (nscan <= kScanOneMax) {
-        k_scan_one<<<1, kScanThreads, 0, s>>>(g.delims, (uint32_t)nscan);
+        launch_after(k_scan_one, 1, kScanThreads, 0, s, g.delims, (uint32_t)nscan);
     } else {
-        k_scan_partial<<<nblk, kScanThreads, 0, s>>>(g.delims, nscan, g.scan_tmp);
-        k_scan_sums<<<1, kScanThreads, 0, s>>>(g.scan_tmp, nblk);
-        k_scan_final<<<nblk, kScanThreads, 0, s>>>(g.delims, nscan, g.scan_tmp);
+        launch_after(k_scan_partial, nblk, kScanThreads, 0, s, g.delims, nscan, g.scan_tmp);
+        launch_after(k_scan_sums, 1, kScanThreads, 0, s, g.scan_tmp, nblk);
+        launch_after(k_scan_final, nblk, kScanThreads, 0, s, g.delims, nscan, g.scan_tmp);
     }
-    k_scatter<<<(g.total + 255) / 256, 256, 0, s>>>(g);
-    k_bin_order<<<(unsigned)((g.total_bins + 255) / 256), 256, 0, s>>>(g);
-    k_gather<<<(g.total + 255) / 256, 256, 0, s>>>(g);
+    launch_after(k_scatter, (g.total + 255) / 256, 256, 0, s, g);
+    launch_after(k_bin_order, (unsigned)((g.total_bins + 255) / 256), 256, 0, s, g);
+    launch_after(k_gather, (g.total + 255) / 256, 256, 0, s, g);
     if (forked) cudaStreamWaitEvent(s, join, 0);
     return cudaGetLastError();
 }
