@@ -211,22 +211,17 @@ struct Engine {
     size_t rq_cap = 0;
     uint32_t* d_rcell = nullptr;
     size_t rcell_cap = 0;
-    uint32_t* d_rcnt = nullptr;
-    size_t rcnt_cap = 0;
-    uint64_t* d_roffs = nullptr;
-    size_t roffs_cap = 0;
-    uint64_t* d_rtmp = nullptr;
-    size_t rtmp_cap = 0;
+    // offsets, scan scratch, error words, counts and listed results of a query in
+    // one block (an allocation costs a first query 13 to 60 us)
+    uint64_t* d_rwork = nullptr;
+    size_t rwork_cap = 0;
     uint32_t* d_rout = nullptr;
-    uint32_t* d_rstage = nullptr; // results listed by the first pass
-    size_t rstage_cap = 0;
     size_t rout_cap = 0;
     short4* d_rtab = nullptr;
     size_t rtab_cap = 0;
     uint32_t rtab_len = 0;
     bool rtab_valid = false;
     uint64_t rtab_radius_bits = 0;
-    int* d_rerr = nullptr;
     int sm_count = 0;
     unsigned long long* d_bnd = nullptr;   // bin boundaries per axis (3 x cpd order codes)
     size_t bnd_cap = 0;
@@ -298,8 +293,8 @@ struct Engine {
         h_ret = nullptr;
         for (auto& l : d_list) dfree(l);
         dfree(d_counters); dfree(d_work); dfree(d_offs); dfree(d_cnbr); dfree(d_carea); dfree(d_csr_tmp);
-        dfree(d_rq); dfree(d_rcell); dfree(d_rcnt); dfree(d_roffs); dfree(d_rtmp); dfree(d_rstage); dfree(d_rout); dfree(d_rtab);
-        dfree(d_rerr); dfree(d_gtab); dfree(d_bnd); dfree(d_qbin); dfree(d_qrank); dfree(d_qorder); dfree(d_qcnt); dfree(d_qcoff); dfree(d_qtmp);
+        dfree(d_rq); dfree(d_rcell); dfree(d_rwork); dfree(d_rout); dfree(d_rtab);
+        dfree(d_gtab); dfree(d_bnd); dfree(d_qbin); dfree(d_qrank); dfree(d_qorder); dfree(d_qcnt); dfree(d_qcoff); dfree(d_qtmp);
         dfree(d_sample); dfree(d_occ);
         if (own_stream && stream) cudaStreamDestroy(stream);
         stream = nullptr;
@@ -1181,7 +1176,6 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     std::lock_guard<std::mutex> lock(E.query_mu);
     CU(cudaSetDevice(E.device));
     if (!E.sm_count) CU(cudaDeviceGetAttribute(&E.sm_count, cudaDevAttrMultiProcessorCount, E.device));
-    if (!E.d_rerr) TRY(dalloc(&E.d_rerr, 2));
     RadiusParams p{};
     p.desc = E.d_desc;
     p.delims = E.d_delims;
@@ -1193,8 +1187,8 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     p.xyz = E.d_xyz;
     p.nq = (uint32_t)nq;
     p.radius = radius;
+    p.radius2 = radius * radius;
     p.group = group;
-    p.err = E.d_rerr;
     if (!by_cell) {
         if (on_device) {
             p.qxyz = qxyz;
@@ -1275,24 +1269,33 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
         p.rtab = E.d_rtab;
         p.rtab_len = E.rtab_len;
     }
-    TRY(ensure(&E.d_rcnt, E.rcnt_cap, nq + 1));
-    TRY(ensure(&E.d_roffs, E.roffs_cap, nq + 1));
+    // One block: offsets, scan scratch, error words, counts, and the listed
+    // results.  These go into the face pool instead while that holds no faces (an
+    // allocation of some MB costs a handle's first query 60 to 90 us).  The list is
+    // bounded, and there is none when memory is short: the second pass then finds
+    // the results again.
     const size_t tmp_words = csr_tmp_words((uint32_t)std::max<size_t>(nq, 1));
-    TRY(ensure(&E.d_rtmp, E.rtmp_cap, tmp_words));
-    p.count = E.d_rcnt;
-    p.offs = E.d_roffs;
-    if (out && cap && nq && E.hgrid_valid) {
-        // a bounded workspace, and none when memory is short: the second pass
-        // then finds the results again
-        const size_t len = radius_stage_len(mode, (uint32_t)nq, E.total, D, radius), entries = len * ((nq + 31) / 32 * 32);
-        if (len && entries <= kMaxStage && ensure(&E.d_rstage, E.rstage_cap, entries) == TESS_OK) {
-            p.stage = E.d_rstage;
-            p.stage_len = (uint32_t)len;
-        }
+    const size_t head = (nq + 1) + tmp_words + 1 + (nq + 2) / 2;
+    size_t len = out && cap && nq && E.hgrid_valid ? radius_stage_len(mode, (uint32_t)nq, E.total, D, radius) : 0;
+    const size_t entries = len * ((nq + 31) / 32 * 32);
+    if (entries > kMaxStage) len = 0;
+    const bool in_pool = len && !E.computed && entries <= 2 * E.face_cap;
+    if (!len || in_pool || ensure(&E.d_rwork, E.rwork_cap, head + (entries + 1) / 2) != TESS_OK) {
         cudaGetLastError();   // leave no error behind a failed allocation
+        if (!in_pool) len = 0;
+        TRY(ensure(&E.d_rwork, E.rwork_cap, head));
     }
+    uint64_t* const d_roffs = E.d_rwork;
+    uint64_t* const d_rtmp = d_roffs + nq + 1;
+    int* const d_rerr = reinterpret_cast<int*>(d_rtmp + tmp_words);
+    uint32_t* const d_rcnt = reinterpret_cast<uint32_t*>(d_rtmp + tmp_words + 1);
+    p.count = d_rcnt;
+    p.offs = d_roffs;
+    p.err = d_rerr;
+    p.stage = in_pool ? reinterpret_cast<uint32_t*>(E.d_farea) : reinterpret_cast<uint32_t*>(E.d_rwork + head);
+    p.stage_len = (uint32_t)len;
     const int blocks = (int)std::max<size_t>(1, std::min<size_t>((nq + 7) / 8, (size_t)E.sm_count * 16));
-    CU(cudaMemsetAsync(E.d_rerr, 0, 2 * sizeof(int), E.stream));
+    CU(cudaMemsetAsync(d_rerr, 0, 2 * sizeof(int), E.stream));
     const bool timing = E.cfg.flags & TESS_FLAG_TIMING;
     TimingEvents tev;
     cudaEvent_t* ev = tev.e;
@@ -1325,13 +1328,13 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
             p.qorder = E.d_qorder;
         }
         CU(launch_radius(p, mode, false, blocks, E.stream));
-        CU(launch_csr_offsets(E.d_rcnt, (uint32_t)nq, E.d_roffs, E.d_rtmp, E.stream));
+        CU(launch_csr_offsets(d_rcnt, (uint32_t)nq, d_roffs, d_rtmp, E.stream));
         if (timing) CU(cudaEventRecord(ev[1], E.stream));
-        CU(cudaMemcpyAsync(E.h_ret + RET_TOTAL, E.d_roffs + nq, sizeof(uint64_t), cudaMemcpyDeviceToHost, E.stream));
+        CU(cudaMemcpyAsync(E.h_ret + RET_TOTAL, d_roffs + nq, sizeof(uint64_t), cudaMemcpyDeviceToHost, E.stream));
         E.launches += 4;
     }
     int err[2];
-    CU(cudaMemcpyAsync(E.h_ret + RET_ERR, E.d_rerr, sizeof(err), cudaMemcpyDeviceToHost, E.stream));
+    CU(cudaMemcpyAsync(E.h_ret + RET_ERR, d_rerr, sizeof(err), cudaMemcpyDeviceToHost, E.stream));
     CU(cudaStreamSynchronize(E.stream));
     if (nq) memcpy(&tot, E.h_ret + RET_TOTAL, sizeof(tot));
     memcpy(err, E.h_ret + RET_ERR, sizeof(err));
@@ -1340,7 +1343,7 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     if (total) *total = (size_t)tot;
     if (offs) {
         if (nq) {
-            TRY(copy_async(E, offs, E.d_roffs, sizeof(uint64_t) * (nq + 1)));
+            TRY(copy_async(E, offs, d_roffs, sizeof(uint64_t) * (nq + 1)));
         } else if (on_device) {
             CU(cudaMemsetAsync(offs, 0, sizeof(uint64_t), E.stream));
         } else {

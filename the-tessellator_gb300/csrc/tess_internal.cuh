@@ -268,7 +268,7 @@ struct RadiusParams {
     const double* qxyz;         // query positions (AoS), or null: queries are cells
     const uint32_t* qcell;      // cloud query cells (original index), or null: every cell
     uint32_t nq;
-    double radius;
+    double radius, radius2;     // and its square
     int64_t group;              // cloud only: < 0 keeps every group
     const short4* rtab;         // cloud only: bin offsets with key <= radius, search order
     uint32_t rtab_len;
@@ -295,9 +295,9 @@ struct RadiusParams {
     const unsigned long long* bnd;
 };
 
-// RadiusParams::stage_len for a batch of nq queries of a diagram of n points:
-// room for half as many results again as a uniform density gives a query (its
-// Poisson tail: 16 on top); 0: nothing is listed.
+// RadiusParams::stage_len for a batch of nq queries of a diagram of n points: six
+// standard deviations above the results that a uniform density gives a query; 0:
+// nothing is listed.
 uint32_t radius_stage_len(int mode, uint32_t nq, uint32_t n, const DiagDesc& D, double radius);
 
 // Fills RadiusParams::bnd for diagram 0 (3 * cpd entries).

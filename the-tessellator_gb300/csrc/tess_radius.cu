@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(256) k_radius(RadiusParams p) {
     const uint32_t pt_base = D.pt_base;
     const double sz0 = D.size[0], sz1 = D.size[1], sz2 = D.size[2];
     const double r = p.radius;
-    const double r2 = sq_rn(r);
+    const double r2 = p.radius2;
     // Per-lane axis for the spread evaluation of the query's bin indices:
     // lanes 0-2 the query's own bin (x, y, z), lanes 3-5 the box's low end,
     // lanes 6-8 its high end (celery.rs:753-778); other lanes repeat lane % 3.
@@ -428,7 +428,7 @@ __device__ __forceinline__ float sqrt_near(float x) {
 // Whether point s is within the radius of query q, exactly (rare).
 __device__ __noinline__ bool exact_query(const RadiusParams& p, uint32_t q, uint32_t s) {
     const double* c = p.qxyz + 3 * (size_t)q;
-    return exact_within(p, c[0], c[1], c[2], sq_rn(p.radius), s);
+    return exact_within(p, c[0], c[1], c[2], p.radius2, s);
 }
 
 // RQ_REAL_RADIUS and RQ_CELL_RADIUS with one query per lane: the same rows and
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kLaneThreads, 6) k_radius_lane(RadiusParams p)
     const uint64_t bin_base = D.bin_base;
     const uint32_t pt_base = D.pt_base;
     const double x = p.qxyz[3 * (size_t)q], y = p.qxyz[3 * (size_t)q + 1], z = p.qxyz[3 * (size_t)q + 2];
-    const float fr = (float)p.radius, r2f = (float)sq_rn(p.radius);
+    const float fr = (float)p.radius, r2f = (float)p.radius2;
 
     // The query in FP32, relative to the diagram's centre and in bins.  Its place
     // in bins is known within feps: 2^-23 of the position, 2^-24 of the corner
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(kLaneThreads, 6) k_radius_lane(RadiusParams p)
                 from = T == p.gtab_z ? p.gtab_z + 1 : gz_need + 1;
             }
             for (int gz = from; gz <= gz_need; ++gz) {
-                if (!(gap_ds(gx, gy, gz, D.size[0], D.size[1], D.size[2]) <= sq_rn(p.radius))) break;
+                if (!(gap_ds(gx, gy, gz, D.size[0], D.size[1], D.size[2]) <= p.radius2)) break;
                 T = gz;
             }
             kl = max(kl, zi - T - 1);
@@ -869,7 +869,7 @@ uint32_t radius_stage_len(int mode, uint32_t nq, uint32_t n, const DiagDesc& D, 
     double mean = n * 4.1887902047863910 * radius * radius * radius;
     for (int a = 0; a < 3; ++a) mean /= D.size[a] * D.cpd;
     if (!(mean >= 0.0 && mean <= 200.0)) return 0;
-    return ((uint32_t)(1.6 * mean) + 16 + 7) / 8 * 8;
+    return ((uint32_t)std::ceil(mean + 6.0 * std::sqrt(mean)) + 7) / 8 * 8;
 }
 
 cudaError_t launch_radius(const RadiusParams& p, int mode, bool fill, int blocks, cudaStream_t s) {
