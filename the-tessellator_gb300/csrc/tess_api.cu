@@ -1158,7 +1158,7 @@ constexpr size_t kMaxRadiusTable = (size_t)1 << 26;
 // order, 524,288 290 and 288, 1,000,000 460 and 428).
 constexpr size_t kOrderMin = 65536, kOrderMinLane = 524288;
 // Most entries (of 4 bytes) of the lists that a radius query's first pass keeps.
-constexpr size_t kMaxStage = (size_t)1 << 29;
+constexpr size_t kMaxStage = (size_t)1 << 30;
 // Largest gap table (entries of int16) for box queries; beyond it the
 // kernel evaluates the gap distance per bin in FP64.
 constexpr size_t kMaxGapTable = 65536;

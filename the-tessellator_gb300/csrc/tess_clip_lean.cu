@@ -29,7 +29,8 @@
 // way with the vertices in registers (12.9 k warp instructions per cell, 16
 // warps per SM), 11.9 ms with a candidate per lane, 10.6 ms with the bins taken
 // as rows (three batches a cell instead of five) and the undecided vertices
-// found at the cut instead of in every test.  The code has to stay small: past
+// found at the cut instead of in every test, 9.9 ms as it stands (9.6 k warp
+// instructions a cell, 78% of the issue slots).  The code has to stay small: past
 // about 40 KB of it the warps, each at another place, wait for instructions.
 //
 // With the FP64 finish (MIXED and the FP64 form) the faces' planes, vertices,

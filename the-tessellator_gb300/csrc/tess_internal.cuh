@@ -35,7 +35,7 @@ enum CellStatus : uint8_t {
     ST_DEGEN = 4,       // inconsistent topology (degenerate input) -> FP64 re-run / error
     ST_POOL = 5,        // face pool full -> host grows the pool
     ST_VERIFY = 6,      // FP32 vertex failed the FP64 check -> FP64 re-run
-    ST_DENSE = 7,       // crowded own bin (lean first pass) -> seeded re-run
+    ST_DENSE = 7,       // crowded own bin (plain first pass) -> seeded re-run
     ST_PENDING = 255    // not computed yet
 };
 
@@ -361,7 +361,7 @@ struct ClipParams {
     unsigned int* list_fp64_count;
     uint32_t* list_cap;           // capacity overflow cells or null
     unsigned int* list_cap_count;
-    uint32_t* list_dense;         // lean first pass: cells of crowded bins, or null
+    uint32_t* list_dense;         // plain pass: cells of crowded bins, or null
     unsigned int* list_dense_count;
     unsigned int* flag_count;     // careful pass over every cell: cells with an undecided FP32 test
     unsigned int* fail_count;     // cells left with an error status
