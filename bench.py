@@ -48,18 +48,18 @@ WORKLOADS = {
 RADIUS_METRIC = "radius queries/sec on 1 GB300 (find_neighbors_in_real_radius, FP64, exact)"
 
 # DRAM traffic per launch from ncu captures of the same kernels on GB300.  The
-# clipping pass was captured at 1,000,000 cells (dram__bytes_read.sum 79.7 MB +
-# dram__bytes_write.sum 171.0 MB in 16.44 ms) and is scaled by cells: its
+# clipping pass was captured at 1,000,000 cells (dram__bytes_read.sum 54.7 MB +
+# dram__bytes_write.sum 167.0 MB in 9.87 ms) and is scaled by cells: its
 # traffic is its output plus L2 misses, both per cell.  The radius passes were
-# captured at full size (16,777,216 queries, radius 0.006).
-NCU_CLIP_BYTES_PER_CELL = (79.678720e6 + 171.049728e6) / 1_000_000
+# captured at 1,000,000 queries with 16 results each, and are scaled by queries.
+NCU_CLIP_BYTES_PER_CELL = (54.693376e6 + 167.044352e6) / 1_000_000
 # Warp instructions of the same capture (smsp__inst_executed.sum), per cell: the
 # kernel is bound by instruction issue, so this gives its issue roofline.
-NCU_CLIP_INST_PER_CELL = 12_904_248_352 / 1_000_000
-NCU_RADIUS_BYTES = {"count": 3.846207488e9 + 0.50285184e9, "fill": 6.337812736e9 + 1.53743616e9}
-# DRAM traffic of the 11 binning launches (read 651.8 MB + write 183.7 MB) at
+NCU_CLIP_INST_PER_CELL = 9_612_786_773 / 1_000_000
+NCU_RADIUS_BYTES = {"count": (88.877312e6 + 58.024192e6) / 1_000_000, "fill": (134.081536e6 + 41.526528e6) / 1_000_000}
+# DRAM traffic of the 10 binning launches (read 692.9 MB + write 208.6 MB) at
 # 4,194,304 uniform points, scaled by points: every term is per point or per bin.
-NCU_GRID_BYTES_PER_POINT = (651.8e6 + 183.7e6) / 4_194_304
+NCU_GRID_BYTES_PER_POINT = (692.9e6 + 208.6e6) / 4_194_304
 
 
 def l2_note(input_bytes, written_bytes):
@@ -560,7 +560,7 @@ def run_ours(args, ws, rank, local):
         "gpu_launches": launches, "clocks": clocks, "e2e": e2e,
         "passes_ms": {"grid": float(np.mean(grid_ms)), "clip_first_pass": float(np.mean(clip_ms)),
                       "reruns": float(np.mean(rerun_ms)), "csr": float(np.mean(csr_ms))},
-        "reruns": {"fp32_hybrid": int(st1["rerun_fp64"]), "fp64_full": int(st1["rerun_fp64_full"]),
+        "reruns": {"undecided": int(st1["rerun_fp64"]), "fp64_full": int(st1["rerun_fp64_full"]),
                    "capacity": int(st1["rerun_capacity"]),
                    "failed": int(st1["failed"]), "guard": int(st1["rerun_guard"]),
                    "verify": int(st1["rerun_verify"]), "degenerate": int(st1["rerun_degenerate"]),
@@ -585,20 +585,20 @@ def run_ours(args, ws, rank, local):
         if batched is None:
             achieved = fpc * n / (np.mean(clip_ms) / 1e3) / 1e12
             out["roofline"] = {
-                "kernel": "k_clip<float,2,lean> (first clipping pass)", "bound": "fp32", "achieved": achieved,
+                "kernel": "k_lean (first clipping pass)", "bound": "fp32", "achieved": achieved,
                 "peak": peak_fp32, "unit": "TFLOP/s", "frac": achieved / peak_fp32,
                 "traffic": NCU_CLIP_BYTES_PER_CELL * n,
                 "traffic_source": "ncu DRAM bytes at 1,000,000 cells, scaled by cells",
                 "flops_per_cell": fpc,
                 "peak_source": f"nominal: {nsm} SMs x 128 FP32 lanes x 2 x {sm_mhz:.0f} MHz (sampled SM clock)",
             }
-            # issue roofline of the FP32 lean pass (its ncu instruction count):
+            # issue roofline of the FP32 first pass (its ncu instruction count):
             # warp instructions per second against one per cycle per scheduler
             iach = NCU_CLIP_INST_PER_CELL * n / (np.mean(clip_ms) / 1e3) / 1e12
             ipeak = nsm * 4 * sm_mhz * 1e6 / 1e12
             if prec == "fp32":
                 out["roofline_issue"] = {
-                    "kernel": "k_clip<float,2,lean> (first clipping pass)", "bound": "issue", "achieved": iach,
+                    "kernel": "k_lean (first clipping pass)", "bound": "issue", "achieved": iach,
                     "peak": ipeak, "unit": "T warp-instructions/s", "frac": iach / ipeak,
                     "instructions_per_cell": NCU_CLIP_INST_PER_CELL,
                     "source": "ncu smsp__inst_executed.sum at 1,000,000 cells, scaled by cells; peak = "
@@ -608,11 +608,11 @@ def run_ours(args, ws, rank, local):
             gbytes = (24 + 24 + 4) * n + 8 * nbins
             hbm = peaks.get("hbm_gbs", 6800.0)
             gach = gbytes / (np.mean(grid_ms) / 1e3) / 1e9
-            out["roofline_grid"] = {"kernel": "binning pass (11 launches)", "bound": "hbm", "achieved": gach,
+            out["roofline_grid"] = {"kernel": "binning pass (10 launches)", "bound": "hbm", "achieved": gach,
                                     "peak": hbm, "unit": "GB/s", "frac": gach / hbm,
                                     "algorithmic_bytes": gbytes, "peak_source": src,
                                     "traffic": NCU_GRID_BYTES_PER_POINT * n,
-                                    "traffic_source": "ncu DRAM bytes of the 11 launches at 4,194,304 points, "
+                                    "traffic_source": "ncu DRAM bytes of the 10 launches at 4,194,304 points, "
                                                       "scaled by points"}
     if rank == 0 and gpu_res is not None:
         try:
@@ -702,7 +702,7 @@ def clustered_leg(args, T, cfg, stream, local, rank):
     leg = {"workload": WORKLOADS["clustered"]["desc"], "value": n / (mms / 1e3), "unit": "cells/s",
            "ms_per_step": mms, "steps": steps, "precision": PREC_DESC["fp32"],
            "passes_ms": {"grid": st["ms_grid"], "clip_first_pass": st["ms_clip"], "reruns": st["ms_rerun"]},
-           "reruns": {"fp32_hybrid": int(st["rerun_fp64"]), "fp64_full": int(st["rerun_fp64_full"]),
+           "reruns": {"undecided": int(st["rerun_fp64"]), "fp64_full": int(st["rerun_fp64_full"]),
                       "capacity": int(st["rerun_capacity"]), "dense_cells": int(st["dense_cells"]),
                       "failed": int(st["failed"]), "rerun_fraction": int(st["rerun_fp64"]) / n}}
     base = None
@@ -791,7 +791,7 @@ def batched_leg(args, T, cfg, stream, local, rank):
                "value": n / (mms / 1e3), "unit": "cells/s", "ms_per_step": mms, "steps": steps,
                "precision": PREC_DESC["fp32"], "graph": "bin + clip + re-runs of every diagram in one CUDA graph",
                "diagram_sizes": {"min": int(sizes.min()), "median": int(np.median(sizes)), "max": int(sizes.max())},
-               "reruns": {"fp32_hybrid": int(st["rerun_fp64"]), "fp64_full": int(st["rerun_fp64_full"]),
+               "reruns": {"undecided": int(st["rerun_fp64"]), "fp64_full": int(st["rerun_fp64_full"]),
                           "capacity": int(st["rerun_capacity"]), "failed": int(st["failed"])},
                "e2e": {"value": n / e2e_s, "unit": "cells/s", "ms_per_step": e2e_s * 1e3,
                        "h2d_bytes_per_step": int(pts.nbytes), "d2h_bytes_per_step": int(12 * used + 20 * n),
@@ -951,9 +951,9 @@ def run_radius(args, ws, rank, local):
     bytes_count = (24 + 24 + 4) * n
     bytes_fill = (24 + 24 + 8) * n + 4 * total
     if f_ms >= c_ms:
-        kname, kbytes, kms, kkey = "k_radius<REAL_RADIUS, fill>", bytes_fill, f_ms, "fill"
+        kname, kbytes, kms, kkey = "k_radius_place (listed results to their places)", bytes_fill, f_ms, "fill"
     else:
-        kname, kbytes, kms, kkey = "k_radius<REAL_RADIUS, count> + offsets scan", bytes_count, c_ms, "count"
+        kname, kbytes, kms, kkey = "k_radius_lane<REAL_RADIUS> (count and list) + offsets scan", bytes_count, c_ms, "count"
     ach = kbytes / (kms / 1e3) / 1e9
     out = {
         "metric": RADIUS_METRIC, "value": n * ws / (ms / 1e3), "unit": "queries/s", "n_gpus": ws,
@@ -963,13 +963,13 @@ def run_radius(args, ws, rank, local):
                    "queries": n, "radius": radius, "results": int(total),
                    "parallelism": "replicas",
                    "l2": l2_note(pts.nbytes, 4 * 16 * len(pts)),
-                   "step": "count pass + scan + fill pass, queries and outputs resident in HBM"},
+                   "step": "counting and listing pass + scan + placing pass, queries and outputs resident in HBM"},
         "gpu_launches": launches, "clocks": clocks, "e2e": e2e,
         "passes_ms": {"count_and_scan": c_ms, "fill": f_ms},
         "roofline": {"kernel": kname, "bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s",
                      "frac": ach / hbm,
-                     "traffic": NCU_RADIUS_BYTES[kkey] if n == w["n"] else None,
-                     "traffic_source": "ncu DRAM bytes of the same launch at 16,777,216 queries",
+                     "traffic": NCU_RADIUS_BYTES[kkey] * n,
+                     "traffic_source": "ncu DRAM bytes of the same kernel at 1,000,000 queries, scaled by queries",
                      "algorithmic_bytes": kbytes, "peak_source": src},
     }
     if rank == 0 and not args.no_cpu_baseline:
