@@ -1,6 +1,6 @@
 // tess_clip_impl.cuh -- the FP64 clipping kernel: one Voronoi cell per warp, for
-// the cells that the FP32 passes (tess_clip_lean.cu) do not settle and for
-// single-cell geometry.
+// the cells that the FP32 passes (tess_clip_lean.cu) do not settle, single-cell
+// geometry included.
 //
 // The GPU form of Cell::compute_voronoi_cell (interface.rs:257-313) with
 // Polyhedron::cut_with_plane (polyhedron.rs:438-642), ExpandingSearch
