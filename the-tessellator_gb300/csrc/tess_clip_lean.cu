@@ -733,7 +733,14 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                     keep = jp != gs && r2 > dup2 && r2 < lim;
                     near = jp != gs && !(r2 > dup2);
                     if (keep && P.target_group >= 0) keep = (int64_t)(P.sgroup ? P.sgroup[jp] : 0u) == P.target_group;
-                    if constexpr (SEED) keep = keep && (!bounded || reaches(rx, ry, rz, r2));
+                    if constexpr (SEED && MODE != kDense) keep = keep && (!bounded || reaches(rx, ry, rz, r2));
+                }
+                // (few of a crowded bin's 32 are within twice the radius, often none:
+                // 2,097,152 clustered points, passes after the first: 47.0 -> 45.3
+                // ms with this and the early end below; 44.1 with ranges read one
+                // after the other, but inputs of 100,000 points 3% slower)
+                if constexpr (MODE == kDense) {
+                    if (bounded && __any_sync(FULL, keep)) keep = keep && reaches(rx, ry, rz, r2);
                 }
                 return heads;
             };
@@ -754,13 +761,18 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 do {
                     const unsigned heads = load();
                     const unsigned kk = __ballot_sync(FULL, keep);
+                    anynear |= near;
+                    if (MODE == kDense && !kk) {
+                        before += __popc(heads);
+                        w0 += 32;
+                        continue;
+                    }
                     if (nk + __popc(kk) > 32u) break;
                     if (keep) {
                         const unsigned at = nk + __popc(kk & lt);
                         S.cand[at] = make_float4(rx, ry, rz, r2);
                         S.candj[at] = jp;
                     }
-                    anynear |= near;
                     nk += __popc(kk);
                     before += __popc(heads);
                     w0 += 32;
