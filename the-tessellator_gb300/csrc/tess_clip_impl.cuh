@@ -1159,6 +1159,7 @@ __device__ void run_cell(const ClipParams& P, Smem<K>& S, uint32_t gs, int lane,
             S.ncnt[lane] = nc;
             S.nd[lane] = dn;
             S.pending = __ballot_sync(FULL, nc >= P.seed_min && dn < INFINITY);
+            __syncwarp();
             ph = 0;
         }
     }

@@ -662,6 +662,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
         if constexpr (COUNT) ++W.batches;
         {
             const unsigned nz = __ballot_sync(FULL, bcnt > 0);
+            __syncwarp();                         // the last batch's offsets are read
             if (bcnt) S.boff[__popc(nz & lt)] = bbeg - pref;
         }
         }
@@ -671,6 +672,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
         const bool bounded = SEED && (crowded || total >= 256);
         unsigned w0 = 0;
         do {
+            __syncwarp();                         // the last window's candidates are read
             float rx, ry, rz, r2;
             uint32_t jp;
             bool keep, near;
@@ -863,6 +865,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                     if (f >= kPlanes) {
                         // the table is full: an id that no live vertex has any
                         // more (planes cut away entirely leave them behind)
+                        __syncwarp();             // the last cut's vertices are written
                         uint32_t u0 = 0x3Fu, u1 = 0, u2 = 0;       // the walls stay
 #pragma unroll 1
                         for (int k = 0; k < 2; ++k)
@@ -897,6 +900,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 }
                 gen = (gen + 1) & 0xFFu;
                 if (gen == 0) {
+                    __syncwarp();                 // the last cut's ring is read
 #pragma unroll 1
                     for (int i = lane; i < kPlanes; i += 32) S.map[i] = 0;
                     gen = 1;
