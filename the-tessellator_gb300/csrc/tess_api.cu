@@ -778,7 +778,6 @@ tess_status engine_compute(Engine& E, int precision, double radius, int64_t grou
         const unsigned* counts = nullptr;
         int gerr = 0;
         TRY(read_back(E, &counts, &used, &gerr));
-        if (gerr == 2) return fail(TESS_E_CUDA, "shell table exceeded its capacity");
         if (gerr == 1) {
             // the device points were rebuilt without a check and hold a
             // non-finite coordinate: the clipping kernels did nothing
@@ -1937,7 +1936,6 @@ static tess_status batch_run(tess_batch* b, int prec) {
         E.computed = false;
         return fail(TESS_E_INVALID, "input coordinates must be finite");
     }
-    if (gerr == 2) return fail(TESS_E_CUDA, "shell table exceeded its capacity");
     if (used > E.face_cap && host) {
         // the caller's pool: report the size needed
         E.pool_need = used;

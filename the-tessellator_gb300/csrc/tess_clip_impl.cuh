@@ -832,9 +832,12 @@ __device__ void run_cell(const ClipParams& P, Smem<K>& S, uint32_t gs, int lane,
 
     // ---- the walk over bins in shell order (celery.rs:1023-1075) ----
     const int cpd = D.cpd;
-    const int cbx = axis_index(sx, D.glo[0], D.ghi[0], D.inv[0], cpd);
-    const int cby = axis_index(sy, D.glo[1], D.ghi[1], D.inv[1], cpd);
-    const int cbz = axis_index(sz, D.glo[2], D.ghi[2], D.inv[2], cpd);
+    // (an axis without extent has all its points in the last bin, and its offsets
+    // count nothing in a key: a position beside it searches from there)
+    auto bin_on = [&](double x, int a) {
+        return D.ghi[a] > D.glo[a] ? axis_index(x, D.glo[a], D.ghi[a], D.inv[a], cpd) : cpd - 1;
+    };
+    const int cbx = bin_on(sx, 0), cby = bin_on(sy, 1), cbz = bin_on(sz, 2);
     const double radius = P.search_radius;
     const bool has_radius = radius >= 0.0;
     const int64_t tgroup = P.target_group;

@@ -532,6 +532,11 @@ __global__ void k_inverse(const uint32_t* sorted, uint32_t* inv, uint32_t n, int
 // the triples' sizes, and the offsets of equal keys order themselves by
 // counting.  Sorting all offsets in shared memory, with an FP64 key each, took
 // 97 us a block; this takes 13.
+//
+// On an axis without extent every offset has the key of its other two, so a
+// plane of points (5,000 offsets) or a line (6,900) has more than kMaxTable
+// entries.  The table then ends with the last key whose offsets all fit, and
+// tab_kmax says so: the walk goes on ring by ring beyond it.
 constexpr int kTabThreads = 1024;
 constexpr int kTabGaps = 9;          // gap counts per axis: 0 .. table_gaps (at most 8)
 __global__ void __launch_bounds__(kTabThreads) k_table(GridBuffers g) {
@@ -542,6 +547,7 @@ __global__ void __launch_bounds__(kTabThreads) k_table(GridBuffers g) {
     __shared__ uint32_t start[kTabThreads];      // first entry of the r-th triple
     __shared__ uint16_t code[kMaxTable];         // an entry's offset, lexicographic
     __shared__ uint16_t rank[kMaxTable];         // ... and the place of its triple
+    __shared__ int ends;                         // more than fit: the triple where the table ends
     const int d = blockIdx.x, t = threadIdx.x, lane = t & 31;
     DiagDesc& D = g.diags[d];
     const int c = D.cheb, side = 2 * c + 1;
@@ -612,8 +618,17 @@ __global__ void __launch_bounds__(kTabThreads) k_table(GridBuffers g) {
     const uint32_t beg = wsum[t >> 5] + inc - cnt;
     start[t] = beg;
     const uint32_t total = wsum[32], cap = min((uint32_t)kMaxTable, D.tab_cap);
-    if (total > cap && t == 0) atomicExch(g.error_flag, 2);
-    const uint32_t m = min(total, cap);
+    uint32_t m = total;
+    if (total > cap) {
+        if (t == 0) ends = 0;
+        __syncthreads();
+        if (kept && beg <= cap && t > 0 && skey[t - 1] != key) atomicMax(&ends, t);
+        __syncthreads();
+        m = start[ends];
+        // (not even the first key's, sides below 1e-162: the own bin alone)
+        if (t == 0) D.tab_kmax = ends ? __longlong_as_double((long long)skey[ends - 1]) : -1.0;
+        if (t == 0 && !ends) g.table[D.tab_base] = TabEntry{-1.0f, 0, 0, 0, 0};
+    }
     for (uint32_t q = 0; q < cnt; ++q) {
         if (beg + q >= m) break;
         const int i = pick(gi, q / (w1 * w2)), j = pick(gj, (q / w2) % w1), k = pick(gk, q % w2);
@@ -642,7 +657,7 @@ __global__ void __launch_bounds__(kTabThreads) k_table(GridBuffers g) {
         te.pad = 0;
         g.table[D.tab_base + at] = te;
     }
-    if (t == 0) D.tab_len = m;
+    if (t == 0) D.tab_len = max(m, 1u);
 }
 
 }  // namespace
