@@ -61,7 +61,9 @@ typedef enum {
      * FP64 finish: every vertex is solved in FP64 from its three face planes,
      * and face areas and volumes are computed in FP64 from those vertices.
      * (As TESS_PRECISION_FP64, without the reference's tolerance in the plane
-     * tests.)  Single-cell geometry queries run in FP64 in every precision. */
+     * tests.)  Single-cell geometry queries finish in FP64 in every precision;
+     * their plane tests are the FP32 form's with TESS_PRECISION_FP32_GUARD and
+     * the FP64 form's otherwise. */
     TESS_PRECISION_MIXED = 2
 } tess_precision;
 

@@ -1106,17 +1106,18 @@ tess_status engine_autotune(Engine& E, int precision, bool batch, const char* ca
 }
 
 // One cell's full geometry in E.h_geo, which the caller holds E.query_mu for: the
-// cell alone through the careful pass's FP64 finish (in every precision), and
-// through the FP64 clipping when that cannot settle it, written by the kernel
-// into mapped memory.
-tess_status engine_geo(Engine& E, const size_t* i, const double* point, double radius, int64_t group, const double* lo,
+// cell alone through the careful pass's FP64 finish (in every precision, with the
+// FP32 form's decisions in that form, so that its faces are those of a whole
+// compute), and through the FP64 clipping when that cannot settle it, written by
+// the kernel into mapped memory.
+tess_status engine_geo(Engine& E, int precision, const size_t* i, const double* point, double radius, int64_t group, const double* lo,
                        const double* hi) {
     CU(cudaSetDevice(E.device));
     ClipParams p = base_params(E);
     p.search_radius = radius;
     p.has_radius = radius >= 0.0;
     p.target_group = group;
-    p.tol = kFp64Tol;
+    p.tol = precision == TESS_PRECISION_FP32_GUARD ? 0.f : kFp64Tol;
     p.total = 1;
     p.geo = E.d_geo;
     if (i) {
@@ -1683,7 +1684,7 @@ tess_status tess_cell_original_index(const tess_diagram* d, size_t i, size_t* or
 
 // Cell i of the last compute, in E.h_geo (E.query_mu held).
 static tess_status geo_for(tess_diagram* d, size_t i) {
-    return engine_geo(d->E, &i, nullptr, d->E.last_radius, d->E.last_group, nullptr, nullptr);
+    return engine_geo(d->E, d->E.last_precision, &i, nullptr, d->E.last_radius, d->E.last_group, nullptr, nullptr);
 }
 
 tess_status tess_cell_vertices(tess_diagram* d, size_t i, double* xyz, size_t cap, size_t* count) {
@@ -1740,7 +1741,7 @@ static tess_status single_cell(tess_diagram* d, const size_t* i, const double* p
         return fail(TESS_E_INVALID, "point must be finite");
     }
     std::lock_guard<std::mutex> lock(d->E.query_mu);
-    TRY(engine_geo(d->E, i, i ? nullptr : p, search_radius, target_group, lo, hi));
+    TRY(engine_geo(d->E, (int)precision, i, i ? nullptr : p, search_radius, target_group, lo, hi));
     geo_to_public(*d->E.h_geo, out);
     return TESS_OK;
 }
