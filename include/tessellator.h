@@ -53,9 +53,10 @@ typedef enum {
      * decided in FP32 where the test is beyond its error bound and the
      * reference's 1e-12 tolerance, else in FP64: the same decisions. */
     TESS_PRECISION_FP64 = 0,
-    /* FP32 clipping; a plane-side test inside the guard band is settled in
-     * FP64, and a cell whose FP32 vertices fail the check is re-run in FP64.
-     * Volumes and areas are accumulated in FP64. */
+    /* FP32 clipping; a cell with a plane-side test inside the guard band, or
+     * whose FP32 vertices fail the check, has that test settled or is re-run in
+     * FP64, and its faces and volume computed in FP64.  Volumes are accumulated
+     * in FP64. */
     TESS_PRECISION_FP32_GUARD = 1,
     /* The FP32 + guard clipping (its exact topology and re-runs) with an
      * FP64 finish: every vertex is solved in FP64 from its three face planes,

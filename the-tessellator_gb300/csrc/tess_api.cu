@@ -125,9 +125,15 @@ static_assert(RET_FLAG < RET_TOTAL && 4 * (RET_ERR + 2) <= RET_BYTES, "layout of
 // Up to this many cells the careful pass runs over all of them: a few waves of
 // warps, whose time is a cell's latency, and a second pass over a few cells
 // would add its own (uniform points, careful alone against plain and careful:
-// 3,000 0.113 / 0.134 ms, 10,000 0.205 / 0.204, 30,000 0.52 / 0.41).  Such
-// inputs have one launch of the FP64 clipping behind it, not two.
-constexpr uint32_t kCarefulMax = 8192;
+// 3,000 0.113 / 0.134 ms, 10,000 0.205 / 0.204, 30,000 0.52 / 0.41, each with the
+// finish of the form).  The careful pass finishes in FP64: where the form does
+// not ask for that, the line lies lower (FP32, 3,000 0.128 / 0.134 ms, 8,000
+// 0.216 / 0.19).  Such inputs have one launch of the FP64 clipping behind it, not
+// two.
+constexpr uint32_t kCarefulMax = 8192, kCarefulMax32 = 4096;
+bool careful_alone(uint32_t n, int precision) {
+    return n <= (precision == TESS_PRECISION_FP32_GUARD ? kCarefulMax32 : kCarefulMax);
+}
 // The FP64 form's first pass runs in FP32 (tess_clip_lean.cu): a vertex whose
 // distance from a plane is within the FP32 error bound plus this is left to
 // the FP64 clipping, so that every decision the FP32 pass takes is the one the
@@ -707,18 +713,19 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
     uint32_t* const lcap = norerun ? nullptr : L[L_FULL];
     // The FP32 first pass hands cells of crowded bins to the dense pass and both
     // hand cells with an undecided plane test to the careful pass, which settles
-    // those tests in FP64; what that cannot settle, and cells beyond 64 vertices
+    // those tests in FP64 and finishes the cell in FP64, whatever the form: such
+    // cells are ill-conditioned.  What that cannot settle, and cells beyond 64 vertices
     // or 96 planes, are clipped in FP64 at 128 and 255 vertices.
-    const bool small = (sample ? nsample : E.total) <= kCarefulMax;
+    const bool small = careful_alone(sample ? nsample : E.total, precision);
     if (small) {
-        TRY(pass(1, 2, kFormCareful | X, sample, nullptr, L[L_FULL], cnt + L_FULL, lcap, cnt + L_FULL, nullptr, cur + C_DENSE));
+        TRY(pass(1, 2, kFormCareful | kFormExact, sample, nullptr, L[L_FULL], cnt + L_FULL, lcap, cnt + L_FULL, nullptr, cur + C_DENSE));
     } else {
         TRY(pass(1, 2, kFormLean | X, sample, nullptr, L[L_CARE], cnt + L_CARE, lcap, cnt + L_FULL, L[L_DENSE], cnt + L_DENSE));
     }
     if (timing) CU(cudaEventRecord(ev[1], E.stream));
     if (!small) {
         TRY(pass(1, 2, kFormDense | X, L[L_DENSE], cnt + L_DENSE, L[L_CARE], cnt + L_CARE, lcap, cnt + L_FULL));
-        TRY(pass(1, 2, kFormCareful | X, L[L_CARE], cnt + L_CARE, L[L_FULL], cnt + L_FULL, lcap, cnt + L_FULL));
+        TRY(pass(1, 2, kFormCareful | kFormExact, L[L_CARE], cnt + L_CARE, L[L_FULL], cnt + L_FULL, lcap, cnt + L_FULL));
     }
     if (s0 < 8 && !small) {
         TRY(pass(0, 4, kFormStd, L[L_FULL], cnt + L_FULL, nullptr, nullptr, norerun ? nullptr : L[L_CAP64], cnt + L_CAP64));
@@ -1892,8 +1899,9 @@ static tess_status batch_run(tess_batch* b, int prec) {
     if (stale) {
         // warm the per-kernel attributes and occupancy queries outside capture
         for (int k : {4, 8}) E.blocks(k, kFormStd);
-        for (int f : {(int)kFormLean, (int)kFormDense, (int)kFormCareful})
+        for (int f : {(int)kFormLean, (int)kFormDense})
             for (int x : {0, (int)kFormExact}) E.blocks(2, f | x);
+        E.blocks(2, kFormCareful | kFormExact);
         if (G) cudaGraphExecDestroy(G);
         G = nullptr;
         cudaGraph_t g = nullptr;
@@ -1925,7 +1933,7 @@ static tess_status batch_run(tess_batch* b, int prec) {
         CU(cudaEventRecord(ev.e[0], E.stream));
     }
     CU(cudaGraphLaunch(G, E.stream));
-    E.launches += grid_launches(E.total_bins, E.ndiag) + (E.total <= kCarefulMax ? 2 : (E.cfg.slots_per_lane >= 8 ? 4 : 5)) + 1;
+    E.launches += grid_launches(E.total_bins, E.ndiag) + (careful_alone(E.total, prec) ? 2 : (E.cfg.slots_per_lane >= 8 ? 4 : 5)) + 1;
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     unsigned long long used = 0;
     const unsigned* counts = nullptr;

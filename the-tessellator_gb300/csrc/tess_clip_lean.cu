@@ -60,7 +60,7 @@ constexpr int kNearZ = 2;      // the first three batches take the bins up to th
 //   kDense    over the cells of crowded bins: seeded, points gathered
 //   kCareful  as kDense, and undecided tests are settled in FP64 in place: over
 //             the cells the others handed on, or over every cell of a small
-//             input.  (An instance of its own: the settling makes the code
+//             input.  Always with the FP64 finish.  (An instance of its own: the settling makes the code
 //             half as large again, and the dense pass waits for instructions.)
 //   kGeo      one cell with its geometry (single-cell queries): careful, the
 //             site may be any position and the container any box
@@ -343,6 +343,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
     const unsigned lt = (1u << lane) - 1u;
     const uint32_t pt_base = D.pt_base;
     constexpr bool COUNT = MODE != kPlain, SEED = MODE >= kDense, CAREFUL = MODE >= kCareful, GEO = MODE == kGeo;
+    static_assert(EXACT || !CAREFUL, "cells with undecided tests finish in FP64");
     // a coordinate relative to the centre of the points as an FP32 pair
     auto pair = [&](double x, int a, float& h, float& l) {
         const double u = x - D.ctr[a];
@@ -1573,13 +1574,13 @@ int blocks_for(int wpb, int device) {
 }  // namespace cliplean
 
 // form: kFormLean (the plain pass; with TESS_FLAG_COUNTERS its counting
-// instance, the results are the same), kFormDense or kFormCareful, with
-// kFormExact for the FP64 finish.
+// instance, the results are the same) or kFormDense, with kFormExact for the FP64
+// finish, or kFormCareful | kFormExact.
 cudaError_t launch_clip_lean(const ClipParams& p, int form, int wpb, int blocks, cudaStream_t s) {
     using namespace cliplean;
     const bool x = form & kFormExact;
     switch (form & 3) {
-        case kFormCareful: return x ? launch<true, kCareful>(p, wpb, blocks, s) : launch<false, kCareful>(p, wpb, blocks, s);
+        case kFormCareful: return launch<true, kCareful>(p, wpb, blocks, s);
         case kFormDense: return x ? launch<true, kDense>(p, wpb, blocks, s) : launch<false, kDense>(p, wpb, blocks, s);
         default: break;
     }
@@ -1597,7 +1598,7 @@ int clip_blocks_lean(int form, int wpb, int device) {
     using namespace cliplean;
     const bool x = form & kFormExact;
     switch (form & 3) {
-        case kFormCareful: return x ? blocks_for<true, kCareful>(wpb, device) : blocks_for<false, kCareful>(wpb, device);
+        case kFormCareful: return blocks_for<true, kCareful>(wpb, device);
         case kFormDense: return x ? blocks_for<true, kDense>(wpb, device) : blocks_for<false, kDense>(wpb, device);
         default: return x ? blocks_for<true, kPlain>(wpb, device) : blocks_for<false, kPlain>(wpb, device);
     }

@@ -400,7 +400,8 @@ struct ClipParams {
 //   kFormStd      FP64 clipping (tess_clip_f64.cu), for what neither settles
 //                 and for single cells;
 //   kFormExact    a flag on the first three: faces, vertices, areas and volume
-//                 computed in FP64 (the MIXED and FP64 forms)
+//                 computed in FP64 (the MIXED and FP64 forms, and always the careful
+//                 pass)
 enum ClipForm : int { kFormLean = 0, kFormStd = 1, kFormDense = 2, kFormCareful = 3, kFormExact = 4 };
 cudaError_t launch_clip_lean(const ClipParams& p, int form, int wpb, int blocks, cudaStream_t s);
 // One cell with its geometry into p.geo (readable by the host once the stream
