@@ -76,8 +76,8 @@ typedef enum {
 #define TESS_FLAG_SMALL_FACE_POOL 4u  /* start the face pool at 1,024 faces, so a compute
                                          overflows it and grows it (tess_stats.face_pool_regrows) */
 #define TESS_FLAG_NO_CAPACITY_RERUN 8u /* skip the larger-capacity re-runs: a cell that outgrows
-                                          the first pass's vertex or face slots is reported as
-                                          failed (TESS_E_OVERFLOW, volume 0, no faces) */
+                                          32 x slots_per_lane vertices (255 with 8) is reported
+                                          as failed (TESS_E_OVERFLOW, volume 0, no faces) */
 #define TESS_FLAG_AUTOTUNE 16u  /* the first compute of a handle autotunes its launch knobs
                                    (tess_diagram_autotune / tess_batch_autotune with the default
                                    cache file) before it runs */

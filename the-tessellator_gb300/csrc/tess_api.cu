@@ -707,10 +707,10 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
     };
     uint32_t* const* L = E.d_list;
     if (timing) CU(cudaEventRecord(ev[0], E.stream));
-    // without capacity re-runs, the capacity lists are left out: an overflowing
-    // cell is then reported as failed
+    // without capacity re-runs, the lists beyond the configured slots are left out:
+    // an overflowing cell is then reported as failed
     const bool norerun = E.cfg.flags & TESS_FLAG_NO_CAPACITY_RERUN;
-    uint32_t* const lcap = norerun ? nullptr : L[L_FULL];
+    uint32_t* const lcap = norerun && s0 == 2 ? nullptr : L[L_FULL];
     // The FP32 first pass hands cells of crowded bins to the dense pass and both
     // hand cells with an undecided plane test to the careful pass, which settles
     // those tests in FP64 and finishes the cell in FP64, whatever the form: such
@@ -727,7 +727,7 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
         TRY(pass(1, 2, kFormDense | X, L[L_DENSE], cnt + L_DENSE, L[L_CARE], cnt + L_CARE, lcap, cnt + L_FULL));
         TRY(pass(1, 2, kFormCareful | kFormExact, L[L_CARE], cnt + L_CARE, L[L_FULL], cnt + L_FULL, lcap, cnt + L_FULL));
     }
-    if (s0 < 8 && !small) {
+    if (s0 < 8 && (!small || norerun)) {
         TRY(pass(0, 4, kFormStd, L[L_FULL], cnt + L_FULL, nullptr, nullptr, norerun ? nullptr : L[L_CAP64], cnt + L_CAP64));
         TRY(pass(0, 8, kFormStd, L[L_CAP64], cnt + L_CAP64, nullptr, nullptr, nullptr, nullptr));
     } else {
