@@ -269,7 +269,10 @@ tess_status tess_volumes(tess_diagram* d, double* volumes);
 tess_status tess_neighbors_csr(tess_diagram* d, uint64_t* offs, int32_t* nbr, double* area,
                                size_t cap, size_t* total);
 /* Device pointers to the same results (valid until the next compute or
- * destroy): volumes[n], offs[n+1], nbr[total], area[total]. */
+ * destroy): volumes[n], offs[n+1], nbr[total], area[total].  On return all are
+ * complete when the handle runs on its own stream; on the caller's stream
+ * (tess_config.stream) volumes and offs are, and nbr and area are complete in
+ * the order of that stream. */
 tess_status tess_results_device(tess_diagram* d, const double** volumes, const uint64_t** offs,
                                 const int32_t** nbr, const double** area, size_t* total);
 /* tess_diagram_compute_all with every cell's results delivered to the
@@ -377,7 +380,7 @@ tess_status tess_batch_neighbors_csr(tess_batch* b, uint64_t* offs, int32_t* nbr
                                      size_t cap, size_t* total);
 /* Device pointers to the same results (valid until the next compute, update
  * or destroy): volumes[total points], offs[total points + 1], nbr[faces],
- * area[faces]; the batch form of tess_results_device. */
+ * area[faces], complete as tess_results_device's; its batch form. */
 tess_status tess_batch_results_device(tess_batch* b, const double** volumes, const uint64_t** offs,
                                       const int32_t** nbr, const double** area, size_t* total);
 tess_status tess_batch_destroy(tess_batch* b);

@@ -196,7 +196,7 @@ struct Engine {
     // 16-byte aligned block of C_BYTES, and the bounds' error flag behind it)
     unsigned* h_ret = nullptr;
     unsigned* d_ret = nullptr;
-    cudaEvent_t ev_bounds = nullptr;
+    cudaEvent_t ev_bounds = nullptr, ev_offs = nullptr;
     uint32_t* d_list[L_COUNT] = {};
     unsigned* d_counters = nullptr;   // C_* above
     unsigned long long* d_work = nullptr;  // work counters (TESS_FLAG_COUNTERS)
@@ -308,8 +308,9 @@ struct Engine {
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         if (ev_bounds) cudaEventDestroy(ev_bounds);
+        if (ev_offs) cudaEventDestroy(ev_offs);
         side = nullptr;
-        ev_fork = ev_join = ev_bounds = nullptr;
+        ev_fork = ev_join = ev_bounds = ev_offs = nullptr;
     }
 
     int blocks(int slots, int form) {
@@ -412,6 +413,7 @@ tess_status engine_init(Engine& E, const tess_config* cfg, std::vector<DiagDesc>
     CU(cudaEventCreateWithFlags(&E.ev_fork, cudaEventDisableTiming));
     CU(cudaEventCreateWithFlags(&E.ev_join, cudaEventDisableTiming));
     CU(cudaEventCreateWithFlags(&E.ev_bounds, cudaEventDisableTiming));
+    CU(cudaEventCreateWithFlags(&E.ev_offs, cudaEventDisableTiming));
     CU(cudaHostAlloc((void**)&E.h_ret, RET_BYTES + sizeof(GeoOut), cudaHostAllocMapped));
     CU(cudaHostGetDevicePointer((void**)&E.d_ret, E.h_ret, 0));
     E.h_geo = reinterpret_cast<GeoOut*>(reinterpret_cast<char*>(E.h_ret) + RET_BYTES);
@@ -846,6 +848,7 @@ tess_status engine_csr(Engine& E) {
     if (timing) CU(ev.create(2));
     if (timing) CU(cudaEventRecord(ev.e[0], E.stream));
     CU(launch_csr_offsets(E.d_nface, E.total, E.d_offs, E.d_csr_tmp, E.stream));
+    CU(cudaEventRecord(E.ev_offs, E.stream));
     // every face of the pool belongs to one cell: their number is the last offset
     const uint64_t total = E.stats.faces;
     if (total > E.csr_cap || !E.d_cnbr) {
@@ -1799,10 +1802,10 @@ tess_status tess_neighbors_csr(tess_diagram* d, uint64_t* offs, int32_t* nbr, do
 }
 
 // Results handed out as device pointers: on the library's own stream, which the
-// caller cannot order against, they are complete; on the caller's stream they
-// are in its order.
+// caller cannot order against, they are complete; on the caller's stream the
+// volumes and offsets are, the faces are in its order.
 static tess_status results_ready(Engine& E) {
-    if (E.own_stream) CU(cudaStreamSynchronize(E.stream));
+    CU(E.own_stream ? cudaStreamSynchronize(E.stream) : cudaEventSynchronize(E.ev_offs));
     return TESS_OK;
 }
 
