@@ -117,7 +117,8 @@ enum { L_DENSE = 0, L_CARE = 1, L_FULL = 2, L_CAP64 = 3, L_COUNT = 4 };
 // status code was given to, in the FP32 and in the FP64 passes.
 enum { C_CURSOR = 0, C_LIST = 16, C_FAIL = 20, C_FLAG = 21, C_DENSE = 22, C_REASON32 = 32, C_REASON64 = 40,
        C_TOTAL = 48,      // cleared for each compute, with the face cursor behind it ...
-       C_FACES = 48, C_ERR = 50, C_BYTES = 208 };   // ... and the binning's error flag, read back together
+       C_FACES = 48, C_ERR = 50, C_TABLE = 51,       // ... the binning's error flag and the shell table's
+       C_BYTES = 208 };                              // length, all read back together
 // Behind them in E.h_ret: the binning's early error flag, and a radius query's
 // total and error words.
 enum { RET_FLAG = C_BYTES / 4, RET_TOTAL = 56, RET_ERR = 58, RET_BYTES = 256 };
@@ -516,6 +517,7 @@ GridBuffers grid_buffers(Engine& E) {
     g.table = E.d_table;
     g.table_gaps = E.cfg.table_gaps;
     g.error_flag = E.d_err;
+    g.table_len = E.d_counters + C_TABLE;
     g.host_flag = reinterpret_cast<int*>(E.d_ret + RET_FLAG);
     g.check = E.d_check;
     return g;
@@ -758,6 +760,7 @@ void read_counts(Engine& E, const unsigned* c, uint64_t faces) {
     const uint64_t cap32 = (uint64_t)r32[ST_VCAP] + r32[ST_PCAP];
     E.stats.cells = E.total;
     E.stats.faces = faces;
+    if (E.ndiag == 1) E.stats.table_entries = c[C_TABLE];
     E.stats.rerun_fp64 = (uint64_t)c[C_LIST + L_CARE] + c[C_FLAG];
     E.stats.rerun_fp64_full = (uint64_t)c[C_LIST + L_FULL] - std::min<uint64_t>(cap32, c[C_LIST + L_FULL]);
     E.stats.dense_cells = (uint64_t)c[C_LIST + L_DENSE] + c[C_DENSE];
@@ -1594,13 +1597,6 @@ tess_status tess_host_free(void* ptr) {
 tess_status tess_diagram_stats(const tess_diagram* d, tess_stats* out) {
     if (!d || !out) return fail(TESS_E_INVALID, "NULL argument");
     *out = d->E.stats;
-    if (d->E.stats.cells) {     // the shell table's length of the last binning
-        DiagDesc D;
-        CU(cudaSetDevice(d->E.device));
-        CU(cudaStreamSynchronize(d->E.stream));
-        CU(cudaMemcpy(&D, d->E.d_desc, sizeof(D), cudaMemcpyDeviceToHost));
-        out->table_entries = D.tab_len;
-    }
     out->launches = d->E.launches;
     return TESS_OK;
 }

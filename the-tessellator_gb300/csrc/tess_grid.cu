@@ -658,6 +658,7 @@ __global__ void __launch_bounds__(kTabThreads) k_table(GridBuffers g) {
         g.table[D.tab_base + at] = te;
     }
     if (t == 0) D.tab_len = max(m, 1u);
+    if (t == 0 && d == 0) *g.table_len = max(m, 1u);
 }
 
 }  // namespace

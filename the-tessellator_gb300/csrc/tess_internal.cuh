@@ -217,6 +217,7 @@ struct GridBuffers {
     TabEntry* table;
     int table_gaps;
     int* error_flag;            // set when an input coordinate is not finite
+    unsigned* table_len;        // entries of the first diagram's shell table
     int* host_flag;             // its value after the bounds, in mapped host memory, or null
     int* check;                 // checked build: the check word
 };
