@@ -263,6 +263,7 @@ struct Engine {
     uint64_t launches = 0;    // kernels launched so far (all passes)
     cudaGraphExec_t graph = nullptr;
     int graph_precision = -1;
+    uint64_t graph_launches = 0, graph_host_launches = 0;   // kernels of the graphs
     // the batch graph captured with a caller's face pool
     // (tess_batch_compute_to_host): its pointers, capacity and precision
     cudaGraphExec_t graph_host = nullptr;
@@ -1151,11 +1152,13 @@ tess_status engine_geo(Engine& E, int precision, const size_t* i, const double* 
         }
     }
     CU(launch_cell_lean(p, E.stream));
+    E.launches += 1;
     CU(cudaStreamSynchronize(E.stream));
     if (E.h_geo->status != ST_OK) {
         CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * C_TOTAL, E.stream));
         p.cursor = E.d_counters;
         CU(launch_clip(p, 8, kFormStd, 1, 1, E.stream));
+        E.launches += 1;
         CU(cudaStreamSynchronize(E.stream));
     }
     TRY(check_word(E));
@@ -1338,14 +1341,14 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
             o.scan_tmp = E.d_qtmp;
             const int eblocks = (int)std::min<size_t>((nq + 255) / 256, (size_t)E.sm_count * 8);
             CU(launch_query_order(p, o, eblocks, E.stream));
-            E.launches += 5;
+            E.launches += 2 + csr_offset_launches(o.ncoarse);
             p.qorder = E.d_qorder;
         }
         CU(launch_radius(p, mode, false, blocks, E.stream));
         CU(launch_csr_offsets(d_rcnt, (uint32_t)nq, d_roffs, d_rtmp, E.stream));
         if (timing) CU(cudaEventRecord(ev[1], E.stream));
         CU(cudaMemcpyAsync(E.h_ret + RET_TOTAL, d_roffs + nq, sizeof(uint64_t), cudaMemcpyDeviceToHost, E.stream));
-        E.launches += 4;
+        E.launches += 1 + csr_offset_launches((uint32_t)nq);
     }
     int err[2];
     CU(cudaMemcpyAsync(E.h_ret + RET_ERR, d_rerr, sizeof(err), cudaMemcpyDeviceToHost, E.stream));
@@ -1382,7 +1385,7 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     if (timing) CU(cudaEventRecord(ev[1], E.stream));
     CU(launch_radius(p, mode, true, blocks, E.stream));
     if (timing) CU(cudaEventRecord(ev[2], E.stream));
-    E.launches += 1;
+    E.launches += p.stage_len && p.unlisted ? 2 : 1;
     if (!on_device) TRY(copy_async(E, out, E.d_rout, sizeof(uint32_t) * tot));
     CU(cudaStreamSynchronize(E.stream));
     if (timing) E.stats.ms_query_fill = tev.ms(1, 2);
@@ -1892,6 +1895,7 @@ static tess_status batch_run(tess_batch* b, int prec) {
     const bool host = E.pool_fixed;
     cudaGraphExec_t& G = host ? E.graph_host : E.graph;
     int& gprec = host ? E.graph_host_precision : E.graph_precision;
+    uint64_t& glaunches = host ? E.graph_host_launches : E.graph_launches;
     const bool stale = !G || gprec != prec ||
                        (host && (E.graph_host_nbr != E.d_fnbr || E.graph_host_area != E.d_farea ||
                                  E.graph_host_cap != E.face_cap));
@@ -1908,7 +1912,10 @@ static tess_status batch_run(tess_batch* b, int prec) {
         tess_status st = TESS_OK;
         cudaError_t ce = launch_grid_build(grid_buffers(E), E.stream, E.side, E.ev_fork, E.ev_join);
         if (ce != cudaSuccess) st = fail(TESS_E_CUDA, "capture: %s", cudaGetErrorString(ce));
+        const uint64_t launched = E.launches;
         if (st == TESS_OK) st = enqueue_passes(E, prec, -1.0, -1, false, nullptr);
+        glaunches = grid_launches(E.total_bins, E.ndiag) + (E.launches - launched);
+        E.launches = launched;
         cudaError_t ee = cudaStreamEndCapture(E.stream, &g);
         if (st != TESS_OK) {
             if (g) cudaGraphDestroy(g);
@@ -1932,7 +1939,7 @@ static tess_status batch_run(tess_batch* b, int prec) {
         CU(cudaEventRecord(ev.e[0], E.stream));
     }
     CU(cudaGraphLaunch(G, E.stream));
-    E.launches += grid_launches(E.total_bins, E.ndiag) + (careful_alone(E.total, prec) ? 2 : (E.cfg.slots_per_lane >= 8 ? 4 : 5)) + 1;
+    E.launches += glaunches;
     if (timing) CU(cudaEventRecord(ev.e[1], E.stream));
     unsigned long long used = 0;
     const unsigned* counts = nullptr;
