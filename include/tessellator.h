@@ -309,7 +309,13 @@ tess_status tess_host_free(void* ptr);
  * larger buffer; the results are deterministic).  With on_device = 1 every
  * array argument is a device pointer; otherwise host memory.  These need only
  * the grid, not compute_all.  radius follows the reference's arithmetic for
- * any value, NaN and negative included. */
+ * any value, NaN and negative included.
+ * The handle keeps its work buffers for later queries until it is destroyed:
+ * 12 bytes a query (24 for large batches, and host arrays' copies), and for a
+ * call of tess_find_neighbors_in_radius with real_radius = 1, 8,192 queries or
+ * more and an output, lists of at most 4 GiB (4 bytes for each of 1.5 to 4 times
+ * the results that a uniform density gives).  Where memory for the lists is
+ * short the query runs without them. */
 
 /* Celery::find_cells_in_radius (celery.rs:753-796) for query positions
  * xyz[nq][3]: the bins (id = i*cpd^2 + j*cpd + k) of the box [q - r, q + r]

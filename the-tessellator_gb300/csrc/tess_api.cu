@@ -16,6 +16,7 @@
 #include <sys/stat.h>
 #include <unistd.h>
 
+#include "tess_grow.h"
 #include "tess_internal.cuh"
 #include "tessellator.h"
 
@@ -93,12 +94,14 @@ void dfree(T*& p) {
 // Device buffer of at least `need` elements (contents not kept).
 template <typename T>
 tess_status ensure(T** p, size_t& cap, size_t need) {
-    if (*p && need <= cap) return TESS_OK;
-    dfree(*p);
-    const size_t c = std::max(need, cap + cap / 2);
-    TRY(dalloc(p, c));
-    cap = c;
-    return TESS_OK;
+    return grow_buffer(
+        p, cap, need,
+        [](T** q, size_t n) {
+            const tess_status st = dalloc(q, n);
+            if (st != TESS_OK) cudaGetLastError();   // leave no error behind a failed allocation
+            return st;
+        },
+        [](T*& q) { dfree(q); });
 }
 
 // cells_per_dimension = (n / density).cbrt() as usize + 1 (celery.rs:159-160),
@@ -1298,7 +1301,6 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     if (entries > kMaxStage) len = 0;
     const bool in_pool = len && !E.computed && entries <= 2 * E.face_cap;
     if (!len || in_pool || ensure(&E.d_rwork, E.rwork_cap, head + (entries + 1) / 2) != TESS_OK) {
-        cudaGetLastError();   // leave no error behind a failed allocation
         if (!in_pool) len = 0;
         TRY(ensure(&E.d_rwork, E.rwork_cap, head));
     }
