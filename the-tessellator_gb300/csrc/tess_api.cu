@@ -706,6 +706,9 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
         p.cursor = cur + C_CURSOR + cursor++;
         p.list_fp64 = l64;
         p.list_fp64_count = c64;
+        p.list_near = E.d_list[L_FULL];
+        p.list_near_count = cnt + L_FULL;
+        p.work_most = (sample ? nsample : E.total) / 2;
         p.list_cap = lcap;
         p.list_cap_count = ccap;
         p.reasons = cur + (prec == 1 ? C_REASON32 : C_REASON64);

@@ -52,6 +52,13 @@ using namespace clipk;
 constexpr int kSlots = 64;     // vertex slots
 constexpr int kPlanes = 96;    // planes, walls included
 constexpr int kNearZ = 2;      // the first three batches take the bins up to this offset along z
+// Careful: a cell with more cuts than this that have undecided tests goes to the
+// FP64 clipping, which takes such a cell faster (a simple cubic lattice of 1,000
+// points, a compute: 423 us when every test is settled, 423 / 298 / 197 / 133 / 114
+// from 16 / 8 / 4 / 2 / 1 on).  Crystals with motion of 2e-3 seldom have more than
+// three (64^3: 4.62 ms from 1,000 / 16 / 8 / 4 on, 4.66 from 2, 4.84 from 1); the
+// tails of clustered points do (8,000: 3.5 ms from 16, 3.8 from 4).
+constexpr int kSettleMax = 4;
 
 // Instances of the pass:
 //   kPlain    over every cell; a cell with an undecided test or a crowded own
@@ -469,7 +476,8 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
     uint32_t nbeg = 0, ncnt = 0;
     float nd = INFINITY;
     unsigned pending = 0;
-    bool undec = false;              // careful: a test was settled in FP64
+    bool undec = false;              // careful: a test was settled in FP64 ...
+    int settled = 0;                 // ... in so many cuts
     if constexpr (SEED) {
         const int ti = lane / 9 - 1, tj = (lane / 3) % 3 - 1, tk = lane % 3 - 1;
         const int x = cbx + ti, y = cby + tj, z = cbz + tk;
@@ -533,7 +541,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 }
             }
             if (__any_sync(FULL, near)) {
-                status = ST_GUARD;
+                status = ST_NEAR;
                 break;
             }
             total = 32;
@@ -800,7 +808,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
             }
             // (near-)coincident points are decided in FP64
             if (__any_sync(FULL, near)) {
-                status = ST_GUARD;
+                status = ST_NEAR;
                 break;
             }
             unsigned km = __ballot_sync(FULL, keep);      // candidates within reach
@@ -973,6 +981,10 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                         break;
                     }
                     undec = true;
+                    if (!GEO && ++settled > kSettleMax) {
+                        status = ST_GUARD;
+                        break;
+                    }
                     // settle the touched vertices in FP64, one lane each, and
                     // choose again
                     uint32_t d0 = 0, d1 = 0;
@@ -1412,17 +1424,22 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
         // as the first pass, it counts what the plain pass would hand on
         if (lane == 0 && !P.work) {
             if (crowded) atomicAdd(P.list_dense_count, 1u);
-            else if (undec || status == ST_GUARD || status == ST_DEGEN || status == ST_VERIFY) atomicAdd(P.flag_count, 1u);
+            else if (undec || status == ST_GUARD || status == ST_NEAR || status == ST_DEGEN || status == ST_VERIFY) atomicAdd(P.flag_count, 1u);
         }
     }
     if (status != ST_OK) {
         if (lane == 0) {
             uint32_t* list = nullptr;
             unsigned* count = nullptr;
-            if (P.reasons) atomicAdd(&P.reasons[status & 7], 1u);
+            if (P.reasons) atomicAdd(&P.reasons[status == ST_NEAR ? ST_GUARD : status], 1u);
             if (status == ST_GUARD || status == ST_DEGEN || status == ST_VERIFY) {
                 list = P.list_fp64;
                 count = P.list_fp64_count;
+            } else if (status == ST_NEAR) {
+                // the careful pass would meet the same point
+                list = P.list_near;
+                count = P.list_near_count;
+                if (!CAREFUL) atomicAdd(P.flag_count, 1u);
             } else if (status == ST_DENSE) {
                 list = P.list_dense;
                 count = P.list_dense_count;
@@ -1485,6 +1502,19 @@ __global__ void __launch_bounds__(128, MODE == kCareful ? 4 : 5) k_lean(ClipPara
     Work W;
     int d = 0;                                    // diagram of the last cell
     const unsigned total = P.work_count ? *P.work_count : P.total;
+    if constexpr (MODE == kCareful) {
+        // most cells undecided (lattices): all of them are the FP64 clipping's (a simple
+        // cubic one of 125,000 points: 20.5 -> 4.8 ms; moved by 1e-4: 7.9 -> 6.4)
+        if (P.work_count && total > P.work_most) {
+            for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < ((total + 31u) & ~31u); i += gridDim.x * blockDim.x) {
+                unsigned at = 0;
+                if (lane == 0) at = atomicAdd(P.list_fp64_count, min(32u, total - i));
+                at = __shfl_sync(FULL, at, 0) + lane;
+                if (i < total) P.list_fp64[tess_chk(at, P.npts, P.check, CK_LIST)] = P.work[i];
+            }
+            return;
+        }
+    }
     // the next cell's number is fetched while a cell is worked on
     unsigned w = 0;
     if (lane == 0) w = atomicAdd(P.cursor, 1u);

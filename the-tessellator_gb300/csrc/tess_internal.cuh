@@ -35,7 +35,8 @@ enum CellStatus : uint8_t {
     ST_DEGEN = 4,       // inconsistent topology (degenerate input) -> FP64 re-run / error
     ST_POOL = 5,        // face pool full -> host grows the pool
     ST_VERIFY = 6,      // FP32 vertex failed the FP64 check -> FP64 re-run
-    ST_DENSE = 7,       // crowded own bin (plain first pass) -> seeded re-run
+    ST_DENSE = 7,       // crowded own bin or long batch (plain pass) -> seeded pass
+    ST_NEAR = 8,        // a (near-)coincident point (FP32 passes) -> FP64 clipping
     ST_PENDING = 255    // not computed yet
 };
 
@@ -360,6 +361,9 @@ struct ClipParams {
     // routing of failed cells
     uint32_t* list_fp64;          // guard / degenerate cells (FP32 pass) or null
     unsigned int* list_fp64_count;
+    uint32_t* list_near;          // cells with a (near-)coincident point
+    unsigned int* list_near_count;
+    unsigned work_most;           // careful pass over a list longer than this: it hands all of it on
     uint32_t* list_cap;           // capacity overflow cells or null
     unsigned int* list_cap_count;
     uint32_t* list_dense;         // plain pass: cells of crowded bins, or null
