@@ -14,7 +14,7 @@ def compute(tess, pts, prec):
 
 
 @pytest.mark.parametrize("prec", ["fp32", "mixed", "fp64"])
-@pytest.mark.parametrize("m", [10, 17, 21, 27])
+@pytest.mark.parametrize("m", [10, 17, 21, 27, 33])
 def test_exact_lattice(tess, m, prec):
     g = np.arange(m) + 0.5
     pts = np.stack(np.meshgrid(g, g, g, indexing="ij"), axis=-1).reshape(-1, 3) / m

@@ -113,12 +113,12 @@ int64_t cells_per_dim(uint64_t n, double density) {
 }
 
 // Work lists: DENSE (cells of crowded bins), CARE (cells with undecided plane
-// tests), FULL (cells for the FP64 clipping), CAP64 (those beyond its first
-// capacity).
-enum { L_DENSE = 0, L_CARE = 1, L_FULL = 2, L_CAP64 = 3, L_COUNT = 4 };
+// tests), FULL (cells for the FP64 clipping), CAP and CAP64 (cells beyond 64 and
+// 128 vertices).
+enum { L_DENSE = 0, L_CARE = 1, L_FULL = 2, L_CAP = 3, L_CAP64 = 4, L_COUNT = 5 };
 // d_counters: pass cursors, then list lengths and counts, then the cells each
 // status code was given to, in the FP32 and in the FP64 passes.
-enum { C_CURSOR = 0, C_LIST = 16, C_FAIL = 20, C_FLAG = 21, C_DENSE = 22, C_REASON32 = 32, C_REASON64 = 40,
+enum { C_CURSOR = 0, C_LIST = 16, C_FAIL = 21, C_FLAG = 22, C_DENSE = 23, C_REASON32 = 32, C_REASON64 = 40,
        C_TOTAL = 48,      // cleared for each compute, with the face cursor behind it ...
        C_FACES = 48, C_ERR = 50, C_TABLE = 51,       // ... the binning's error flag and the shell table's
        C_BYTES = 208 };                              // length, all read back together
@@ -133,11 +133,26 @@ static_assert(RET_FLAG < RET_TOTAL && 4 * (RET_ERR + 2) <= RET_BYTES, "layout of
 // finish of the form).  The careful pass finishes in FP64: where the form does
 // not ask for that, the line lies lower (FP32, 3,000 0.128 / 0.134 ms, 8,000
 // 0.216 / 0.19).  Such inputs have one launch of the FP64 clipping behind it, not
-// two.
+// two or three.
 constexpr uint32_t kCarefulMax = 8192, kCarefulMax32 = 4096;
 bool careful_alone(uint32_t n, int precision) {
     return n <= (precision == TESS_PRECISION_FP32_GUARD ? kCarefulMax32 : kCarefulMax);
 }
+// Careful pass: a cell with more cuts than this that have undecided tests goes to the
+// FP64 clipping, which takes such a cell faster.  Where the pass runs over all cells,
+// a simple cubic lattice of 1,000 points takes 423 us when every test is settled, 423
+// / 298 / 197 / 133 / 114 from 16 / 8 / 4 / 2 / 1 on, and crystals with motion of 2e-3,
+// whose cells seldom have more than three, are slower from 2 on.  Over a list it is
+// the tails of clustered points that have more (100,000: 42 ms from 16, 47 from 4).
+constexpr int kSettleMost = 16, kSettleMostAlone = 4;
+// The FP64 clipping at 64 vertices works on twice as many cells at a time as at 128, but
+// a cell that outgrows it is clipped twice, one after the other.  It takes lists
+// longer than what the 128-vertex form works on at a time (50,000 points in
+// near-coincident pairs 3.96 -> 3.20 ms, a simple cubic lattice of 125,000 4.79 ->
+// 3.99; 100,000 clustered points, whose list has 250 cells: 42 ms, 58 if it took
+// them), in inputs of more than kClip64Min points: the launch costs 6 us (10,000
+// points 203 -> 209, 60,000 704 -> 710).
+constexpr uint32_t kClip64Min = 32768;
 // The FP64 form's first pass runs in FP32 (tess_clip_lean.cu): a vertex whose
 // distance from a plane is within the FP32 error bound plus this is left to
 // the FP64 clipping, so that every decision the FP32 pass takes is the one the
@@ -274,7 +289,7 @@ struct Engine {
     const void* graph_host_nbr = nullptr;
     const void* graph_host_area = nullptr;
     uint64_t graph_host_cap = 0;
-    int blocks_cache[3][8] = {};   // [FP64 4 slots, FP64 8 slots, FP32][form, with the exact flag]
+    int blocks_cache[4][8] = {};   // [FP64 2, 4, 8 slots, FP32][form, with the exact flag]
     // allocated capacities of the grid arrays a re-grid may grow
     uint64_t delims_alloc = 0, table_alloc = 0;
     // autotuning: the timing sample, the occupancy counters, and whether the
@@ -319,16 +334,14 @@ struct Engine {
     }
 
     int blocks(int slots, int form) {
-        int& b = blocks_cache[form == kFormStd ? (slots <= 4 ? 0 : 1) : 2][form];
+        int& b = blocks_cache[form == kFormStd ? (slots <= 2 ? 0 : (slots <= 4 ? 1 : 2)) : 3][form];
         if (!b) b = clip_blocks_for(slots, form, wpb_for(slots, form), device);
         return b;
     }
     int wpb_for(int slots, int form) const {
         int w = cfg.warps_per_block;
-        if ((form & 3) != kFormStd) w = std::min(w, 4);   // their launch bound
-        if (slots >= 8) w = std::min(w, 2);
-        else if (slots >= 4) w = std::min(w, 4);
-        return std::max(1, w);
+        // their launch bounds and shared memory
+        return std::max(1, std::min(w, (form & 3) != kFormStd ? 4 : (slots <= 2 ? 8 : (slots <= 4 ? 4 : 2))));
     }
 };
 
@@ -709,6 +722,7 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
         p.list_near = E.d_list[L_FULL];
         p.list_near_count = cnt + L_FULL;
         p.work_most = (sample ? nsample : E.total) / 2;
+        p.settle_most = work && wcount ? kSettleMost : kSettleMostAlone;
         p.list_cap = lcap;
         p.list_cap_count = ccap;
         p.reasons = cur + (prec == 1 ? C_REASON32 : C_REASON64);
@@ -721,28 +735,49 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
     // without capacity re-runs, the lists beyond the configured slots are left out:
     // an overflowing cell is then reported as failed
     const bool norerun = E.cfg.flags & TESS_FLAG_NO_CAPACITY_RERUN;
-    uint32_t* const lcap = norerun && s0 == 2 ? nullptr : L[L_FULL];
+    const int lc = s0 == 2 ? L_CAP : L_FULL;
+    uint32_t* const lcap = norerun && s0 == 2 ? nullptr : L[lc];
+    unsigned* const ccap = cnt + lc;
     // The FP32 first pass hands cells of crowded bins to the dense pass and both
     // hand cells with an undecided plane test to the careful pass, which settles
     // those tests in FP64 and finishes the cell in FP64, whatever the form: such
-    // cells are ill-conditioned.  What that cannot settle, and cells beyond 64 vertices
-    // or 96 planes, are clipped in FP64 at 128 and 255 vertices.
+    // cells are ill-conditioned.  What that cannot settle is clipped in FP64, and so are
+    // cells beyond 64 vertices or 96 planes, at 128 and 255 vertices.
     const bool small = careful_alone(sample ? nsample : E.total, precision);
     if (small) {
-        TRY(pass(1, 2, kFormCareful | kFormExact, sample, nullptr, L[L_FULL], cnt + L_FULL, lcap, cnt + L_FULL, nullptr, cur + C_DENSE));
+        TRY(pass(1, 2, kFormCareful | kFormExact, sample, nullptr, L[L_FULL], cnt + L_FULL, lcap, ccap, nullptr, cur + C_DENSE));
     } else {
-        TRY(pass(1, 2, kFormLean | X, sample, nullptr, L[L_CARE], cnt + L_CARE, lcap, cnt + L_FULL, L[L_DENSE], cnt + L_DENSE));
+        TRY(pass(1, 2, kFormLean | X, sample, nullptr, L[L_CARE], cnt + L_CARE, lcap, ccap, L[L_DENSE], cnt + L_DENSE));
     }
     if (timing) CU(cudaEventRecord(ev[1], E.stream));
     if (!small) {
-        TRY(pass(1, 2, kFormDense | X, L[L_DENSE], cnt + L_DENSE, L[L_CARE], cnt + L_CARE, lcap, cnt + L_FULL));
-        TRY(pass(1, 2, kFormCareful | kFormExact, L[L_CARE], cnt + L_CARE, L[L_FULL], cnt + L_FULL, lcap, cnt + L_FULL));
+        TRY(pass(1, 2, kFormDense | X, L[L_DENSE], cnt + L_DENSE, L[L_CARE], cnt + L_CARE, lcap, ccap));
+        TRY(pass(1, 2, kFormCareful | kFormExact, L[L_CARE], cnt + L_CARE, L[L_FULL], cnt + L_FULL, lcap, ccap));
     }
-    if (s0 < 8 && (!small || norerun)) {
-        TRY(pass(0, 4, kFormStd, L[L_FULL], cnt + L_FULL, nullptr, nullptr, norerun ? nullptr : L[L_CAP64], cnt + L_CAP64));
-        TRY(pass(0, 8, kFormStd, L[L_CAP64], cnt + L_CAP64, nullptr, nullptr, nullptr, nullptr));
+    // The FP64 clipping: lists {cells, beyond 64, beyond 128 vertices}
+    struct Work { int list; unsigned least; int list2; unsigned most2; };
+    auto clip64 = [&](int slots, Work w, bool last, int next = 0) -> tess_status {
+        base.work_least = w.least;
+        base.work2 = w.most2 ? L[w.list2] : nullptr;
+        base.work2_count = cnt + w.list2;
+        base.work2_most = w.most2;
+        return pass(0, slots, kFormStd, L[w.list], cnt + w.list, nullptr, nullptr, last ? nullptr : L[next], cnt + next);
+    };
+    const unsigned all = ~0u;
+    if (s0 == 2 && norerun) {
+        TRY(clip64(2, {L_FULL}, true));
+    } else if (s0 == 2 && small) {
+        TRY(clip64(8, {L_CAP, 0, L_FULL, all}, true));
+    } else if (s0 == 2) {
+        const unsigned few = (sample ? nsample : E.total) <= kClip64Min ? all : (unsigned)(E.blocks(4, kFormStd) * E.wpb_for(4, kFormStd));
+        if (few != all) TRY(clip64(2, {L_FULL, few}, false, L_CAP));
+        TRY(clip64(4, {L_CAP, 0, L_FULL, few}, false, L_CAP64));
+        TRY(clip64(8, {L_CAP64}, true));
+    } else if (s0 == 4 && (!small || norerun)) {
+        TRY(clip64(4, {L_FULL}, norerun, L_CAP64));
+        if (!norerun) TRY(clip64(8, {L_CAP64}, true));
     } else {
-        TRY(pass(0, 8, kFormStd, L[L_FULL], cnt + L_FULL, nullptr, nullptr, nullptr, nullptr));
+        TRY(clip64(8, {L_FULL}, true));
     }
     if (timing) CU(cudaEventRecord(ev[2], E.stream));
     return TESS_OK;
@@ -765,13 +800,14 @@ tess_status read_back(Engine& E, const unsigned** counts, unsigned long long* fa
 void read_counts(Engine& E, const unsigned* c, uint64_t faces) {
     const unsigned *r32 = c + C_REASON32, *r64 = c + C_REASON64;
     const uint64_t cap32 = (uint64_t)r32[ST_VCAP] + r32[ST_PCAP];
+    const int s0 = E.cfg.slots_per_lane;
     E.stats.cells = E.total;
     E.stats.faces = faces;
     if (E.ndiag == 1) E.stats.table_entries = c[C_TABLE];
     E.stats.rerun_fp64 = (uint64_t)c[C_LIST + L_CARE] + c[C_FLAG];
-    E.stats.rerun_fp64_full = (uint64_t)c[C_LIST + L_FULL] - std::min<uint64_t>(cap32, c[C_LIST + L_FULL]);
+    E.stats.rerun_fp64_full = (uint64_t)c[C_LIST + L_FULL] - (s0 == 2 ? 0 : std::min<uint64_t>(cap32, c[C_LIST + L_FULL]));
     E.stats.dense_cells = (uint64_t)c[C_LIST + L_DENSE] + c[C_DENSE];
-    E.stats.rerun_capacity = cap32 + c[C_LIST + L_CAP64];
+    E.stats.rerun_capacity = (s0 == 2 ? c[C_LIST + L_CAP] : cap32) + (uint64_t)c[C_LIST + L_CAP64];
     E.stats.failed = c[C_FAIL];
     E.stats.rerun_guard = (uint64_t)r32[ST_GUARD] + r64[ST_GUARD];
     E.stats.rerun_verify = (uint64_t)r32[ST_VERIFY] + r64[ST_VERIFY];
@@ -1906,7 +1942,7 @@ static tess_status batch_run(tess_batch* b, int prec) {
                                  E.graph_host_cap != E.face_cap));
     if (stale) {
         // warm the per-kernel attributes and occupancy queries outside capture
-        for (int k : {4, 8}) E.blocks(k, kFormStd);
+        for (int k : {2, 4, 8}) E.blocks(k, kFormStd);
         for (int f : {(int)kFormLean, (int)kFormDense})
             for (int x : {0, (int)kFormExact}) E.blocks(2, f | x);
         E.blocks(2, kFormCareful | kFormExact);

@@ -1501,15 +1501,16 @@ __global__ void __launch_bounds__(K == 2 ? 256 : 128, K == 2 ? 2 : 1) k_clip(Cli
     extern __shared__ __align__(16) unsigned char smraw[];
     Smem<K>& S = reinterpret_cast<Smem<K>*>(smraw)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    if (P.grid_err && *P.grid_err == 1) return;   // non-finite input: nothing to clip
+    const unsigned n1 = P.work_count ? *P.work_count : P.total, n2 = P.work2 ? *P.work2_count : 0u;
+    unsigned total = (P.work_least && n1 <= P.work_least ? 0u : n1) + (n2 <= P.work2_most ? n2 : 0u);
+    if (P.grid_err && *P.grid_err == 1) total = 0;   // non-finite input: nothing to clip
     Work W;
-    for (;;) {
+    while (total) {
         unsigned w = 0;
         if (lane == 0) w = atomicAdd(P.cursor, 1u);
         w = __shfl_sync(FULL, w, 0);
-        const unsigned total = P.work_count ? *P.work_count : P.total;
         if (w >= total) break;
-        const uint32_t gs = P.work ? P.work[w] : w;
+        const uint32_t gs = w >= n1 ? P.work2[w - n1] : (P.work ? P.work[w] : w);
         run_cell<K, GEO>(P, S, gs, lane, W);
     }
     if (P.work_ctr && lane == 0) {

@@ -52,13 +52,6 @@ using namespace clipk;
 constexpr int kSlots = 64;     // vertex slots
 constexpr int kPlanes = 96;    // planes, walls included
 constexpr int kNearZ = 2;      // the first three batches take the bins up to this offset along z
-// Careful: a cell with more cuts than this that have undecided tests goes to the
-// FP64 clipping, which takes such a cell faster (a simple cubic lattice of 1,000
-// points, a compute: 423 us when every test is settled, 423 / 298 / 197 / 133 / 114
-// from 16 / 8 / 4 / 2 / 1 on).  Crystals with motion of 2e-3 seldom have more than
-// three (64^3: 4.62 ms from 1,000 / 16 / 8 / 4 on, 4.66 from 2, 4.84 from 1); the
-// tails of clustered points do (8,000: 3.5 ms from 16, 3.8 from 4).
-constexpr int kSettleMax = 4;
 
 // Instances of the pass:
 //   kPlain    over every cell; a cell with an undecided test or a crowded own
@@ -67,8 +60,9 @@ constexpr int kSettleMax = 4;
 //   kDense    over the cells of crowded bins: seeded, points gathered
 //   kCareful  as kDense, and undecided tests are settled in FP64 in place: over
 //             the cells the others handed on, or over every cell of a small
-//             input.  Always with the FP64 finish.  (An instance of its own: the settling makes the code
-//             half as large again, and the dense pass waits for instructions.)
+//             input.  Always with the FP64 finish.  (An instance of its own: the
+//             settling makes the code half as large again, and the dense pass
+//             waits for instructions.)
 //   kGeo      one cell with its geometry (single-cell queries): careful, the
 //             site may be any position and the container any box
 enum Mode : int { kPlain = 0, kCount = 1, kDense = 2, kCareful = 3, kGeo = 4 };
@@ -981,7 +975,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                         break;
                     }
                     undec = true;
-                    if (!GEO && ++settled > kSettleMax) {
+                    if (!GEO && ++settled > P.settle_most) {
                         status = ST_GUARD;
                         break;
                     }

@@ -347,6 +347,12 @@ struct ClipParams {
     // work: sorted positions to process
     const uint32_t* work;          // null: 0 .. total-1
     const uint32_t* work_count;    // null: total
+    // FP64 clipping: a list not longer than work_least is left to the next pass, which
+    // takes it as its second one (work2) when it is not longer than work2_most
+    unsigned work_least;
+    const uint32_t* work2;
+    const uint32_t* work2_count;
+    unsigned work2_most;
     uint32_t total;
     unsigned int* cursor;          // work cursor (zeroed before launch)
     // results, indexed by point (concatenated original order)
@@ -364,6 +370,7 @@ struct ClipParams {
     uint32_t* list_near;          // cells with a (near-)coincident point
     unsigned int* list_near_count;
     unsigned work_most;           // careful pass over a list longer than this: it hands all of it on
+    int settle_most;              // careful pass: a cell with more such cuts is handed on
     uint32_t* list_cap;           // capacity overflow cells or null
     unsigned int* list_cap_count;
     uint32_t* list_dense;         // plain pass: cells of crowded bins, or null
@@ -416,7 +423,7 @@ cudaError_t launch_cell_lean(const ClipParams& p, cudaStream_t s);
 int clip_blocks_lean(int form, int wpb, int device);
 cudaError_t launch_clip_f64(const ClipParams& p, int slots, int wpb, int blocks, cudaStream_t s);
 int clip_blocks_f64(int slots, int wpb, int device);
-// slots (kFormStd): vertex slots per lane, 4 or 8.
+// slots (kFormStd): vertex slots per lane, 2, 4 or 8.
 cudaError_t launch_clip(const ClipParams& p, int slots, int form, int warps_per_block, int blocks, cudaStream_t s);
 int clip_blocks_for(int slots, int form, int warps_per_block, int device);
 // CSR offsets (3 launches) and the gather into them (1 launch).
