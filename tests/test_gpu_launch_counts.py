@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
     (1000, False, 1 + 1 + 1 + 1),            # count, scan, copy of the offsets, fill
     (16384, False, 1 + 1 + 1 + 1),
     (16385, False, 1 + 3 + 1 + 1),
-    (16384, True, 1 + 1 + 1 + 2),            # the listed results to their places, the others found again
+    (262_144, True, 1 + 3 + 1 + 2),          # the listed results to their places, the others found again
     (600_000, False, 3 + 1 + 3 + 1 + 1),     # order: bins, scan, scatter
 ])
 def test_radius_queries(tess, nq, crowd, want):

@@ -535,6 +535,8 @@ GridBuffers grid_buffers(Engine& E) {
     g.table_gaps = E.cfg.table_gaps;
     g.error_flag = E.d_err;
     g.table_len = E.d_counters + C_TABLE;
+    const double fill = (double)E.total / (double)E.total_bins;
+    g.crowded = (uint32_t)(fill + 6.0 * std::sqrt(fill)) + 1u;
     g.host_flag = reinterpret_cast<int*>(E.d_ret + RET_FLAG);
     g.check = E.d_check;
     return g;
@@ -1335,7 +1337,9 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     // the results again.
     const size_t tmp_words = csr_tmp_words((uint32_t)std::max<size_t>(nq, 1));
     const size_t head = (nq + 1) + tmp_words + 1 + (nq + 2) / 2;
-    size_t len = out && cap && nq && E.hgrid_valid ? radius_stage_len(mode, (uint32_t)nq, E.total, D, radius) : 0;
+    // (D is valid: the gap table's build, of this binning, has read it)
+    p.lanes = mode != RQ_CLOUD && E.hgrid_valid && radius_lanes(mode, (uint32_t)nq, E.total, D);
+    size_t len = out && cap && p.lanes ? radius_stage_len(mode, E.total, D, radius) : 0;
     const size_t entries = len * ((nq + 31) / 32 * 32);
     if (entries > kMaxStage) len = 0;
     const bool in_pool = len && !E.computed && entries <= 2 * E.face_cap;
@@ -1362,7 +1366,7 @@ tess_status engine_radius(Engine& E, int mode, bool by_cell, const double* qxyz,
     uint64_t tot = 0;
     if (nq) {
         if (timing) CU(cudaEventRecord(ev[0], E.stream));
-        if (nq >= (mode == RQ_CELL_RADIUS || mode == RQ_REAL_RADIUS ? kOrderMinLane : kOrderMin) && (p.qxyz || p.qcell)) {
+        if (nq >= (p.lanes ? kOrderMinLane : kOrderMin) && (p.qxyz || p.qcell)) {
             // process large batches in coarse-bin order: neighbouring warps then
             // read the same candidate bins
             QueryOrder o{};

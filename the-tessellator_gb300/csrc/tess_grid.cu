@@ -71,6 +71,7 @@ __device__ __forceinline__ void grid_params(const GridBuffers& g, int t) {
     D.inv_s[a] = ext > 0.0 ? inv_f : 0.f;
     if (a != 0) return;
     D.lean_ok = quad == 7u;
+    D.crowd = 0;
     // (x - glo) * inv from the FP32 pairs: one rounding of the difference, one
     // of inv, one of the product (u = 2^-24 each, relative to the result, at
     // most cpd bins), with a factor 4 in hand
@@ -409,8 +410,10 @@ __global__ void __launch_bounds__(256) k_bin_order(GridBuffers g) {
     __syncthreads();
     const uint64_t b0 = (uint64_t)blockIdx.x * blockDim.x;
     const uint64_t b = b0 + threadIdx.x;
+    uint32_t crowd = 0;
     if (b < g.total_bins) {
         const uint32_t beg = g.delims[b], end = g.delims[b + 1];
+        if (end - beg > g.crowded) crowd = end - beg;
         if (end - beg > 32) {
             big[atomicAdd(&nbig, 1u)] = threadIdx.x;
         } else if (end - beg >= 2) {
@@ -425,6 +428,9 @@ __global__ void __launch_bounds__(256) k_bin_order(GridBuffers g) {
             }
         }
     }
+    // how evenly the points fill the grid (radius queries, of one diagram)
+    crowd = __reduce_add_sync(0xffffffffu, crowd);
+    if (crowd && g.ndiag == 1 && (threadIdx.x & 31) == 0) atomicAdd(&g.diags[0].crowd, crowd);
     __syncthreads();
     const uint32_t nb = nbig;
     for (uint32_t q = 0; q < nb; ++q) {

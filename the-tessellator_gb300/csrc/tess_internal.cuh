@@ -102,6 +102,7 @@ struct DiagDesc {
     float inv_s[3];                      // inverse bin sides, 0 on an axis without extent
     float frac_eps;                      // bound on the FP32 in-bin position's error, in bins
     int32_t has_extent;                  // some bin side is nonzero (min_size > 0)
+    uint32_t crowd;                      // points in bins of more than GridBuffers::crowded (a single diagram's)
     int32_t lean_ok;                     // inv_s and size_f are in FP32's normal range (or 0)
 };
 
@@ -219,6 +220,7 @@ struct GridBuffers {
     int table_gaps;
     int* error_flag;            // set when an input coordinate is not finite
     unsigned* table_len;        // entries of the first diagram's shell table
+    uint32_t crowded;           // a bin's points that evenly spread points do not reach
     int* host_flag;             // its value after the bounds, in mapped host memory, or null
     int* check;                 // checked build: the check word
 };
@@ -290,6 +292,7 @@ struct RadiusParams {
     // place i of the processing order, at stage[(i / 32 * stage_len + k) * 32 + i % 32]
     uint32_t* stage;
     uint32_t stage_len;
+    int lanes;                  // a lane per query
     int unlisted;               // fill pass: some query has more results than are listed
     int gtab_tie;               // some squared gap distance is at most 1% above radius^2
     // bin boundaries per axis: bnd[a * cpd + i] (1 <= i < cpd) is the order
@@ -300,7 +303,9 @@ struct RadiusParams {
 // RadiusParams::stage_len for a batch of nq queries of a diagram of n points: six
 // standard deviations above the results that a uniform density gives a query; 0:
 // nothing is listed.
-uint32_t radius_stage_len(int mode, uint32_t nq, uint32_t n, const DiagDesc& D, double radius);
+uint32_t radius_stage_len(int mode, uint32_t n, const DiagDesc& D, double radius);
+// Whether a batch of nq queries takes a lane per query (else a warp).
+bool radius_lanes(int mode, uint32_t nq, uint32_t n, const DiagDesc& D);
 
 // Fills RadiusParams::bnd for diagram 0 (3 * cpd entries).
 cudaError_t launch_axis_bounds(const DiagDesc* desc, int cpd, unsigned long long* bnd, cudaStream_t s);

@@ -36,10 +36,6 @@ namespace tess {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-// Queries from which a lane answers one.  1,000,000 points, 16 results each,
-// whole calls: 4,000 queries 89 us by warps and 109 by lanes, 8,192 about 105 and
-// 104, 16,384 137 and 120, 65,535 213 and 112.
-constexpr uint32_t kLaneMin = 8192;
 constexpr uint32_t kLongRun = 64;     // points of a row from which a warp shares them
 constexpr int kLaneThreads = 128;     // threads of such a block
 constexpr int kLaneRows = 16;         // rows listed at a time
@@ -803,7 +799,7 @@ __global__ void __launch_bounds__(256) k_query_scatter(uint32_t nq, QueryOrder o
 template <int MODE>
 cudaError_t launch_mode(const RadiusParams& p, bool fill, int blocks, cudaStream_t s) {
     if constexpr (MODE == RQ_REAL_RADIUS || MODE == RQ_CELL_RADIUS) {
-        if (p.nq >= kLaneMin) {
+        if (p.lanes) {
             const unsigned nb = (unsigned)(((uint64_t)p.nq + kLaneThreads - 1) / kLaneThreads);
             if (fill && p.stage_len) {
                 k_radius_place<<<nb, kLaneThreads, 0, s>>>(p);
@@ -864,8 +860,24 @@ struct RadiusEntry {
 
 }  // namespace
 
-uint32_t radius_stage_len(int mode, uint32_t nq, uint32_t n, const DiagDesc& D, double radius) {
-    if (mode != RQ_REAL_RADIUS || nq < kLaneMin) return 0;
+// Queries from which a lane answers one.  Whole calls on an evenly filled grid, by
+// warps and by lanes, 1,000,000 points and 16 results each: 4,000 queries 89 and 109
+// us, 8,192 about 105 and 104, 16,384 137 and 120, 65,535 213 and 112; every point
+// of the bins instead: 8,192 59 and 75, 16,384 74 and 78, 32,768 85 and 80.
+// Where points crowd, a lane in the crowd keeps its warp waiting: 200,000 points, 90%
+// of them in 64 clusters, 19 results each: 8,192 queries 153 and 468, 65,536 475 and
+// 563, 131,072 805 and 923, 262,144 1,473 and 1,360, 600,000 3,146 and 1,925; 10%
+// in the clusters 95 and 206, 223 and 222, 338 and 342, 565 and 478, 1,134 and 520;
+// every point of the bins, 615 of them: 600,000 1,299 and 4,090.
+constexpr uint32_t kLaneMin = 8192, kLaneMinCell = 16384, kLaneMinCrowded = 262144;
+bool radius_lanes(int mode, uint32_t nq, uint32_t n, const DiagDesc& D) {
+    const bool even = D.crowd <= n / 64;
+    if (mode == RQ_REAL_RADIUS) return nq >= (even ? kLaneMin : kLaneMinCrowded);
+    return mode == RQ_CELL_RADIUS && even && nq >= kLaneMinCell;
+}
+
+uint32_t radius_stage_len(int mode, uint32_t n, const DiagDesc& D, double radius) {
+    if (mode != RQ_REAL_RADIUS) return 0;
     double mean = n * 4.1887902047863910 * radius * radius * radius;
     for (int a = 0; a < 3; ++a) mean /= D.size[a] * D.cpd;
     if (!(mean >= 0.0 && mean <= 200.0)) return 0;
