@@ -64,3 +64,15 @@ def test_single_cell(tess):
         start = d.stats()["launches"]
         d.get_cell_at_index(4).compute_voronoi_cell()
         assert d.stats()["launches"] == start + 1
+
+
+@pytest.mark.parametrize("p,launches", [((0.4, 0.5, 0.6), 1), ((0.4, 0.5, 1.6), 1), ((0.4, 0.5, 1.0), 1), ((-1e-9, 0.5, 0.6), 1)])
+def test_cell_at_a_position(tess, oracle_mod, p, launches):
+    """Inside the container, above it, on its wall, just below it: one launch each."""
+    pts = np.random.default_rng(7).random((1000, 3))
+    ref = oracle_mod.Diagram(pts, lo=[0, 0, 0], hi=[1, 1, 1]).cell_at(list(p))
+    with tess.Diagram(pts, container=tess.Polyhedron(0, 0, 0, 1, 1, 1)) as d:
+        start = d.stats()["launches"]
+        cell = d.get_cell_at_particle(list(p)).compute_voronoi_cell()
+        assert d.stats()["launches"] == start + launches
+        assert cell.compute_neighbors() == ref.ids.tolist()

@@ -1195,10 +1195,17 @@ tess_status engine_geo(Engine& E, int precision, const size_t* i, const double* 
             p.box[3 + a] = hi[a];
         }
     }
-    CU(launch_cell_lean(p, E.stream));
-    E.launches += 1;
-    CU(cudaStreamSynchronize(E.stream));
-    if (E.h_geo->status != ST_OK) {
+    // (the careful pass leaves a position outside the container to the FP64 clipping:
+    // 50 us with it, 40 without)
+    bool in = true;
+    for (int a = 0; point && a < 3; ++a)
+        in = in && point[a] > (lo ? lo[a] : E.hdesc[0].blo[a]) && point[a] < (hi ? hi[a] : E.hdesc[0].bhi[a]);
+    if (in) {
+        CU(launch_cell_lean(p, E.stream));
+        E.launches += 1;
+        CU(cudaStreamSynchronize(E.stream));
+    }
+    if (!in || E.h_geo->status != ST_OK) {
         CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * C_TOTAL, E.stream));
         p.cursor = E.d_counters;
         CU(launch_clip(p, 8, kFormStd, 1, 1, E.stream));
