@@ -97,7 +97,8 @@ typedef struct {
     double bin_density;
     /* Extent of the precomputed shell table, in bins of gap (>= 1). */
     int32_t table_gaps;
-    /* Warps per block of the clipping kernel (1..32). */
+    /* Warps per block of the clipping kernels, at most (1..32): the FP32 passes take up
+     * to 4, the FP64 clipping up to 8, 4 or 2 at 64, 128 or 255 vertices. */
     int32_t warps_per_block;
     /* Vertex slots per lane (2, 4 or 8).  The FP32 passes hold 64 vertices;
      * cells beyond that are clipped in FP64 at 128 and then 255, with 8 at
@@ -400,7 +401,7 @@ tess_status tess_batch_destroy(tess_batch* b);
  * the whole box and every diagram of a batch).  Results never depend on
  * them: they change how the work is laid out, not what is computed. */
 typedef struct {
-    int32_t warps_per_block;   /* chosen warps per block of the clipping kernel      */
+    int32_t warps_per_block;   /* chosen warps per block (tess_config)               */
     int32_t crowded_bin;       /* chosen crowded-bin threshold (tess_config)        */
     double bin_density;        /* batch: chosen points per bin of the batch's grid;
                                   diagram: the Celery grid's density, unchanged, as
@@ -408,7 +409,8 @@ typedef struct {
     double ms_chosen;          /* the sample's compute time with the chosen knobs   */
     double ms_default;         /* ... with the default knobs                        */
     uint64_t sample_cells;     /* cells in the timing sample                         */
-    int32_t trials;            /* candidate knob sets timed (0: read from the cache) */
+    int32_t trials;            /* candidate knob sets compared (0: read from the cache);
+                                  those that launch the same kernels are timed once  */
     int32_t from_cache;        /* 1: the choice came from the cache file             */
     uint32_t max_bin_points;   /* the input's most crowded bin (points)             */
     double crowded_fraction;   /* share of points in bins of >= 12 points           */

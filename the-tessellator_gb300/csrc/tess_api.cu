@@ -1056,9 +1056,11 @@ tess_status time_sample(Engine& E, int precision, uint32_t m, float* ms) {
 // Choose warps per block, the crowded-bin threshold and (batches) the grid
 // density by timing each candidate on an evenly spaced sample of up to
 // 262,144 cells in bin order (the whole box, every diagram), two runs each,
-// the faster counted.  Candidates: warps per block {4, 8} (the clipping
-// kernel's launch bound allows 8 at most), crowded bin {12, 8, 24, 48},
-// density {0.6, 1.25, 2.5} points per bin (batches).
+// the faster counted.  Candidates: warps per block {8, 4}, crowded bin {12, 8, 24,
+// 48}, density {1.25, 0.6, 2.5} points per bin (batches), the default first; another
+// is taken when it is 1% faster.  Only the FP64 clipping at 64 vertices takes 8 warps a
+// block (Engine::wpb_for): where the sample does not reach that size, 4 launches what
+// 8 does and has its times.
 tess_status engine_autotune(Engine& E, int precision, bool batch, const char* cache_path, tess_tuning* out) {
     if (!E.built) return fail(TESS_E_STATE, "the grid is not built");
     if (precision != TESS_PRECISION_FP64 && precision != TESS_PRECISION_FP32_GUARD && precision != TESS_PRECISION_MIXED)
@@ -1124,20 +1126,24 @@ tess_status engine_autotune(Engine& E, int precision, bool batch, const char* ca
             if (layout_grid(probe, de, E.cfg.table_gaps, &nb, &nt) != TESS_OK) continue;   // too many bins
             TRY(engine_regrid(E, de));
         }
+        float first[4];
         for (int w : wpbs)
-            for (int c : crowds) {
+            for (int k = 0; k < 4; ++k) {
+                const int c = crowds[k];
                 E.cfg.warps_per_block = w;
                 E.cfg.crowded_bin = c;
                 std::memset(E.blocks_cache, 0, sizeof(E.blocks_cache));
-                float t = INFINITY;
-                for (int rep = 0; rep < 2; ++rep) {
+                const bool known = w != wpbs[0] && !(E.cfg.slots_per_lane == 2 && m > kClip64Min);
+                float t = known ? first[k] : INFINITY;
+                for (int rep = 0; rep < 2 && !known; ++rep) {
                     float ms = 0.f;
                     TRY(time_sample(E, precision, m, &ms));
                     t = std::min(t, ms);
                 }
+                if (w == wpbs[0]) first[k] = t;
                 ++T.trials;
                 if (de == 1.25 && w == 8 && c == kDefaultCrowdedBin) T.ms_default = t;
-                if (t < best) {
+                if (t < 0.99f * best) {
                     best = t;
                     bw = w;
                     bc = c;
