@@ -687,8 +687,8 @@ ClipParams base_params(Engine& E) {
 }
 
 // The fixed launch sequence of one compute (no host synchronisation):
-// first pass, capacity re-runs, FP64 re-runs.  Counters: cursor c at
-// d_counters[c], list counts at d_counters[16 + list].
+// the FP32 passes, then the FP64 clipping over what they hand on.  d_counters holds
+// a cursor per pass, list counts and reasons (C_*).
 tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t group, bool timing,
                            cudaEvent_t* ev, const uint32_t* sample = nullptr, uint32_t nsample = 0) {
     unsigned* cur = E.d_counters;

@@ -14,8 +14,7 @@
 //   - its plane triple (a, b, c), ordered counter-clockwise seen from outside,
 //   - its three neighbours: adj[i] is the vertex across the edge (t[i], t[i+1]).
 // The half-edge pools of the reference (pool.rs) become these fixed-capacity
-// slot arrays; a cell that outgrows them is flagged and re-run at a larger
-// capacity.
+// slot arrays; a cell that outgrows them is listed for a larger capacity.
 //
 // Cutting by a bisector (vector3.rs:223-239):
 //   1. every lane classifies its vertices, sd = n.v - offset, Outside when
@@ -57,9 +56,6 @@ constexpr unsigned FULL = 0xffffffffu;
 // FP32 form: relative error constant of a vertex solved from its three planes
 // (a few FP32 roundings of the plane data and of Cramer's rule).
 constexpr float kVertexErr = 1.5e-6f;
-// Load the next batch's table entries and bin ranges before cutting the
-// current batch (overlaps their latency, costs registers).
-constexpr bool kPrefetch = true;
 // Pre-test a window's candidates against the live vertices when at least
 // this many are within twice the cell radius.
 constexpr int kPretestMin = 2;
@@ -857,11 +853,9 @@ __device__ void run_cell(const ClipParams& P, Smem<K>& S, uint32_t gs, int lane,
     auto run_window = [&](bool keep, double rx, double ry, double rz, double r2, uint32_t j, int32_t cid) -> int {
         unsigned km = __ballot_sync(FULL, keep);
         // Pre-test the window at once: each lane tests its own candidate's
-        // bisector against every live vertex (read from the shared
-        // mirror).  A bisector with no vertex Outside cuts nothing now and
-        // nothing later (the cell only shrinks), so only possible cutters
-        // (and guard-band cases, which the serial test reports) go on to
-        // the serial nearest-first loop.  Same arithmetic as cut().
+        // bisector against every live vertex.  A bisector with no vertex
+        // Outside cuts nothing now and nothing later (the cell only shrinks), so
+        // only possible cutters go on to the serial nearest-first loop.
         if (__popc(km) >= kPretestMin) {
             bool maycut = false;
             if (keep) {
@@ -885,23 +879,6 @@ __device__ void run_cell(const ClipParams& P, Smem<K>& S, uint32_t gs, int lane,
                     }
                 }
                 maycut = out;
-            } else if (keep) {
-                double nx_, ny_, nz_, off_, rn_;
-                bisector(rx, ry, rz, r2, nx_, ny_, nz_, off_, rn_);
-                bool out = false, amb = false;
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    uint32_t m = C.lm[k];
-                    while (m) {
-                        const int sl = k * 32 + __ffs(m) - 1;
-                        m &= m - 1u;
-                        const double sd = sdist(nx_, ny_, nz_, off_, S.vx[sl], S.vy[sl], S.vz[sl]);
-                        // any vertex beyond the plane may be cut (the serial
-                        // test applies the tolerance)
-                        out |= sd > 0.0;
-                    }
-                }
-                maycut = out || amb;
             }
             km = __ballot_sync(FULL, keep && maycut);
         }
@@ -1367,21 +1344,9 @@ __device__ void run_cell(const ClipParams& P, Smem<K>& S, uint32_t gs, int lane,
             return;
         }
         if (lane == 0) {
-            uint32_t* list = nullptr;
-            unsigned* count = nullptr;
-            if (P.reasons) atomicAdd(&P.reasons[status & 7], 1u);
-            if (status == ST_DEGEN) {
-                list = P.list_fp64;
-                count = P.list_fp64_count;
-            } else if (status == ST_VCAP || status == ST_PCAP) {
-                list = P.list_cap;
-                count = P.list_cap_count;
-            } else if (status == ST_DENSE) {
-                list = P.list_dense;
-                count = P.list_dense_count;
-            }
-            if (list) {
-                list[tess_chk(atomicAdd(count, 1u), P.npts, P.check, CK_LIST)] = gs;
+            if (P.reasons) atomicAdd(&P.reasons[status], 1u);
+            if ((status == ST_VCAP || status == ST_PCAP) && P.list_cap) {
+                P.list_cap[tess_chk(atomicAdd(P.list_cap_count, 1u), P.npts, P.check, CK_LIST)] = gs;
                 P.status[orig] = ST_PENDING;
             } else {
                 P.status[orig] = (uint8_t)status;

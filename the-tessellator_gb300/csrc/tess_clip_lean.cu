@@ -488,7 +488,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
     }
     const float fx = fminf(fmaxf(px - (float)cbx, 0.f), 1.f), fy = fminf(fmaxf(py - (float)cby, 0.f), 1.f);
     const float fz = fminf(fmaxf(pz - (float)cbz, 0.f), 1.f);
-    // Careful: when the own bin is crowded, it and the crowded bins around it
+    // Dense and careful: when the own bin is crowded, it and the crowded bins around it
     // are seeded first, nearest first: each lane takes the nearest point of its
     // stride of the bin, and the 32 are cut as one window.  Otherwise windows
     // in storage order meet the nearest points late, after many cuts by farther
@@ -521,7 +521,7 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
     if (!(R2 >= FLT_MIN)) status = ST_GUARD;
     if (GEO && !(R2 < 1e30f)) status = ST_GUARD;
     while (status == ST_OK) {
-        float sx_ = 0.f, sy_ = 0.f, sz_ = 0.f, s2_ = INFINITY;   // careful: my seed
+        float sx_ = 0.f, sy_ = 0.f, sz_ = 0.f, s2_ = INFINITY;   // my seed
         uint32_t sj_ = 0;
         unsigned total, pref = 0;
         uint32_t bbeg = 0, bcnt = 0;
@@ -582,7 +582,13 @@ __device__ __forceinline__ void run_lean(const ClipParams& P, Lean& S, uint32_t 
                 const float rx_ = rc * inx + feps, ry_ = rc * iny + feps, rz_ = rc * inz + feps;
                 const float far = fmaxf(fmaxf(rx_ + fx, rx_ + 1.f - fx), fmaxf(ry_ + fy, ry_ + 1.f - fy));
                 if (m == 2 && !(far >= 2.f)) m = 3;
-                if (m == 3 && !(fmaxf(rz_ + fz, rz_ + 1.f - fz) >= (float)(kNearZ + 1))) m = 4;
+                // (batch 3 goes on once begun, while the ends are in reach: a point of it
+                // that cuts leaves a face at half its distance, so twice the radius
+                // reaches the ends still; ring 4 begins at its first row in any case)
+                if (m == 3 && !(fmaxf(rz_ + fz, rz_ + 1.f - fz) >= (float)(kNearZ + 1))) {
+                    m = 4;
+                    ring0 = 0;
+                }
                 // a cell that a search radius leaves open reaches far: its rings end
                 // with the radius (50,000 points, radius 0: 3.1 -> 0.6 ms)
                 if (P.has_radius) m = radius_next(D, P.search_radius, m);

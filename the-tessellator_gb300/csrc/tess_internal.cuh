@@ -29,12 +29,13 @@ constexpr int kMaxTable = 4096;             // shell-table entries per diagram (
 // Per-cell status codes written by the clipping kernels.
 enum CellStatus : uint8_t {
     ST_OK = 0,
-    ST_GUARD = 1,       // FP32 plane-side test inside the guard band -> FP64 re-run
-    ST_VCAP = 2,        // vertex capacity exceeded -> larger capacity re-run
-    ST_PCAP = 3,        // face (plane) capacity exceeded -> larger capacity re-run
-    ST_DEGEN = 4,       // inconsistent topology (degenerate input) -> FP64 re-run / error
+    ST_GUARD = 1,       // plane-side test inside the guard band (plain, dense) -> careful
+                        // pass; not to be settled there -> FP64 clipping
+    ST_VCAP = 2,        // vertex capacity exceeded -> FP64 clipping, larger
+    ST_PCAP = 3,        // face (plane) capacity exceeded -> FP64 clipping, larger
+    ST_DEGEN = 4,       // inconsistent topology -> as ST_GUARD; FP64 clipping: error
     ST_POOL = 5,        // face pool full -> host grows the pool
-    ST_VERIFY = 6,      // FP32 vertex failed the FP64 check -> FP64 re-run
+    ST_VERIFY = 6,      // FP32 vertex failed the FP64 check -> as ST_GUARD
     ST_DENSE = 7,       // crowded own bin or long batch (plain pass) -> seeded pass
     ST_NEAR = 8,        // a (near-)coincident point (FP32 passes) -> FP64 clipping
     ST_PENDING = 255    // not computed yet
@@ -53,7 +54,7 @@ enum CheckSite : int {
     CK_BIN = 1,     // a bin of the grid
     CK_SLOT = 2,    // a vertex slot or free-slot stack entry of a cell
     CK_PLANE = 3,   // a plane of a cell
-    CK_LIST = 4,    // an entry of a re-run list
+    CK_LIST = 4,    // an entry of a work list
     CK_FACE = 5,    // a face of the face pool
     CK_GRID = 6     // a position of the binning pass's sort
 };
@@ -370,7 +371,7 @@ struct ClipParams {
     unsigned long long* face_cursor;
     uint64_t face_cap;
     // routing of failed cells
-    uint32_t* list_fp64;          // guard / degenerate cells (FP32 pass) or null
+    uint32_t* list_fp64;          // FP32 passes: guard, degenerate and verify cells
     unsigned int* list_fp64_count;
     uint32_t* list_near;          // cells with a (near-)coincident point
     unsigned int* list_near_count;
