@@ -128,13 +128,11 @@ enum { RET_FLAG = C_BYTES / 4, RET_TOTAL = 56, RET_ERR = 58, RET_BYTES = 256 };
 static_assert(RET_FLAG < RET_TOTAL && 4 * (RET_ERR + 2) <= RET_BYTES, "layout of the read-back block");
 // Up to this many cells the careful pass runs over all of them: a few waves of
 // warps, whose time is a cell's latency, and a second pass over a few cells
-// would add its own (uniform points, careful alone against plain and careful:
-// 3,000 0.113 / 0.134 ms, 10,000 0.205 / 0.204, 30,000 0.52 / 0.41, each with the
-// finish of the form).  The careful pass finishes in FP64: where the form does
-// not ask for that, the line lies lower (FP32, 3,000 0.128 / 0.134 ms, 8,000
-// 0.216 / 0.19).  Such inputs have one launch of the FP64 clipping behind it, not
-// two or three.
-constexpr uint32_t kCarefulMax = 8192, kCarefulMax32 = 4096;
+// would add its own.  Uniform points, computes, careful alone against plain and
+// careful: MIXED and FP64, 4,500 141 / 176 us, 6,000 168 / 174, 8,000 211 / 226,
+// 10,000 even; FP32, where the careful pass finishes in FP64 for nothing, 4,500 142
+// / 158, 5,500 163 / 166, 6,500 181 / 177, 8,000 213 / 198.
+constexpr uint32_t kCarefulMax = 8192, kCarefulMax32 = 5632;
 bool careful_alone(uint32_t n, int precision) {
     return n <= (precision == TESS_PRECISION_FP32_GUARD ? kCarefulMax32 : kCarefulMax);
 }
@@ -689,15 +687,22 @@ ClipParams base_params(Engine& E) {
     return p;
 }
 
-// The fixed launch sequence of one compute (no host synchronisation):
-// the FP32 passes, then the FP64 clipping over what they hand on.  d_counters holds
-// a cursor per pass, list counts and reasons (C_*).
-tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t group, bool timing,
+// Cells beyond 128 vertices are rare: a compute that the host waits for launches the
+// pass over them when it has seen some (PASSES_FIRST, then PASSES_LAST); a captured
+// sequence has it always.
+enum Passes { PASSES_ALL, PASSES_FIRST, PASSES_LAST };
+
+// The launch sequence of one compute (no host synchronisation): the FP32 passes, then
+// the FP64 clipping over what they hand on.  d_counters holds a cursor per pass, list
+// counts and reasons (C_*).
+tess_status enqueue_passes(Engine& E, Passes which, int precision, double radius, int64_t group, bool timing,
                            cudaEvent_t* ev, const uint32_t* sample = nullptr, uint32_t nsample = 0) {
     unsigned* cur = E.d_counters;
     unsigned* cnt = E.d_counters + C_LIST;
-    CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * C_TOTAL + sizeof(unsigned long long), E.stream));
-    if (E.cfg.flags & TESS_FLAG_COUNTERS) CU(cudaMemsetAsync(E.d_work, 0, sizeof(unsigned long long) * 8, E.stream));
+    if (which != PASSES_LAST) {
+        CU(cudaMemsetAsync(E.d_counters, 0, sizeof(unsigned) * C_TOTAL + sizeof(unsigned long long), E.stream));
+        if (E.cfg.flags & TESS_FLAG_COUNTERS) CU(cudaMemsetAsync(E.d_work, 0, sizeof(unsigned long long) * 8, E.stream));
+    }
     ClipParams base = base_params(E);
     base.search_radius = radius;
     base.has_radius = radius >= 0.0;
@@ -736,13 +741,31 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
         return TESS_OK;
     };
     uint32_t* const* L = E.d_list;
-    if (timing) CU(cudaEventRecord(ev[0], E.stream));
     // without capacity re-runs, the lists beyond the configured slots are left out:
     // an overflowing cell is then reported as failed
     const bool norerun = E.cfg.flags & TESS_FLAG_NO_CAPACITY_RERUN;
     const int lc = s0 == 2 ? L_CAP : L_FULL;
     uint32_t* const lcap = norerun && s0 == 2 ? nullptr : L[lc];
     unsigned* const ccap = cnt + lc;
+    // a launch of the FP64 clipping over a list, and a second one of at most most2 cells
+    struct Work { int list; unsigned least; int list2; unsigned most2; };
+    auto clip64 = [&](int slots, Work w, bool last, int next = 0) -> tess_status {
+        base.work_least = w.least;
+        base.work2 = w.most2 ? L[w.list2] : nullptr;
+        base.work2_count = cnt + w.list2;
+        base.work2_most = w.most2;
+        return pass(0, slots, kFormStd, L[w.list], cnt + w.list, nullptr, nullptr, last ? nullptr : L[next], cnt + next);
+    };
+    auto largest = [&]() -> tess_status {
+        cursor = C_LIST - C_CURSOR - 1;
+        return clip64(8, {L_CAP64}, true);
+    };
+    if (which == PASSES_LAST) {
+        TRY(largest());
+        if (timing) CU(cudaEventRecord(ev[2], E.stream));
+        return TESS_OK;
+    }
+    if (timing) CU(cudaEventRecord(ev[0], E.stream));
     // The FP32 first pass hands cells of crowded bins to the dense pass and both
     // hand cells with an undecided plane test to the careful pass, which settles
     // those tests in FP64 and finishes the cell in FP64, whatever the form: such
@@ -759,31 +782,23 @@ tess_status enqueue_passes(Engine& E, int precision, double radius, int64_t grou
         TRY(pass(1, 2, kFormDense | X, L[L_DENSE], cnt + L_DENSE, L[L_CARE], cnt + L_CARE, lcap, ccap));
         TRY(pass(1, 2, kFormCareful | kFormExact, L[L_CARE], cnt + L_CARE, L[L_FULL], cnt + L_FULL, lcap, ccap));
     }
-    // The FP64 clipping: lists {cells, beyond 64, beyond 128 vertices}
-    struct Work { int list; unsigned least; int list2; unsigned most2; };
-    auto clip64 = [&](int slots, Work w, bool last, int next = 0) -> tess_status {
-        base.work_least = w.least;
-        base.work2 = w.most2 ? L[w.list2] : nullptr;
-        base.work2_count = cnt + w.list2;
-        base.work2_most = w.most2;
-        return pass(0, slots, kFormStd, L[w.list], cnt + w.list, nullptr, nullptr, last ? nullptr : L[next], cnt + next);
-    };
+    // (FULL at 64 and 128 vertices, CAP at 128, CAP64 at 255)
     const unsigned all = ~0u;
+    bool more = false;
     if (s0 == 2 && norerun) {
         TRY(clip64(2, {L_FULL}, true));
-    } else if (s0 == 2 && small) {
-        TRY(clip64(8, {L_CAP, 0, L_FULL, all}, true));
     } else if (s0 == 2) {
         const unsigned few = (sample ? nsample : E.total) <= kClip64Min ? all : (unsigned)(E.blocks(4, kFormStd) * E.wpb_for(4, kFormStd));
         if (few != all) TRY(clip64(2, {L_FULL, few}, false, L_CAP));
         TRY(clip64(4, {L_CAP, 0, L_FULL, few}, false, L_CAP64));
-        TRY(clip64(8, {L_CAP64}, true));
-    } else if (s0 == 4 && (!small || norerun)) {
+        more = true;
+    } else if (s0 == 4) {
         TRY(clip64(4, {L_FULL}, norerun, L_CAP64));
-        if (!norerun) TRY(clip64(8, {L_CAP64}, true));
+        more = !norerun;
     } else {
         TRY(clip64(8, {L_FULL}, true));
     }
+    if (more && which == PASSES_ALL) TRY(largest());
     if (timing) CU(cudaEventRecord(ev[2], E.stream));
     return TESS_OK;
 }
@@ -847,11 +862,15 @@ tess_status engine_compute(Engine& E, int precision, double radius, int64_t grou
     TimingEvents ev;
     if (timing) CU(ev.create(3));
     for (int attempt = 0; attempt < 4; ++attempt) {
-        TRY(enqueue_passes(E, precision, radius, group, timing, ev.e));
         unsigned long long used = 0;
         const unsigned* counts = nullptr;
         int gerr = 0;
+        TRY(enqueue_passes(E, PASSES_FIRST, precision, radius, group, timing, ev.e));
         TRY(read_back(E, &counts, &used, &gerr));
+        if (counts[C_LIST + L_CAP64]) {
+            TRY(enqueue_passes(E, PASSES_LAST, precision, radius, group, timing, ev.e));
+            TRY(read_back(E, &counts, &used, &gerr));
+        }
         if (gerr == 1) {
             // the device points were rebuilt without a check and hold a
             // non-finite coordinate: the clipping kernels did nothing
@@ -1048,7 +1067,7 @@ tess_status time_sample(Engine& E, int precision, uint32_t m, float* ms) {
     CU(ev.create(2));
     for (int attempt = 0; attempt < 4; ++attempt) {
         CU(cudaEventRecord(ev.e[0], E.stream));
-        TRY(enqueue_passes(E, precision, -1.0, -1, false, nullptr, E.d_sample, m));
+        TRY(enqueue_passes(E, PASSES_ALL, precision, -1.0, -1, false, nullptr, E.d_sample, m));
         CU(cudaEventRecord(ev.e[1], E.stream));
         unsigned long long used = 0;
         CU(cudaMemcpyAsync(&used, E.d_fcursor, sizeof(used), cudaMemcpyDeviceToHost, E.stream));
@@ -1987,7 +2006,7 @@ static tess_status batch_run(tess_batch* b, int prec) {
         cudaError_t ce = launch_grid_build(grid_buffers(E), E.stream, E.side, E.ev_fork, E.ev_join);
         if (ce != cudaSuccess) st = fail(TESS_E_CUDA, "capture: %s", cudaGetErrorString(ce));
         const uint64_t launched = E.launches;
-        if (st == TESS_OK) st = enqueue_passes(E, prec, -1.0, -1, false, nullptr);
+        if (st == TESS_OK) st = enqueue_passes(E, PASSES_ALL, prec, -1.0, -1, false, nullptr);
         glaunches = grid_launches(E.total_bins, E.ndiag) + (E.launches - launched);
         E.launches = launched;
         cudaError_t ee = cudaStreamEndCapture(E.stream, &g);
