@@ -52,10 +52,10 @@ RADIUS_METRIC = "radius queries/sec on 1 GB300 (find_neighbors_in_real_radius, F
 # dram__bytes_write.sum 167.0 MB in 9.87 ms) and is scaled by cells: its
 # traffic is its output plus L2 misses, both per cell.  The radius passes were
 # captured at 1,000,000 queries with 16 results each, and are scaled by queries.
-NCU_CLIP_BYTES_PER_CELL = (54.693376e6 + 167.044352e6) / 1_000_000
+NCU_CLIP_BYTES_PER_CELL = (55.570688e6 + 167.587328e6) / 1_000_000
 # Warp instructions of the same capture (smsp__inst_executed.sum), per cell: the
 # kernel is bound by instruction issue, so this gives its issue roofline.
-NCU_CLIP_INST_PER_CELL = 9_612_786_773 / 1_000_000
+NCU_CLIP_INST_PER_CELL = 9_635_499_419 / 1_000_000
 NCU_RADIUS_BYTES = {"count": (88.877312e6 + 58.024192e6) / 1_000_000, "fill": (134.081536e6 + 41.526528e6) / 1_000_000}
 # DRAM traffic of the 10 binning launches (read 692.9 MB + write 208.6 MB) at
 # 4,194,304 uniform points, scaled by points: every term is per point or per bin.
@@ -648,7 +648,7 @@ def run_ours(args, ws, rank, local):
 
 VOL_BAR = {"fp32": 1e-6, "mixed": 1e-11, "fp64": 1e-12}
 PREC_DESC = {"fp32": "FP32 + FP64 guard re-run", "fp64": "FP64",
-             "mixed": "FP32 + FP64 guard re-run, FP64-accurate finish (two FP64-residual Newton steps "
+             "mixed": "FP32 + FP64 guard re-run, FP64-accurate finish (an FP64 Newton step "
                       "per vertex, FP64 areas and volumes)"}
 
 

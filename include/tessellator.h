@@ -84,14 +84,16 @@ typedef enum {
 
 typedef struct {
     /* FP32 form, guard band: a plane test of vertex v against the bisector of
-     * the site and a point at offset r is undecided (the cell re-runs in FP64)
-     * when |signed distance| <= e_v + guard_rel * (|v|_1 + |r|) plus a small
-     * term for the FP32 split of the positions, with e_v the vertex's tracked
-     * error bound (distances normalised by |r|).  The FP32 rounding of a test
-     * stays below 3e-7 (|v|_1 + |r|): keep guard_rel at or above that. */
+     * the site and a point at offset r is undecided (settled in FP64, or the
+     * cell clipped in FP64) when |signed distance| <= e_v + guard_rel * (|v|_1
+     * + |r|) plus a small term for the FP32 split of the positions, with e_v the
+     * vertex's tracked error bound (distances normalised by |r|).  The FP32
+     * rounding of a test stays below 3e-7 (|v|_1 + |r|): keep guard_rel at or
+     * above that. */
     double guard_rel;
     /* FP32 form, final check: the FP64 correction of every vertex must stay
-     * within 2 e_v + verify_rel * R, else the cell re-runs in FP64. */
+     * within 2 e_v + verify_rel * R, else the cell is computed again with its
+     * undecided tests settled and its results in FP64. */
     double verify_rel;
     /* Points per bin; the reference's cell_density() is 1.25 (celery.rs:185-188). */
     double bin_density;
@@ -144,9 +146,10 @@ typedef struct {
     /* of the rerun_fp64 cells, those that settling single tests in FP64 did
      * not finish, clipped in FP64 as a whole */
     uint64_t rerun_fp64_full;
-    /* FP32 form: cells whose own bin is crowded (>= crowded_bin points), taken out of
-     * the first pass and computed by a pass that first cuts by the nearest
-     * point of each lane's stride of that bin */
+    /* cells whose own bin is crowded (>= crowded_bin points) or with 1,024 points
+     * or more in one batch of bins (beside a cluster), taken out of the first
+     * pass and computed by a pass that first cuts by the nearest point of each
+     * lane's stride of a crowded own bin */
     uint64_t dense_cells;
     /* times the face pool was found too small and grown, followed by a
      * recompute, since the handle was created */

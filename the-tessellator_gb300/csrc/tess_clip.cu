@@ -120,9 +120,7 @@ __global__ void __launch_bounds__(kCsrThreads) k_csr_one(const uint32_t* cnt, ui
 // One warp per C consecutive cells: their CSR range is contiguous, so the
 // warp writes it as one coalesced stream; each output element finds its cell
 // (lane) by a binary search over the warp's prefix sums of the face counts
-// and reads from that cell's contiguous run in the face pool.  C = 32 where
-// that fills the GPU; small inputs take C = 4 (1,000 cells: 4 blocks of 16 us
-// with 32 a warp).
+// and reads from that cell's contiguous run in the face pool (kCsrWide: which C).
 template <int C>
 __global__ void __launch_bounds__(256) k_csr_gather(const uint32_t* cnt, const uint64_t* fstart,
                                                     const int32_t* fnbr, const double* farea, uint32_t n,
@@ -178,9 +176,10 @@ int clip_blocks_for(int slots, int form, int wpb, int device) {
     return clip_blocks_f64(slots, wpb, device);
 }
 
-// From this many cells a warp of the gather takes 32 (38,912 warps fill the GPU's
-// 152 x 64 four times over), below it 4.
-constexpr uint32_t kCsrWide = 262144;
+// From this many cells a warp of the gather takes 32, below it 4.  Offsets and gather,
+// 32 and 4 cells a warp: 1,000 cells 18 and 10 us, 131,072 27 and 24, 200,000 30 and
+// 32, 262,144 37 and 41, 1,000,000 135 and 151.
+constexpr uint32_t kCsrWide = 196608;
 
 uint64_t csr_offset_launches(uint32_t n) { return n <= kCsrOneMax ? 1 : 3; }
 
