@@ -99,3 +99,17 @@ def test_identical_points_seen_from_outside(tess, oracle_mod):
             cell, ref = d.get_cell_at_particle(p).compute_voronoi_cell(), r.cell_at(p)
             assert cell.compute_neighbors() == ref.ids.tolist()
             assert math.isclose(cell.compute_volume(), ref.volume, rel_tol=1e-12)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+def test_keys_that_underflow(tess, oracle_mod, prec):
+    """Sides of 1e-171: every key is 0, and no whole key fits the table.  The oracle's cells (nothing cuts within the
+    reference's tolerance)."""
+    pts = np.random.default_rng(5).random((1300, 3)) * 1e-170
+    box = [1e-170] * 3
+    ro, ri = oracle_mod.Diagram(pts, lo=[0, 0, 0], hi=box).compute_all()[1:3]
+    with tess.Diagram(pts, container=tess.Polyhedron(0, 0, 0, *box)) as d:
+        d.compute_all(prec)
+        offs, nbr, _ = d.neighbors_csr()
+        assert d.stats()["table_entries"] == 1
+    assert np.array_equal(offs.astype(np.int64), ro) and np.array_equal(nbr.astype(np.int64), ri)

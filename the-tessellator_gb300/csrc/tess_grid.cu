@@ -631,10 +631,11 @@ __global__ void __launch_bounds__(kTabThreads) k_table(GridBuffers g) {
         if (kept && beg <= cap && t > 0 && skey[t - 1] != key) atomicMax(&ends, t);
         __syncthreads();
         m = start[ends];
-        // (not even the first key's, sides below 1e-162: the own bin alone)
         if (t == 0) D.tab_kmax = ends ? __longlong_as_double((long long)skey[ends - 1]) : -1.0;
-        if (t == 0 && !ends) g.table[D.tab_base] = TabEntry{-1.0f, 0, 0, 0, 0};
     }
+    // (not even the first key's, sides below 1e-162, or no key is a number, sides
+    // beyond FP64's range: the own bin alone)
+    if (t == 0 && m == 0) g.table[D.tab_base] = TabEntry{-1.0f, 0, 0, 0, 0};
     for (uint32_t q = 0; q < cnt; ++q) {
         if (beg + q >= m) break;
         const int i = pick(gi, q / (w1 * w2)), j = pick(gj, (q / w2) % w1), k = pick(gk, q % w2);
