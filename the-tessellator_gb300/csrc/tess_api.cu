@@ -138,10 +138,12 @@ bool careful_alone(uint32_t n, int precision) {
 }
 // Careful pass: a cell with more cuts than this that have undecided tests goes to the
 // FP64 clipping, which takes such a cell faster.  Where the pass runs over all cells,
-// a simple cubic lattice of 1,000 points takes 423 us when every test is settled, 423
-// / 298 / 197 / 133 / 114 from 16 / 8 / 4 / 2 / 1 on, and crystals with motion of 2e-3,
-// whose cells seldom have more than three, are slower from 2 on.  Over a list it is
-// the tails of clustered points that have more (100,000: 42 ms from 16, 47 from 4).
+// 1,000 points of a simple cubic lattice take 423 us when every test is settled and 182
+// / 157 / 130 / 105 from 4 / 3 / 2 / 1 on, 8,000 of a crystal with motion of 2e-3 315 /
+// 312 / 307 / 300, uniform points the same; 4 is the least that still settles a good
+// part of a lattice's cells in place (659 of 2,000 of a BCC one, 4 from 3 on, none
+// below).  Over a list it is the tails of clustered points that have more (100,000:
+// 42 ms from 16, 47 from 4).
 constexpr int kSettleMost = 16, kSettleMostAlone = 4;
 // The FP64 clipping at 64 vertices works on twice as many cells at a time as at 128, but
 // a cell that outgrows it is clipped twice, one after the other.  It takes lists
